@@ -35,6 +35,7 @@ struct Decoder {
   float2 *hdr_a = nullptr, *hdr_b = nullptr;
   float2* best = nullptr;  // per-CTA argmax candidates of the lm_head kernel
   float *part_o = nullptr, *part_ml = nullptr;  // per-split attention partials (decode)
+  uint8_t* kv_split = nullptr;  // a layer's keys and values as operands of the prompt attention
   int attn_chunk = 32, attn_splits = 1;
   void* ws = nullptr;  // workspace of the public forward (prefill)
   size_t ws_bytes = 0;
