@@ -128,7 +128,8 @@ MLLMB200_API int mllmb200_w4a32_linear_forward(const float* x_dev, const void* t
 
 /* Same, with the kernel family forced (tests and benchmarks):
  * 0 auto, 1 streaming GEMV (M <= 4: ONE launch, x quantized inside it, ws_dev unused), 2 SIMT dp4a GEMM,
- * 3 tcgen05 kind::i8 GEMM (exact int32 group sums, as the reference), 4 tcgen05 fp16 GEMM (M >= 64: group
+ * 3 tcgen05 tile GEMM (M <= 64 kind::i8, exact int32 group sums; above, fp16 operands with exact products and chunks
+ * of K summed in tensor memory, the chunks in fp32 registers), 4 tcgen05 fp16 GEMM (M >= 64: group
  * scales folded into an fp16 weight operand - exact for bf16-encoded scales, rounded to fp16's 11 bits
  * (relative error <= 2^-11 per weight) for MLLMB200_SCALE_FP16 - fp32 accumulation over all of K in
  * tensor memory; same 1e-3*rms bound; auto never picks it; launches that would fill less than half of the SMs

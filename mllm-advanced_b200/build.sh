@@ -11,7 +11,7 @@ WHAT="${1:-all}"
 OUT="$HERE/lib"
 OBJ="$HERE/build"
 CORE=(host_pack.cpp c_api.cu device_status.cu repack.cu act_quant.cu gemv.cu gemv_stream.cu gemm_stream.cu gemm_simt.cu gemm_tc.cu
-      gemm_tcf16.cu decoder_kernels.cu decoder_attn.cu decoder_attn_prefill.cu decoder_sample.cu decoder.cu decoder_batch.cu decoder_persistent.cu conv3d.cu
+      gemm_tcf16.cu gemm_chunk.cu decoder_kernels.cu decoder_attn.cu decoder_attn_prefill.cu decoder_sample.cu decoder.cu decoder_batch.cu decoder_persistent.cu conv3d.cu
       host_pack_a16.cpp w4a16.cu c_api_a16.cu tp.cu)
 [ -f "$HERE/csrc/no_alloc.cu" ] && CORE+=(no_alloc.cu)
 LM=(lm/lm_engine.cu lm/lm_linear.cu lm/lm_norm.cu lm/lm_attn.cu lm/lm_latent.cu lm/lm_moe.cu lm/lm_retention.cu device_status.cu decoder_sample.cu)

@@ -246,12 +246,17 @@ __global__ void __launch_bounds__(256) act_quant_reflayout_kernel(const float* _
   for (int i = threadIdx.x; i < k; i += blockDim.x) dst[8 + i] = (uint8_t)(int8_t)act_quant_value(row[i], p);
 }
 
-// The same for the fp16 tensor-core path (gemm_tcf16.cu): the zero-point-corrected values a_q + a_off
+// The same for the fp16 tensor-core paths (gemm_chunk.cu, gemm_tcf16.cu): the zero-point-corrected values a_q + a_off
 // are written as fp16 (exact) in 512-byte canonical K-major blocks [group][row / 8]: 4 chunks of 128 bytes, chunk c =
 // 8 rows x 16 bytes holding k = 8c + {0,4,1,5,2,6,3,7} - the order in which the weight side's
 // nibble unpack (two nibbles 16 bits apart per half2) produces its elements.
-constexpr int kF16RowsPerCta = 4;   // rows 4i .. 4i+3 sit side by side in a block: 64-byte pieces
+// Bound: at small M a chain of latencies (row in, min/max across the CTA, blocks out), at large M the memory.  A thread
+// keeps its items of the row (8 values of K each) in registers between the two halves of the work, up to K = 10240; the
+// rest of a longer row is read again.  Two rows per CTA: their 16-byte pieces fill a 32-byte sector.  Measured (B200)
+// with four rows per CTA and every row read twice / as it is: M = 64, K = 1536 3.6 / 2.7 us, K = 8960 8.2 / 4.7 us.
+constexpr int kF16RowsPerCta = 2;
 constexpr int kF16WarpsPerRow = 8;
+constexpr int kF16Items = 5;
 __global__ void __launch_bounds__(kF16RowsPerCta * kF16WarpsPerRow * 32) act_quant_blocks_f16_kernel(
     const float* __restrict__ x, int m_total, int k, int ldx, int num_groups, int m8_pad, uint8_t* __restrict__ blocks,
     float2* __restrict__ hdr, int use_pdl, int* __restrict__ clear_ints, int clear_count) {
@@ -266,30 +271,46 @@ __global__ void __launch_bounds__(kF16RowsPerCta * kF16WarpsPerRow * 32) act_qua
   if (blockIdx.x == 0)
     for (int i = threadIdx.x; i < clear_count; i += blockDim.x) clear_ints[i] = 0;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int r = warp & (kF16RowsPerCta - 1), part = warp / kF16RowsPerCta;
+  const int r = warp % kF16RowsPerCta, part = warp / kF16RowsPerCta;
   const int m = blockIdx.x * kF16RowsPerCta + r;
   const bool live = m < m_total;
   const float* row = x + (size_t)(live ? m : 0) * ldx;
   const bool vec = ((reinterpret_cast<uintptr_t>(row) & 15u) == 0);
-  float mn = 3.402823466e+38f, mx = -3.402823466e+38f;
-  if (live) {
-    const int stride = 32 * kF16WarpsPerRow, first = part * 32 + lane;
-    if (vec) {
-      const float4* r4 = reinterpret_cast<const float4*>(row);
-      for (int i = first; i < (k >> 2); i += stride) {
-        const float4 v = r4[i];
-        mn = fminf(mn, fminf(fminf(v.x, v.y), fminf(v.z, v.w)));
-        mx = fmaxf(mx, fmaxf(fmaxf(v.x, v.y), fmaxf(v.z, v.w)));
-      }
-      for (int i = (k & ~3) + first; i < k; i += stride) {
-        mn = fminf(mn, row[i]);
-        mx = fmaxf(mx, row[i]);
-      }
+  constexpr int kStride = kF16WarpsPerRow * 32;
+  const int items = num_groups * 4, first = part * 32 + lane;  // item = 8 consecutive k = one 16-byte chunk of a block
+  auto load = [&](int item, float (&f)[8]) {
+    const int k0 = item * 8;
+    if (vec && k0 + 8 <= k) {
+      const float4 a = *reinterpret_cast<const float4*>(row + k0);
+      const float4 b = *reinterpret_cast<const float4*>(row + k0 + 4);
+      f[0] = a.x, f[1] = a.y, f[2] = a.z, f[3] = a.w, f[4] = b.x, f[5] = b.y, f[6] = b.z, f[7] = b.w;
     } else {
-      for (int i = first; i < k; i += stride) {
-        mn = fminf(mn, row[i]);
-        mx = fmaxf(mx, row[i]);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) f[j] = k0 + j < k ? row[k0 + j] : 0.0f;
+    }
+  };
+  float mn = 3.402823466e+38f, mx = -3.402823466e+38f;
+  auto extend = [&](int item, const float (&f)[8]) {
+    const int left = k - item * 8;
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+      if (j < left) {
+        mn = fminf(mn, f[j]);
+        mx = fmaxf(mx, f[j]);
       }
+  };
+  float v[kF16Items][8];
+  if (live) {
+#pragma unroll
+    for (int i = 0; i < kF16Items; ++i)
+      if (first + i * kStride < items) load(first + i * kStride, v[i]);
+#pragma unroll
+    for (int i = 0; i < kF16Items; ++i)
+      if (first + i * kStride < items) extend(first + i * kStride, v[i]);
+    for (int item = first + kF16Items * kStride; item < items; item += kStride) {
+      float f[8];
+      load(item, f);
+      extend(item, f);
     }
   }
 #pragma unroll
@@ -309,31 +330,27 @@ __global__ void __launch_bounds__(kF16RowsPerCta * kF16WarpsPerRow * 32) act_qua
   }
   const ActQuantParams p = act_quant_params(mn, mx);
   if (live && lane == 0 && part == 0) hdr[m] = make_float2(p.recip_scale, __int_as_float(-p.nzp));
-  // padding rows (m >= m_total, inside the padded tile) are written as zeros: the tensor core reads them.
-  // One thread per (K-group, 8-element chunk): 4 x the parallelism of one thread per group.
-  for (int it = part * 32 + lane; it < num_groups * 4; it += 32 * kF16WarpsPerRow) {
-    const int g = it >> 2, c = it & 3;
-    const int kc = g * kGroup + c * 8;
-    uint8_t* blk = blocks + ((size_t)g * m8_pad + (m >> 3)) * 512 + (m & 7) * 16;
-    float f[8];
-    if (live && vec && kc + 8 <= k) {
-      const float4 a = *reinterpret_cast<const float4*>(row + kc);
-      const float4 b = *reinterpret_cast<const float4*>(row + kc + 4);
-      f[0] = a.x, f[1] = a.y, f[2] = a.z, f[3] = a.w, f[4] = b.x, f[5] = b.y, f[6] = b.z, f[7] = b.w;
-    } else {
-#pragma unroll
-      for (int jj = 0; jj < 8; ++jj) f[jj] = (live && kc + jj < k) ? row[kc + jj] : 0.0f;
-    }
+  // padding rows (m >= m_total, inside the padded tile) are written as zeros: the tensor core reads them
+  auto store = [&](int item, const float (&f)[8]) {
+    const int left = live ? k - item * 8 : 0;
     __align__(16) __half h[8];
 #pragma unroll
-    for (int jj = 0; jj < 8; ++jj) {
+    for (int j = 0; j < 8; ++j) {
       // a_q + a_off (= a_q - zero point), |.| <= 255: exact in fp16, and exactly the factor the reference
       // multiplies the weight with, so no zero-point correction term (and none of its cancellation) is left
-      const int q = (live && kc + jj < k) ? act_quant_value(f[jj], p) - p.nzp : 0;
-      const int pos = (jj < 4) ? 2 * jj : 2 * (jj - 4) + 1;  // chunk order {0,4,1,5,2,6,3,7}
-      h[pos] = __int2half_rn(q);
+      const int q = j < left ? act_quant_value(f[j], p) - p.nzp : 0;
+      h[(j < 4) ? 2 * j : 2 * (j - 4) + 1] = __int2half_rn(q);  // chunk order {0,4,1,5,2,6,3,7}
     }
-    *reinterpret_cast<uint4*>(blk + c * 128) = *reinterpret_cast<const uint4*>(h);
+    uint8_t* blk = blocks + ((size_t)(item >> 2) * m8_pad + (m >> 3)) * 512 + (m & 7) * 16;
+    *reinterpret_cast<uint4*>(blk + (item & 3) * 128) = *reinterpret_cast<const uint4*>(h);
+  };
+#pragma unroll
+  for (int i = 0; i < kF16Items; ++i)
+    if (first + i * kStride < items) store(first + i * kStride, v[i]);
+  for (int item = first + kF16Items * kStride; item < items; item += kStride) {
+    float f[8] = {};
+    if (live) load(item, f);
+    store(item, f);
   }
 }
 

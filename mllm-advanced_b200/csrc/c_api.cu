@@ -9,7 +9,7 @@ namespace mllmb200 {
 // repack.cu
 __global__ void repack_cells_kernel(const uint8_t*, const uint16_t*, int, int, int, int, int, uint8_t*);
 __global__ void repack_rowdata_kernel(const uint8_t*, const float*, int, int, int, int, uint32_t, float*, float*,
-                                      unsigned int*);
+                                      unsigned int*, unsigned int*);
 __global__ void unpack_cells_kernel(const uint8_t*, int, int, int, int, uint8_t*, uint16_t*);
 __global__ void unpack_bias_kernel(const float*, int, float*);
 // act_quant.cu
@@ -53,6 +53,12 @@ cudaError_t launch_act_quant_mma(const float*, int, int, int, uint8_t*, float2*,
 cudaError_t launch_w4a32_gemm_stream(const uint8_t*, const float2*, int, int, int, const void* const*, float* const*,
                                      const int*, const int*, int, cudaStream_t);
 constexpr int kStreamGemmMinM = 5, kStreamGemmMaxM = 64;  // batch sizes the streaming tensor-core GEMM takes by default
+
+// gemm_chunk.cu: kernel id 3 from kChunkMinM rows on.  Up to 64 rows gemm_tc.cu, whose int8 activations take half of the
+// workspace (M = 65, 1536 x 1536: 18.7 us with gemm_tc.cu, 13.7 with gemm_chunk.cu; 17920 x 1536: 36 and 24).
+cudaError_t launch_w4a32_gemm_chunk(const uint8_t*, const float2*, int, int, int, const void* const*, float* const*, const int*,
+                                    const int*, int, cudaStream_t);
+constexpr int kChunkMinM = 65;
 
 cudaError_t read_device_status(cudaStream_t, int* status);
 
@@ -137,7 +143,8 @@ int mllmb200_w4a32_repack_device(const void* blob_dev, int N, int K, int scale_m
       tiled + th.cells_off, has_bias ? reinterpret_cast<const float*>(blob + bh.bias_off) : nullptr, row_begin,
       row_count, (int)th.num_groups, (int)th.num_panels, (uint32_t)scale_mode,
       reinterpret_cast<float*>(tiled + th.zsum_off), reinterpret_cast<float*>(tiled + th.bias_off),
-      reinterpret_cast<unsigned int*>(tiled + offsetof(TiledHeader, max_scale_bits)));
+      reinterpret_cast<unsigned int*>(tiled + offsetof(TiledHeader, max_scale_bits)),
+      reinterpret_cast<unsigned int*>(tiled + offsetof(TiledHeader, min_row_scale_not)));
   if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(e);
   return MLLMB200_OK;
 }
@@ -205,6 +212,17 @@ static int quantize_into_ws(const float* x_dev, void* ws_dev, int M, int K, int 
   return e == cudaSuccess ? MLLMB200_OK : cuda_fail(e);
 }
 
+// One quantization and one launch of the chunked tile GEMM for up to four matrices that share x.
+static int chunk_forward(const float* x_dev, int M, int K, int ldx, int count, const void* const* tiled_dev, float* const* y_dev,
+                         const int* N, const int* ldy, void* ws_dev, int use_pdl, cudaStream_t st) {
+  if (!ws_dev || (reinterpret_cast<uintptr_t>(ws_dev) & 255u)) return MLLMB200_INVALID_ARG;
+  uint8_t* blocks = static_cast<uint8_t*>(ws_dev);
+  float2* hdr = reinterpret_cast<float2*>(blocks + ws_rec_bytes(M, K));
+  cudaError_t e = launch_act_quant_blocks_f16(x_dev, M, (M + 7) / 8 * 8, K, ldx, blocks, hdr, st, use_pdl);
+  if (e == cudaSuccess) e = launch_w4a32_gemm_chunk(blocks, hdr, M, K, count, tiled_dev, y_dev, N, ldy, use_pdl, st);
+  return e == cudaSuccess ? MLLMB200_OK : cuda_fail(e);
+}
+
 int mllmb200_w4a32_linear_forward_ex(const float* x_dev, const void* tiled_dev, float* y_dev, void* ws_dev, int M,
                                      int K, int N, int ldx, int ldy, int kernel, void* stream) {
   if (!x_dev || !tiled_dev || !y_dev || M <= 0 || K <= 0 || N <= 0 || ldx < K || ldy < N) return MLLMB200_INVALID_ARG;
@@ -234,6 +252,8 @@ int mllmb200_w4a32_linear_forward_ex(const float* x_dev, const void* tiled_dev, 
   }
   if (kernel == 6 && !w4a32_gemv_supported(M, K, N)) return MLLMB200_UNSUPPORTED;
   if (kernel == 3 && !w4a32_gemm_tc_supported(M, K, N)) return MLLMB200_UNSUPPORTED;
+  if (kernel == 3 && M >= kChunkMinM)
+    return chunk_forward(x_dev, M, K, ldx, 1, &tiled_dev, &y_dev, &N, &ldy, ws_dev, use_pdl, st);
   if (kernel == 4) {  // fp16 tensor-core path: its own activation layout
     if (!w4a32_gemm_tcf16_supported(M, K, N)) return MLLMB200_UNSUPPORTED;
     if (!ws_dev || (reinterpret_cast<uintptr_t>(ws_dev) & 255u)) return MLLMB200_INVALID_ARG;
@@ -338,6 +358,8 @@ int mllmb200_w4a32_linear_forward_grouped(const float* x_dev, int M, int K, int 
   }
   bool all8 = count > 1;
   for (int i = 0; i < count; ++i) all8 = all8 && mllmb200_w4a32_select_kernel(M, K, N[i]) == 3;
+  if (all8 && M >= kChunkMinM)
+    return chunk_forward(x_dev, M, K, ldx, count, tiled_dev, y_dev, N, ldy, ws_dev, (flags >> 8) & 1, st_grp);
   if (all8) {
     if (!ws_dev || (reinterpret_cast<uintptr_t>(ws_dev) & 255u)) return MLLMB200_INVALID_ARG;
     uint8_t* blocks = static_cast<uint8_t*>(ws_dev);

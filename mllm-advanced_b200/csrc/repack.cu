@@ -46,7 +46,7 @@ __global__ void repack_cells_kernel(const uint8_t* __restrict__ nibbles, const u
 __global__ void repack_rowdata_kernel(const uint8_t* __restrict__ cells, const float* __restrict__ bias_src,
                                       int row_begin, int row_count, int num_groups, int num_panels,
                                       uint32_t scale_mode, float* __restrict__ zsum, float* __restrict__ bias_dst,
-                                      unsigned int* __restrict__ max_scale_bits) {
+                                      unsigned int* __restrict__ max_scale_bits, unsigned int* __restrict__ min_row_scale_not) {
   const int warps_per_block = blockDim.x >> 5;
   const int lane = threadIdx.x & 31;
   const int padded_rows = num_panels * kPanelRows;
@@ -79,6 +79,7 @@ __global__ void repack_rowdata_kernel(const uint8_t* __restrict__ cells, const f
     }
     if (lane == 0) {
       if (max_scale_bits != nullptr && row < row_count) atomicMax(max_scale_bits, __float_as_uint(smax));  // non-negative floats order as integers
+      if (min_row_scale_not != nullptr && row < row_count && smax > 0.0f) atomicMax(min_row_scale_not, ~__float_as_uint(smax));
       zsum[row] = (float)acc;
       bias_dst[row] = (bias_src != nullptr && row < row_count) ? bias_src[row_begin + row] : 0.0f;
     }

@@ -1,0 +1,90 @@
+"""The tile GEMM of M >= 65 (fp16 operands, chunks of K summed in tensor memory, the rest in fp32 registers) at the edges of
+its tiles, chunks and forms, against the same sums in 64 bits from the oracle's quantized activations.
+
+Bar on the 2-norm of the error: operands and products are exact, so what rounds is the addition: inside a chunk at most 48
+truncated ones (768 values of K, 16 an instruction), each off by at most 2^-23 of a running sum that is on average 2/3 of
+the chunk's, half of that on average: 48 / 3 * 2^-23; then one addition per chunk and the epilogue, 2^-24 each."""
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+import mllm_b200 as mb  # noqa: E402
+from oracle_lib import Oracle  # noqa: E402
+
+
+def _weights64(blob, mode):
+    nib, sc, bias = mb.blob_sections(blob)
+    n, k = mb.blob_info(blob)[:2]
+    q = np.stack([nib & 15, nib >> 4], axis=-1).reshape(n, -1)[:, :k].astype(np.float64) - 8
+    s = sc.view(np.float16).astype(np.float64) if mode == mb.SCALE_FP16 else (sc.astype(np.uint32) << 16).view(np.float32).astype(np.float64)
+    return q * np.repeat(s, 32, axis=1)[:, :k], bias
+
+
+def _acts64(orc, x):
+    m, k = x.shape
+    raw = np.ascontiguousarray(orc.quant_act(x)).reshape(m, -1).view(np.uint8)
+    head = np.ascontiguousarray(raw[:, :8])
+    recip, off = head.view(np.float32)[:, :1].astype(np.float64), head.view(np.int32)[:, 1:].astype(np.float64)
+    return (raw[:, 8:8 + k].view(np.int8).astype(np.float64) + off) * recip
+
+
+def _run(m, k, ns, mode=mb.SCALE_BF16_TRUNC, small_row=False):
+    orc, rng = Oracle(), np.random.default_rng(m + 3 * k + ns[0])
+    x = rng.standard_normal((m, k)).astype(np.float32)
+    x[7], x[8] = np.abs(x[7]) + 1, 0
+    xd, a = torch.from_numpy(x).cuda(), _acts64(orc, x)
+    wts = []
+    for i, n in enumerate(ns):
+        w = (rng.standard_normal((n, k)) * 0.02).astype(np.float32)
+        if small_row:
+            w[n // 2] *= 1e-12
+        blob = mb.quant_prepack(w, None if i else (rng.standard_normal(n) * 0.1).astype(np.float32), scale_mode=mode)
+        w64, bias = _weights64(blob, mode)
+        wts.append((mb.W4A32Weights.from_blob(blob), w64, bias))
+    outs = mb.linear_forward_grouped(xd, [w for w, _, _ in wts], pdl=True)
+    mb.check_device_status()
+    bar = (48 / 3 + (k + 127) // 128 / 2 + 2) * 2.0 ** -23
+    for (wt, w64, bias), y in zip(wts, outs):
+        want = a @ w64.T + (0 if bias is None else bias)
+        d = y.cpu().numpy() - want
+        assert np.linalg.norm(d) <= bar * np.linalg.norm(want), (wt.n, np.linalg.norm(d) / np.linalg.norm(want))
+        if small_row and bias is None:  # a row by itself: its accuracy does not depend on the other rows' scales
+            r = wt.n // 2
+            assert np.linalg.norm(d[:, r]) <= bar * np.linalg.norm(want[:, r])
+        buf = torch.full((m, wt.n + 24), float("nan"), device="cuda")
+        mb.linear_forward(xd, wt, out=buf[:, :wt.n])  # the same bits by itself, and nothing outside of its columns
+        mb.check_device_status()
+        assert torch.equal(buf[:, :wt.n], y) and bool(torch.isnan(buf[:, wt.n:]).all())
+
+
+# single CTAs (few tiles) and pairs; rows and columns over and under a tile, a second CTA of a pair without rows, K under a
+# group, under a stage, at chunk lengths of 1, 2, 4 and 6 quads, and one stage more than a whole chunk
+@pytest.mark.parametrize("m,k,ns", [(65, 1536, (256, 40)), (65, 96, (12900,)), (130, 1176, (40,)), (256, 31, (40,)), (257, 70, (129, 33)),
+                                    (300, 896, (200,)), (256, 1056, (12800,)), (385, 96, (12900,)), (511, 1536, (6400, 130)),
+                                    (640, 2176, (4480,)), (271, 8224, (12832,)), (520, 8960, (384,))])
+def test_tiles_chunks_and_forms(m, k, ns):
+    _run(m, k, ns)
+
+
+# fp16-encoded scales: rounded product and remainder, two passes over every stage, chunks of 2 stages and more
+@pytest.mark.parametrize("m,k,ns", [(256, 70, (12800,)), (300, 896, (200,)), (256, 928, (12800,)), (512, 4160, (6400,))])
+def test_fp16_scales(m, k, ns):
+    _run(m, k, ns, mb.SCALE_FP16)
+
+
+@pytest.mark.parametrize("ns", [(96, 64), (64, 12800)])
+def test_a_row_of_tiny_weights(ns):
+    _run(256, 512, ns, small_row=True)
+
+
+def test_row_shards_are_slices():
+    """A shard small enough for single CTAs gives the bits of the whole matrix, which takes pairs."""
+    rng = np.random.default_rng(5)
+    m, k, n = 300, 2080, 12800
+    x = torch.from_numpy(rng.standard_normal((m, k)).astype(np.float32)).cuda()
+    blob = mb.quant_prepack((rng.standard_normal((n, k)) * 0.02).astype(np.float32))
+    whole = mb.linear_forward(x, mb.W4A32Weights.from_blob(blob))
+    part = mb.linear_forward(x, mb.W4A32Weights.from_blob(blob, row_begin=6400, row_count=300))
+    assert torch.equal(part, whole[:, 6400:6700])
