@@ -37,6 +37,18 @@ __global__ void attn_decode_partial_kernel(const float*, const float*, const flo
                                            int, int, int, float*, float*, float*, float*, int, int);
 __global__ void attn_combine_quant_kernel(const float*, const float*, const int*, int, int, int, int, int, float*, uint8_t*,
                                           float2*, int);
+__global__ void rope_kv_append_kernel(const float*, const float*, int, const float*, const float*, const int*, int,
+                                      float*, float*);
+template <int D>
+__global__ void attention_prefill_kernel(const float*, int, int, const float*, const float*, const int*, int, int, const float*,
+                                         const float*, float*, int);
+size_t attention_prefill_smem_bytes(int head_dim);
+int attention_prefill_rows();
+int attention_prefill_threads();
+// Prompts up to here keep the fp32 attention on the CUDA cores (decoder_attn.cu): the tensor-core kernels' chain of set-up,
+// splitting and tile latencies costs 19 us a layer whatever the length, these 16 us for 40 tokens of the 1.5B decoder and
+// 85 for 512, where the tensor-core kernels take 31.
+constexpr int kShortPrompt = 96;
 size_t prefill_attention_scratch_bytes(int kv_heads, int head_dim, int max_ctx);
 cudaError_t prefill_attention_configure(int head_dim);
 cudaError_t launch_prefill_attention(const float*, const float*, const float*, int, int, int, int, const float*, const float*, int, float*,
@@ -194,8 +206,22 @@ int prefill_into(Decoder* d, const int* tokens_dev, const float* embeds_dev, int
       const int tn[3] = {QD, KD, KD};
       DEC_ST(mllmb200_w4a32_linear_forward_grouped(d->xn, n, H, H, 3, tw, ty, tn, tn, d->ws, 5, s));
     }
-    DEC_CHECK(launch_prefill_attention(d->q, d->k, d->v, n, c.q_heads, c.kv_heads, c.head_dim, d->sin_t, d->cos_t, c.max_ctx, cache_k[l],
-                                       cache_v[l], d->kv_split, d->attn, s));
+    if (n <= kShortPrompt) {
+      rope_kv_append_kernel<<<dim3(c.kv_heads, n), c.head_dim, 0, s>>>(d->k, d->v, KD, d->sin_t, d->cos_t, d->zero, c.max_ctx,
+                                                                      cache_k[l], cache_v[l]);
+      const int rows = attention_prefill_rows();  // query rows per CTA, one warp each
+      const dim3 grid((n + rows - 1) / rows, c.kv_heads);
+      const size_t smem = attention_prefill_smem_bytes(c.head_dim);
+      if (c.head_dim == 128)
+        attention_prefill_kernel<128><<<grid, attention_prefill_threads(), smem, s>>>(d->q, QD, n, d->sin_t, d->cos_t, d->zero, c.max_ctx,
+                                                               c.q_heads / c.kv_heads, cache_k[l], cache_v[l], d->attn, QD);
+      else
+        attention_prefill_kernel<64><<<grid, attention_prefill_threads(), smem, s>>>(d->q, QD, n, d->sin_t, d->cos_t, d->zero, c.max_ctx,
+                                                              c.q_heads / c.kv_heads, cache_k[l], cache_v[l], d->attn, QD);
+    } else {
+      DEC_CHECK(launch_prefill_attention(d->q, d->k, d->v, n, c.q_heads, c.kv_heads, c.head_dim, d->sin_t, d->cos_t, c.max_ctx, cache_k[l],
+                                         cache_v[l], d->kv_split, d->attn, s));
+    }
     DEC_ST(mllmb200_w4a32_linear_forward_ex(d->attn, L.w[kO], d->o, d->ws, n, QD, H, QD, H, 5, s));
     add_rmsnorm_quant_kernel<<<n, 256, 0, s>>>(d->h, d->o, L.ln2, c.eps, H, d->h, d->xn, nullptr, nullptr, 0);
     {  // gate and up likewise
