@@ -64,22 +64,6 @@ __global__ void set_int_kernel(int* dst, int v) { *dst = v; }
 
 namespace {
 
-// launch with the programmatic-dependent-launch attribute (the kernels call griddepcontrol themselves)
-template <class... KArgs, class... Args>
-cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid;
-  cfg.blockDim = block;
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = s;
-  cudaLaunchAttribute attr;
-  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr.val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = &attr;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
-}
-
 #define DEC_CHECK(expr)                     \
   do {                                      \
     cudaError_t e__ = (expr);               \
@@ -198,40 +182,41 @@ int prefill_into(Decoder* d, const int* tokens_dev, const float* embeds_dev, int
     DEC_CHECK(cudaMemcpyAsync(d->h, embeds_dev, (size_t)n * H * sizeof(float), cudaMemcpyDeviceToDevice, s));
   for (int l = 0; l < c.layers; ++l) {
     const Layer& L = d->layers[l];
-    add_rmsnorm_quant_kernel<<<n, 256, 0, s>>>(d->h, l == 0 ? nullptr : d->down, L.ln1, c.eps, H, d->h, d->xn, nullptr,
-                                               nullptr, 0);
+    DEC_CHECK(launch_pdl(add_rmsnorm_quant_kernel, dim3(n), dim3(256), 0, s, d->h, l == 0 ? nullptr : d->down, L.ln1, c.eps, H, d->h,
+                         d->xn, nullptr, nullptr, 1));
     {  // q, k, v share one quantization of the normalized rows
       const void* tw[3] = {L.w[kQ], L.w[kK], L.w[kV]};
       float* ty[3] = {d->q, d->k, d->v};
       const int tn[3] = {QD, KD, KD};
-      DEC_ST(mllmb200_w4a32_linear_forward_grouped(d->xn, n, H, H, 3, tw, ty, tn, tn, d->ws, 5, s));
+      DEC_ST(mllmb200_w4a32_linear_forward_grouped(d->xn, n, H, H, 3, tw, ty, tn, tn, d->ws, 5 | 0x100, s));
     }
     if (n <= kShortPrompt) {
-      rope_kv_append_kernel<<<dim3(c.kv_heads, n), c.head_dim, 0, s>>>(d->k, d->v, KD, d->sin_t, d->cos_t, d->zero, c.max_ctx,
-                                                                      cache_k[l], cache_v[l]);
+      DEC_CHECK(launch_pdl(rope_kv_append_kernel, dim3(c.kv_heads, n), dim3(c.head_dim), 0, s, d->k, d->v, KD, d->sin_t, d->cos_t, d->zero,
+                           c.max_ctx, cache_k[l], cache_v[l]));
       const int rows = attention_prefill_rows();  // query rows per CTA, one warp each
       const dim3 grid((n + rows - 1) / rows, c.kv_heads);
       const size_t smem = attention_prefill_smem_bytes(c.head_dim);
       if (c.head_dim == 128)
-        attention_prefill_kernel<128><<<grid, attention_prefill_threads(), smem, s>>>(d->q, QD, n, d->sin_t, d->cos_t, d->zero, c.max_ctx,
-                                                               c.q_heads / c.kv_heads, cache_k[l], cache_v[l], d->attn, QD);
+        DEC_CHECK(launch_pdl(attention_prefill_kernel<128>, grid, dim3(attention_prefill_threads()), smem, s, d->q, QD, n, d->sin_t, d->cos_t, d->zero, c.max_ctx,
+                                                               c.q_heads / c.kv_heads, cache_k[l], cache_v[l], d->attn, QD));
       else
-        attention_prefill_kernel<64><<<grid, attention_prefill_threads(), smem, s>>>(d->q, QD, n, d->sin_t, d->cos_t, d->zero, c.max_ctx,
-                                                              c.q_heads / c.kv_heads, cache_k[l], cache_v[l], d->attn, QD);
+        DEC_CHECK(launch_pdl(attention_prefill_kernel<64>, grid, dim3(attention_prefill_threads()), smem, s, d->q, QD, n, d->sin_t, d->cos_t, d->zero, c.max_ctx,
+                                                              c.q_heads / c.kv_heads, cache_k[l], cache_v[l], d->attn, QD));
     } else {
       DEC_CHECK(launch_prefill_attention(d->q, d->k, d->v, n, c.q_heads, c.kv_heads, c.head_dim, d->sin_t, d->cos_t, c.max_ctx, cache_k[l],
                                          cache_v[l], d->kv_split, d->attn, s));
     }
-    DEC_ST(mllmb200_w4a32_linear_forward_ex(d->attn, L.w[kO], d->o, d->ws, n, QD, H, QD, H, 5, s));
-    add_rmsnorm_quant_kernel<<<n, 256, 0, s>>>(d->h, d->o, L.ln2, c.eps, H, d->h, d->xn, nullptr, nullptr, 0);
+    DEC_ST(mllmb200_w4a32_linear_forward_ex(d->attn, L.w[kO], d->o, d->ws, n, QD, H, QD, H, 5 | 0x100, s));
+    DEC_CHECK(launch_pdl(add_rmsnorm_quant_kernel, dim3(n), dim3(256), 0, s, d->h, d->o, L.ln2, c.eps, H, d->h, d->xn, nullptr, nullptr, 1));
     {  // gate and up likewise
       const void* tw[2] = {L.w[kGate], L.w[kUp]};
       float* ty[2] = {d->gate, d->up};
       const int tn[2] = {I, I};
-      DEC_ST(mllmb200_w4a32_linear_forward_grouped(d->xn, n, H, H, 2, tw, ty, tn, tn, d->ws, 5, s));
+      DEC_ST(mllmb200_w4a32_linear_forward_grouped(d->xn, n, H, H, 2, tw, ty, tn, tn, d->ws, 5 | 0x100, s));
     }
-    silu_mul_quant_kernel<<<n, 512, (size_t)I * sizeof(float), s>>>(d->gate, d->up, I, d->act, nullptr, nullptr, 0);
-    DEC_ST(mllmb200_w4a32_linear_forward_ex(d->act, L.w[kDown], d->down, d->ws, n, I, H, I, H, 5, s));
+    DEC_CHECK(launch_pdl(silu_mul_quant_kernel, dim3(n), dim3(512), (size_t)I * sizeof(float), s, d->gate, d->up, I, d->act, nullptr,
+                         nullptr, 1));
+    DEC_ST(mllmb200_w4a32_linear_forward_ex(d->act, L.w[kDown], d->down, d->ws, n, I, H, I, H, 5 | 0x100, s));
   }
   // only the last position feeds the sampler (the reference computes all rows and reads the last)
   const size_t last = (size_t)(n - 1) * H;

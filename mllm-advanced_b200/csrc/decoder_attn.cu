@@ -31,6 +31,8 @@ __global__ void rope_kv_append_kernel(const float* __restrict__ k_new, const flo
                                       const float* __restrict__ sin_t, const float* __restrict__ cos_t,
                                       const int* __restrict__ pos0_ptr, int max_ctx, float* __restrict__ cache_k,
                                       float* __restrict__ cache_v) {
+  pdl_launch_dependents();
+  pdl_wait_prior();
   const int h = blockIdx.x, s = blockIdx.y, d = threadIdx.x, D = blockDim.x, half = D >> 1;
   const int pos = *pos0_ptr + s;  // the position lives in device memory so that one CUDA graph serves every step
   if (pos >= max_ctx) return;
@@ -88,6 +90,8 @@ __global__ void __launch_bounds__(kPfThreads) attention_prefill_kernel(
     const int* __restrict__ pos0_ptr, int max_ctx, int group, const float* __restrict__ cache_k,
     const float* __restrict__ cache_v, float* __restrict__ out, int ldo) {
   extern __shared__ __align__(16) uint8_t pf_smem[];
+  pdl_launch_dependents();
+  pdl_wait_prior();
   PrefillAttnSmem<D>& sm = *reinterpret_cast<PrefillAttnSmem<D>*>(pf_smem);
   constexpr int HALF = D / 2, NG = kPfThreads / (D / 4), QPT = (kPfRows * kAttnMaxGroup + NG - 1) / NG;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;

@@ -20,6 +20,7 @@
 // the tensor pipe).  Tiles are dispatched longest causal range first.
 #include <cuda_fp16.h>
 
+#include "decoder_state.h"
 #include "device_common.cuh"
 #include "tcgen05_common.cuh"
 
@@ -68,6 +69,8 @@ __global__ void __launch_bounds__(kPsThreads) prefill_kv_split_kernel(
     uint8_t* __restrict__ tiles, float2* __restrict__ tile_scales) {
   using L = PaLayout<D>;
   constexpr int HALF = D / 2, KI = kPaKeys * HALF / 4 / kPsThreads, VI = kPaKeys * D / 4 / kPsThreads;
+  pdl_launch_dependents();
+  pdl_wait_prior();
   extern __shared__ __align__(16) float ps_smem[];
   float(*s_k)[D + 1] = reinterpret_cast<float(*)[D + 1]>(ps_smem);
   float(*s_v)[D + 1] = s_k + kPaKeys;
@@ -165,6 +168,8 @@ __global__ void __launch_bounds__(kPaThreads, 1) attention_prefill_tc_kernel(
     int kv_heads, const uint8_t* __restrict__ tiles, const float2* __restrict__ tile_scales, float* __restrict__ out, int ldo) {
   using L = PaLayout<D>;
   constexpr int HALF = D / 2, QD = HALF / 2, kStages = L::kStages;  // QD: rotated pairs per thread
+  pdl_launch_dependents();
+  pdl_wait_prior();
   extern __shared__ __align__(128) uint8_t pa_smem[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(pa_smem) + 1023) & ~uintptr_t(1023));
   uint64_t* k_full = reinterpret_cast<uint64_t*>(smem);
@@ -422,15 +427,16 @@ cudaError_t configure() {
   return cudaFuncSetAttribute(attention_prefill_tc_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, PaLayout<D>::kTotal);
 }
 template <int D>
-void launch(const float* q, const float* k, const float* v, int n, int q_heads, int kv_heads, const float* sin_t, const float* cos_t,
+cudaError_t launch(const float* q, const float* k, const float* v, int n, int q_heads, int kv_heads, const float* sin_t, const float* cos_t,
             int max_ctx, float* cache_k, float* cache_v, uint8_t* scratch, float* out, cudaStream_t s) {
   const int tiles = (n + kPaKeys - 1) / kPaKeys, group = q_heads / kv_heads, tokens = 128 / group;
   float2* scales = reinterpret_cast<float2*>(scratch);
   uint8_t* ops = scratch + (size_t)kPaMaxTiles * kv_heads * sizeof(float2);
-  prefill_kv_split_kernel<D><<<dim3(tiles, kv_heads), kPsThreads, ps_smem_bytes(D), s>>>(k, v, kv_heads * D, n, sin_t, cos_t, max_ctx, cache_k, cache_v,
-                                                                                      ops, scales);
-  attention_prefill_tc_kernel<D><<<(n + tokens - 1) / tokens * kv_heads, kPaThreads, PaLayout<D>::kTotal, s>>>(
-      q, q_heads * D, n, sin_t, cos_t, group, kv_heads, ops, scales, out, q_heads * D);
+  const cudaError_t e = launch_pdl(prefill_kv_split_kernel<D>, dim3(tiles, kv_heads), dim3(kPsThreads), ps_smem_bytes(D), s, k, v, kv_heads * D, n,
+                                   sin_t, cos_t, max_ctx, cache_k, cache_v, ops, scales);
+  if (e != cudaSuccess) return e;
+  return launch_pdl(attention_prefill_tc_kernel<D>, dim3((n + tokens - 1) / tokens * kv_heads), dim3(kPaThreads), PaLayout<D>::kTotal, s, q,
+                    q_heads * D, n, sin_t, cos_t, group, kv_heads, ops, scales, out, q_heads * D);
 }
 }  // namespace
 
@@ -446,9 +452,9 @@ cudaError_t prefill_attention_configure(int head_dim) { return head_dim == 128 ?
 cudaError_t launch_prefill_attention(const float* q, const float* k, const float* v, int n, int q_heads, int kv_heads, int head_dim,
                                      const float* sin_t, const float* cos_t, int max_ctx, float* cache_k, float* cache_v, uint8_t* scratch,
                                      float* out, cudaStream_t s) {
-  if (head_dim == 128) launch<128>(q, k, v, n, q_heads, kv_heads, sin_t, cos_t, max_ctx, cache_k, cache_v, scratch, out, s);
-  else launch<64>(q, k, v, n, q_heads, kv_heads, sin_t, cos_t, max_ctx, cache_k, cache_v, scratch, out, s);
-  return cudaGetLastError();
+  return head_dim == 128
+             ? launch<128>(q, k, v, n, q_heads, kv_heads, sin_t, cos_t, max_ctx, cache_k, cache_v, scratch, out, s)
+             : launch<64>(q, k, v, n, q_heads, kv_heads, sin_t, cos_t, max_ctx, cache_k, cache_v, scratch, out, s);
 }
 
 }  // namespace mllmb200
