@@ -330,7 +330,8 @@ __global__ void __launch_bounds__(kTcThreads, 1) lm_gemm_tc_kernel(const __grid_
   __shared__ uint32_t tmem_slot;
   __shared__ volatile int gave_up;
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(tc_smem_raw) + 1023) & ~(uintptr_t)1023);
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  // (warp-uniform for the compiler, here and in the MMA warp)
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
   int mt = (M + kTileM - 1) / kTileM;
   const int nt = (N + BN - 1) / BN, kt = K / kTileK;
   int a_rows = M >= kTileM ? kTileM : (M + 15) / 16 * 16;  // rows of x that are loaded at all
@@ -352,7 +353,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) lm_gemm_tc_kernel(const __grid_
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = tmem_slot;
+  const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_slot, 0);
   pdl_launch_dependents();
   auto k_range = [&](int split, int& k0, int& k1) {
     k0 = (int)((long long)kt * split / splits);
@@ -407,6 +408,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) lm_gemm_tc_kernel(const __grid_
   } else if (warp == 1) {
     const bool leader = elect_one_sync();
     const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(kTileM >> 4) << 24);
+    const uint32_t smem0 = (smem_u32(tc_smem_raw) + 1023u) & ~1023u;
     int it = 0, t = 0;
     bool ok = true;
     if (GROUPED) grouped_start();
@@ -414,18 +416,18 @@ __global__ void __launch_bounds__(kTcThreads, 1) lm_gemm_tc_kernel(const __grid_
       int k0, k1;
       k_range(item / (mt * nt), k0, k1);
       const int buf = t & 1;
-      if (t >= 2 && (gave_up || !mbar_wait_bounded(&acc_empty[buf], ((t >> 1) & 1) ^ 1))) ok = false;
+      if (t >= 2) ok = __all_sync(0xffffffffu, !gave_up && mbar_wait_bounded(&acc_empty[buf], ((t >> 1) & 1) ^ 1));
       tc_fence_after();
       for (int k = k0; k < k1 && ok; ++k, ++it) {
         const int st = it % S::kStages;
-        if (gave_up || !mbar_wait_bounded(&full[st], (it / S::kStages) & 1)) {
-          ok = false;
-          break;
-        }
+        ok = __all_sync(0xffffffffu, !gave_up && mbar_wait_bounded(&full[st], (it / S::kStages) & 1));
+        if (!ok) break;
         tc_fence_after();
+        // The instructions' operands are values of the whole warp, computed outside of the elected lane's branch: they issue
+        // faster than from the registers of a diverged lane (prompt of 1500 tokens, 28 layers of width 1536: 8.94 / 8.70 ms).
+        const uint32_t a = smem0 + (uint32_t)(st * S::kStageBytes);
+        const uint64_t ad = swizzled_desc(a), bd = swizzled_desc(a + kABytes);
         if (leader) {
-          const uint32_t a = smem_u32(smem + (size_t)st * S::kStageBytes);
-          const uint64_t ad = swizzled_desc(a), bd = swizzled_desc(a + kABytes);
 #pragma unroll
           for (int j = 0; j < kTileK / 16; ++j)
             tc_mma_f16(tmem + buf * BN, ad + j * 2, bd + j * 2, idesc, (k > k0 || j > 0) ? 1u : 0u);
