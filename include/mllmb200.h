@@ -135,8 +135,7 @@ MLLMB200_API int mllmb200_w4a32_linear_forward(const float* x_dev, const void* t
  * tensor memory; same 1e-3*rms bound; auto never picks it; launches that would fill less than half of the SMs
  * split K between two CTAs per output tile, and y holds one half's partial sums for a moment during the
  * call - deterministic, but y is scratch until the call's work on the stream has finished), 5 fastest: kernel 4
- * for M >= 128, at 65 <= M < 128 for K > 4096, at M = 64 for matrices (or groups) of at least 8192 rows with K <= 4096;
- * else auto,
+ * for M >= 128 and, at 64 <= M < 128, for matrices (or groups) of at least 8192 rows with K <= 4096; else auto,
  * 6 the two-launch GEMV (activation-quantization kernel + one-shot GEMV), kept for comparison,
  * 7 streaming tensor-core GEMM for small batches (M <= 64; what auto picks for 5 <= M <= 64): the weight cells are
  * spread over all SMs as in the GEMV, the per-group integer products run as mma.sync u8 x s8 (exact int32 group
@@ -388,7 +387,8 @@ MLLMB200_API int mllmb200_qwen2_batch_read(void* handle, int seq, int first, int
  *   linear_forward_tp  y[:, r N/g : (r+1) N/g] = x W_r^T + b_r on this rank, delivered to all ranks:
  *                    gather_mode 2 = the kernels' epilogues store every finished element into every rank's buffer
  *                    (plain stores over NVLink while other tiles are still computed: the single-launch GEMV for
- *                    M <= 4, the fp16 tensor-core GEMM for kernel policies 4 / 5 at M >= 128; other kernels
+ *                    M <= 4, the fp16 tensor-core GEMM for kernel policies 4 / 5 at M >= 128, and from M = 64 for
+ *                    shards of at least 8192 rows with K <= 4096; other kernels
  *                    compute the block and push it with strided device copies), then each rank flags every peer
  *                    and waits - bounded, MLLMB200_TIMEOUT through mllmb200_check_device_status - for theirs;
  *                    1 = NCCL baseline (ncclAllGather of the blocks + a re-assembly kernel; needs the

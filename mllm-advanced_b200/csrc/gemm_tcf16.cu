@@ -652,16 +652,15 @@ int w4a32_gemm_tcf16_m_pad(int m, int n) {
 }
 int w4a32_gemm_tcf16_m_pad_max(int m) { return (m + 255) / 256 * 256; }
 bool w4a32_gemm_tcf16_supported(int m, int k, int n) { return m >= 64 && k >= 1 && n >= 1 && (m + 63) / 64 <= 65535; }
-// Shapes on which this path is at least as fast as the int8 path (measured on the Qwen2-1.5B layer
-// shapes at M = 512: 17 vs 18 us for N = 1536 / 256, 24 vs 60 us for N = 8960, 59 vs 68 us for K = 8960).
-// At M = 64 only where the weight tiles alone fill the GPU and K is short (gate / up of the 1.5B model, alone or grouped: 17
-// vs 30 us against the streaming small-batch GEMM); narrow or long-K matrices stay there.  At 64 < M < 128 only for a long
-// K, which it splits between two CTAs (1536 x 8960: see gemm_chunk.cu's 53 us at M = 65); shorter ones take gemm_chunk.cu
-// (9728 x 896, M = 65: 16 us here, 11 there; 17920 x 1536 24 with either).
+// Where the "fastest" policy (5) takes this kernel: from 128 rows on (1.5B layer shapes, M = 512, against the default, which is
+// gemm_chunk.cu: 8960 x 1536 26 vs 29 us, 17920 x 1536 39 vs 50, 1536 x 8960 42 vs 63; 1536 x 1536 20 vs 19); below that only
+// where the weight tiles alone fill the GPU and K is short (gate / up of the 1.5B model, alone or grouped: M = 64 17 vs 30 us
+// against the streaming small-batch GEMM, M = 65 to 127 15 vs 16 to 17 us against gemm_chunk.cu).  Narrow or long-K matrices
+// stay with the default there: ONE truncated fp32 sum over a long K is off by 4.3e-7 at K = 8960 (gemm_chunk.cu 9.6e-8, int32
+// group sums 1.4e-7), and fp16-encoded scales are rounded here, not there.
 bool w4a32_gemm_tcf16_preferred(int m, int k, int n) {
   if (!w4a32_gemm_tcf16_supported(m, k, n)) return false;
-  if (m == 64) return MLLMB200_TF_SMALL_M && n >= 8192 && k <= 4096;
-  return m >= 128 || k > 4096;
+  return m >= 128 || (MLLMB200_TF_SMALL_M && n >= 8192 && k <= 4096);
 }
 
 // Up to four matrices that share x in ONE launch (their weight tiles side by side in the grid):
