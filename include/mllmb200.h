@@ -127,9 +127,10 @@ MLLMB200_API int mllmb200_w4a32_linear_forward(const float* x_dev, const void* t
                                                void* stream);
 
 /* Same, with the kernel family forced (tests and benchmarks):
- * 0 auto, 1 streaming GEMV (M <= 4: ONE launch, x quantized inside it, ws_dev unused), 2 SIMT dp4a GEMM,
- * 3 tcgen05 tile GEMM (M <= 64 kind::i8, exact int32 group sums; above, fp16 operands with exact products and chunks
- * of K summed in tensor memory, the chunks in fp32 registers), 4 tcgen05 fp16 GEMM (M >= 64: group
+ * 0 auto (kernel 1, 7, 3 or 2 up to 64 rows; from 65 rows on a tcgen05 GEMM with fp16 operands and exact products:
+ * chunks of K summed in tensor memory, the chunks in fp32 registers; closer to the exact sum than kernels 2 and 3, not
+ * their bits), 1 streaming GEMV (M <= 4: ONE launch, x quantized inside it, ws_dev unused), 2 SIMT dp4a GEMM,
+ * 3 tcgen05 kind::i8 GEMM (M >= 17: exact int32 group sums, as the reference), 4 tcgen05 fp16 GEMM (M >= 64: group
  * scales folded into an fp16 weight operand - exact for bf16-encoded scales, rounded to fp16's 11 bits
  * (relative error <= 2^-11 per weight) for MLLMB200_SCALE_FP16 - fp32 accumulation over all of K in
  * tensor memory; same 1e-3*rms bound; auto never picks it; launches that would fill less than half of the SMs
@@ -159,7 +160,8 @@ MLLMB200_API int mllmb200_w4a32_linear_forward_grouped(const float* x_dev, int M
                                                        const int* N, const int* ldy, void* ws_dev, int flags,
                                                        void* stream);
 
-/* Which kernel family `kernel = 0` picks for a shape (1, 2 or 3 as above). */
+/* Which kernel family `kernel = 0` picks for a shape: 1, 2 or 7 as above, 3 the tcgen05 tile GEMMs (up to 64 rows kernel 3
+ * itself, above the form with chunked sums). */
 MLLMB200_API int mllmb200_w4a32_select_kernel(int M, int K, int N);
 
 /* Several INDEPENDENT linears in one launch: count in [1,8] matrices [N[i], K[i]], each with its own

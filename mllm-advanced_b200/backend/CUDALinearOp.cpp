@@ -206,8 +206,9 @@ void CUDAW4A32LinearOp::forward(const std::vector<Tensor>& inputs, std::vector<T
   // grow once and keep: the reference allocates a workspace tensor on every call (LinearOp.cpp:41-43)
   if (need > workspace_bytes_) growWorkspace(need);
   auto& be = registeredW4A32Backend();
+  const int policy = be.linearKernelPolicy() == 3 && m < 65 ? 0 : be.linearKernelPolicy();
   MLLMB200_CHECK(mllmb200_w4a32_linear_forward_ex(x.ptr<float>(), tiled_dev_, y.ptr<float>(), workspace_dev_, m, k_, n_, k_,
-                                                  n_, be.linearKernelPolicy(), be.stream()));
+                                                  n_, policy, be.stream()));
 }
 
 }  // namespace mllm::cuda

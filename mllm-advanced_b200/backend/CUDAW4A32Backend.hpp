@@ -55,8 +55,9 @@ class CUDAW4A32Backend final : public BackendBase {
   void deviceFree(void* ptr);
 
   // Kernel policy of CUDAW4A32LinearOp::forward for M >= 65 (the `kernel` argument of
-  // mllmb200_w4a32_linear_forward_ex): 0 = the exact int8 tensor-core path (default: the reference's
-  // arithmetic), 5 = the fastest path (fp16 tensor-core kernel for M >= 128, same 1e-3 * rms bound).
+  // mllmb200_w4a32_linear_forward_ex): 0 = the default (fp16 tensor-core products, all exact, summed in fp32 chunk by
+  // chunk), 3 = int8 tensor cores with the reference's exact int32 group sums (fewer rows: as 0, whose kernels keep those
+  // sums there), 5 = the fastest path (one fp32 sum over all of K for M >= 128, same 1e-3 * rms bound).
   void setLinearKernelPolicy(int policy) { linear_policy_ = policy; }
   [[nodiscard]] int linearKernelPolicy() const { return linear_policy_; }
 

@@ -54,8 +54,8 @@ cudaError_t launch_w4a32_gemm_stream(const uint8_t*, const float2*, int, int, in
                                      const int*, const int*, int, cudaStream_t);
 constexpr int kStreamGemmMinM = 5, kStreamGemmMaxM = 64;  // batch sizes the streaming tensor-core GEMM takes by default
 
-// gemm_chunk.cu: kernel id 3 from kChunkMinM rows on.  Up to 64 rows gemm_tc.cu, whose int8 activations take half of the
-// workspace (M = 65, 1536 x 1536: 18.7 us with gemm_tc.cu, 13.7 with gemm_chunk.cu; 17920 x 1536: 36 and 24).
+// gemm_chunk.cu: what the default runs from kChunkMinM rows on where select_kernel says 3 (M = 65, 1536 x 1536: 18.7 us with
+// gemm_tc.cu, 13.7 with gemm_chunk.cu; 17920 x 1536: 36 and 24).  Kernel 3 by name is gemm_tc.cu at any M.
 cudaError_t launch_w4a32_gemm_chunk(const uint8_t*, const float2*, int, int, int, const void* const*, float* const*, const int*,
                                     const int*, int, cudaStream_t);
 constexpr int kChunkMinM = 65;
@@ -234,7 +234,8 @@ int mllmb200_w4a32_linear_forward_ex(const float* x_dev, const void* tiled_dev, 
   kernel &= 0xFF;
   if (kernel < 0 || kernel > 7) return MLLMB200_INVALID_ARG;
   if (kernel == 5) kernel = w4a32_gemm_tcf16_preferred(M, K, N) ? 4 : 0;  // "fastest": fp16 path where it wins
-  if (kernel == 0) kernel = mllmb200_w4a32_select_kernel(M, K, N);
+  const bool by_default = kernel == 0;
+  if (by_default) kernel = mllmb200_w4a32_select_kernel(M, K, N);
   if (kernel == 1) {  // single launch: x is quantized inside the GEMV, no workspace
     if (!w4a32_gemv_stream_supported(M, 1, &K, &N)) return MLLMB200_UNSUPPORTED;
     const cudaError_t e1 =
@@ -252,7 +253,7 @@ int mllmb200_w4a32_linear_forward_ex(const float* x_dev, const void* tiled_dev, 
   }
   if (kernel == 6 && !w4a32_gemv_supported(M, K, N)) return MLLMB200_UNSUPPORTED;
   if (kernel == 3 && !w4a32_gemm_tc_supported(M, K, N)) return MLLMB200_UNSUPPORTED;
-  if (kernel == 3 && M >= kChunkMinM)
+  if (kernel == 3 && by_default && M >= kChunkMinM)
     return chunk_forward(x_dev, M, K, ldx, 1, &tiled_dev, &y_dev, &N, &ldy, ws_dev, use_pdl, st);
   if (kernel == 4) {  // fp16 tensor-core path: its own activation layout
     if (!w4a32_gemm_tcf16_supported(M, K, N)) return MLLMB200_UNSUPPORTED;
@@ -327,10 +328,10 @@ int mllmb200_w4a32_linear_forward_grouped(const float* x_dev, int M, int K, int 
     cudaError_t e = launch_w4a32_gemv_grouped(a_rec, a_hdr, M, K, count, tiled_dev, y_dev, N, ldy, (flags >> 8) & 1, st);
     return e == cudaSuccess ? MLLMB200_OK : cuda_fail(e);
   }
-  // Larger M: the matrices share ONE quantization of x.  With the "fastest" policy (5) and M >= 128 they
-  // also share ONE launch of the fp16 tensor-core kernel (their tiles side by side in the grid: q, k, v
-  // alone fill 16 + 2 + 2 tiles); with the default policy, or when the fp16 path does not apply, they
-  // run as separate int8 tensor-core launches behind one quantization, or as ordinary forwards.
+  // Larger M: the matrices share ONE quantization of x.  From M = 65 they also share ONE launch, their tiles side by
+  // side in the grid (q, k, v alone fill 16 + 2 + 2): of gemm_tcf16.cu where the "fastest" policy (5) takes it, else of
+  // gemm_chunk.cu.  Below, what the streaming kernel does not take runs as separate int8 tensor-core launches behind one
+  // quantization, or as ordinary forwards.
   const int policy = flags & 0xFF;  // 0 auto, 5 fastest (as the kernel argument of linear_forward_ex)
   if (policy != 0 && policy != 5) return MLLMB200_INVALID_ARG;
   cudaStream_t st_grp = static_cast<cudaStream_t>(stream);

@@ -1,5 +1,5 @@
-// tcgen05 (5th-generation tensor core) W4A32 GEMM for 17 <= M <= 64, sm_100a: kernel id 3 there, and the
-// default where the streaming kernel does not take K.
+// tcgen05 (5th-generation tensor core) W4A32 GEMM for M >= 17, sm_100a: kernel id 3, and the default up to
+// 64 rows where the streaming kernel does not take K (from 65 rows on the default is gemm_chunk.cu).
 //
 // The reference quantizes activations to int8 per row and accumulates every 32-wide K-group in
 // int32 before applying that group's weight scale (tests/Arm/KaiLinearTest.hpp:338-373 of the

@@ -109,3 +109,32 @@ def test_fastest_policy_below_128_rows_is_as_close_as_int32_sums(m, k, n, mode):
     grouped = mb.linear_forward_grouped(xd, [wt, wt], policy=mb.KERNEL_FASTEST)
     mb.check_device_status()
     assert err(single) <= 1.2 * exact_sums and all(err(y) <= 1.2 * exact_sums for y in grouped)
+
+
+@pytest.mark.parametrize("m,k,n", [(65, 1536, 96), (130, 1176, 200), (512, 96, 160)])
+def test_kernel_3_keeps_int32_group_sums_at_any_m(m, k, n):
+    """Kernel 3 by name is the int8 kernel with the reference's arithmetic: exact int32 sums of a K-group, one fused
+    multiply-add with the group's scale each, in K order.  Bit for bit (a 64-bit sum rounded to 32 is the fused operation:
+    products of 21 + 8 bits are exact)."""
+    orc, rng = Oracle(), np.random.default_rng(m + k)
+    x = rng.standard_normal((m, k)).astype(np.float32)
+    bias = (rng.standard_normal(n) * 0.1).astype(np.float32)
+    blob = mb.quant_prepack((rng.standard_normal((n, k)) * 0.02).astype(np.float32), bias)
+    raw = np.ascontiguousarray(orc.quant_act(x)).reshape(m, -1).view(np.uint8)
+    head = np.ascontiguousarray(raw[:, :8])
+    a = np.zeros((m, (k + 31) // 32 * 32))
+    a[:, :k] = raw[:, 8:8 + k].view(np.int8)
+    nib, sc, _ = mb.blob_sections(blob)
+    u = np.zeros((n, a.shape[1]))
+    u[:, :k] = np.stack([nib & 15, nib >> 4], axis=-1).reshape(n, -1)[:, :k].astype(np.float64) - 8
+    s = (sc.reshape(n, -1).astype(np.uint32) << 16).view(np.float32).astype(np.float64)
+    acc, zsum = np.zeros((m, n), np.float32), np.zeros(n)
+    for g in range(s.shape[1]):
+        ug = u[:, 32 * g:32 * g + 32]
+        acc = (a[:, 32 * g:32 * g + 32] @ ug.T * s[:, g] + acc).astype(np.float32)
+        zsum += ug.sum(1) * s[:, g]
+    acc = (head.view(np.int32)[:, 1:].astype(np.float64) * zsum.astype(np.float32) + acc).astype(np.float32)
+    want = (head.view(np.float32)[:, :1].astype(np.float64) * acc + bias).astype(np.float32)
+    y = mb.linear_forward(torch.from_numpy(x).cuda(), mb.W4A32Weights.from_blob(blob), kernel=mb.KERNEL_TC)
+    mb.check_device_status()
+    assert np.array_equal(y.cpu().numpy(), want)
