@@ -321,8 +321,9 @@ int w4a32_gemm_tc_m_pad(int m) { return (m + 63) / 64 * 64; }
 
 bool w4a32_gemm_tc_supported(int m, int k, int n) {
   // one CTA per SM holds 128 KB+ of shared memory and all tensor memory it allocates; any K, any N.
-  // Below ~17 rows the GEMV / SIMT paths are the better fit.
-  return m >= 17 && k >= 1 && n >= 1 && (size_t)((m + 127) / 128) <= 65535;
+  // Below ~17 rows the GEMV / SIMT paths are the better fit.  At most 65535 tiles of 64 rows along the grid's y; the fp16
+  // tile GEMMs' activation blocks have their room in the workspace up to the same M.
+  return m >= 17 && k >= 1 && n >= 1 && m <= 65535 * 64;
 }
 
 cudaError_t launch_w4a32_gemm_tc(const uint8_t* a_blocks, const float2* a_hdr, const void* tiled, float* y, int m, int k,

@@ -119,6 +119,18 @@ def test_default_kernel_by_batch_size():
     assert L.mllmb200_w4a32_select_kernel(8, 32768, 64) == mb.KERNEL_STREAM_TC               # ... but those of 8 rows do
 
 
+def test_workspace_covers_the_tile_gemms_up_to_their_last_row():
+    """Where the default takes a tile GEMM above 64 rows, the workspace holds its fp16 activation blocks (64 bytes per row and
+    K-group, rows in eights) and the rows' headers; beyond the rows that its launch can cover it takes no tile GEMM."""
+    last = 65535 * 64
+    for m in (65, last - 1, last, last + 1, 2 * last, 2 * last + 1):
+        for k in (32, 96):
+            taken = mb.lib().mllmb200_w4a32_select_kernel(m, k, 32) == mb.KERNEL_TC
+            assert taken == (m <= last), m
+            if taken:
+                assert mb.workspace_size(m, k) >= (k // 32) * ((m + 7) // 8 * 8) * 64 + m * 8, (m, k)
+
+
 def test_gemv_plan_replay_covers_every_cell_once():
     """The streaming GEMV's work decomposition, replayed on the host with the kernel's own walk: every weight
     cell requested and consumed once, every activation group a CTA reads quantized by it, every panel finished
