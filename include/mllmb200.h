@@ -417,6 +417,14 @@ MLLMB200_API void mllmb200_w4a32_tp_destroy(void* handle);
  * NULL) is 1.  The kernel returns normally; nothing faults. */
 MLLMB200_API int mllmb200_selftest_wait_timeout(long long limit_ticks, int* gave_up_dev, void* stream);
 
+/* The Qwen2 decoder's prompt attention by itself (tests): causal, n tokens from position 0, RoPE with the given tables.
+ * form: 0 = what a prompt of n tokens takes, 1 = fp32 on the CUDA cores, 2 = tensor cores.  q_dev and out_dev
+ * [n, q_heads * head_dim], k_dev and v_dev [n, kv_heads * head_dim], sin_dev and cos_dev [n, head_dim / 2], caches
+ * [kv_heads][n][head_dim].  The limits are the decoder's; allocates its scratch memory and synchronizes `stream`. */
+MLLMB200_API int mllmb200_selftest_prompt_attention(const float* q_dev, const float* k_dev, const float* v_dev, int n, int q_heads,
+                                                    int kv_heads, int head_dim, const float* sin_dev, const float* cos_dev, int form,
+                                                    float* cache_k_dev, float* cache_v_dev, float* out_dev, void* stream);
+
 /* Device-side status word (bounded waits that ran out, bad tile headers).  Synchronizes `stream`,
  * reads and clears the word.  0 = clean. */
 MLLMB200_API int mllmb200_check_device_status(void* stream);

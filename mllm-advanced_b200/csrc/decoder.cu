@@ -45,9 +45,10 @@ __global__ void attention_prefill_kernel(const float*, int, int, const float*, c
 size_t attention_prefill_smem_bytes(int head_dim);
 int attention_prefill_rows();
 int attention_prefill_threads();
-// Prompts up to here keep the fp32 attention on the CUDA cores (decoder_attn.cu): the tensor-core kernels' chain of set-up,
-// splitting and tile latencies costs 19 us a layer whatever the length, these 16 us for 40 tokens of the 1.5B decoder and
-// 85 for 512, where the tensor-core kernels take 31.
+// Prompts up to here keep the fp32 attention on the CUDA cores (decoder_attn_rows.cuh).  Its time grows by blocks of 32
+// positions, the tensor-core kernels' by tiles of 64 from a chain of set-up, splitting and tile latencies.  A layer's two
+// kernels, fp32 / tensor cores, us: 12 heads of 128 at 64 tokens 15 / 18, 96 20 / 20, 97 24 / 20, 512 87 / 31; 14 heads of 64
+// at 96 13 / 14, 97 16 / 14, 512 54 / 24; 16 heads of 128 on 4 at 96 18 / 20, 97 22 / 20.
 constexpr int kShortPrompt = 96;
 size_t prefill_attention_scratch_bytes(int kv_heads, int head_dim, int max_ctx);
 cudaError_t prefill_attention_configure(int head_dim);
@@ -59,6 +60,7 @@ __global__ void act_quant_records_kernel(const float*, int, int, int, uint8_t*, 
 cudaError_t launch_w4a32_gemv_grouped(const uint8_t*, const float2*, int, int, int, const void* const*, float* const*,
                                       const int*, const int*, int, cudaStream_t);
 cudaError_t launch_act_quant_records(const float*, int, int, int, uint8_t*, float2*, int, int, cudaStream_t);
+int record_cuda_failure(cudaError_t e);  // c_api.cu
 
 __global__ void set_int_kernel(int* dst, int v) { *dst = v; }
 
@@ -165,6 +167,33 @@ int check_ready(Decoder* d) {
   return MLLMB200_OK;
 }
 
+static cudaError_t prompt_attention_configure(int head_dim) {
+  const cudaError_t e = head_dim == 128 ? cudaFuncSetAttribute(attention_prefill_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                               (int)attention_prefill_smem_bytes(128))
+                                        : cudaFuncSetAttribute(attention_prefill_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                               (int)attention_prefill_smem_bytes(64));
+  return e == cudaSuccess ? prefill_attention_configure(head_dim) : e;
+}
+// A layer's attention over a prompt of n tokens from position 0 (*zero): rotated keys and values into the cache, the
+// attention's rows into out.  tensor_cores: decoder_attn_prefill.cu, else fp32 on the CUDA cores.
+static cudaError_t prompt_attention(bool tensor_cores, const float* q, const float* k, const float* v, int n, int q_heads, int kv_heads,
+                                    int head_dim, const float* sin_t, const float* cos_t, const int* zero, int max_ctx, float* cache_k,
+                                    float* cache_v, uint8_t* scratch, float* out, cudaStream_t s) {
+  if (tensor_cores)
+    return launch_prefill_attention(q, k, v, n, q_heads, kv_heads, head_dim, sin_t, cos_t, max_ctx, cache_k, cache_v, scratch, out, s);
+  const int QD = q_heads * head_dim, group = q_heads / kv_heads;
+  const cudaError_t e = launch_pdl(rope_kv_append_kernel, dim3(kv_heads, n), dim3(head_dim), 0, s, k, v, kv_heads * head_dim, sin_t, cos_t,
+                                   zero, max_ctx, cache_k, cache_v);
+  if (e != cudaSuccess) return e;
+  const int rows = attention_prefill_rows();  // query rows per CTA
+  const dim3 grid((n + rows - 1) / rows, kv_heads), block(attention_prefill_threads());
+  const size_t smem = attention_prefill_smem_bytes(head_dim);
+  return head_dim == 128 ? launch_pdl(attention_prefill_kernel<128>, grid, block, smem, s, q, QD, n, sin_t, cos_t, zero, max_ctx, group,
+                                      cache_k, cache_v, out, QD)
+                         : launch_pdl(attention_prefill_kernel<64>, grid, block, smem, s, q, QD, n, sin_t, cos_t, zero, max_ctx, group,
+                                      cache_k, cache_v, out, QD);
+}
+
 // The prompt pass of the batch-1 decoder, writing keys / values into the given per-layer caches
 // ([kv_heads][max_ctx][D] each) and the sampled token and position into the given words: the decoder's own for
 // mllmb200_qwen2_prefill, a sequence's for the batched decoder (decoder_batch.cu).  Exactly one of tokens_dev
@@ -190,22 +219,8 @@ int prefill_into(Decoder* d, const int* tokens_dev, const float* embeds_dev, int
       const int tn[3] = {QD, KD, KD};
       DEC_ST(mllmb200_w4a32_linear_forward_grouped(d->xn, n, H, H, 3, tw, ty, tn, tn, d->ws, 5 | 0x100, s));
     }
-    if (n <= kShortPrompt) {
-      DEC_CHECK(launch_pdl(rope_kv_append_kernel, dim3(c.kv_heads, n), dim3(c.head_dim), 0, s, d->k, d->v, KD, d->sin_t, d->cos_t, d->zero,
-                           c.max_ctx, cache_k[l], cache_v[l]));
-      const int rows = attention_prefill_rows();  // query rows per CTA, one warp each
-      const dim3 grid((n + rows - 1) / rows, c.kv_heads);
-      const size_t smem = attention_prefill_smem_bytes(c.head_dim);
-      if (c.head_dim == 128)
-        DEC_CHECK(launch_pdl(attention_prefill_kernel<128>, grid, dim3(attention_prefill_threads()), smem, s, d->q, QD, n, d->sin_t, d->cos_t, d->zero, c.max_ctx,
-                                                               c.q_heads / c.kv_heads, cache_k[l], cache_v[l], d->attn, QD));
-      else
-        DEC_CHECK(launch_pdl(attention_prefill_kernel<64>, grid, dim3(attention_prefill_threads()), smem, s, d->q, QD, n, d->sin_t, d->cos_t, d->zero, c.max_ctx,
-                                                              c.q_heads / c.kv_heads, cache_k[l], cache_v[l], d->attn, QD));
-    } else {
-      DEC_CHECK(launch_prefill_attention(d->q, d->k, d->v, n, c.q_heads, c.kv_heads, c.head_dim, d->sin_t, d->cos_t, c.max_ctx, cache_k[l],
-                                         cache_v[l], d->kv_split, d->attn, s));
-    }
+    DEC_CHECK(prompt_attention(n > kShortPrompt, d->q, d->k, d->v, n, c.q_heads, c.kv_heads, c.head_dim, d->sin_t, d->cos_t, d->zero, c.max_ctx,
+                               cache_k[l], cache_v[l], d->kv_split, d->attn, s));
     DEC_ST(mllmb200_w4a32_linear_forward_ex(d->attn, L.w[kO], d->o, d->ws, n, QD, H, QD, H, 5 | 0x100, s));
     DEC_CHECK(launch_pdl(add_rmsnorm_quant_kernel, dim3(n), dim3(256), 0, s, d->h, d->o, L.ln2, c.eps, H, d->h, d->xn, nullptr, nullptr, 1));
     {  // gate and up likewise

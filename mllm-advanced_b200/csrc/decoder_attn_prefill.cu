@@ -3,11 +3,20 @@
 //   RoPE (half-split) and the cache append          mllm/Backends/Arm/Kernels/rope.cpp:20-87, Ops/KVCacheOp.cpp:15-72
 //
 // The two products run as tcgen05.mma kind::f16 on operands split in two, x 2^E = hi + lo with hi = fp16(x 2^E) and
-// lo = fp16(x 2^E - hi): 22 significant bits, the rest below 2^-24 |x|; hi hi + hi lo + lo hi drops less than 2^-24 of
-// a product.  2^E (one per query row, one per 64-position tile of K and of V, the tile's largest magnitude at 2^13)
-// keeps both halves clear of fp16's range and of its subnormals whatever the size of the numbers.  Every product is
-// exact in the fp32 accumulator; a tile's P.V leaves tensor memory after 64 positions and is added in registers, so
-// that no sum runs through more than 64 (scores: D) additions on the tensor core.
+// lo = fp16(x 2^E - hi).  2^E (one per query row, one per 64-position tile of K and of V, the largest magnitude at 2^13) keeps
+// hi clear of fp16's range and subnormals; what is lost of x is at most 2^-22 |x|, or 2^-38 of the row's or tile's largest
+// magnitude where that is more; hi hi + hi lo + lo hi drops at most 2^-22 of a product.  Every product is exact in the fp32
+// accumulator; a tile's P.V leaves tensor memory after 64 positions and is added in registers, so that no sum runs through
+// more than 64 (scores: D) additions on the tensor core.  Error of the output against 64 bits (2-norm, all rows, 12 heads of
+// 128), this kernel / fp32 on the CUDA cores: normal q, k, v at 97, 512, 1900, 6000 tokens 2.4, 3.1, 3.3, 3.4e-7 / 2.5, 3.5,
+// 4.4, 6.1e-7; eight times larger scores 4.6, 6.0, 7.5, 8.7e-7 / 8.1, 11.9, 15.6, 18.4e-7; values of one sign, which the
+// truncated sums shrink, 1.6, 1.9, 2.1, 2.3e-7 / 1.2, 2.4, 4.6, 8.1e-7.
+//
+// One power of two for a tile ties its positions together, those included that a row must not see.  So a tile whose rows of K
+// or V differ by more than 2^14 in magnitude, or that holds infinities or NaN, is marked unfit, and the CTAs that reach it
+// take the fp32 arithmetic of decoder_attn_rows.cuh (512 tokens, 12 heads of 128: 500 us a layer instead of 26; the fp32
+// kernel, whose grid is finer, 85).  Below that, what a position loses to its neighbours' size is at most 2^-24 of its own
+// largest element, which is what fp32 itself keeps.
 //
 // prefill_kv_split_kernel rotates the keys, appends keys and values to the cache and leaves both as ready operands
 // (canonical K-major core matrices; V transposed), 64 positions per tile.  attention_prefill_tc_kernel: a CTA owns the
@@ -20,6 +29,7 @@
 // the tensor pipe).  Tiles are dispatched longest causal range first.
 #include <cuda_fp16.h>
 
+#include "decoder_attn_rows.cuh"
 #include "decoder_state.h"
 #include "device_common.cuh"
 #include "tcgen05_common.cuh"
@@ -60,8 +70,19 @@ __device__ __forceinline__ void pa_split(float a, float b, uint32_t& hi, uint32_
   lo = *reinterpret_cast<const uint32_t*>(&l);
 }
 
+__device__ __forceinline__ uint32_t pa_magnitude(float x) { return __float_as_uint(x) & 0x7FFFFFFFu; }  // orders like |x|, infinities and NaN on top
+template <int LANES>
+__device__ __forceinline__ uint32_t pa_row_max(uint32_t m, int lane) {  // over the LANES lanes that share a row
+  return __reduce_max_sync(LANES == 32 ? 0xffffffffu : ((1u << (LANES & 31)) - 1u) << (lane & ~(LANES - 1)), m);
+}
+// A tile's keys or values that one power of two does not serve: rows whose largest magnitudes (bits; of the smallest non-zero
+// one, less 1) are more than a factor of 2^14 apart, infinities, NaN, nothing but numbers below 2^-113.
+__device__ __forceinline__ bool pa_unfit(uint32_t largest, uint32_t smallest_less_1) {
+  return largest != 0 && (largest >= 0x7F800000u || largest < (14u << 23) || (smallest_less_1 >> 23) + 14 < largest >> 23);
+}
+
 // grid (tiles, kv heads): rotates 64 new keys, appends keys and values at positions 64 tile .. to the cache
-// [kv_heads][max_ctx][D] and writes the tile's operands and {2^-E of K, 2^-E of V}.
+// [kv_heads][max_ctx][D] and writes the tile's operands and {2^-E of K, 2^-E of V} (zeros: the tile is unfit).
 template <int D>
 __global__ void __launch_bounds__(kPsThreads) prefill_kv_split_kernel(
     const float* __restrict__ k_new, const float* __restrict__ v_new, int ld, int n, const float* __restrict__ sin_t,
@@ -74,7 +95,7 @@ __global__ void __launch_bounds__(kPsThreads) prefill_kv_split_kernel(
   extern __shared__ __align__(16) float ps_smem[];
   float(*s_k)[D + 1] = reinterpret_cast<float(*)[D + 1]>(ps_smem);
   float(*s_v)[D + 1] = s_k + kPaKeys;
-  __shared__ float s_mx[2][kPsThreads / 32];
+  __shared__ uint4 s_mx[kPsThreads / 32];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int tile = blockIdx.x, h = blockIdx.y, p0 = tile * kPaKeys;
   float4 x0[KI], x1[KI], sn[KI], cs[KI], vv[VI];
@@ -95,50 +116,56 @@ __global__ void __launch_bounds__(kPsThreads) prefill_kv_split_kernel(
     const int idx = tid + u * kPsThreads, j = idx / (D / 4), d = idx % (D / 4) * 4;
     vv[u] = p0 + j < n ? *reinterpret_cast<const float4*>(v_new + (size_t)(p0 + j) * ld + h * D + d) : make_float4(0.f, 0.f, 0.f, 0.f);
   }
-  float mk = 0.0f, mv = 0.0f;
+  uint32_t mk = 0, nk = ~0u, mv = 0, nv = ~0u;  // bits of the largest and the smallest of the rows' largest magnitudes (rows of zeros aside)
 #pragma unroll
   for (int u = 0; u < KI; ++u) {
     const int idx = tid + u * kPsThreads, j = idx / (HALF / 4), d = idx % (HALF / 4) * 4;
     const float a[4] = {x0[u].x, x0[u].y, x0[u].z, x0[u].w}, b[4] = {x1[u].x, x1[u].y, x1[u].z, x1[u].w};
     const float s[4] = {sn[u].x, sn[u].y, sn[u].z, sn[u].w}, c[4] = {cs[u].x, cs[u].y, cs[u].z, cs[u].w};
     float y0[4], y1[4];
+    uint32_t m = 0;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       y0[i] = a[i] * c[i] - b[i] * s[i];
       y1[i] = a[i] * s[i] + b[i] * c[i];
       s_k[j][d + i] = y0[i];
       s_k[j][d + HALF + i] = y1[i];
-      mk = fmaxf(mk, fmaxf(fabsf(y0[i]), fabsf(y1[i])));
+      m = max(m, max(pa_magnitude(y0[i]), pa_magnitude(y1[i])));
     }
     if (p0 + j < n) {
       float* dst = cache_k + ((size_t)h * max_ctx + p0 + j) * D + d;
       *reinterpret_cast<float4*>(dst) = make_float4(y0[0], y0[1], y0[2], y0[3]);
       *reinterpret_cast<float4*>(dst + HALF) = make_float4(y1[0], y1[1], y1[2], y1[3]);
     }
+    m = pa_row_max<HALF / 4>(m, lane);
+    mk = max(mk, m), nk = min(nk, m - 1);
   }
 #pragma unroll
   for (int u = 0; u < VI; ++u) {
     const int idx = tid + u * kPsThreads, j = idx / (D / 4), d = idx % (D / 4) * 4;
     const float a[4] = {vv[u].x, vv[u].y, vv[u].z, vv[u].w};
+    uint32_t m = 0;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       s_v[j][d + i] = a[i];
-      mv = fmaxf(mv, fabsf(a[i]));
+      m = max(m, pa_magnitude(a[i]));
     }
     if (p0 + j < n) *reinterpret_cast<float4*>(cache_v + ((size_t)h * max_ctx + p0 + j) * D + d) = vv[u];
+    m = pa_row_max<D / 4>(m, lane);
+    mv = max(mv, m), nv = min(nv, m - 1);
   }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    mk = fmaxf(mk, __shfl_xor_sync(0xffffffffu, mk, o));
-    mv = fmaxf(mv, __shfl_xor_sync(0xffffffffu, mv, o));
-  }
-  if (lane == 0) s_mx[0][warp] = mk, s_mx[1][warp] = mv;
+  mk = __reduce_max_sync(0xffffffffu, mk), nk = __reduce_min_sync(0xffffffffu, nk);
+  mv = __reduce_max_sync(0xffffffffu, mv), nv = __reduce_min_sync(0xffffffffu, nv);
+  if (lane == 0) s_mx[warp] = make_uint4(mk, nk, mv, nv);
   __syncthreads();
 #pragma unroll
-  for (int w = 0; w < kPsThreads / 32; ++w) mk = fmaxf(mk, s_mx[0][w]), mv = fmaxf(mv, s_mx[1][w]);
-  const int ek = pa_exponent(mk), ev = pa_exponent(mv);
+  for (int w = 0; w < kPsThreads / 32; ++w) {
+    const uint4 o = s_mx[w];
+    mk = max(mk, o.x), nk = min(nk, o.y), mv = max(mv, o.z), nv = min(nv, o.w);
+  }
+  const int ek = pa_exponent(__uint_as_float(mk)), ev = pa_exponent(__uint_as_float(mv));
   const size_t at = (size_t)h * gridDim.x + tile;
-  if (tid == 0) tile_scales[at] = make_float2(pa_pow2(-ek), pa_pow2(-ev));
+  if (tid == 0) tile_scales[at] = pa_unfit(mk, nk) || pa_unfit(mv, nv) ? make_float2(0.0f, 0.0f) : make_float2(pa_pow2(-ek), pa_pow2(-ev));
   uint8_t* out = tiles + at * L::kTileBytes;
   const float fk = pa_pow2(ek), fv = pa_pow2(ev);
   // 16 bytes per item: 8 dimensions of one key; 8 keys of one dimension
@@ -161,11 +188,25 @@ __global__ void __launch_bounds__(kPsThreads) prefill_kv_split_kernel(
   }
 }
 
+// The rows [s0, end) on the CUDA cores, by 256 threads.
+template <int D>
+__device__ __forceinline__ void prefill_rows_fp32(PrefillAttnSmem<D>& sm, int tid, const float* q, int ldq, int s0, int end, int kvh,
+                                               const float* sin_t, const float* cos_t, int max_ctx, int group, const float* cache_k,
+                                               const float* cache_v, float* out, int ldo) {
+  static_assert(kPfRowThreads<2> == 256 && sizeof(PrefillAttnSmem<D>) <= (size_t)PaLayout<D>::kStages * PaLayout<D>::kTileBytes, "fits the rings");
+  for (int next; s0 < end; s0 = next) {
+    next = min(end, (s0 / kPfRows + 1) * kPfRows);  // the tiles of attention_prefill_kernel: an infinity reaches no other rows than there
+    prefill_attn_rows<D, 2>(sm, tid, [] { asm volatile("bar.sync 5, 256;" ::: "memory"); }, q, ldq, s0, next, kvh, sin_t, cos_t, 0, max_ctx,
+                            group, cache_k, cache_v, out, ldo);
+  }
+}
+
 // q: rows of ldq floats (token s at position s); out: rows of ldo floats.  grid: (row tiles x kv heads), 1-D.
 template <int D>
 __global__ void __launch_bounds__(kPaThreads, 1) attention_prefill_tc_kernel(
     const float* __restrict__ q, int ldq, int n, const float* __restrict__ sin_t, const float* __restrict__ cos_t, int group,
-    int kv_heads, const uint8_t* __restrict__ tiles, const float2* __restrict__ tile_scales, float* __restrict__ out, int ldo) {
+    int kv_heads, const uint8_t* __restrict__ tiles, const float2* __restrict__ tile_scales, int max_ctx,
+    const float* __restrict__ cache_k, const float* __restrict__ cache_v, float* __restrict__ out, int ldo) {
   using L = PaLayout<D>;
   constexpr int HALF = D / 2, QD = HALF / 2, kStages = L::kStages;  // QD: rotated pairs per thread
   pdl_launch_dependents();
@@ -207,17 +248,25 @@ __global__ void __launch_bounds__(kPaThreads, 1) attention_prefill_tc_kernel(
     mbar_init(q_ready, 8);
     mbar_fence_init();
   }
-  for (int i = tid; i < nt; i += kPaThreads) s_scales[i] = scales[i];
+  bool unfit = false;
+  for (int i = tid; i < nt; i += kPaThreads) {
+    s_scales[i] = scales[i];
+    unfit = unfit || s_scales[i].x == 0.0f;
+  }
   if (warp == 9) {
     tmem_alloc(tmem_slot, 512);
     tmem_relinquish();
   }
   tc_fence_before();
-  __syncthreads();
+  unfit = __syncthreads_or(unfit) != 0;
   tc_fence_after();
   const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);
 
-  if (warp == 8) {
+  if (unfit) {
+    if (warp < 8)
+      prefill_rows_fp32<D>(*reinterpret_cast<PrefillAttnSmem<D>*>(ring), tid, q, ldq, s0, last + 1, kvh, sin_t, cos_t, max_ctx, group, cache_k,
+                           cache_v, out, ldo);
+  } else if (warp == 8) {
     // ------------------------------------------------------------ producer
     if (lane == 0) {
       constexpr uint32_t kBytes = 2 * L::kOpBytes;
@@ -436,7 +485,7 @@ cudaError_t launch(const float* q, const float* k, const float* v, int n, int q_
                                    sin_t, cos_t, max_ctx, cache_k, cache_v, ops, scales);
   if (e != cudaSuccess) return e;
   return launch_pdl(attention_prefill_tc_kernel<D>, dim3((n + tokens - 1) / tokens * kv_heads), dim3(kPaThreads), PaLayout<D>::kTotal, s, q,
-                    q_heads * D, n, sin_t, cos_t, group, kv_heads, ops, scales, out, q_heads * D);
+                    q_heads * D, n, sin_t, cos_t, group, kv_heads, ops, scales, max_ctx, cache_k, cache_v, out, q_heads * D);
 }
 }  // namespace
 
