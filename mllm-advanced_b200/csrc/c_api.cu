@@ -144,7 +144,7 @@ int mllmb200_w4a32_repack_device(const void* blob_dev, int N, int K, int scale_m
       row_count, (int)th.num_groups, (int)th.num_panels, (uint32_t)scale_mode,
       reinterpret_cast<float*>(tiled + th.zsum_off), reinterpret_cast<float*>(tiled + th.bias_off),
       reinterpret_cast<unsigned int*>(tiled + offsetof(TiledHeader, max_scale_bits)),
-      reinterpret_cast<unsigned int*>(tiled + offsetof(TiledHeader, min_row_scale_not)));
+      reinterpret_cast<unsigned int*>(tiled + offsetof(TiledHeader, low_bit)));
   if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(e);
   return MLLMB200_OK;
 }

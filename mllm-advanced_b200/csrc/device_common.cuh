@@ -146,6 +146,15 @@ __device__ __forceinline__ float decode_scale(uint32_t raw16, uint32_t scale_mod
   return scale_mode == 2u ? as_f16 : as_bf16;
 }
 
+// TiledHeader::low_bit of one scale
+__device__ __forceinline__ uint32_t scale_low_bit(float s) {
+  const uint32_t b = __float_as_uint(s) & 0x7FFFFFFFu;
+  if (b == 0) return 0;
+  if (b >= 0x7F800000u) return kScaleNoNumber;
+  const int e = max((int)(b >> 23), 1) - 150;  // exponent of the last place
+  return (uint32_t)(512 - e - (b & 0x7FFFFFu ? __ffs(b) - 1 : 23));
+}
+
 // ------------------------------------------------------------------ activation quantization
 // Per-row parameters of the dynamic asymmetric int8 quantization
 // (reference project: tests/Arm/KaiLinearTest.hpp:163-205).  Every operation is a separately

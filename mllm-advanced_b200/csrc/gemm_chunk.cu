@@ -4,10 +4,12 @@
 //   A[n, k] = fp16( (u[n,k] - 8) * s[n, group(k)] * 2^E[n] )      B[m, k] = fp16( a_q[m, k] + a_off[m] )
 //   y[m, n] = lhs_scale[m] * 2^-E[n] * sum_k A[n,k] B[m,k] + bias[n]
 //
-// (reference project tests/Arm/KaiLinearTest.hpp:338-377, production call kai_linear.cpp:350-398).  Both operands hold
-// their values exactly: |a_q + a_off| <= 255, and (u - 8) * s has at most 3 + 8 significant bits for a bf16-encoded
-// scale.  E is the matrix' exponent (its largest |scale| comes to [2^10, 2^11)); where the rows' largest scales differ by
-// more than 2^12, which the repack notes, E[n] is the row's own, so that a row of tiny scales keeps its accuracy.
+// (reference project tests/Arm/KaiLinearTest.hpp:338-377, production call kai_linear.cpp:350-398).  B is exact: |a_q + a_off| <=
+// 255.  A is exact too: (u - 8) * s has at most 3 + 8 significant bits for a bf16-encoded scale, and E brings the matrix'
+// largest |scale| to [2^10, 2^11) as long as no bit of any scale then falls below fp16's last place, 2^-24, which the repack
+// notes (bf16-encoded scales: largest and smallest up to 2^27 apart).  Where one does, E[n] is the row's own; rows with more
+// than that between their own scales, or with an infinity or NaN among them, are summed on the CUDA cores instead
+// (ck_row_sum; the tensor core's sums of such a row are not used).
 // An fp16-encoded scale needs 14 bits: those matrices go through every K-tile twice, once with the rounded product and
 // once with its (exact) remainder.  All products are exact in fp32; what rounds is the addition.
 //
@@ -140,21 +142,51 @@ __device__ __forceinline__ void ck_mma(uint32_t d, uint32_t a, uint64_t b_desc, 
   else
     tc_mma_f16_ts(d, a, b_desc, idesc, accumulate);
 }
-// 2^E for row `lane` of a panel
+// 2^E that brings a largest |scale| (its bits) to [2^10, 2^11); 2^E and 2^-E stay normal
+__device__ __forceinline__ int ck_exponent(uint32_t top) { return min(10 - ((int)(top >> 23) - 127), 126); }
+// the bits of all scales times 2^E lie at 2^-24 or above: fp16 holds them and their products with u - 8
+__device__ __forceinline__ bool ck_fits(uint32_t low_bit, int e) { return low_bit <= (uint32_t)(512 + 24 + e); }
+// 2^E for row `lane` of a panel: the matrix' exponent, or (rare) the row's own where that one does not fit all scales.  0: nor does the row's
 __device__ __forceinline__ float ck_up(const uint8_t* tiled, int panel, int lane, int num_groups, uint32_t scale_mode) {
   const TiledHeader* h = reinterpret_cast<const TiledHeader*>(tiled);
-  uint32_t top = h->max_scale_bits;
-  const uint32_t low = ~h->min_row_scale_not;
-  if (low != ~0u && (low >> 23) + 12 < top >> 23) {  // rare: the row's own largest finite |scale|
+  int e = ck_exponent(h->max_scale_bits);
+  if (!ck_fits(h->low_bit, e)) {
     const uint8_t* cell = tiled + sizeof(TiledHeader) + (size_t)panel * num_groups * kCellBytes + kCellNibbleBytes + lane * 2;
+    uint32_t low = 0;
     float mx = 0.0f;
     for (int g = 0; g < num_groups; ++g, cell += kCellBytes) {
       const float s = fabsf(decode_scale(*reinterpret_cast<const uint16_t*>(cell), scale_mode));
       if (s <= 3.402823466e+38f) mx = fmaxf(mx, s);
+      low = max(low, scale_low_bit(s));
     }
-    top = __float_as_uint(mx);
+    e = ck_exponent(__float_as_uint(mx));
+    if (!ck_fits(low, e)) return 0.0f;
   }
-  return __uint_as_float((uint32_t)(min(10 - ((int)(top >> 23) - 127), 126) + 127) << 23);  // (126: 2^E and 2^-E stay normal)
+  return __uint_as_float((uint32_t)(e + 127) << 23);
+}
+// One sum as the reference forms it, for rows whose scales fit no common exponent (or hold infinities): the K-groups' integer
+// sums, exact in fp32, times their scales.  cell: the row's 16 bytes in its panel's first cell; scale: its scale there;
+// x: the row's 16 bytes in the first activation block.
+__device__ __forceinline__ float ck_row_sum(const uint8_t* cell, const uint8_t* scale, const uint8_t* x, size_t x_stride, int num_groups,
+                                            uint32_t scale_mode) {
+  float acc = 0.0f;
+#pragma unroll 1
+  for (int g = 0; g < num_groups; ++g, cell += kCellBytes, scale += kCellBytes, x += x_stride) {
+    float sum = 0.0f;
+#pragma unroll 1
+    for (int c = 0; c < 4; ++c) {
+      const uint32_t w = *reinterpret_cast<const uint32_t*>(cell + c * 4);
+      const __half2* h = reinterpret_cast<const __half2*>(x + c * 128);  // k = 8c + {0,4}, {1,5}, {2,6}, {3,7}
+#pragma unroll
+      for (int t = 0; t < 4; ++t) {
+        const float2 v = __half22float2(h[t]);
+        sum = fmaf((float)((int)(w >> (4 * t) & 15u) - 8), v.x, sum);
+        sum = fmaf((float)((int)(w >> (4 * t + 16) & 15u) - 8), v.y, sum);
+      }
+    }
+    acc = fmaf(sum, decode_scale(*reinterpret_cast<const uint16_t*>(scale), scale_mode), acc);
+  }
+  return acc;
 }
 __device__ __forceinline__ float ck_clamp(float v) {  // clamp_flt_max: only infinities lie outside
   return fabsf(v) > 3.402823466e+38f ? copysignf(3.402823466e+38f, v) : v;
@@ -426,7 +458,17 @@ __global__ void __launch_bounds__(kCkThreads, 1) w4a32_gemm_chunk_kernel(const _
     if (tid < m_here) s_scale[tid] = x_scale;
     asm volatile("bar.sync 1, %0;" ::"n"(kCkDqWarps * 32) : "memory");
     const float down = __uint_as_float((254u << 23) - __float_as_uint(up));  // 1 / up
-    if (ok && live) {
+    if (ok && live && up == 0.0f) {
+      const uint8_t* cell = pr.tiled + sizeof(TiledHeader) + (size_t)(panel0 + rset) * p.num_groups * kCellBytes;
+#pragma unroll 1
+      for (int i = 0; i < kCols; ++i) {
+        const int col = first_col(i / kSlotWarpCols) + i % kSlotWarpCols, m = m0 + col;
+        if (col >= m_here) continue;
+        const float sum = ck_row_sum(cell + lane * 16, cell + kCellNibbleBytes + lane * 2, p.a_blocks + (size_t)(m >> 3) * 512 + (m & 7) * 16,
+                                     (size_t)p.m8 * 512, p.num_groups, scale_mode);
+        pr.y[(size_t)m * pr.ldy + n] = ck_clamp(fmaf(sum, s_scale[col], bs));
+      }
+    } else if (ok && live) {
 #pragma unroll
       for (int j = 0; j < kCols / kSlotWarpCols; ++j) {
         const int col0 = first_col(j);

@@ -57,10 +57,11 @@ struct TiledHeader {
   uint32_t magic, version, n, k, num_groups, num_panels, scale_mode, has_bias;
   uint64_t cells_off, zsum_off, bias_off, total_bytes;
   uint32_t max_scale_bits;  // fp32 bits of the largest |group scale| of the matrix (written by the repack kernel)
-  uint32_t min_row_scale_not;  // ~ the fp32 bits of the smallest of the rows' largest |scales| (rows of zeros aside; 0: none)
+  uint32_t low_bit;         // 512 - exponent of the lowest bit set in any scale (0: zeros only); kScaleNoNumber: an infinity or NaN among them
   uint8_t pad[256 - 32 - 32 - 8];
 };
 static_assert(sizeof(TiledHeader) == 256, "tiled header is 256 bytes");
+constexpr uint32_t kScaleNoNumber = 0x7FFFFFFFu;
 
 inline TiledHeader make_tiled_header(int n, int k, int scale_mode, int has_bias) {
   TiledHeader h{};

@@ -138,3 +138,39 @@ def test_kernel_3_keeps_int32_group_sums_at_any_m(m, k, n):
     y = mb.linear_forward(torch.from_numpy(x).cuda(), mb.W4A32Weights.from_blob(blob), kernel=mb.KERNEL_TC)
     mb.check_device_status()
     assert np.array_equal(y.cpu().numpy(), want)
+
+
+@pytest.mark.parametrize("mode", [mb.SCALE_BF16_TRUNC, mb.SCALE_FP16])
+@pytest.mark.parametrize("m,k,n", [(70, 200, 150), (300, 256, 12810)])
+def test_scales_far_apart_and_no_numbers(m, k, n, mode):
+    """Group scales that no common power of two brings into fp16 together, in other rows and within a row, and scales that are
+    infinite or NaN: the reference's arithmetic, as if every row were by itself.  Activations that are zero except in the
+    groups of tiny scales show those rows' small sums by themselves."""
+    orc, rng = Oracle(), np.random.default_rng(m + k)
+    groups = (k + 31) // 32
+    nib = (rng.integers(1, 16, (n, (k + 1) // 2)) | rng.integers(1, 16, (n, (k + 1) // 2)) << 4).astype(np.uint8)
+    s = (rng.random((n, groups)) + 0.5) * 2.0 ** (-18 if mode == mb.SCALE_FP16 else -40)
+    far = [1, 40, 70, n - 1]
+    s[far, 0] = 50000 if mode == mb.SCALE_FP16 else 2.0 ** 20  # more than 2^27 above the row's other scales
+    s[45], s[46] = 3000, 0                                     # rows of another size; a row of zeros
+    s[90, 2], s[91, 1], s[92, 3] = np.inf, -np.inf, np.nan
+    s16 = s.astype(np.float16).view(np.uint16) if mode == mb.SCALE_FP16 else (s.astype(np.float32).view(np.uint32) >> 16).astype(np.uint16)
+    x = rng.standard_normal((m, k)).astype(np.float32)
+    x[m // 2:, :32] = 0
+    x[m // 2:, 32:] = np.abs(x[m // 2:, 32:])
+    blob = mb.prepack_from_quantized(nib, s16, n, k, None, mode)
+    y = mb.linear_forward(torch.from_numpy(x).cuda(), mb.W4A32Weights.from_blob(blob)).cpu().numpy()
+    mb.check_device_status()
+    want = orc.linear(x, nib, s16, None, mode)
+    assert np.array_equal(np.isnan(y), np.isnan(want)) and np.isnan(want[:, 92]).all() and np.abs(want[:, 90]).max() == np.finfo(np.float32).max
+    numbers = [r for r in range(n) if r not in (90, 91, 92)]
+    assert np.array_equal(np.abs(y[:, 90:92]), np.abs(want[:, 90:92]), equal_nan=True)
+    assert np.array_equal(np.sign(y[:, 90:92]), np.sign(want[:, 90:92]), equal_nan=True)
+    # The bar of test_tiles_chunks_and_forms for every row's two halves, against 64 bits
+    s64 = s16.view(np.float16).astype(np.float64) if mode == mb.SCALE_FP16 else (s16.astype(np.uint32) << 16).view(np.float32).astype(np.float64)
+    u = np.stack([nib & 15, nib >> 4], axis=-1).reshape(n, -1)[:, :k].astype(np.float64) - 8
+    exact = _acts64(orc, x) @ (u[numbers] * np.repeat(s64.reshape(n, -1)[numbers], 32, axis=1)[:, :k]).T
+    bar = (48 / 3 + (k + 127) // 128 / 2 + 2) * 2.0 ** -23
+    for half in (slice(0, m // 2), slice(m // 2, m)):
+        d = np.linalg.norm(y[half][:, numbers] - exact[half], axis=0)
+        assert (d <= bar * np.linalg.norm(exact[half], axis=0)).all()
