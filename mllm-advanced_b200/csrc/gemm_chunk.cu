@@ -10,8 +10,8 @@
 // notes (bf16-encoded scales: largest and smallest up to 2^27 apart).  Where one does, E[n] is the row's own; rows with more
 // than that between their own scales, or with an infinity or NaN among them, are summed on the CUDA cores instead
 // (ck_row_sum; the tensor core's sums of such a row are not used).
-// An fp16-encoded scale needs 14 bits: those matrices go through every K-tile twice, once with the rounded product and
-// once with its (exact) remainder.  All products are exact in fp32; what rounds is the addition.
+// An fp16-encoded scale needs 14 bits: those matrices go through every K-tile twice, once with the scale's first 8 bits and
+// once with the rest.  All products are exact in fp32; what rounds is the addition.
 //
 // The tensor core truncates where it adds, which shrinks a sum of 1024 values by about 5e-8 and one of 8960 by 4e-7:
 // more than fp32 additions of rounded group sums are off.  So a sum stays in tensor memory for one CHUNK of K only and is
@@ -26,12 +26,16 @@
 //   warp 17    MMA issuer (one elected lane; of CTA 0 for a pair) and tensor-memory owner
 // A pair multiplies four stages (256 values of K) for the first half of its columns, then for the second: while one half's
 // finished chunk is fetched the other half's products run, and the next four stages are dequantized.
-// Bound: instruction issue of the dequantization (16 warps x ~150 instructions per two K-groups) next to the tensor pipe.
-// Measured (B200, quantization of x included), the int8 tile GEMM (gemm_tc.cu) / this kernel: 8960 x 1536, M = 512 61 / 27 us;
-// 28672 x 8192, M = 512 765 / 313 us, M = 2048 2857 / 1020 us (943 TFLOP/s); 1536 x 8960 (single CTAs), M = 512 77 / 62 us;
+// Bound: the dequantization warps' chain (wait, load, ~150 instructions per two K-groups, store, arrive) and the hand-offs around
+// it, next to the tensor pipe: without its tensor-core instructions a launch on 1536 x 8960 takes 51 of 54 us at M = 65 and 57
+// of 63 at M = 512, without the operand's stores to tensor memory or without the sums' fetches as long as with them.
+// Measured (B200, quantization of x included), the int8 tile GEMM (gemm_tc.cu) / this kernel: 8960 x 1536, M = 512 63 / 28 us;
+// 28672 x 8192, M = 512 762 / 308 us, M = 2048 2848 / 995 us (967 TFLOP/s); 1536 x 8960 (single CTAs), M = 512 78 / 62 us;
 // error against 64 bits (2-norm) 6.0e-8 / 5.3e-8 at K = 1536, 1.29e-7 / 9.4e-8 at K = 8192.  M = 65, 17920 x 1536
-// 36 / 24 us; the three matrices of q, k, v, M = 65 (one launch instead of three) 47 / 14 us.  At M <= 64 the streaming
+// 33 / 24 us; the three matrices of q, k, v, M = 65 (one launch instead of three) 47 / 14 us.  At M <= 64 the streaming
 // kernel (gemm_stream.cu) mostly stays ahead: it needs no 128-row tiles (1536 x 1536, M = 48: 8 us, here 14).
+// fp16-encoded scales, us: 1536 x 1536, M = 65 19.4, 1536 x 8960, M = 512 87, 8960 x 1536, M = 512 38 (27, 110 and 47 with
+// finished chunks fetched in front of every turn and a wait of the MMA issuer for either part).
 #include <cuda_fp16.h>
 
 #include "device_common.cuh"
@@ -106,7 +110,8 @@ __device__ __noinline__ bool ck_wait_slow(uint32_t bar, uint32_t parity) {
 }
 __device__ __forceinline__ bool ck_wait(uint32_t bar, uint32_t parity) {
   bool ok = ck_try_wait(bar, parity);
-  if (!ok) ok = ck_wait_slow(bar, parity);
+  if (__all_sync(0xffffffffu, ok)) return true;
+  ok = ok || ck_wait_slow(bar, parity);
   return __all_sync(0xffffffffu, ok);
 }
 // arrival on this CTA's barrier, or (a pair) on the one of CTA 0 that has its place there
@@ -188,6 +193,11 @@ __device__ __forceinline__ float ck_row_sum(const uint8_t* cell, const uint8_t* 
   }
   return acc;
 }
+// (the single-CTA form is 3 % slower with it in line, the pair form 1 % with a call: registers of the loop in front of it)
+__device__ __noinline__ float ck_row_sum_call(const uint8_t* cell, const uint8_t* scale, const uint8_t* x, size_t x_stride, int num_groups,
+                                            uint32_t scale_mode) {
+  return ck_row_sum(cell, scale, x, x_stride, num_groups, scale_mode);
+}
 __device__ __forceinline__ float ck_clamp(float v) {  // clamp_flt_max: only infinities lie outside
   return fabsf(v) > 3.402823466e+38f ? copysignf(3.402823466e+38f, v) : v;
 }
@@ -225,9 +235,12 @@ __global__ void __launch_bounds__(kCkThreads, 1) w4a32_gemm_chunk_kernel(const _
   if (!tiled_header_ok_cta(pr.tiled, pr.n, p.k)) return;  // the same answer in both CTAs of a pair
   const int panel0 = ((bx - pr.tile_begin) * (kPair ? 2 : 1) + rank) * kCkPanels, n0 = panel0 * kPanelRows;
   const int k_tiles = (p.num_groups + kGroups - 1) / kGroups;
-  const int chunk_tiles = p.chunk_quads * (kCkQuad / kGroups);
   const uint32_t scale_mode = reinterpret_cast<const TiledHeader*>(pr.tiled)->scale_mode;
-  const int parts = scale_mode == 2u ? 2 : 1;  // fp16-encoded scales: every stage twice (rounded product, remainder)
+  const int parts = scale_mode == 2u ? 2 : 1;  // fp16-encoded scales: every stage twice
+  // With two parts a turn of the dequant warps waits for MMAs of the span before, and those of a pair for the fetch of the
+  // chunk before theirs, which comes behind the turn: no chunk ends inside a span.
+  const int chunk_tiles = max(p.chunk_quads, parts) * (kCkQuad / kGroups);
+  static_assert(2 * kCkQuad / kGroups % kSpan == 0 && 4 * kCkQuad / kGroups % kSpan == 0 && 6 * kCkQuad / kGroups % kSpan == 0, "chunks of whole spans");
   const int m_here = min(NT, p.m - m0);
 
   if (tid == 0) {
@@ -296,8 +309,9 @@ __global__ void __launch_bounds__(kCkThreads, 1) w4a32_gemm_chunk_kernel(const _
       uint32_t accumulate = 0;
       for (int it = 0; it < k_tiles && ok;) {
         const int steps = min(kStep, left);
-        for (int v = it * parts; v < (it + steps) * parts && ok; ++v)
-          // arrived on by warps that saw raw_full complete: orders the stage's copies too
+        for (int v = it * parts + parts - 1; v < (it + steps) * parts && ok; v += parts)
+          // arrived on by warps that saw raw_full complete: orders the stage's copies too.  (Of two parts the last: the
+          // same warps wrote the first before it.)
           ok = ck_wait(a_full + (uint32_t)(v % kAStages) * 8, (uint32_t)(v / kAStages) & 1u);
         left -= steps;
 #pragma unroll
@@ -386,10 +400,7 @@ __global__ void __launch_bounds__(kCkThreads, 1) w4a32_gemm_chunk_kernel(const _
     const int own = kPair ? turn : turn >> 1, half = kPair ? 0 : turn & 1;  // stage of a span, pair of its K-groups
     const uint32_t raw_off = (uint32_t)((rset * kGroups + half * 2) * kCellBytes);
     for (int span = 0; span < k_tiles && ok; span += kSpan) {
-      // Chunks that ended before this span are fetched behind this span's turn: the MMA issuer has work meanwhile.  With
-      // two parts a span fills the operand ring, and the MMAs it waits for may wait for those chunks: fetched first.
-      if (parts == 2)
-        while (ok && drained_end <= span) drain();
+      // chunks that ended before this span are fetched behind this span's turn: the MMA issuer has work meanwhile
       const int it = span + own;
       if (it < k_tiles) {
         const uint32_t s = (uint32_t)it % kStages;
@@ -425,15 +436,17 @@ __global__ void __launch_bounds__(kCkThreads, 1) w4a32_gemm_chunk_kernel(const _
                   areg[c * 4 + t] = *reinterpret_cast<const uint32_t*>(&v);
                 }
             } else {
-              const __half2 s2 = __float2half2_rn(decode_scale(sc16, 2u) * up), off = __floats2half2_rn(1032.0f, 1032.0f);
+              // the scale's first 8 bits in the first part, the up to 3 that are left in the second: as above
+              const float s = decode_scale(sc16, 2u), top = __uint_as_float(__float_as_uint(s) & 0xFFFF0000u);
+              const float s_up = (part == 0 ? top : s - top) * up;
+              const __half2 s4 = __float2half2_rn(4.0f * s_up), c24 = __float2half2_rn(-24.0f * s_up);
 #pragma unroll
               for (int c = 0; c < 4; ++c)
 #pragma unroll
                 for (int t = 0; t < 4; ++t) {
-                  const uint32_t bits = ((ws[c] >> (4 * t)) & 0x000F000Fu) | 0x64006400u;  // 1024 + u
-                  const __half2 u8 = __hsub2(*reinterpret_cast<const __half2*>(&bits), off);
-                  const __half2 hi = __hmul2(u8, s2);
-                  const __half2 v = part == 0 ? hi : __hfma2(u8, s2, __hneg2(hi));
+                  const uint32_t moved = t == 0 ? ws[c] << 6 : t == 1 ? ws[c] << 2 : t == 2 ? ws[c] >> 2 : ws[c] >> 6;
+                  const uint32_t bits = (moved & 0x03C003C0u) | 0x44004400u;
+                  const __half2 v = __hfma2(*reinterpret_cast<const __half2*>(&bits), s4, c24);
                   areg[c * 4 + t] = *reinterpret_cast<const uint32_t*>(&v);
                 }
             }
@@ -464,7 +477,7 @@ __global__ void __launch_bounds__(kCkThreads, 1) w4a32_gemm_chunk_kernel(const _
       for (int i = 0; i < kCols; ++i) {
         const int col = first_col(i / kSlotWarpCols) + i % kSlotWarpCols, m = m0 + col;
         if (col >= m_here) continue;
-        const float sum = ck_row_sum(cell + lane * 16, cell + kCellNibbleBytes + lane * 2, p.a_blocks + (size_t)(m >> 3) * 512 + (m & 7) * 16,
+        const float sum = (kPair ? ck_row_sum : ck_row_sum_call)(cell + lane * 16, cell + kCellNibbleBytes + lane * 2, p.a_blocks + (size_t)(m >> 3) * 512 + (m & 7) * 16,
                                      (size_t)p.m8 * 512, p.num_groups, scale_mode);
         pr.y[(size_t)m * pr.ldy + n] = ck_clamp(fmaf(sum, s_scale[col], bs));
       }
