@@ -251,16 +251,17 @@ __global__ void __launch_bounds__(256) act_quant_reflayout_kernel(const float* _
 // 8 rows x 16 bytes holding k = 8c + {0,4,1,5,2,6,3,7} - the order in which the weight side's
 // nibble unpack (two nibbles 16 bits apart per half2) produces its elements.
 // Bound: at small M a chain of latencies (row in, min/max across the CTA, blocks out), at large M the memory.  A thread
-// keeps its items of the row (8 values of K each) in registers between the two halves of the work, up to K = 10240; the
-// rest of a longer row is read again.  Two rows per CTA: their 16-byte pieces fill a 32-byte sector.  Measured (B200)
-// with four rows per CTA and every row read twice / as it is: M = 64, K = 1536 3.6 / 2.7 us, K = 8960 8.2 / 4.7 us.
-constexpr int kF16RowsPerCta = 2;
-constexpr int kF16WarpsPerRow = 8;
-constexpr int kF16Items = 5;
-__global__ void __launch_bounds__(kF16RowsPerCta * kF16WarpsPerRow * 32) act_quant_blocks_f16_kernel(
+// keeps its items of the row (8 values of K each) in registers between the two halves of the work; the rest of a longer row
+// is read again.  Rows of a CTA fill 16-byte pieces of the same lines.  Two forms: two rows by 8 warps each, ITEMS = 5, as
+// long as that is one wave of CTAs (one per SM); above, four rows by 4 warps each, ITEMS = 4, which leaves more CTAs per SM.
+// Measured (B200), us, four rows by 8 warps with every row read twice / two rows / four rows: M = 256, K = 1536 5.3 / 4.2 / 4.2,
+// K = 8960 10.3 / 6.3 / 10.3; M = 512, K = 1536 5.2 / 6.2 / 4.2, K = 8960 10.4 / 10.4 / 10.4; M = 2048, K = 96 8.3 / 12.4 / 6.2,
+// K = 1536 12.4 / 14.4 / 8.3, K = 8960 36.9 / 32.9 / 29.0.
+template <int ROWS, int WARPS, int ITEMS>
+__global__ void __launch_bounds__(ROWS * WARPS * 32) act_quant_blocks_f16_kernel(
     const float* __restrict__ x, int m_total, int k, int ldx, int num_groups, int m8_pad, uint8_t* __restrict__ blocks,
     float2* __restrict__ hdr, int use_pdl, int* __restrict__ clear_ints, int clear_count) {
-  __shared__ float s_mm[kF16RowsPerCta][kF16WarpsPerRow][2];
+  __shared__ float s_mm[ROWS][WARPS][2];
   if (use_pdl) {
     // x may be the previous kernel's output, and that kernel may still be reading the blocks this one overwrites:
     // nothing happens before it has finished; the kernel behind this one may set itself up meanwhile
@@ -271,12 +272,12 @@ __global__ void __launch_bounds__(kF16RowsPerCta * kF16WarpsPerRow * 32) act_qua
   if (blockIdx.x == 0)
     for (int i = threadIdx.x; i < clear_count; i += blockDim.x) clear_ints[i] = 0;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int r = warp % kF16RowsPerCta, part = warp / kF16RowsPerCta;
-  const int m = blockIdx.x * kF16RowsPerCta + r;
+  const int r = warp % ROWS, part = warp / ROWS;
+  const int m = blockIdx.x * ROWS + r;
   const bool live = m < m_total;
   const float* row = x + (size_t)(live ? m : 0) * ldx;
   const bool vec = ((reinterpret_cast<uintptr_t>(row) & 15u) == 0);
-  constexpr int kStride = kF16WarpsPerRow * 32;
+  constexpr int kStride = WARPS * 32;
   const int items = num_groups * 4, first = part * 32 + lane;  // item = 8 consecutive k = one 16-byte chunk of a block
   auto load = [&](int item, float (&f)[8]) {
     const int k0 = item * 8;
@@ -299,15 +300,15 @@ __global__ void __launch_bounds__(kF16RowsPerCta * kF16WarpsPerRow * 32) act_qua
         mx = fmaxf(mx, f[j]);
       }
   };
-  float v[kF16Items][8];
+  float v[ITEMS][8];
   if (live) {
 #pragma unroll
-    for (int i = 0; i < kF16Items; ++i)
+    for (int i = 0; i < ITEMS; ++i)
       if (first + i * kStride < items) load(first + i * kStride, v[i]);
 #pragma unroll
-    for (int i = 0; i < kF16Items; ++i)
+    for (int i = 0; i < ITEMS; ++i)
       if (first + i * kStride < items) extend(first + i * kStride, v[i]);
-    for (int item = first + kF16Items * kStride; item < items; item += kStride) {
+    for (int item = first + ITEMS * kStride; item < items; item += kStride) {
       float f[8];
       load(item, f);
       extend(item, f);
@@ -324,7 +325,7 @@ __global__ void __launch_bounds__(kF16RowsPerCta * kF16WarpsPerRow * 32) act_qua
   }
   __syncthreads();
 #pragma unroll
-  for (int q = 0; q < kF16WarpsPerRow; ++q) {
+  for (int q = 0; q < WARPS; ++q) {
     mn = fminf(mn, s_mm[r][q][0]);
     mx = fmaxf(mx, s_mm[r][q][1]);
   }
@@ -345,21 +346,21 @@ __global__ void __launch_bounds__(kF16RowsPerCta * kF16WarpsPerRow * 32) act_qua
     *reinterpret_cast<uint4*>(blk + (item & 3) * 128) = *reinterpret_cast<const uint4*>(h);
   };
 #pragma unroll
-  for (int i = 0; i < kF16Items; ++i)
+  for (int i = 0; i < ITEMS; ++i)
     if (first + i * kStride < items) store(first + i * kStride, v[i]);
-  for (int item = first + kF16Items * kStride; item < items; item += kStride) {
+  for (int item = first + ITEMS * kStride; item < items; item += kStride) {
     float f[8] = {};
     if (live) load(item, f);
     store(item, f);
   }
 }
 
-cudaError_t launch_act_quant_blocks_f16(const float* x, int m, int m_pad, int k, int ldx, uint8_t* blocks, float2* hdr,
-                                        cudaStream_t stream, int use_pdl, int* clear_ints, int clear_count) {
-  const int num_groups = (k + kGroup - 1) / kGroup;
+template <int ROWS, int WARPS, int ITEMS>
+static cudaError_t launch_blocks_f16_t(const float* x, int m, int m_pad, int k, int ldx, uint8_t* blocks, float2* hdr, cudaStream_t stream,
+                                       int use_pdl, int* clear_ints, int clear_count) {
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(m_pad / kF16RowsPerCta), 1, 1);
-  cfg.blockDim = dim3(kF16RowsPerCta * kF16WarpsPerRow * 32, 1, 1);
+  cfg.gridDim = dim3((unsigned)(m_pad / ROWS), 1, 1);
+  cfg.blockDim = dim3(ROWS * WARPS * 32, 1, 1);
   cfg.stream = stream;
   cudaLaunchAttribute attr;
   if (use_pdl) {
@@ -368,8 +369,14 @@ cudaError_t launch_act_quant_blocks_f16(const float* x, int m, int m_pad, int k,
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
   }
-  return cudaLaunchKernelEx(&cfg, act_quant_blocks_f16_kernel, x, m, k, ldx, num_groups, m_pad / 8, blocks, hdr, use_pdl,
-                            clear_ints, clear_ints != nullptr ? clear_count : 0);
+  return cudaLaunchKernelEx(&cfg, act_quant_blocks_f16_kernel<ROWS, WARPS, ITEMS>, x, m, k, ldx, (k + kGroup - 1) / kGroup, m_pad / 8, blocks,
+                            hdr, use_pdl, clear_ints, clear_ints != nullptr ? clear_count : 0);
+}
+// m_pad: a multiple of 8
+cudaError_t launch_act_quant_blocks_f16(const float* x, int m, int m_pad, int k, int ldx, uint8_t* blocks, float2* hdr,
+                                        cudaStream_t stream, int use_pdl, int* clear_ints, int clear_count) {
+  if (m_pad > 2 * 148) return launch_blocks_f16_t<4, 4, 4>(x, m, m_pad, k, ldx, blocks, hdr, stream, use_pdl, clear_ints, clear_count);
+  return launch_blocks_f16_t<2, 8, 5>(x, m, m_pad, k, ldx, blocks, hdr, stream, use_pdl, clear_ints, clear_count);
 }
 
 // m8_pad == 0: 48-byte records; m8_pad > 0: canonical 256-byte blocks with m8_pad blocks per K-group.

@@ -174,3 +174,21 @@ def test_scales_far_apart_and_no_numbers(m, k, n, mode):
     for half in (slice(0, m // 2), slice(m // 2, m)):
         d = np.linalg.norm(y[half][:, numbers] - exact[half], axis=0)
         assert (d <= bar * np.linalg.norm(exact[half], axis=0)).all()
+
+
+# The quantization in front of it: two rows per CTA up to 296 padded rows, four above; K within the registers of both forms
+# (4096, 10240 values), one more, and beyond; rows of x on 16-byte boundaries or not
+@pytest.mark.parametrize("m,k", [(296, 70), (297, 70), (295, 4096), (299, 4096), (299, 4097), (290, 10240), (290, 10244), (513, 8965)])
+@pytest.mark.parametrize("offset", [0, 1])
+def test_quantization_forms(m, k, offset):
+    orc, rng = Oracle(), np.random.default_rng(m + k)
+    buf = rng.standard_normal((m, k + 4 + offset)).astype(np.float32)
+    x = np.ascontiguousarray(buf[:, offset:offset + k])
+    x[3], x[m - 1] = 0, np.abs(x[m - 1])
+    buf[:, offset:offset + k] = x
+    blob = mb.quant_prepack((rng.standard_normal((33, k)) * 0.02).astype(np.float32))
+    y = mb.linear_forward(torch.from_numpy(buf).cuda()[:, offset:offset + k], mb.W4A32Weights.from_blob(blob)).cpu().numpy()
+    mb.check_device_status()
+    want = _acts64(orc, x) @ _weights64(blob, mb.SCALE_BF16_TRUNC)[0].T
+    bar = (48 / 3 + (k + 127) // 128 / 2 + 2) * 2.0 ** -23
+    assert (np.linalg.norm(y - want, axis=1) <= bar * np.linalg.norm(want, axis=1)).all()
