@@ -141,9 +141,11 @@ MLLMB200_API int mllmb200_w4a32_linear_forward(const float* x_dev, const void* t
  * 7 streaming tensor-core GEMM for small batches (M <= 64; what auto picks for 5 <= M <= 64): the weight cells are
  * spread over all SMs as in the GEMV, the per-group integer products run as mma.sync u8 x s8 (exact int32 group
  * sums, as the reference), clusters split K where the quantized activations of a whole row do not fit one CTA.
- * OR 0x100 into `kernel` to allow programmatic dependent launch (kernels 1, 4, 5, 6, 7): the kernel then
- * requests its (constant) weights while the previous kernel of the stream still runs and reads x only
- * after that kernel has completed. */
+ * OR 0x100 into `kernel` to allow programmatic dependent launch (kernels 1, 4, 5, 6, 7 and the default from 65 rows
+ * on): the kernel then requests its (constant) weights while the previous kernel of the stream still runs and reads x
+ * only after that kernel has completed.
+ * OR 0x200 into `kernel` where the matrix was packed with MLLMB200_SCALE_FP16: a hint, results are right with and
+ * without it.  From 65 rows on the default then runs kernel 3 where that is the faster one (few tiles). */
 MLLMB200_API int mllmb200_w4a32_linear_forward_ex(const float* x_dev, const void* tiled_dev, float* y_dev,
                                                   void* ws_dev, int M, int K, int N, int ldx, int ldy,
                                                   int kernel, void* stream);
@@ -153,8 +155,8 @@ MLLMB200_API int mllmb200_w4a32_linear_forward_ex(const float* x_dev, const void
  * [1,4], all with the same K.  For M <= 4 this is a single kernel launch that quantizes x once per
  * CTA and streams all the weight matrices; for larger M the matrices share one quantization of x
  * when they take the same tensor-core path, else it is `count` ordinary forwards.
- * flags: bit 8 = allow programmatic dependent launch; low byte = kernel policy: 0 auto, 5 fastest
- * (as linear_forward_ex's kernel argument), 6 the two-launch GEMV (M <= 4 only). */
+ * flags: bits 8 and 9 as linear_forward_ex's kernel argument; low byte = kernel policy: 0 auto, 5 fastest
+ * (as there), 6 the two-launch GEMV (M <= 4 only). */
 MLLMB200_API int mllmb200_w4a32_linear_forward_grouped(const float* x_dev, int M, int K, int ldx, int count,
                                                        const void* const* tiled_dev, float* const* y_dev,
                                                        const int* N, const int* ldy, void* ws_dev, int flags,

@@ -72,7 +72,7 @@ void CUDAW4A32LinearOp::growWorkspace(size_t need) {
   workspace_bytes_ = need;
 }
 
-void* uploadW4A32Weights(Tensor& weight, Tensor& bias, bool want_bias, int n, int k, const std::string& name) {
+void* uploadW4A32Weights(Tensor& weight, Tensor& bias, bool want_bias, int n, int k, const std::string& name, int* scale_mode_out) {
   std::vector<unsigned char> owned;  // holds the blob when it is produced here
   const void* blob = nullptr;
   size_t blob_bytes = 0;
@@ -97,6 +97,7 @@ void* uploadW4A32Weights(Tensor& weight, Tensor& bias, bool want_bias, int n, in
   int bn = 0, bk = 0, scale_mode = 0, has_bias = 0;
   MLLMB200_CHECK(mllmb200_w4a32_blob_info(blob, blob_bytes, &bn, &bk, &scale_mode, &has_bias));
   if (bn != n || bk != k) { MLLM_ERROR_EXIT(kError, "{}: blob is {}x{} but the layer is {}x{}", name, bn, bk, n, k); }
+  if (scale_mode_out != nullptr) *scale_mode_out = scale_mode;
 
   auto& be = registeredW4A32Backend();
   auto stream = static_cast<cudaStream_t>(be.stream());
@@ -162,8 +163,10 @@ void CUDAW4A32LinearOp::load(const std::shared_ptr<ParameterLoader>& ploader) {
     MLLM_RT_ASSERT_EQ(shape[0], n_);
     MLLM_RT_ASSERT_EQ(shape[1], k_);
   }
+  int scale_mode = MLLMB200_SCALE_BF16_TRUNC;
   tiled_dev_ = a16_ ? uploadW4A16Weights(weight_, bias_, cargo_.bias, n_, k_, "CUDAW4A32LinearOp " + name())
-                    : uploadW4A32Weights(weight_, bias_, cargo_.bias, n_, k_, "CUDAW4A32LinearOp " + name());
+                    : uploadW4A32Weights(weight_, bias_, cargo_.bias, n_, k_, "CUDAW4A32LinearOp " + name(), &scale_mode);
+  kernel_flags_ = scale_mode == MLLMB200_SCALE_FP16 ? 0x200 : 0;
 }
 
 void CUDAW4A32LinearOp::reshape(const std::vector<Tensor>& inputs, std::vector<Tensor>& outputs) {
@@ -208,7 +211,7 @@ void CUDAW4A32LinearOp::forward(const std::vector<Tensor>& inputs, std::vector<T
   auto& be = registeredW4A32Backend();
   const int policy = be.linearKernelPolicy() == 3 && m < 65 ? 0 : be.linearKernelPolicy();
   MLLMB200_CHECK(mllmb200_w4a32_linear_forward_ex(x.ptr<float>(), tiled_dev_, y.ptr<float>(), workspace_dev_, m, k_, n_, k_,
-                                                  n_, policy, be.stream()));
+                                                  n_, policy | kernel_flags_, be.stream()));
 }
 
 }  // namespace mllm::cuda

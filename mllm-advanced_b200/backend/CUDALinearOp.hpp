@@ -33,6 +33,7 @@ class CUDAW4A32LinearOp final : public LinearOp {
   void* workspace_dev_ = nullptr;  // quantized activations, grown on demand, reused across calls
   size_t workspace_bytes_ = 0;
   int n_ = 0, k_ = 0;
+  int kernel_flags_ = 0;  // of linear_forward_ex's kernel argument
   bool a16_ = false;  // the W4A16 sibling format
 };
 
@@ -45,7 +46,8 @@ class CUDALinearOpFactory : public TypedOpFactory<OpType::kLinear, LinearOpCargo
 
 // Pre-pack blob (int8 tensor) or fp32 weight of an [n, k] matrix -> device buffer in the tile layout
 // (from the registered backend's allocator; the caller returns it with deviceFree).  Shared with the Conv3D op.
-void* uploadW4A32Weights(Tensor& weight, Tensor& bias, bool want_bias, int n, int k, const std::string& name);
+// scale_mode_out (optional): the encoding of the group scales.
+void* uploadW4A32Weights(Tensor& weight, Tensor& bias, bool want_bias, int n, int k, const std::string& name, int* scale_mode_out = nullptr);
 
 // True for the impl types this op implements (the six f32 W4 Kai tiles; the tile choice is an
 // Arm micro-kernel detail and is ignored here).

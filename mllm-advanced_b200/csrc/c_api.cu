@@ -59,6 +59,12 @@ constexpr int kStreamGemmMinM = 5, kStreamGemmMaxM = 64;  // batch sizes the str
 cudaError_t launch_w4a32_gemm_chunk(const uint8_t*, const float2*, int, int, int, const void* const*, float* const*, const int*,
                                     const int*, int, cudaStream_t);
 constexpr int kChunkMinM = 65;
+// fp16-encoded scales cost the chunked GEMM a second pass over every K-tile.  Where the int8 kernel's tiles (128 x 64) fit one
+// wave it is as fast or faster (us, int8 / chunked: 1536 x 1536, M = 65 18.6 / 19.4, M = 512 19.2 / 22.7; 1536 x 8960, M = 512
+// 78 / 87; 8960 x 1536, M = 128 19.5 / 21.9), from there on slower (8960 x 1536, M = 512 63 / 38; 1536 x 8960, M = 2048
+// 222 / 190).  The host does not see the encoding; callers that know it say so with this flag.
+constexpr int kFlagFp16Scales = 0x200;
+static bool int8_suits_fp16_scales(int m, int n) { return (long long)((n + 127) / 128) * ((m + 63) / 64) <= 148; }
 
 cudaError_t read_device_status(cudaStream_t, int* status);
 
@@ -231,6 +237,7 @@ int mllmb200_w4a32_linear_forward_ex(const float* x_dev, const void* tiled_dev, 
     return MLLMB200_INVALID_ARG;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int use_pdl = (kernel >> 8) & 1;
+  const bool fp16_scales = (kernel & kFlagFp16Scales) != 0;
   kernel &= 0xFF;
   if (kernel < 0 || kernel > 7) return MLLMB200_INVALID_ARG;
   if (kernel == 5) kernel = w4a32_gemm_tcf16_preferred(M, K, N) ? 4 : 0;  // "fastest": fp16 path where it wins
@@ -253,7 +260,7 @@ int mllmb200_w4a32_linear_forward_ex(const float* x_dev, const void* tiled_dev, 
   }
   if (kernel == 6 && !w4a32_gemv_supported(M, K, N)) return MLLMB200_UNSUPPORTED;
   if (kernel == 3 && !w4a32_gemm_tc_supported(M, K, N)) return MLLMB200_UNSUPPORTED;
-  if (kernel == 3 && by_default && M >= kChunkMinM)
+  if (kernel == 3 && by_default && M >= kChunkMinM && !(fp16_scales && int8_suits_fp16_scales(M, N)))
     return chunk_forward(x_dev, M, K, ldx, 1, &tiled_dev, &y_dev, &N, &ldy, ws_dev, use_pdl, st);
   if (kernel == 4) {  // fp16 tensor-core path: its own activation layout
     if (!w4a32_gemm_tcf16_supported(M, K, N)) return MLLMB200_UNSUPPORTED;
@@ -372,7 +379,7 @@ int mllmb200_w4a32_linear_forward_grouped(const float* x_dev, int M, int K, int 
   }
   for (int i = 0; i < count; ++i) {
     const int st = mllmb200_w4a32_linear_forward_ex(x_dev, tiled_dev[i], y_dev[i], ws_dev, M, K, N[i], ldx, ldy[i],
-                                                    (flags & 0x100) | policy, stream);
+                                                    (flags & (0x100 | kFlagFp16Scales)) | policy, stream);
     if (st != MLLMB200_OK) return st;
   }
   return MLLMB200_OK;

@@ -221,7 +221,7 @@ int prefill_into(Decoder* d, const int* tokens_dev, const float* embeds_dev, int
     }
     DEC_CHECK(prompt_attention(n > kShortPrompt, d->q, d->k, d->v, n, c.q_heads, c.kv_heads, c.head_dim, d->sin_t, d->cos_t, d->zero, c.max_ctx,
                                cache_k[l], cache_v[l], d->kv_split, d->attn, s));
-    DEC_ST(mllmb200_w4a32_linear_forward_ex(d->attn, L.w[kO], d->o, d->ws, n, QD, H, QD, H, 5 | 0x100, s));
+    DEC_ST(mllmb200_w4a32_linear_forward_ex(d->attn, L.w[kO], d->o, d->ws, n, QD, H, QD, H, 5 | 0x100 | L.flags[kO], s));
     DEC_CHECK(launch_pdl(add_rmsnorm_quant_kernel, dim3(n), dim3(256), 0, s, d->h, d->o, L.ln2, c.eps, H, d->h, d->xn, nullptr, nullptr, 1));
     {  // gate and up likewise
       const void* tw[2] = {L.w[kGate], L.w[kUp]};
@@ -231,7 +231,7 @@ int prefill_into(Decoder* d, const int* tokens_dev, const float* embeds_dev, int
     }
     DEC_CHECK(launch_pdl(silu_mul_quant_kernel, dim3(n), dim3(512), (size_t)I * sizeof(float), s, d->gate, d->up, I, d->act, nullptr,
                          nullptr, 1));
-    DEC_ST(mllmb200_w4a32_linear_forward_ex(d->act, L.w[kDown], d->down, d->ws, n, I, H, I, H, 5 | 0x100, s));
+    DEC_ST(mllmb200_w4a32_linear_forward_ex(d->act, L.w[kDown], d->down, d->ws, n, I, H, I, H, 5 | 0x100 | L.flags[kDown], s));
   }
   // only the last position feeds the sampler (the reference computes all rows and reads the last)
   const size_t last = (size_t)(n - 1) * H;

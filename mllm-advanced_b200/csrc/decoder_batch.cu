@@ -520,7 +520,7 @@ int enqueue_batched_step(BatchDecoder* b) {
       attn_combine_batched_kernel<<<B, kBatchCombineThreads, (size_t)c.q_heads * b->attn_splits * sizeof(float), s>>>(
           b->part_o, b->part_ml, b->pos, c.max_ctx, b->attn_chunk, b->attn_splits, c.q_heads, c.head_dim, b->attn);
     }
-    BD_ST(mllmb200_w4a32_linear_forward_ex(b->attn, L.w[kO], b->o, b->ws, B, QD, H, QD, H, b->policy | 0x100, s));
+    BD_ST(mllmb200_w4a32_linear_forward_ex(b->attn, L.w[kO], b->o, b->ws, B, QD, H, QD, H, b->policy | 0x100 | L.flags[kO], s));
     add_rmsnorm_quant_kernel<<<B, 256, 0, s>>>(b->h, b->o, L.ln2, c.eps, H, b->h, b->xn, nullptr, nullptr, 0);
     {
       const void* tw[2] = {L.w[kGate], L.w[kUp]};
@@ -529,7 +529,7 @@ int enqueue_batched_step(BatchDecoder* b) {
       BD_ST(mllmb200_w4a32_linear_forward_grouped(b->xn, B, H, H, 2, tw, ty, tn, tn, b->ws, b->policy | 0x100, s));
     }
     silu_mul_quant_kernel<<<B, 512, (size_t)I * sizeof(float), s>>>(b->gate, b->up, I, b->act, nullptr, nullptr, 0);
-    BD_ST(mllmb200_w4a32_linear_forward_ex(b->act, L.w[kDown], b->down, b->ws, B, I, H, I, H, b->policy | 0x100, s));
+    BD_ST(mllmb200_w4a32_linear_forward_ex(b->act, L.w[kDown], b->down, b->ws, B, I, H, I, H, b->policy | 0x100 | L.flags[kDown], s));
   }
   add_rmsnorm_quant_kernel<<<B, 256, 0, s>>>(b->h, b->down, d->final_norm, c.eps, H, nullptr, b->xn, nullptr, nullptr, 0);
   {
@@ -618,7 +618,7 @@ void mllmb200_qwen2_batch_destroy(void* handle) {
   delete b;
 }
 
-// Kernel policy of the M = batch linears (0 auto: exact int32 group sums; 4 / 5: fp16 tensor cores where they apply).
+// Kernel policy of the M = batch linears (0 auto: exact int32 group sums up to 64 sequences, above the GEMM with chunked sums; 4 / 5: fp16 tensor cores where they apply).
 int mllmb200_qwen2_batch_set_policy(void* handle, int policy) {
   auto* b = static_cast<BatchDecoder*>(handle);
   if (!b || (policy != 0 && policy != 4 && policy != 5)) return MLLMB200_INVALID_ARG;

@@ -17,6 +17,7 @@ constexpr int kHeadCtas = 148 * 4;
 
 struct Layer {
   void* w[kNumLinears] = {};
+  int flags[kNumLinears] = {};  // of linear_forward_ex's kernel argument
   float *ln1 = nullptr, *ln2 = nullptr;
   float *cache_k = nullptr, *cache_v = nullptr;
 };

@@ -6,6 +6,7 @@ import numpy as np
 SCALE_BF16_TRUNC, SCALE_BF16_RNE, SCALE_FP16 = 0, 1, 2
 KERNEL_AUTO, KERNEL_GEMV, KERNEL_SIMT, KERNEL_TC, KERNEL_TC_F16, KERNEL_FASTEST, KERNEL_GEMV_2LAUNCH, KERNEL_STREAM_TC = 0, 1, 2, 3, 4, 5, 6, 7
 KERNEL_FLAG_PDL = 0x100
+KERNEL_FLAG_FP16_SCALES = 0x200  # a hint for the choice of the kernel
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 
@@ -169,6 +170,7 @@ class W4A32Weights:
     def __init__(self, tiled, n, k, scale_mode, has_bias, row_begin=0, n_total=None):
         self.tiled, self.n, self.k = tiled, n, k
         self.scale_mode, self.has_bias = scale_mode, has_bias
+        self.kernel_flags = KERNEL_FLAG_FP16_SCALES if scale_mode == SCALE_FP16 else 0
         self.row_begin, self.n_total = row_begin, n if n_total is None else n_total
 
     @staticmethod
@@ -219,7 +221,8 @@ def linear_forward(x, weights, out=None, workspace=None, kernel=KERNEL_AUTO, str
         workspace = _workspace_for(m, k, x.device)
     _check(lib().mllmb200_w4a32_linear_forward_ex(x.data_ptr(), weights.tiled.data_ptr(), out.data_ptr(),
                                                   workspace.data_ptr(), m, k, weights.n, x.stride(0), out.stride(0),
-                                                  kernel | (KERNEL_FLAG_PDL if pdl else 0), _stream_ptr(stream)),
+                                                  kernel | (KERNEL_FLAG_PDL if pdl else 0) | weights.kernel_flags,
+                                                  _stream_ptr(stream)),
            "linear_forward")
     return out
 
@@ -241,7 +244,8 @@ def linear_forward_grouped(x, weights_list, outs=None, workspace=None, stream=No
     ns = (C.c_int * cnt)(*[w.n for w in weights_list])
     ldy = (C.c_int * cnt)(*[o.stride(0) for o in outs])
     _check(lib().mllmb200_w4a32_linear_forward_grouped(x.data_ptr(), m, k, x.stride(0), cnt, tiled, ys, ns, ldy,
-                                                       workspace.data_ptr(), (KERNEL_FLAG_PDL if pdl else 0) | policy,
+                                                       workspace.data_ptr(),
+                                                       (KERNEL_FLAG_PDL if pdl else 0) | policy | weights_list[0].kernel_flags,
                                                        _stream_ptr(stream)), "linear_forward_grouped")
     return outs
 

@@ -159,7 +159,8 @@ def test_scales_far_apart_and_no_numbers(m, k, n, mode):
     x[m // 2:, :32] = 0
     x[m // 2:, 32:] = np.abs(x[m // 2:, 32:])
     blob = mb.prepack_from_quantized(nib, s16, n, k, None, mode)
-    y = mb.linear_forward(torch.from_numpy(x).cuda(), mb.W4A32Weights.from_blob(blob)).cpu().numpy()
+    wt = mb.W4A32Weights.from_blob(blob)
+    y = mb.linear_forward_grouped(torch.from_numpy(x).cuda(), [wt, wt])[1].cpu().numpy()
     mb.check_device_status()
     want = orc.linear(x, nib, s16, None, mode)
     assert np.array_equal(np.isnan(y), np.isnan(want)) and np.isnan(want[:, 92]).all() and np.abs(want[:, 90]).max() == np.finfo(np.float32).max
@@ -192,3 +193,45 @@ def test_quantization_forms(m, k, offset):
     want = _acts64(orc, x) @ _weights64(blob, mb.SCALE_BF16_TRUNC)[0].T
     bar = (48 / 3 + (k + 127) // 128 / 2 + 2) * 2.0 ** -23
     assert (np.linalg.norm(y - want, axis=1) <= bar * np.linalg.norm(want, axis=1)).all()
+
+
+def test_fp16_scales_by_size():
+    """A matrix that says its scales are fp16-encoded takes the int8 kernel while its tiles fit one wave, the GEMM with chunked
+    sums above; matrices of a group share one launch of that (here its single-CTA form).  Both near 64 bits."""
+    orc, rng = Oracle(), np.random.default_rng(3)
+    for m, k, n, int8 in ((148 * 64, 96, 128, True), (148 * 64 + 1, 96, 128, False), (65, 928, 150, True), (300, 928, 3800, False)):
+        x = rng.standard_normal((m, k)).astype(np.float32)
+        blob = mb.quant_prepack((rng.standard_normal((n, k)) * 0.02).astype(np.float32), scale_mode=mb.SCALE_FP16)
+        wt, xd = mb.W4A32Weights.from_blob(blob), torch.from_numpy(x).cuda()
+        y, by_name = mb.linear_forward(xd, wt), mb.linear_forward(xd, wt, kernel=mb.KERNEL_TC)
+        grouped = mb.linear_forward_grouped(xd, [wt, wt], pdl=True)
+        mb.check_device_status()
+        assert torch.equal(y, by_name) == int8, (m, k, n)
+        want = _acts64(orc, x) @ _weights64(blob, mb.SCALE_FP16)[0].T
+        for got in [y] + grouped:
+            assert np.linalg.norm(got.cpu().numpy() - want) <= 1.5e-7 * np.linalg.norm(want), (m, k, n)
+
+
+def test_dependent_launches_in_a_graph():
+    """Quantization and GEMM (pairs, single CTAs) as dependent launches, captured and replayed, give the bits of plain calls."""
+    rng = np.random.default_rng(8)
+    k = 1536
+    wts = [mb.W4A32Weights.from_blob(mb.quant_prepack((rng.standard_normal((n, k)) * 0.02).astype(np.float32))) for n in (12800, 96, 1536)]
+    x = torch.randn((200, k), device="cuda")
+    want = [mb.linear_forward(x, w) for w in wts]
+    outs, s = [torch.zeros_like(y) for y in want], torch.cuda.Stream()
+    ws = torch.empty(mb.workspace_size(200, k), dtype=torch.uint8, device="cuda")
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=s):
+        for _ in range(2):
+            mb.linear_forward_grouped(x, wts[:2], outs=outs[:2], workspace=ws, stream=s, pdl=True)
+            mb.linear_forward(x, wts[2], out=outs[2], workspace=ws, stream=s, pdl=True)
+    for _ in range(3):
+        for y in outs:
+            y.fill_(float("nan"))
+        torch.cuda.synchronize()
+        g.replay()
+        torch.cuda.synchronize()
+        assert all(torch.equal(a, b) for a, b in zip(outs, want))
+    mb.check_device_status()
