@@ -732,9 +732,9 @@ def run_gpu(args):
         stream.synchronize()
         ms_pf = e0.elapsed_time(e1) / 3
         flops = n_pf_layers * sum(2 * PREFILL_M * k * n for _, k, n, _ in LINEARS)
-        kern = {1: "gemv", 2: "simt-dp4a", 3: "tcgen05"}[mb.lib().mllmb200_w4a32_select_kernel(PREFILL_M, 1536, 8960)]
+        kern = {1: "gemv", 2: "simt-dp4a", 3: "tcgen05, chunked fp32 sums"}[mb.lib().mllmb200_w4a32_select_kernel(PREFILL_M, 1536, 8960)]
         line["prefill"] = {"M": PREFILL_M, "layers": n_pf_layers, "ms": ms_pf, "tflops": flops / (ms_pf * 1e-3) / 1e12,
-                           "kernel": kern, "unit": "TOP/s (2*M*N*K int8 ops)",
+                           "kernel": kern, "unit": "TOP/s (2*M*N*K)",
                            "frac_of_bf16_peak": flops / (ms_pf * 1e-3) / 1e12 / tensor_peak, "peak_kind": f"of {peak_kind}"}
         mb.check_device_status()
 
@@ -1217,7 +1217,7 @@ def run_config4(args, torch, mb, gen, hbm_peak, tensor_peak, peak_kind):
     ym = torch.empty((m, n), device="cuda")
     wsm = torch.empty(mb.workspace_size(m, k), dtype=torch.uint8, device="cuda")
     flops = 2.0 * m * n * k
-    for key, kern in (("gemm_M2048_int8", mb.KERNEL_AUTO), ("gemm_M2048_fp16", mb.KERNEL_TC_F16)):
+    for key, kern in (("gemm_M2048_int8", mb.KERNEL_TC), ("gemm_M2048_default", mb.KERNEL_AUTO), ("gemm_M2048_fp16", mb.KERNEL_TC_F16)):
         def gemm_pass(kern=kern):
             with torch.cuda.stream(stream):
                 for w in copies[:2]:

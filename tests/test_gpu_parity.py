@@ -424,9 +424,9 @@ def test_tcgen05_fp16_gemm_other_scale_encodings(orc, m, k, n, mode):
 @pytest.mark.parametrize("policy", [0, 5])
 def test_grouped_prefill_shares_quantization(orc, policy):
     """q/k/v and gate/up at prefill size through the grouped call equal single calls bit for bit:
-    policy 0 = one shared quantization, then one int8 tensor-core launch per matrix; policy 5 = one
-    shared quantization and ONE fp16 tensor-core launch for all matrices (same tile width as the
-    single fp16 calls here, hence the same order of additions)."""
+    one shared quantization and ONE tensor-core launch for all matrices, of the GEMM with chunked sums (policy 0: chunks
+    depend on K alone) or of the one with a single sum (policy 5: same tile width as the single calls here, hence the
+    same order of additions)."""
     rng = np.random.default_rng(91)
     m, k = 300, 1536
     x = rng.standard_normal((m, k)).astype(np.float32)
