@@ -31,7 +31,8 @@
 // of 63 at M = 512, without the operand's stores to tensor memory or without the sums' fetches as long as with them.
 // Measured (B200, quantization of x included), the int8 tile GEMM (gemm_tc.cu) / this kernel: 8960 x 1536, M = 512 63 / 28 us;
 // 28672 x 8192, M = 512 762 / 308 us, M = 2048 2848 / 995 us (967 TFLOP/s); 1536 x 8960 (single CTAs), M = 512 78 / 62 us;
-// error against 64 bits (2-norm) 6.0e-8 / 5.3e-8 at K = 1536, 1.29e-7 / 9.4e-8 at K = 8192.  M = 65, 17920 x 1536
+// error against 64 bits (2-norm) 6.0e-8 / 5.3e-8 at K = 1536, 1.29e-7 / 9.4e-8 at K = 8192; where weights and activations
+// are of one sign throughout, 1.3e-7 / 1.0e-7 at K = 1536, 3.9e-7 / 5.3e-7 at K = 8960.  M = 65, 17920 x 1536
 // 33 / 24 us; the three matrices of q, k, v, M = 65 (one launch instead of three) 47 / 14 us.  At M <= 64 the streaming
 // kernel (gemm_stream.cu) mostly stays ahead: it needs no 128-row tiles (1536 x 1536, M = 48: 8 us, here 14).
 // fp16-encoded scales, us: 1536 x 1536, M = 65 19.4, 1536 x 8960, M = 512 87, 8960 x 1536, M = 512 38 (27, 110 and 47 with
