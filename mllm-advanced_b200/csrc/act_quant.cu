@@ -253,7 +253,9 @@ __global__ void __launch_bounds__(256) act_quant_reflayout_kernel(const float* _
 // Bound: at small M a chain of latencies (row in, min/max across the CTA, blocks out), at large M the memory.  A thread
 // keeps its items of the row (8 values of K each) in registers between the two halves of the work; the rest of a longer row
 // is read again.  Rows of a CTA fill 16-byte pieces of the same lines.  Two forms: two rows by 8 warps each, ITEMS = 5, as
-// long as that is one wave of CTAs (one per SM); above, four rows by 4 warps each, ITEMS = 4, which leaves more CTAs per SM.
+// long as that is one wave of CTAs (one per SM); above, four rows by 4 warps each, ITEMS = 4, which leaves more CTAs per SM,
+// for a long K, of which four rows read half twice, from 768 rows on (a whole prompt of 512 tokens, 28 layers with K = 1536
+// and 8960: two rows throughout 4.87 ms, four rows throughout 4.97, as it is 4.81; 1900 tokens 13.5, 12.65, 12.65).
 // Measured (B200), us, four rows by 8 warps with every row read twice / two rows / four rows: M = 256, K = 1536 5.3 / 4.2 / 4.2,
 // K = 8960 10.3 / 6.3 / 10.3; M = 512, K = 1536 5.2 / 6.2 / 4.2, K = 8960 10.4 / 10.4 / 10.4; M = 2048, K = 96 8.3 / 12.4 / 6.2,
 // K = 1536 12.4 / 14.4 / 8.3, K = 8960 36.9 / 32.9 / 29.0.
@@ -375,7 +377,7 @@ static cudaError_t launch_blocks_f16_t(const float* x, int m, int m_pad, int k, 
 // m_pad: a multiple of 8
 cudaError_t launch_act_quant_blocks_f16(const float* x, int m, int m_pad, int k, int ldx, uint8_t* blocks, float2* hdr,
                                         cudaStream_t stream, int use_pdl, int* clear_ints, int clear_count) {
-  if (m_pad > 2 * 148) return launch_blocks_f16_t<4, 4, 4>(x, m, m_pad, k, ldx, blocks, hdr, stream, use_pdl, clear_ints, clear_count);
+  if (m_pad > 2 * 148 && (k <= 6144 || m_pad > 768)) return launch_blocks_f16_t<4, 4, 4>(x, m, m_pad, k, ldx, blocks, hdr, stream, use_pdl, clear_ints, clear_count);
   return launch_blocks_f16_t<2, 8, 5>(x, m, m_pad, k, ldx, blocks, hdr, stream, use_pdl, clear_ints, clear_count);
 }
 
