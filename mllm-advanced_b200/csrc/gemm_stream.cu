@@ -11,53 +11,56 @@
 // (128 weight rows x all of K per CTA) fill a fraction of the SMs: 12 CTAs for a 1536 x 1536 matrix.  Here the
 // cells of the weight matrix (layout.h: [panel of 32 rows][K-group] x 576 bytes) are spread over all SMs as in the
 // GEMV and the per-group integer products run on the tensor cores:
-//   * work unit = one panel x one K-slice.  A cluster of S CTAs owns panels c, c + C, c + 2C, ...; CTA rank r of it
-//     takes K-groups [r G / S, (r + 1) G / S) of every one of those panels.  S is the smallest size for which the
-//     quantized activations of a K-slice (36 bytes per row and group) fit beside the weight ring in shared memory:
-//     1 for K = 1536 at M = 64, 6 for K = 8960.  They are loaded once per CTA with one bulk copy.
+//   * a cluster of S CTAs keeps one block of at most 32 rows of x (9 .. 64 rows: up to two blocks of even size) and walks
+//     panels; work unit = panel x block.  CTA rank r takes K-groups [r G / S, (r + 1) G / S) of every unit.  Two blocks read
+//     the weights twice from L2, but 1536 x 1536 becomes 96 units on 148 SMs instead of 48 (M = 64: 9.2 -> 6.2 us with the
+//     quantization, in a chain of dependent launches).  S, KS and with them the bits follow from M and K alone: a matrix has
+//     the same bits by itself and in a group.
 //   * a producer warp streams the unit's cells through a ring of 16-group stages (cp.async.bulk + full / empty
 //     mbarriers, weights marked evict-first in L2); under programmatic dependent launch the first stages are
-//     requested before griddepcontrol.wait, the activations after it.
-//   * 8 compute warps: warp (ks, ns) takes the K-groups ks, ks + KS, ... of a stage and the batch columns
-//     [ns, ns + 1) * 8 NTW.  Per cell: 4 word loads = the A fragments of two mma.sync.m16n8k32 (u8 nibbles x s8
-//     activations -> s32; low nibbles are k 0..15, high nibbles k 16..31 of the instruction, which is the byte order
-//     of the activation blocks), accumulator start value -8 * sum(a_q) (the nibbles are stored +8) plus the bits of
-//     12582912.0f, so that the s32 result read as a float is 12582912 + value exactly and one FADD and one FMA with
-//     the row's group scale fold it into the fp32 accumulators.
-//   * at the end of a unit the warps' partial sums meet in shared memory (added in K-slice order); with S > 1
-//     ranks 1.. leave theirs in a double-buffered slot of their own shared memory, signal rank 0 through an
-//     mbarrier in ITS shared memory, and rank 0 adds them in rank order through distributed-shared-memory loads:
-//     deterministic.  Rank 0 (or the only CTA) applies zero-point term, row scale and bias and stores y.
+//     requested before griddepcontrol.wait, the activations after it, in four parts of which the first is enough to start.
+//   * 8 compute warps: warp ks takes the K-groups ks, ks + 8 of a stage.  A cell: one ldmatrix.x4 = the words of four rows
+//     per lane; two LOP3 and a shift make the A fragments of two mma.sync.m16n8k32 (s8: 16 (nibble - 8) in the high half
+//     of each byte, so no zero-point term per group; low nibbles are k 0..15, high nibbles k 16..31 of the instruction, the
+//     byte order of the activation blocks).  The accumulator starts at the bits of 786432.0f, whose last place is 1/16: the
+//     s32 result read as a float is 786432 + group sum exactly (|16 sum| <= 2^19 < 2^22).  One packed add and one packed
+//     FMA (two columns each) fold it into the fp32 sums.
+//   * at the end of a unit the warps' sums meet in shared memory, [slice][column][row], and are added in pairs.  Three
+//     epilogue warps do that beside the next unit's products; where no cluster has a second unit, the compute warps do it
+//     themselves (eight are faster than three: 0.4 us).  With S > 1 ranks 1.. leave theirs in a double-buffered slot of
+//     their own shared memory, signal rank 0 through an mbarrier in ITS shared memory, and rank 0 adds them in rank order
+//     through distributed-shared-memory loads: deterministic.  Rank 0 (or the only CTA) applies zero-point term, row scale
+//     and bias and stores four rows of a column at a time.
+// What bounds it (M = 64, K = 1536, cycles of an SM): a cell takes 115, of which its tensor instructions need 32 and its
+// packed FP32 instructions 32; the rest is issue (about 80 slots) and dependences.  More warps (16), registers filled one
+// stage ahead and 64 columns per warp were each as slow or slower.  With u8 nibbles, a zero-point term per group, scalar
+// FP32 and 32-bit loads a cell took 150.  us a call with its quantization, before -> now, chain of dependent launches:
+//   1536 -> 17920  M = 8 10.4 -> 10.7, 24 15.5 -> 12.4, 48 22.5 -> 19.7, 64 25.8 -> 21.9
+//   8960 -> 1536   M = 8 12.3 -> 11.4, 24 18.7 -> 11.1, 48 22.7 -> 17.1, 64 30.6 -> 19.3
+//   8192 -> 28672  M = 8 46 -> 46, 24 90 -> 62, 64 292 -> 130
 // Every wait is bounded; a cluster leaves together (one cluster barrier at the end) so that no CTA's shared memory
 // disappears under a peer.
 #include <algorithm>
+#include <type_traits>
 
 #include "device_common.cuh"
 
 namespace mllmb200 {
 
-#ifdef MLLMB200_MS_TRACE
-extern __device__ unsigned long long* g_gs_trace;  // development build only: stamps of CTA 0 into the GEMV trace buffer
-#define MS_STAMP(i, v) do { if (blockIdx.x == 0 && tid == 0 && g_gs_trace != nullptr) g_gs_trace[1 + (i)] = (unsigned long long)(v); } while (0)
-#else
-#define MS_STAMP(i, v) do { } while (0)
-#endif
-
-#ifndef MLLMB200_MS_WARPS
-#define MLLMB200_MS_WARPS 8
-#endif
-constexpr int kMsCWarps = MLLMB200_MS_WARPS;  // compute warps (16 were measured 7 % slower than 8)
-constexpr int kMsCThreads = kMsCWarps * 32;
-constexpr int kMsThreads = kMsCThreads + 32;  // + the producer warp
+constexpr int kMsCWarps = 8;                  // compute warps
+constexpr int kMsEWarps = 3;                  // epilogue warps; with the producer warp between them 12 warps, 3 per scheduler
+constexpr int kMsThreads = (kMsCWarps + 1 + kMsEWarps) * 32;
 constexpr int kMsBlockGroups = 16;            // K-groups per ring stage
 constexpr int kMsStageBytes = kMsBlockGroups * kCellBytes;  // 9216
-constexpr int kMsStages = kMsCWarps > 8 ? 4 : 6;
+constexpr int kMsMaxStages = 6, kMsMinStages = 3;
+constexpr int kMsActChunks = 4;               // parts in which a CTA's activations arrive
 constexpr int kMsMaxProblems = 4;
 constexpr int kMsMaxCluster = 8;
-constexpr int kMsActRowBytes = 36;            // per activation row and K-group: 16 + 16 bytes of int8 and the -8 * sum word
-constexpr size_t kMsActBudget = 112 * 1024;   // shared memory for the activations of a CTA's K-slice
+constexpr int kMsActRowBytes = 32;            // per activation row and K-group: 16 + 16 bytes of int8
 constexpr int kMsMaxM = 64;
-constexpr int kMsSlotsPerThread = kMsMaxM * 8 / kMsCThreads;  // float4 result slots of a unit per compute thread (2)
+constexpr int kMsMaxTiles = 4;                // tiles of 8 rows that a CTA multiplies a cell with
+constexpr int kMsRedCol = 36;                 // floats per column of a panel's sums (32 rows; 36 keep the stores free of bank conflicts)
+constexpr size_t kMsSmemMax = 227 * 1024;
 
 struct MsProblem {
   const uint8_t* tiled;  // TiledHeader at offset 0
@@ -66,47 +69,46 @@ struct MsProblem {
   size_t zsum_off, bias_off;
 };
 struct MsParams {
-  const uint8_t* acts;   // [num_groups][ m_pad x 16 (low words) | m_pad x 16 (high words) | m_pad x 4 (-8 * sum) ]
+  const uint8_t* acts;   // per block of rows: [num_groups][ rows x 16 (low words) | rows x 16 (high words) ]
   const float2* a_hdr;   // [m] {lhs_scale, a_off bits}
   int m, m_pad, k, num_groups;
-  int cluster_size, num_clusters, total_panels, num_problems, use_pdl;
+  int num_blocks;  // blocks of 8 NT rows (the last may have fewer)
+  int cluster_size, num_clusters, total_panels, num_problems, stages, one_unit, use_pdl;  // one_unit: no cluster has more than one panel
   MsProblem prob[kMsMaxProblems];
 };
 
 struct MsSmem {
   size_t bars, hdr, flags, acts, ring, red, psum, total;
 };
-__host__ __device__ inline MsSmem ms_smem_layout(int m_pad, int groups_per_rank, int cluster_size, int ks) {
+__host__ __device__ inline MsSmem ms_smem_layout(int rows, int groups_per_rank, int cluster_size, int stages) {
   MsSmem L;
   size_t off = 0;
   L.bars = off;
-  off += 256;  // full[6], empty[6], act, peer_full[2], peer_free[2]
+  off += 256;  // full[6], empty[6], act[4], peer_full[2], peer_free[2], red_full, red_free
   L.hdr = off;
-  off += (size_t)m_pad * 8;
+  off += (size_t)rows * 8;
   L.flags = off;
-  off += 16;
+  off += 32;
   L.acts = off;
-  off += (size_t)groups_per_rank * m_pad * kMsActRowBytes;
+  off += (size_t)groups_per_rank * rows * kMsActRowBytes;
   off = (off + 127) & ~(size_t)127;
   L.ring = off;
-  off += (size_t)kMsStages * kMsStageBytes;
+  off += (size_t)stages * kMsStageBytes;
   L.red = off;
-  off += (size_t)ks * m_pad * 32 * 4;
+  off += (size_t)kMsCWarps * rows * kMsRedCol * 4;
   L.psum = off;
-  if (cluster_size > 1) off += (size_t)2 * m_pad * 32 * 4;
+  if (cluster_size > 1) off += (size_t)2 * rows * 32 * 4;
   L.total = off;
   return L;
 }
 
-__device__ __forceinline__ uint32_t ms_lds32(uint32_t a) {
-  uint32_t v;
-  asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a));
-  return v;
+__device__ __forceinline__ void ms_ldsm4(uint32_t (&v)[4], uint32_t a) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
+               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3])
+               : "r"(a));
 }
-__device__ __forceinline__ uint2 ms_lds64(uint32_t a) {
-  uint2 v;
-  asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(a));
-  return v;
+__device__ __forceinline__ void ms_ldsm2(uint32_t& v0, uint32_t& v1, uint32_t a) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x2.shared.b16 {%0, %1}, [%2];" : "=r"(v0), "=r"(v1) : "r"(a));
 }
 __device__ __forceinline__ uint32_t ms_lds16(uint32_t a) {
   uint32_t v;
@@ -145,68 +147,95 @@ __device__ __forceinline__ bool ms_mbar_wait_cluster_bounded(uint64_t* bar, uint
   }
   return true;
 }
-// D (s32, 16 x 8) = A (u8, 16 x 32, row-major) * B (s8, 32 x 8, column-major) + C, where C holds c0 in the columns
-// 2 (lane % 4) and c1 in the columns 2 (lane % 4) + 1 of both of the lane's rows
-__device__ __forceinline__ void ms_mma_u8s8(int (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1, int c0, int c1) {
-  asm("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%10, %11, %10, %11};"
-      : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3])
-      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "r"(c0), "r"(c1));
+__device__ __forceinline__ uint64_t ms_pack(uint32_t lo, uint32_t hi) {
+  uint64_t v;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "r"(lo), "r"(hi));
+  return v;
 }
-__device__ __forceinline__ void ms_compute_sync() { asm volatile("bar.sync 1, %0;" ::"n"(kMsCThreads) : "memory"); }
+__device__ __forceinline__ void ms_unpack(uint64_t v, uint32_t& lo, uint32_t& hi) { asm("mov.b64 {%0, %1}, %2;" : "=r"(lo), "=r"(hi) : "l"(v)); }
+__device__ __forceinline__ uint64_t ms_add2(uint64_t a, uint64_t b) {
+  uint64_t v;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(v) : "l"(a), "l"(b));
+  return v;
+}
+__device__ __forceinline__ void ms_fma2(uint64_t& acc, uint64_t a, uint64_t b) { asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b)); }
+constexpr uint32_t kMsMagic = 0x49400000u;                      // 786432.0f
+constexpr uint64_t kMsMinusMagic2 = 0xC9400000C9400000ull;      // -786432.0f twice
+// D (s32, 16 x 8) = A (s8, 16 x 32, row-major) * B (s8, 32 x 8, column-major) + c (the bits of 786432.0f)
+__device__ __forceinline__ void ms_mma_s8(uint32_t (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1, const uint32_t (&c)[4]) {
+  asm("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%10, %11, %12, %13};"
+      : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "r"(c[0]), "r"(c[1]), "r"(c[2]), "r"(c[3]));
+}
 
-// NTW: 8-column tiles of the batch per warp (1, 2, 4); NS: warps side by side along the batch (1, 2).
-// The other kMsCWarps / NS warps split the K-groups of a stage.
-template <int NTW, int NS>
+// NT: 8-column tiles of a block of the batch
+template <int NT>
 __global__ void __launch_bounds__(kMsThreads, 1) w4a32_gemm_stream_kernel(const __grid_constant__ MsParams p) {
-  constexpr int KS = kMsCWarps / NS;
+  constexpr int KS = kMsCWarps, ROWS = NT * 8;  // (KS: warps that share the K-groups of a stage)
   extern __shared__ __align__(128) uint8_t ms_smem[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int S = p.cluster_size, G = p.num_groups, m_pad = p.m_pad;
+  const int S = p.cluster_size, G = p.num_groups;
   const uint32_t rank = S > 1 ? cluster_ctarank() : 0u;
-  const int cluster = (int)blockIdx.x / S;
+  // a cluster keeps one block of the batch's rows and walks panels
+  const int cluster = (int)blockIdx.x / S, blk = cluster % p.num_blocks;
+  const int first_row = blk * ROWS, n_tiles = min(NT, (p.m_pad >> 3) - blk * NT), rows = n_tiles * 8, m_here = min(rows, p.m - first_row);
   const int g_lo = (int)(((long long)rank * G) / S), g_hi = (int)(((long long)(rank + 1) * G) / S);
   const int ng = g_hi - g_lo;
-  const MsSmem Lo = ms_smem_layout(m_pad, (G + S - 1) / S, S, KS);
+  const MsSmem Lo = ms_smem_layout(ROWS, (G + S - 1) / S, S, p.stages);
+  const int NST = p.stages, panel_step = p.num_clusters / p.num_blocks;
+  const int act_chunk = ((ng + kMsActChunks - 1) / kMsActChunks + 15) & ~15;  // K-groups
   uint64_t* full = reinterpret_cast<uint64_t*>(ms_smem + Lo.bars);
-  uint64_t* empty = full + kMsStages;
-  uint64_t* act_bar = empty + kMsStages;
-  uint64_t* peer_full = act_bar + 1;   // [2] rank 0: the other ranks' partial sums of a unit are in place
+  uint64_t* empty = full + kMsMaxStages;
+  uint64_t* act_bar = empty + kMsMaxStages;
+  uint64_t* peer_full = act_bar + kMsActChunks;   // [2] rank 0: the other ranks' partial sums of a unit are in place
   uint64_t* peer_free = peer_full + 2; // [2] ranks 1..: rank 0 has read the slot
+  uint64_t* red_full = peer_free + 2;  // the warps' sums of a unit are in place
+  uint64_t* red_free = red_full + 1;   // ... and have been read
   float2* s_hdr = reinterpret_cast<float2*>(ms_smem + Lo.hdr);
-  volatile int* flags = reinterpret_cast<volatile int*>(ms_smem + Lo.flags);
+  volatile int* flags = reinterpret_cast<volatile int*>(ms_smem + Lo.flags);  // bad header, wait ran out, -, -, scale encodings
   uint8_t* acts = ms_smem + Lo.acts;
   uint8_t* ring = ms_smem + Lo.ring;
   float* red = reinterpret_cast<float*>(ms_smem + Lo.red);
   float* psum = reinterpret_cast<float*>(ms_smem + Lo.psum);
-  const size_t group_bytes = (size_t)m_pad * kMsActRowBytes;
+  const size_t group_bytes = (size_t)rows * kMsActRowBytes;
+  const uint8_t* acts_from = p.acts + (size_t)G * first_row * kMsActRowBytes;
 
-  MS_STAMP(0, clock64());
   if (p.use_pdl) pdl_launch_dependents();
   if (tid == 0) {
-    for (int i = 0; i < kMsStages; ++i) {
+    for (int i = 0; i < NST; ++i) {
       mbar_init(&full[i], 1);
       mbar_init(&empty[i], kMsCWarps);
     }
-    mbar_init(act_bar, 1);
+    for (int i = 0; i < kMsActChunks; ++i) mbar_init(&act_bar[i], 1);
     for (int i = 0; i < 2; ++i) {
       mbar_init(&peer_full[i], (uint32_t)max(S - 1, 1));
       mbar_init(&peer_free[i], 1);
     }
+    mbar_init(red_full, kMsCWarps);
+    mbar_init(red_free, kMsEWarps);
     mbar_fence_init();
+    flags[1] = 0;  // set when a wait ran out
+    flags[2] = (int)kMsMagic;
+  }
+  if (warp == 1) {
     // tile headers: checked before a single byte of a matrix is requested
     int bad = 0;
-    for (int i = 0; i < p.num_problems; ++i) {
-      const uint4 h = *reinterpret_cast<const uint4*>(p.prob[i].tiled);  // magic, version, n, k
-      if (h.x != kTiledMagic || h.z != (uint32_t)p.prob[i].n || h.w != (uint32_t)p.k) bad = 1;
+    if (lane < p.num_problems) {
+      const uint4* at = reinterpret_cast<const uint4*>(p.prob[lane].tiled);
+      const uint4 h = at[0], h2 = at[1];  // magic, version, n, k; groups, panels, scale mode, bias
+      bad = h.x != kTiledMagic || h.z != (uint32_t)p.prob[lane].n || h.w != (uint32_t)p.k;
+      flags[4 + lane] = h2.z == 2u;
     }
-    if (bad) atomicOr(&g_device_status, kDevStatusBadHeader);
-    flags[0] = bad;  // 1: nothing is done
-    flags[1] = 0;    // set when a wait ran out
+    bad = __any_sync(0xffffffffu, bad);
+    if (lane == 0) {
+      if (bad) atomicOr(&g_device_status, kDevStatusBadHeader);
+      flags[0] = bad;  // 1: nothing is done
+    }
   }
   __syncthreads();
   if (S > 1) cluster_sync_all();  // every CTA of the cluster runs and has its barriers initialised
   const bool run = flags[0] == 0;
-  const int first_unit = run ? cluster : p.total_panels;
+  const int first_panel = run ? cluster / p.num_blocks : p.total_panels;
 
   auto problem_of = [&](int u) {
     int pi = 0;
@@ -214,6 +243,80 @@ __global__ void __launch_bounds__(kMsThreads, 1) w4a32_gemm_stream_kernel(const 
     for (int i = 1; i < kMsMaxProblems; ++i)
       if (i < p.num_problems && u >= p.prob[i].panel_begin) pi = i;
     return pi;
+  };
+
+  // A unit's outputs from the warps' sums, by THREADS threads (t: this one's number; a multiple of 8, so a thread's tasks are
+  // the same 4 rows of the panel in different columns).  sums: waits for them; read: they may be overwritten.
+  auto finish = [&](auto threads, int t, int u, int unit_index, bool& ok, auto sums, auto read) {
+    constexpr int THREADS = decltype(threads)::value, TRIPS = (ROWS * 8 + THREADS - 1) / THREADS;
+    const MsProblem& pr = p.prob[problem_of(u)];
+    // the rows' constants are requested now and used behind the unit
+    const int n = (u - pr.panel_begin) * kPanelRows + 4 * (t & 7), n_end = pr.n, ldy = pr.ldy;
+    float* const y = pr.y + n + (size_t)first_row * ldy;
+    float4 zs = make_float4(0.0f, 0.0f, 0.0f, 0.0f), bs = zs;
+    if (rank == 0) {
+      zs = *reinterpret_cast<const float4*>(pr.tiled + pr.zsum_off + (size_t)n * 4);
+      bs = *reinterpret_cast<const float4*>(pr.tiled + pr.bias_off + (size_t)n * 4);
+    }
+    const int buf = unit_index & 1;
+    ok = sums() && ok;
+    float4 v[TRIPS];
+#pragma unroll
+    for (int i = 0; i < TRIPS; ++i) {
+      const int col = (t + i * THREADS) >> 3;
+      if (col < m_here) {
+        const float* from = red + (size_t)col * kMsRedCol + 4 * (t & 7);
+        float4 o[KS];
+#pragma unroll
+        for (int r = 0; r < KS; ++r) o[r] = *reinterpret_cast<const float4*>(from + (size_t)r * ROWS * kMsRedCol);
+#pragma unroll
+        for (int d = 1; d < KS; d *= 2)  // pairs, pairs of pairs ..: less rounding than one after the other
+#pragma unroll
+          for (int r = 0; r < KS; r += 2 * d) o[r].x += o[r + d].x, o[r].y += o[r + d].y, o[r].z += o[r + d].z, o[r].w += o[r + d].w;
+        v[i] = o[0];
+      }
+    }
+    read();
+    // ranks 1..: the slot written two units ago must have been read by rank 0
+    if (S > 1 && rank != 0 && unit_index >= 2 && ok)
+      ok = ms_mbar_wait_cluster_bounded(&peer_free[buf], (uint32_t)((unit_index >> 1) - 1) & 1u);
+    if (S > 1 && rank == 0 && ok) ok = ms_mbar_wait_cluster_bounded(&peer_full[buf], (uint32_t)(unit_index >> 1) & 1u);
+#pragma unroll
+    for (int i = 0; i < TRIPS; ++i) {
+      const int col = (t + i * THREADS) >> 3;
+      if (col < m_here) {
+        float* slot = psum + ((size_t)(buf * ROWS + col) * 8 + (t & 7)) * 4;
+        if (S > 1 && rank != 0) *reinterpret_cast<float4*>(slot) = v[i];
+        else if (ok) {
+          for (uint32_t r = 1; r < (uint32_t)S; ++r) {
+            const float4 o = ms_ld_cluster_f32x4(map_to_cta(slot, r));
+            v[i].x += o.x, v[i].y += o.y, v[i].z += o.z, v[i].w += o.w;
+          }
+          const float2 hc = s_hdr[col];
+          const float off = (float)__float_as_int(hc.y);
+          v[i].x = clamp_flt_max(fmaf(fmaf(off, zs.x, v[i].x), hc.x, bs.x));
+          v[i].y = clamp_flt_max(fmaf(fmaf(off, zs.y, v[i].y), hc.x, bs.y));
+          v[i].z = clamp_flt_max(fmaf(fmaf(off, zs.z, v[i].z), hc.x, bs.z));
+          v[i].w = clamp_flt_max(fmaf(fmaf(off, zs.w, v[i].w), hc.x, bs.w));
+          float* to = y + (size_t)col * ldy;
+          if (n + 4 <= n_end && (reinterpret_cast<uintptr_t>(to) & 15u) == 0) *reinterpret_cast<float4*>(to) = v[i];
+          else {
+            if (n < n_end) to[0] = v[i].x;
+            if (n + 1 < n_end) to[1] = v[i].y;
+            if (n + 2 < n_end) to[2] = v[i].z;
+            if (n + 3 < n_end) to[3] = v[i].w;
+          }
+        }
+      }
+    }
+    if (S > 1) {
+      asm volatile("bar.sync 1, %0;" ::"n"(THREADS) : "memory");
+      if (t == 0) {
+        if (rank != 0) ms_mbar_arrive_remote(&peer_full[buf], 0);  // our partial sums of this unit are in place
+        else
+          for (uint32_t r = 1; r < (uint32_t)S; ++r) ms_mbar_arrive_remote(&peer_free[buf], r);
+      }
+    }
   };
 
   if (warp == kMsCWarps) {
@@ -225,19 +328,20 @@ __global__ void __launch_bounds__(kMsThreads, 1) w4a32_gemm_stream_kernel(const 
       bool acts_requested = false;
       auto request_acts = [&] {
         if (p.use_pdl) pdl_wait_prior();  // the activation blocks come from the kernel before this one
-        const uint32_t bytes = (uint32_t)((size_t)ng * group_bytes);
-        mbar_arrive_expect_tx(act_bar, bytes);
-        bulk_g2s(acts, p.acts + (size_t)g_lo * group_bytes, bytes, act_bar);
+        for (int i = 0, g = 0; g < ng; ++i, g += act_chunk) {
+          const uint32_t bytes = (uint32_t)((size_t)min(act_chunk, ng - g) * group_bytes);
+          mbar_arrive_expect_tx(&act_bar[i], bytes);
+          bulk_g2s(acts + (size_t)g * group_bytes, acts_from + (size_t)(g_lo + g) * group_bytes, bytes, &act_bar[i]);
+        }
         acts_requested = true;
       };
       bool ok = true;
-      for (int u = first_unit; u < p.total_panels && ok; u += p.num_clusters) {
-        const int pi = problem_of(u);
-        const MsProblem& pr = p.prob[pi];
-        const uint8_t* panel_cells = pr.tiled + sizeof(TiledHeader) + (size_t)(u - pr.panel_begin) * G * kCellBytes;
+      for (int u = first_panel; u < p.total_panels && ok; u += panel_step) {
+        const MsProblem& pr = p.prob[problem_of(u)];
+        const uint8_t* cells = pr.tiled + sizeof(TiledHeader) + (size_t)(u - pr.panel_begin) * G * kCellBytes;
         for (int b = g_lo; b < g_hi; b += kMsBlockGroups) {
-          if (issued == kMsStages && !acts_requested) request_acts();  // the ring is full of weights: now the activations
-          if (issued >= kMsStages) {
+          if (issued == NST && !acts_requested) request_acts();  // the ring is full of weights: now the activations
+          if (issued >= NST) {
             if (!mbar_wait_bounded(&empty[st], ph ^ 1u)) {
               flags[1] = 1;
               ok = false;
@@ -246,224 +350,197 @@ __global__ void __launch_bounds__(kMsThreads, 1) w4a32_gemm_stream_kernel(const 
           }
           const uint32_t bytes = (uint32_t)(min(kMsBlockGroups, g_hi - b) * kCellBytes);
           mbar_arrive_expect_tx(&full[st], bytes);
-          bulk_g2s_hint(ring + (size_t)st * kMsStageBytes, panel_cells + (size_t)b * kCellBytes, bytes, &full[st], stream_once);
+          bulk_g2s_hint(ring + (size_t)st * kMsStageBytes, cells + (size_t)b * kCellBytes, bytes, &full[st], stream_once);
           ++issued;
-          if (++st == kMsStages) {
+          if (++st == NST) {
             st = 0;
             ph ^= 1u;
           }
         }
       }
-      if (!acts_requested) request_acts();  // (also when there is no unit: the compute warps wait for it)
+      if (!acts_requested && run) request_acts();
     }
     __syncwarp();
-  } else {
+  } else if (warp < kMsCWarps) {
     // =============================== compute warps ===============================
-    const int ks = warp % KS, ns = warp / KS;
-    const int g8 = lane >> 2, c4 = lane & 3;
-    const int n_tiles = m_pad >> 3;
-    MS_STAMP(1, clock64());
-    if (p.use_pdl) pdl_wait_prior();
-    MS_STAMP(2, clock64());
-    for (int i = tid; i < m_pad; i += kMsCThreads) s_hdr[i] = i < p.m ? p.a_hdr[i] : make_float2(0.0f, 0.0f);
-    bool ok = ng <= 0 || mbar_wait_bounded(act_bar, 0);  // also publishes nothing else: s_hdr is read after the first unit's barrier
-    MS_STAMP(3, clock64());
-    long long wait_full = 0, t_loop = 0, t_tail = 0;
+    const int ks = warp, g8 = lane >> 2;
+    bool ok = true;
+    if (p.one_unit) {  // these warps write the outputs themselves
+      if (p.use_pdl) pdl_wait_prior();
+      for (int i = tid; i < m_here; i += kMsCWarps * 32) s_hdr[i] = p.a_hdr[first_row + i];
+    }
+    int acts_here = 0;  // K-groups of the activations that have arrived
     const uint32_t ring_s = smem_u32(ring), acts_s = smem_u32(acts), red_s = smem_u32(red);
-    const uint32_t lo_off = (uint32_t)(g8 * 16 + c4 * 4);                  // this lane's word of a row block
-    const uint32_t hi_base = (uint32_t)m_pad * 16, sum_base = (uint32_t)m_pad * 32;
+    // matrices of an ldmatrix.x4 of the activations: low and high words of tile t, low and high words of tile t + 1
+    const uint32_t b_lane = (uint32_t)(((lane >> 4) * 8 + (lane & 7)) * 16 + ((lane >> 3) & 1) * rows * 16);
 
-    float acc[2][NTW][4];
+    uint64_t acc[2][NT][2];  // pairs of columns: [half][tile][row g8, row g8 + 8]
 #pragma unroll
     for (int h = 0; h < 2; ++h)
 #pragma unroll
-      for (int t = 0; t < NTW; ++t)
+      for (int t = 0; t < NT; ++t) acc[h][t][0] = acc[h][t][1] = 0ull;
+    // the start value of a product, in registers of which the compiler does not know the value: as a constant it would be
+    // written into four registers anew for every product
+    uint32_t magic[4];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) acc[h][t][i] = 0.0f;
+    for (int i = 0; i < 4; ++i) magic[i] = (uint32_t)flags[2];
 
     int st = 0, unit_index = 0;
     uint32_t ph = 0;
-    for (int u = first_unit; u < p.total_panels; u += p.num_clusters, ++unit_index) {
-      const int pi = problem_of(u);
-      const MsProblem& pr = p.prob[pi];
-      const bool f16 = reinterpret_cast<const TiledHeader*>(pr.tiled)->scale_mode == 2u;
-      // the per-row constants of the epilogue are requested now and used after the last stage of the unit
-      const int slots = n_tiles * 64;  // float4 slots of a unit: (column tile, half, lane)
-      const int panel = u - pr.panel_begin;
-      float zs[kMsSlotsPerThread][2], bs[kMsSlotsPerThread][2];
-#pragma unroll
-      for (int q = 0; q < kMsSlotsPerThread; ++q) {
-        const int e4 = tid + q * kMsCThreads;
-        zs[q][0] = zs[q][1] = bs[q][0] = bs[q][1] = 0.0f;
-        if (e4 < slots && rank == 0) {
-          const int row0 = 16 * ((e4 >> 5) & 1) + ((e4 & 31) >> 2);
-          const float* zsum = reinterpret_cast<const float*>(pr.tiled + pr.zsum_off) + (size_t)panel * kPanelRows;
-          const float* bias = reinterpret_cast<const float*>(pr.tiled + pr.bias_off) + (size_t)panel * kPanelRows;
-          zs[q][0] = zsum[row0], zs[q][1] = zsum[row0 + 8];
-          bs[q][0] = bias[row0], bs[q][1] = bias[row0 + 8];
-        }
-      }
-      const long long tl0 = clock64();
+    for (int u = first_panel; u < p.total_panels; u += panel_step, ++unit_index) {
+      const bool f16 = flags[4 + problem_of(u)] != 0;
       for (int b = g_lo; b < g_hi && ok; b += kMsBlockGroups) {
-        const long long tw0 = clock64();
-        if (!mbar_wait_bounded(&full[st], ph)) {
+        if (b - g_lo >= acts_here) {  // (the first unit only)
+          ok = mbar_wait_bounded(&act_bar[(b - g_lo) / act_chunk], 0);
+          acts_here += act_chunk;
+        }
+        if (!ok || !mbar_wait_bounded(&full[st], ph)) {
           ok = false;
           break;
         }
-        wait_full += clock64() - tw0;
         const int cnt = min(kMsBlockGroups, g_hi - b);
         // Two cells per trip (K-groups j and j + KS of the stage), their loads and tensor-core products interleaved:
         // with two warps per scheduler the dependent chain of a single cell would leave the pipes idle.
-        // The accumulator of a product starts at 0x4B400000 - 8 * sum(a_q): the s32 result, read as a float, is then
-        // 12582912 + value exactly (|value| <= 32768), and one FADD replaces the integer-to-float conversion.
         for (int j = ks; j < cnt; j += 2 * KS) {
           const bool two = j + KS < cnt;
-          const uint32_t cell0 = ring_s + (uint32_t)st * kMsStageBytes + (uint32_t)j * kCellBytes;
-          const uint32_t cell1 = two ? cell0 + (uint32_t)KS * kCellBytes : cell0;
-          const uint32_t ag0 = acts_s + (uint32_t)(b - g_lo + j) * (uint32_t)group_bytes;
-          const uint32_t ag1 = two ? ag0 + (uint32_t)KS * (uint32_t)group_bytes : ag0;
+          uint32_t cell[2], act[2];
+          cell[0] = ring_s + (uint32_t)st * kMsStageBytes + (uint32_t)j * kCellBytes;
+          cell[1] = two ? cell[0] + (uint32_t)KS * kCellBytes : cell[0];
+          act[0] = acts_s + (uint32_t)(b - g_lo + j) * (uint32_t)group_bytes;
+          act[1] = two ? act[0] + (uint32_t)KS * (uint32_t)group_bytes : act[0];
           // weights: rows g8, g8 + 8 of either 16-row half; 4 bytes = 8 nibbles = k {4 c4 .. 4 c4 + 3} low and high
-          uint32_t w0[4], w1[4];
-          uint32_t r0[4], r1[4];
+          uint32_t w[2][4], v[2][4], x[2][NT > 2 ? 2 : 1][4];
 #pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            w0[i] = ms_lds32(cell0 + lo_off + (uint32_t)i * 128);
-            w1[i] = ms_lds32(cell1 + lo_off + (uint32_t)i * 128);
-            r0[i] = ms_lds16(cell0 + kCellNibbleBytes + (uint32_t)(g8 + 8 * i) * 2);
-            r1[i] = ms_lds16(cell1 + kCellNibbleBytes + (uint32_t)(g8 + 8 * i) * 2);
+          for (int c = 0; c < 2; ++c) {
+            ms_ldsm4(w[c], cell[c] + (uint32_t)lane * 16);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) v[c][i] = ms_lds16(cell[c] + kCellNibbleBytes + (uint32_t)(g8 + 8 * i) * 2);
+            // (what lies behind the last tile of an odd number of them - bytes of the next group or of the ring - is not used)
+#pragma unroll
+            for (int t = 0; t < NT; t += 2) {
+              if (NT > 1) ms_ldsm4(x[c][t / 2], act[c] + b_lane + (uint32_t)t * 128);
+              else ms_ldsm2(x[c][0][0], x[c][0][1], act[c] + b_lane);
+            }
           }
-          float sc0[4], sc1[4];
-          uint32_t a0[2][4], a1[2][4];
+          if (f16) {
 #pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            sc0[i] = f16 ? __half2float(__ushort_as_half((unsigned short)r0[i])) : __uint_as_float(r0[i] << 16);
-            sc1[i] = f16 ? __half2float(__ushort_as_half((unsigned short)r1[i])) : __uint_as_float(r1[i] << 16);
-            if (!two) sc1[i] = 0.0f;  // the second cell of an odd trip repeats the first with scale 0
+            for (int c = 0; c < 2; ++c)
+#pragma unroll
+              for (int i = 0; i < 4; ++i) v[c][i] = __float_as_uint(__half2float(__ushort_as_half((unsigned short)v[c][i])));
+          } else {
+#pragma unroll
+            for (int c = 0; c < 2; ++c)
+#pragma unroll
+              for (int i = 0; i < 4; ++i) v[c][i] <<= 16;
           }
+          uint64_t sc[2][4];
+          uint32_t a[2][2][4];
 #pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            a0[h][0] = w0[2 * h] & 0x0F0F0F0Fu, a0[h][1] = w0[2 * h + 1] & 0x0F0F0F0Fu;
-            a0[h][2] = (w0[2 * h] >> 4) & 0x0F0F0F0Fu, a0[h][3] = (w0[2 * h + 1] >> 4) & 0x0F0F0F0Fu;
-            a1[h][0] = w1[2 * h] & 0x0F0F0F0Fu, a1[h][1] = w1[2 * h + 1] & 0x0F0F0F0Fu;
-            a1[h][2] = (w1[2 * h] >> 4) & 0x0F0F0F0Fu, a1[h][3] = (w1[2 * h + 1] >> 4) & 0x0F0F0F0Fu;
-          }
-          constexpr int kMagic = 0x4B400000;  // 12582912.0f: ulp 1 up to +-2^22 around it
+          for (int c = 0; c < 2; ++c)
 #pragma unroll
-          for (int t = 0; t < NTW; ++t) {
-            const int nt = ns * NTW + t;
-            if (nt < n_tiles) {
-              const uint32_t col = (uint32_t)nt * 128 + lo_off;  // 8 rows x 16 bytes per column tile
-              const uint32_t sum_at = sum_base + (uint32_t)(nt * 8 + 2 * c4) * 4;  // -8 * sum(a_q) of columns 2 c4, 2 c4 + 1
-              const uint32_t p0 = ms_lds32(ag0 + col), q0 = ms_lds32(ag0 + hi_base + col);
-              const uint32_t p1 = ms_lds32(ag1 + col), q1 = ms_lds32(ag1 + hi_base + col);
-              const uint2 s0 = ms_lds64(ag0 + sum_at), s1 = ms_lds64(ag1 + sum_at);
-              int d0[2][4], d1[2][4];
+            for (int i = 0; i < 4; ++i) {
+              if (c == 1 && !two) v[c][i] = 0u;  // the second cell of an odd trip repeats the first with scale 0
+              sc[c][i] = ms_pack(v[c][i], v[c][i]);
+              a[c][i >> 1][i & 1] = ((w[c][i] << 4) & 0xF0F0F0F0u) ^ 0x80808080u;
+              a[c][i >> 1][2 + (i & 1)] = (w[c][i] & 0xF0F0F0F0u) ^ 0x80808080u;
+            }
 #pragma unroll
-              for (int h = 0; h < 2; ++h) {
-                ms_mma_u8s8(d0[h], a0[h], p0, q0, (int)s0.x + kMagic, (int)s0.y + kMagic);
-                ms_mma_u8s8(d1[h], a1[h], p1, q1, (int)s1.x + kMagic, (int)s1.y + kMagic);
-              }
+          for (int t = 0; t < NT; ++t) {
+            if (t < n_tiles) {
+              uint32_t d[2][2][4];
 #pragma unroll
               for (int h = 0; h < 2; ++h)
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                  const float f0 = __int_as_float(d0[h][i]) - 12582912.0f, f1 = __int_as_float(d1[h][i]) - 12582912.0f;
-                  acc[h][t][i] = fmaf(f0, sc0[2 * h + (i >> 1)], acc[h][t][i]);
-                  acc[h][t][i] = fmaf(f1, sc1[2 * h + (i >> 1)], acc[h][t][i]);
-                }
+                for (int c = 0; c < 2; ++c) ms_mma_s8(d[c][h], a[c][h], x[c][t / 2][2 * (t & 1)], x[c][t / 2][2 * (t & 1) + 1], magic);
+#pragma unroll
+              for (int c = 0; c < 2; ++c)
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
+#pragma unroll
+                  for (int i = 0; i < 2; ++i)
+                    ms_fma2(acc[h][t][i], ms_add2(ms_pack(d[c][h][2 * i], d[c][h][2 * i + 1]), kMsMinusMagic2), sc[c][2 * h + i]);
             }
           }
         }
         __syncwarp();
         if (lane == 0) mbar_arrive(&empty[st]);
-        if (++st == kMsStages) {
+        if (++st == NST) {
           st = 0;
           ph ^= 1u;
         }
       }
-      const long long tl1 = clock64();
-      t_loop += tl1 - tl0;
-      // ---- end of the unit: the K-slices of the warps meet in shared memory
+      // ---- end of the unit: the K-slices of the warps meet in shared memory, [slice][column][row].  Where more units follow,
+      // the epilogue warps add them while this warp goes on.
+      if (ok && unit_index > 0) ok = mbar_wait_bounded(red_free, (uint32_t)(unit_index - 1) & 1u);
 #pragma unroll
       for (int h = 0; h < 2; ++h)
 #pragma unroll
-        for (int t = 0; t < NTW; ++t) {
-          const int nt = ns * NTW + t;
-          if (nt < n_tiles) {
-            const uint32_t at = red_s + (uint32_t)(((ks * n_tiles + nt) * 2 + h) * 32 + lane) * 16;
-            asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(at), "f"(acc[h][t][0]), "f"(acc[h][t][1]),
-                         "f"(acc[h][t][2]), "f"(acc[h][t][3])
-                         : "memory");
-          }
-          acc[h][t][0] = acc[h][t][1] = acc[h][t][2] = acc[h][t][3] = 0.0f;
-        }
-      ms_compute_sync();
-      const int buf = unit_index & 1;
-      // ranks 1..: the slot written two units ago must have been read by rank 0
-      if (S > 1 && rank != 0 && unit_index >= 2 && ok)
-        ok = ms_mbar_wait_cluster_bounded(&peer_free[buf], (uint32_t)((unit_index >> 1) - 1) & 1u);
-      if (S > 1 && rank == 0 && ok) ok = ms_mbar_wait_cluster_bounded(&peer_full[buf], (uint32_t)(unit_index >> 1) & 1u);
+        for (int t = 0; t < NT; ++t) {
+          if (t < n_tiles) {
 #pragma unroll
-      for (int q = 0; q < kMsSlotsPerThread; ++q) {
-        const int e4 = tid + q * kMsCThreads;
-        if (e4 >= slots) break;
-        float4 v = *reinterpret_cast<const float4*>(red + (size_t)e4 * 4);
-        for (int r = 1; r < KS; ++r) {
-          const float4 o = *reinterpret_cast<const float4*>(red + ((size_t)r * slots + e4) * 4);
-          v.x += o.x, v.y += o.y, v.z += o.z, v.w += o.w;
-        }
-        if (S > 1 && rank != 0) {
-          *reinterpret_cast<float4*>(psum + ((size_t)buf * slots + e4) * 4) = v;
-          continue;
-        }
-        if (S > 1 && ok) {
-          for (uint32_t r = 1; r < (uint32_t)S; ++r) {
-            const float4 o = ms_ld_cluster_f32x4(map_to_cta(psum + ((size_t)buf * slots + e4) * 4, r));
-            v.x += o.x, v.y += o.y, v.z += o.z, v.w += o.w;
+            for (int i = 0; i < 2; ++i) {
+              uint32_t v0, v1;  // columns 8 t + 2 (lane % 4) (+ 1) of row 16 h + 8 i + g8
+              ms_unpack(acc[h][t][i], v0, v1);
+              const uint32_t at = red_s + (uint32_t)((ks * ROWS + 8 * t + 2 * (lane & 3)) * kMsRedCol + 16 * h + 8 * i + g8) * 4;
+              asm volatile("st.shared.u32 [%0], %1;" ::"r"(at), "r"(v0) : "memory");
+              asm volatile("st.shared.u32 [%0], %1;" ::"r"(at + kMsRedCol * 4), "r"(v1) : "memory");
+            }
           }
+          acc[h][t][0] = acc[h][t][1] = 0ull;
         }
-        // epilogue: slot = (column tile nt, half h, lane l): rows 16 h + l / 4 (+ 8), columns 8 nt + 2 (l % 4) (+ 1)
-        const int nt = e4 >> 6, h = (e4 >> 5) & 1, l = e4 & 31;
-        const int row0 = 16 * h + (l >> 2), col0 = 8 * nt + 2 * (l & 3);
-        const float vals[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const int row = row0 + (i >> 1) * 8, col = col0 + (i & 1);
-          const int n = panel * kPanelRows + row;
-          if (n < pr.n && col < p.m && ok) {
-            const float2 hc = s_hdr[col];
-            float o = fmaf((float)__float_as_int(hc.y), zs[q][i >> 1], vals[i]);
-            o = fmaf(o, hc.x, bs[q][i >> 1]);
-            pr.y[(size_t)col * pr.ldy + n] = clamp_flt_max(o);
-          }
-        }
+      if (p.one_unit) {
+        finish(std::integral_constant<int, kMsCWarps * 32>(), tid, u, 0, ok,
+               [] {
+                 asm volatile("bar.sync 1, %0;" ::"n"(kMsCWarps * 32) : "memory");
+                 return true;
+               },
+               [] {});
+        break;
       }
-      ms_compute_sync();  // red (and, for rank 0, the peers' slots) are read: the next unit may overwrite them
-      t_tail += clock64() - tl1;
-      if (S > 1 && tid == 0) {
-        if (rank != 0) ms_mbar_arrive_remote(&peer_full[buf], 0);  // our partial sums of this unit are in place
-        else
-          for (uint32_t r = 1; r < (uint32_t)S; ++r) ms_mbar_arrive_remote(&peer_free[buf], r);
-      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(red_full);
+      if (!ok) break;
     }
     if (!ok && lane == 0) flags[1] = 1;
-    MS_STAMP(4, clock64());
-    MS_STAMP(5, wait_full);
-    MS_STAMP(6, t_loop);
-    MS_STAMP(7, t_tail);
-    MS_STAMP(8, unit_index);
+  } else {
+    // =============================== epilogue warps ===============================
+    constexpr int kEThreads = kMsEWarps * 32;
+    const int et = tid - (kMsCWarps + 1) * 32;
+    bool ok = true;
+    if (!p.one_unit) {
+      if (p.use_pdl) pdl_wait_prior();
+      for (int i = et; i < m_here; i += kEThreads) s_hdr[i] = p.a_hdr[first_row + i];
+      asm volatile("bar.sync 1, %0;" ::"n"(kEThreads) : "memory");
+      int unit_index = 0;
+      for (int u = first_panel; u < p.total_panels; u += panel_step, ++unit_index)  // (to the end also when a wait ran out: the barriers)
+        finish(std::integral_constant<int, kEThreads>(), et, u, unit_index, ok, [&] { return ok && mbar_wait_bounded(red_full, (uint32_t)unit_index & 1u); },
+               [&] {
+                 __syncwarp();
+                 if (lane == 0) mbar_arrive(red_free);
+               });
+    }
+    if (!ok && lane == 0) flags[1] = 1;
   }
   // Leave together: ranks 1.. hold partial sums that rank 0 reads, rank 0 holds the barriers they arrive on.
   __syncthreads();
   if (S > 1) cluster_sync_all();
 }
 
+// Rows of x are cut into blocks of at most four tiles of 8, as even as that goes
+static int ms_block_tiles(int m) {
+  const int tiles = (m + 7) / 8, blocks = (tiles + kMsMaxTiles - 1) / kMsMaxTiles;
+  return (tiles + blocks - 1) / blocks;
+}
+
 // ------------------------------------------------------------------------------------------------ activations
 // Per-row int8 quantization (the arithmetic of act_quant_records_kernel) into the layout above: for K-group g
 // and row m the four low words (even k of each 8-value item) at [g][m][0..16), the four high words (odd k) at
-// [g][m_pad + m] ... , -8 * sum at [g][2 m_pad ... ].  One CTA per row of the padded batch; padding rows are zeros.
-constexpr int kMsQuantThreads = 256;
-__global__ void __launch_bounds__(kMsQuantThreads) act_quant_mma_kernel(const float* __restrict__ x, int m_total, int m_pad,
+// [g][rows + m] of its block of rows.  One CTA per row of the padded batch; padding rows are zeros.  A thread keeps its ITEMS items of 8
+// values in registers between minimum / maximum and quantization (all loads in flight at once); rows that are longer or not
+// 16-byte aligned are read twice.
+constexpr int kMsQuantThreads = 512;
+template <int ITEMS>
+__global__ void __launch_bounds__(kMsQuantThreads) act_quant_mma_kernel(const float* __restrict__ x, int m_total, int m_pad, int block_rows,
                                                                         int k, int ldx, int num_groups,
                                                                         uint8_t* __restrict__ acts, float2* __restrict__ hdr,
                                                                         int use_pdl) {
@@ -472,103 +549,117 @@ __global__ void __launch_bounds__(kMsQuantThreads) act_quant_mma_kernel(const fl
     pdl_launch_dependents();
     pdl_wait_prior();  // x may be the previous kernel's output, and that kernel may still read the blocks we overwrite
   }
-  const int m = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int m = blockIdx.x, tid = threadIdx.x;
   const bool live = m < m_total;
   const float* row = x + (size_t)(live ? m : 0) * ldx;
-  const bool vec = (reinterpret_cast<uintptr_t>(row) & 15u) == 0;
   const int num_items = num_groups * 4;
+  const int first = m / block_rows * block_rows, rows = min(block_rows, m_pad - first);  // the block that holds this row
+  acts += (size_t)num_groups * first * kMsActRowBytes + (size_t)(m - first) * 16;
+  auto store = [&](int item, uint32_t lo, uint32_t hi) {
+    const int g = item >> 2, i = item & 3;
+    uint8_t* at = acts + (size_t)g * rows * kMsActRowBytes;
+    reinterpret_cast<uint32_t*>(at)[i] = lo;
+    reinterpret_cast<uint32_t*>(at + (size_t)rows * 16)[i] = hi;
+  };
+  if (!live) {
+    for (int item = tid; item < num_items; item += kMsQuantThreads) store(item, 0u, 0u);
+    return;
+  }
+  auto value = [&](int at) { return at < k ? row[at] : 0.0f; };
+  const bool keep = (reinterpret_cast<uintptr_t>(row) & 15u) == 0 && num_items <= ITEMS * kMsQuantThreads;
+  float v[ITEMS][8];
   float mn = 3.402823466e+38f, mx = -3.402823466e+38f;
-  if (live) {
-    if (vec) {
-      for (int i = tid; i < (k >> 2); i += kMsQuantThreads) {
-        const float4 v = reinterpret_cast<const float4*>(row)[i];
-        mn = fminf(mn, fminf(fminf(v.x, v.y), fminf(v.z, v.w)));
-        mx = fmaxf(mx, fmaxf(fmaxf(v.x, v.y), fmaxf(v.z, v.w)));
-      }
-      for (int i = (k & ~3) + tid; i < k; i += kMsQuantThreads) {
-        mn = fminf(mn, row[i]);
-        mx = fmaxf(mx, row[i]);
-      }
-    } else {
-      for (int i = tid; i < k; i += kMsQuantThreads) {
-        mn = fminf(mn, row[i]);
-        mx = fmaxf(mx, row[i]);
+  if (keep) {
+#pragma unroll
+    for (int j = 0; j < ITEMS; ++j) {
+      const int k0 = (tid + j * kMsQuantThreads) * 8;
+      if (k0 + 8 <= k) {
+        const float4 a = *reinterpret_cast<const float4*>(row + k0);
+        const float4 b = *reinterpret_cast<const float4*>(row + k0 + 4);
+        v[j][0] = a.x, v[j][1] = a.y, v[j][2] = a.z, v[j][3] = a.w;
+        v[j][4] = b.x, v[j][5] = b.y, v[j][6] = b.z, v[j][7] = b.w;
+      } else {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[j][i] = value(k0 + i);
       }
     }
-  }
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    mn = fminf(mn, __shfl_xor_sync(0xffffffffu, mn, o));
-    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-  }
-  if (lane == 0) {
-    scratch[warp] = mn;
-    scratch[32 + warp] = mx;
-  }
-  __syncthreads();
-  mn = lane < kMsQuantThreads / 32 ? scratch[lane] : 3.402823466e+38f;
-  mx = lane < kMsQuantThreads / 32 ? scratch[32 + lane] : -3.402823466e+38f;
+    for (int j = 0; j < ITEMS; ++j) {
+      const int k0 = (tid + j * kMsQuantThreads) * 8;
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    mn = fminf(mn, __shfl_xor_sync(0xffffffffu, mn, o));
-    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+      for (int i = 0; i < 8; ++i)
+        if (k0 + i < k) {
+          mn = fminf(mn, v[j][i]);
+          mx = fmaxf(mx, v[j][i]);
+        }
+    }
+    const int warp = tid >> 5, lane = tid & 31;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      mn = fminf(mn, __shfl_xor_sync(0xffffffffu, mn, o));
+      mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    }
+    if (lane == 0) {
+      scratch[warp] = mn;
+      scratch[32 + warp] = mx;
+    }
+    __syncthreads();
+    mn = scratch[lane & 15];
+    mx = scratch[32 + (lane & 15)];
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) {
+      mn = fminf(mn, __shfl_xor_sync(0xffffffffu, mn, o));
+      mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    }
+  } else {
+    block_row_minmax(row, k, scratch, mn, mx);
   }
   const ActQuantParams qp = act_quant_params(mn, mx);
-  if (live && tid == 0) hdr[m] = make_float2(qp.recip_scale, __int_as_float(-qp.nzp));
-  const size_t group_bytes = (size_t)m_pad * kMsActRowBytes;
-  for (int base = 0; base < num_items; base += kMsQuantThreads) {  // uniform trip count: full warps at the shuffles
-    const int item = base + tid;
-    const bool valid = item < num_items;
-    const int k0 = item * 8;
-    int q8[8];
-    if (live && valid && vec && k0 + 8 <= k) {
-      const float4 a = *reinterpret_cast<const float4*>(row + k0);
-      const float4 b = *reinterpret_cast<const float4*>(row + k0 + 4);
-      const float f[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+  if (tid == 0) hdr[m] = make_float2(qp.recip_scale, __int_as_float(-qp.nzp));
+  auto emit = [&](int item, const float (&f)[8]) {
+    uint32_t lo = 0, hi = 0;
 #pragma unroll
-      for (int j = 0; j < 8; ++j) q8[j] = act_quant_value(f[j], qp);
-    } else {
-#pragma unroll
-      for (int j = 0; j < 8; ++j) q8[j] = (live && valid && k0 + j < k) ? act_quant_value(row[k0 + j], qp) : 0;
+    for (int i = 0; i < 8; ++i) {
+      const uint32_t q = item * 8 + i < k ? (uint32_t)act_quant_value(f[i], qp) & 0xFFu : 0u;
+      if (i & 1) hi |= q << (4 * (i - 1));
+      else lo |= q << (4 * i);
     }
-    const uint32_t lo = ((uint32_t)q8[0] & 0xFFu) | (((uint32_t)q8[2] & 0xFFu) << 8) | (((uint32_t)q8[4] & 0xFFu) << 16) |
-                        (((uint32_t)q8[6] & 0xFFu) << 24);
-    const uint32_t hi = ((uint32_t)q8[1] & 0xFFu) | (((uint32_t)q8[3] & 0xFFu) << 8) | (((uint32_t)q8[5] & 0xFFu) << 16) |
-                        (((uint32_t)q8[7] & 0xFFu) << 24);
-    int s = q8[0] + q8[1] + q8[2] + q8[3] + q8[4] + q8[5] + q8[6] + q8[7];
-    s += __shfl_xor_sync(0xffffffffu, s, 1);
-    s += __shfl_xor_sync(0xffffffffu, s, 2);
-    if (valid) {
-      const int g = item >> 2, i = item & 3;
-      uint8_t* grp = acts + (size_t)g * group_bytes;
-      reinterpret_cast<uint32_t*>(grp + (size_t)m * 16)[i] = lo;
-      reinterpret_cast<uint32_t*>(grp + (size_t)m_pad * 16 + (size_t)m * 16)[i] = hi;
-      if (i == 0) reinterpret_cast<int*>(grp + (size_t)m_pad * 32)[m] = -8 * s;
+    store(item, lo, hi);
+  };
+  if (keep) {
+#pragma unroll
+    for (int j = 0; j < ITEMS; ++j)
+      if (tid + j * kMsQuantThreads < num_items) emit(tid + j * kMsQuantThreads, v[j]);
+  } else {
+    for (int item = tid; item < num_items; item += kMsQuantThreads) {
+      float f[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) f[i] = value(item * 8 + i);
+      emit(item, f);
     }
   }
 }
 
 // ------------------------------------------------------------------------------------------------ host side
 struct MsPlan {
-  int m_pad, cluster_size, num_clusters, total_panels, ks, ntw, ns;
-  size_t smem;
+  int m_pad, block_tiles, num_blocks, cluster_size, groups_per_rank, stages, total_panels;
 };
 
-template <int NTW, int NS>
+template <int NT>
 static cudaError_t ms_configure() {
   static bool configured[64] = {};
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
   if (dev >= 0 && dev < 64 && configured[dev]) return cudaSuccess;
-  e = cudaFuncSetAttribute(w4a32_gemm_stream_kernel<NTW, NS>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+  e = cudaFuncSetAttribute(w4a32_gemm_stream_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMsSmemMax);
   if (e != cudaSuccess) return e;
   if (dev >= 0 && dev < 64) configured[dev] = true;
   return cudaSuccess;
 }
 
 // clusters of `s` CTAs of this kernel that the current device runs at once (148 / s without a device)
-template <int NTW, int NS>
+template <int NT>
 static int ms_cluster_capacity(int s, size_t smem) {
   if (s <= 1) return 148;
   int n = 0;
@@ -583,30 +674,34 @@ static int ms_cluster_capacity(int s, size_t smem) {
   attr.val.clusterDim.z = 1;
   cfg.attrs = &attr;
   cfg.numAttrs = 1;
-  if (ms_configure<NTW, NS>() != cudaSuccess ||
-      cudaOccupancyMaxActiveClusters(&n, w4a32_gemm_stream_kernel<NTW, NS>, &cfg) != cudaSuccess || n <= 0) {
+  if (ms_configure<NT>() != cudaSuccess ||
+      cudaOccupancyMaxActiveClusters(&n, w4a32_gemm_stream_kernel<NT>, &cfg) != cudaSuccess || n <= 0) {
     (void)cudaGetLastError();
     n = 148 / s;
   }
   return n;
 }
 
+// Nothing here but the number of panels depends on N: a matrix has the same bits whether it is launched alone or grouped.
+// The limit of K is that of 36 bytes per row and group (what callers' workspaces are made for) in eight shares of 112 KB.
+// The smallest cluster whose shared memory holds the activations, a power of two (us, 8960 -> 1536, M = 16, an earlier form of
+// the kernel: sizes 2 / 3 / 4 / 5 10.4 / 15.4 / 13.0 / 13.3); two from K = 4480 on, where one CTA would walk a unit for longer
+// than the exchange takes (8960 -> 1536, M = 16: 12.7 alone, 10.1; 4864 -> 896, M = 24: 9.8, 8.7), but for a single tile of
+// rows (8192 -> 28672, M = 8: 46 alone, 60).
 static bool ms_shape_plan(int m, int k, int count, const int* n, MsPlan* plan) {
   if (m < 1 || m > kMsMaxM || count < 1 || count > kMsMaxProblems || k < 1) return false;
   const int G = (k + kGroup - 1) / kGroup;
   plan->m_pad = (m + 7) / 8 * 8;
-  const int n_tiles = plan->m_pad / 8;
-  plan->ntw = n_tiles <= 1 ? 1 : (n_tiles <= 2 ? 2 : 4);
-  plan->ns = n_tiles > 4 ? 2 : 1;
-  plan->ks = kMsCWarps / plan->ns;
-  int S = 0;
-  for (int s = 1; s <= kMsMaxCluster; ++s)
-    if ((size_t)((G + s - 1) / s) * plan->m_pad * kMsActRowBytes <= kMsActBudget) {
-      S = s;
-      break;
-    }
-  if (S == 0 || S > G) return false;
-  plan->cluster_size = S;
+  plan->block_tiles = ms_block_tiles(m);
+  plan->num_blocks = (plan->m_pad / 8 + plan->block_tiles - 1) / plan->block_tiles;
+  if ((size_t)((G + kMsMaxCluster - 1) / kMsMaxCluster) * plan->m_pad * 36 > 112 * 1024) return false;
+  plan->stages = 0;
+  for (int s = G >= 140 && plan->m_pad > 8 ? 2 : 1; s <= kMsMaxCluster && plan->stages == 0; s *= 2) {
+    plan->cluster_size = s;
+    plan->groups_per_rank = (G + s - 1) / s;
+    for (int stages = kMsMaxStages; stages >= kMsMinStages && plan->stages == 0; --stages)
+      if (ms_smem_layout(plan->block_tiles * 8, plan->groups_per_rank, s, stages).total <= kMsSmemMax) plan->stages = stages;
+  }
   long long panels = 0;
   for (int i = 0; i < count; ++i) {
     if (n[i] < 1) return false;
@@ -614,8 +709,7 @@ static bool ms_shape_plan(int m, int k, int count, const int* n, MsPlan* plan) {
   }
   if (panels >= (1ll << 30)) return false;
   plan->total_panels = (int)panels;
-  plan->smem = ms_smem_layout(plan->m_pad, (G + S - 1) / S, S, plan->ks).total;
-  return plan->smem <= 227 * 1024;
+  return plan->stages != 0;
 }
 
 bool w4a32_gemm_stream_supported(int m, int k, int count, const int* n) {
@@ -623,9 +717,9 @@ bool w4a32_gemm_stream_supported(int m, int k, int count, const int* n) {
   return m >= 1 && ms_shape_plan(m, k, count, n, &plan);
 }
 
-// bytes of the activation blocks for m rows of k values (rows padded to a multiple of 8)
+// bytes of the activation blocks for m rows of k values (rows padded to a multiple of 8; what workspaces are made for)
 size_t w4a32_gemm_stream_act_bytes(int m, int k) {
-  return (size_t)((k + kGroup - 1) / kGroup) * (size_t)((m + 7) / 8 * 8) * kMsActRowBytes;
+  return (size_t)((k + kGroup - 1) / kGroup) * (size_t)((m + 7) / 8 * 8) * 36;
 }
 
 cudaError_t launch_act_quant_mma(const float* x, int m, int k, int ldx, uint8_t* acts, float2* hdr, int use_pdl,
@@ -642,23 +736,27 @@ cudaError_t launch_act_quant_mma(const float* x, int m, int k, int ldx, uint8_t*
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
   }
-  return cudaLaunchKernelEx(&cfg, act_quant_mma_kernel, x, m, m_pad, k, ldx, num_groups, acts, hdr, use_pdl);
+  return num_groups * 4 <= kMsQuantThreads
+             ? cudaLaunchKernelEx(&cfg, act_quant_mma_kernel<1>, x, m, m_pad, ms_block_tiles(m) * 8, k, ldx, num_groups, acts, hdr, use_pdl)
+             : cudaLaunchKernelEx(&cfg, act_quant_mma_kernel<3>, x, m, m_pad, ms_block_tiles(m) * 8, k, ldx, num_groups, acts, hdr, use_pdl);
 }
 
-template <int NTW, int NS>
+template <int NT>
 static cudaError_t ms_launch_t(MsParams& prm, const MsPlan& plan, cudaStream_t stream) {
-  cudaError_t e = ms_configure<NTW, NS>();
+  cudaError_t e = ms_configure<NT>();
   if (e != cudaSuccess) return e;
   const int S = plan.cluster_size;
   static int capacity[64][kMsMaxCluster + 1] = {};  // per device and cluster size (the largest shared-memory need is assumed)
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) dev = 0;
-  if (capacity[dev][S] == 0) capacity[dev][S] = ms_cluster_capacity<NTW, NS>(S, 227 * 1024);
-  prm.num_clusters = std::max(1, std::min(std::min(capacity[dev][S], 148 / S), plan.total_panels));
+  if (capacity[dev][S] == 0) capacity[dev][S] = ms_cluster_capacity<NT>(S, kMsSmemMax);
+  const int per_block = std::max(1, std::min(capacity[dev][S], 148 / S) / plan.num_blocks);
+  prm.num_clusters = std::min(per_block, plan.total_panels) * plan.num_blocks;
+  prm.one_unit = plan.total_panels <= per_block;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(prm.num_clusters * S), 1, 1);
   cfg.blockDim = dim3(kMsThreads, 1, 1);
-  cfg.dynamicSmemBytes = plan.smem;
+  cfg.dynamicSmemBytes = ms_smem_layout(plan.block_tiles * 8, plan.groups_per_rank, S, plan.stages).total;
   cfg.stream = stream;
   cudaLaunchAttribute attrs[2];
   int na = 0;
@@ -676,7 +774,7 @@ static cudaError_t ms_launch_t(MsParams& prm, const MsPlan& plan, cudaStream_t s
   }
   cfg.attrs = attrs;
   cfg.numAttrs = na;
-  return cudaLaunchKernelEx(&cfg, w4a32_gemm_stream_kernel<NTW, NS>, prm);
+  return cudaLaunchKernelEx(&cfg, w4a32_gemm_stream_kernel<NT>, prm);
 }
 
 // acts / a_hdr: output of launch_act_quant_mma for the same m and k.  Up to four matrices that share them.
@@ -693,6 +791,8 @@ cudaError_t launch_w4a32_gemm_stream(const uint8_t* acts, const float2* a_hdr, i
   prm.k = k;
   prm.num_groups = (k + kGroup - 1) / kGroup;
   prm.cluster_size = plan.cluster_size;
+  prm.num_blocks = plan.num_blocks;
+  prm.stages = plan.stages;
   prm.total_panels = plan.total_panels;
   prm.num_problems = count;
   prm.use_pdl = use_pdl;
@@ -709,11 +809,11 @@ cudaError_t launch_w4a32_gemm_stream(const uint8_t* acts, const float2* a_hdr, i
     prm.prob[i].bias_off = th.bias_off;
     begin += (int)th.num_panels;
   }
-  if (plan.ns == 2) return ms_launch_t<4, 2>(prm, plan, stream);
-  switch (plan.ntw) {
-    case 1: return ms_launch_t<1, 1>(prm, plan, stream);
-    case 2: return ms_launch_t<2, 1>(prm, plan, stream);
-    default: return ms_launch_t<4, 1>(prm, plan, stream);
+  switch (plan.block_tiles) {
+    case 1: return ms_launch_t<1>(prm, plan, stream);
+    case 2: return ms_launch_t<2>(prm, plan, stream);
+    case 3: return ms_launch_t<3>(prm, plan, stream);
+    default: return ms_launch_t<4>(prm, plan, stream);
   }
 }
 
