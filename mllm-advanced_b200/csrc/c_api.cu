@@ -48,6 +48,7 @@ cudaError_t launch_w4a32_gemm_tcf16_grouped(const uint8_t*, const float2*, int, 
 constexpr int kSplitSyncInts = 1024;  // K-split counters of the fp16 tile GEMM at the end of the workspace (two per output tile)
 
 bool w4a32_gemm_stream_supported(int m, int k, int count, const int* n);
+bool w4a32_gemm_stream_preferred(int m, int k, int count, const int* n);
 size_t w4a32_gemm_stream_act_bytes(int m, int k);
 cudaError_t launch_act_quant_mma(const float*, int, int, int, uint8_t*, float2*, int, cudaStream_t);
 cudaError_t launch_w4a32_gemm_stream(const uint8_t*, const float2*, int, int, int, const void* const*, float* const*,
@@ -218,6 +219,17 @@ static int quantize_into_ws(const float* x_dev, void* ws_dev, int M, int K, int 
   return e == cudaSuccess ? MLLMB200_OK : cuda_fail(e);
 }
 
+// One quantization and one launch of the streaming tensor-core GEMM for up to four matrices that share x.
+static int stream_forward(const float* x_dev, int M, int K, int ldx, int count, const void* const* tiled_dev, float* const* y_dev,
+                          const int* N, const int* ldy, void* ws_dev, int use_pdl, cudaStream_t st) {
+  if (!ws_dev || (reinterpret_cast<uintptr_t>(ws_dev) & 255u)) return MLLMB200_INVALID_ARG;
+  uint8_t* acts = static_cast<uint8_t*>(ws_dev);
+  float2* hdr = reinterpret_cast<float2*>(acts + ws_rec_bytes(M, K));
+  cudaError_t e = launch_act_quant_mma(x_dev, M, K, ldx, acts, hdr, use_pdl, st);
+  if (e == cudaSuccess) e = launch_w4a32_gemm_stream(acts, hdr, M, K, count, tiled_dev, y_dev, N, ldy, use_pdl, st);
+  return e == cudaSuccess ? MLLMB200_OK : cuda_fail(e);
+}
+
 // One quantization and one launch of the chunked tile GEMM for up to four matrices that share x.
 static int chunk_forward(const float* x_dev, int M, int K, int ldx, int count, const void* const* tiled_dev, float* const* y_dev,
                          const int* N, const int* ldy, void* ws_dev, int use_pdl, cudaStream_t st) {
@@ -240,7 +252,11 @@ int mllmb200_w4a32_linear_forward_ex(const float* x_dev, const void* tiled_dev, 
   const bool fp16_scales = (kernel & kFlagFp16Scales) != 0;
   kernel &= 0xFF;
   if (kernel < 0 || kernel > 7) return MLLMB200_INVALID_ARG;
-  if (kernel == 5) kernel = w4a32_gemm_tcf16_preferred(M, K, N) ? 4 : 0;  // "fastest": fp16 path where it wins
+  if (kernel == 5) {  // "fastest": the fp16 path or, above the rows of the default, the streaming kernel where they win
+    kernel = w4a32_gemm_tcf16_preferred(M, K, N) ? 4 : 0;
+    if (w4a32_gemm_stream_preferred(M, K, 1, &N))
+      return stream_forward(x_dev, M, K, ldx, 1, &tiled_dev, &y_dev, &N, &ldy, ws_dev, use_pdl, st);
+  }
   const bool by_default = kernel == 0;
   if (by_default) kernel = mllmb200_w4a32_select_kernel(M, K, N);
   if (kernel == 1) {  // single launch: x is quantized inside the GEMV, no workspace
@@ -251,12 +267,7 @@ int mllmb200_w4a32_linear_forward_ex(const float* x_dev, const void* tiled_dev, 
   }
   if (kernel == 7) {  // streaming tensor-core GEMM for small batches: its own activation layout
     if (!w4a32_gemm_stream_supported(M, K, 1, &N)) return MLLMB200_UNSUPPORTED;
-    if (!ws_dev || (reinterpret_cast<uintptr_t>(ws_dev) & 255u)) return MLLMB200_INVALID_ARG;
-    uint8_t* acts = static_cast<uint8_t*>(ws_dev);
-    float2* hdr7 = reinterpret_cast<float2*>(acts + ws_rec_bytes(M, K));
-    cudaError_t e7 = launch_act_quant_mma(x_dev, M, K, ldx, acts, hdr7, use_pdl, st);
-    if (e7 == cudaSuccess) e7 = launch_w4a32_gemm_stream(acts, hdr7, M, K, 1, &tiled_dev, &y_dev, &N, &ldy, use_pdl, st);
-    return e7 == cudaSuccess ? MLLMB200_OK : cuda_fail(e7);
+    return stream_forward(x_dev, M, K, ldx, 1, &tiled_dev, &y_dev, &N, &ldy, ws_dev, use_pdl, st);
   }
   if (kernel == 6 && !w4a32_gemv_supported(M, K, N)) return MLLMB200_UNSUPPORTED;
   if (kernel == 3 && !w4a32_gemm_tc_supported(M, K, N)) return MLLMB200_UNSUPPORTED;
@@ -312,18 +323,13 @@ int mllmb200_w4a32_linear_forward_grouped(const float* x_dev, int M, int K, int 
   int n_group = 0;
   for (int i = 0; i < count; ++i) n_group += N[i];
   // ("fastest" at 64 <= M: wide groups with a short K go to the fp16 tile GEMM further down)
+  const bool stream_fastest = (flags & 0xFF) == 5 && w4a32_gemm_stream_preferred(M, K, count, N);
   const bool tile16_first = (flags & 0xFF) == 5 && count > 1 && w4a32_gemm_tcf16_preferred(M, K, n_group);
-  if (((flags & 0xFF) == 0 || (flags & 0xFF) == 5) && !tile16_first && M >= kStreamGemmMinM && M <= kStreamGemmMaxM &&
-      w4a32_gemm_stream_supported(M, K, count, N)) {  // small batch: one quantization, ONE streaming tensor-core launch
-    if (!ws_dev || (reinterpret_cast<uintptr_t>(ws_dev) & 255u)) return MLLMB200_INVALID_ARG;
-    cudaStream_t st7 = static_cast<cudaStream_t>(stream);
-    uint8_t* acts = static_cast<uint8_t*>(ws_dev);
-    float2* hdr7 = reinterpret_cast<float2*>(acts + ws_rec_bytes(M, K));
-    const int pdl7 = (flags >> 8) & 1;
-    cudaError_t e7 = launch_act_quant_mma(x_dev, M, K, ldx, acts, hdr7, pdl7, st7);
-    if (e7 == cudaSuccess) e7 = launch_w4a32_gemm_stream(acts, hdr7, M, K, count, tiled_dev, y_dev, N, ldy, pdl7, st7);
-    return e7 == cudaSuccess ? MLLMB200_OK : cuda_fail(e7);
-  }
+  // small batch: one quantization, ONE streaming tensor-core launch
+  const bool stream_default = ((flags & 0xFF) == 0 || (flags & 0xFF) == 5) && M >= kStreamGemmMinM && M <= kStreamGemmMaxM &&
+                              w4a32_gemm_stream_supported(M, K, count, N);
+  if (stream_fastest || (stream_default && !tile16_first))
+    return stream_forward(x_dev, M, K, ldx, count, tiled_dev, y_dev, N, ldy, ws_dev, (flags >> 8) & 1, static_cast<cudaStream_t>(stream));
   bool gemv = (flags & 0xFF) == 6;  // the two-launch path (quantization kernel + one-shot GEMV), kept for comparison
   for (int i = 0; i < count && gemv; ++i) gemv = w4a32_gemv_supported(M, K, N[i]);
   if ((flags & 0xFF) == 6 && !gemv) return MLLMB200_UNSUPPORTED;

@@ -1,4 +1,4 @@
-// Streaming W4A32 GEMM for small batches (5 <= M <= 64 activation rows), sm_100a.
+// Streaming W4A32 GEMM for small batches (5 <= M <= 64 activation rows; up to 192 by the "fastest" policy), sm_100a.
 //
 //   y[m,n] = lhs_scale[m] * ( sum_b float(sum_{k in b} a_q[m,k] * w[n,k]) * s[n,b]  +  a_off[m] * zsum[n] ) + bias[n]
 //
@@ -11,7 +11,7 @@
 // (128 weight rows x all of K per CTA) fill a fraction of the SMs: 12 CTAs for a 1536 x 1536 matrix.  Here the
 // cells of the weight matrix (layout.h: [panel of 32 rows][K-group] x 576 bytes) are spread over all SMs as in the
 // GEMV and the per-group integer products run on the tensor cores:
-//   * a cluster of S CTAs keeps one block of at most 32 rows of x (9 .. 64 rows: up to two blocks of even size) and walks
+//   * a cluster of S CTAs keeps one block of at most 32 rows of x (33 rows and more: blocks of even size) and walks
 //     panels; work unit = panel x block.  CTA rank r takes K-groups [r G / S, (r + 1) G / S) of every unit.  Two blocks read
 //     the weights twice from L2, but 1536 x 1536 becomes 96 units on 148 SMs instead of 48 (M = 64: 9.2 -> 6.2 us with the
 //     quantization, in a chain of dependent launches).  S, KS and with them the bits follow from M and K alone: a matrix has
@@ -57,7 +57,7 @@ constexpr int kMsActChunks = 4;               // parts in which a CTA's activati
 constexpr int kMsMaxProblems = 4;
 constexpr int kMsMaxCluster = 8;
 constexpr int kMsActRowBytes = 32;            // per activation row and K-group: 16 + 16 bytes of int8
-constexpr int kMsMaxM = 64;
+constexpr int kMsMaxM = 192, kMsNamedMaxM = 64;  // of a launch; of kernel 7 by name and by default
 constexpr int kMsMaxTiles = 4;                // tiles of 8 rows that a CTA multiplies a cell with
 constexpr int kMsRedCol = 36;                 // floats per column of a panel's sums (32 rows; 36 keep the stores free of bank conflicts)
 constexpr size_t kMsSmemMax = 227 * 1024;
@@ -694,7 +694,7 @@ static bool ms_shape_plan(int m, int k, int count, const int* n, MsPlan* plan) {
   plan->m_pad = (m + 7) / 8 * 8;
   plan->block_tiles = ms_block_tiles(m);
   plan->num_blocks = (plan->m_pad / 8 + plan->block_tiles - 1) / plan->block_tiles;
-  if ((size_t)((G + kMsMaxCluster - 1) / kMsMaxCluster) * plan->m_pad * 36 > 112 * 1024) return false;
+  if (m <= kMsNamedMaxM && (size_t)((G + kMsMaxCluster - 1) / kMsMaxCluster) * plan->m_pad * 36 > 112 * 1024) return false;
   plan->stages = 0;
   for (int s = G >= 140 && plan->m_pad > 8 ? 2 : 1; s <= kMsMaxCluster && plan->stages == 0; s *= 2) {
     plan->cluster_size = s;
@@ -714,7 +714,19 @@ static bool ms_shape_plan(int m, int k, int count, const int* n, MsPlan* plan) {
 
 bool w4a32_gemm_stream_supported(int m, int k, int count, const int* n) {
   MsPlan plan;
-  return m >= 1 && ms_shape_plan(m, k, count, n, &plan);
+  return m >= 1 && m <= kMsNamedMaxM && ms_shape_plan(m, k, count, n, &plan);
+}
+
+// Where the "fastest" policy (5) takes this kernel above 64 rows: matrices, or groups, of at most 4096 rows, whose 128-row tiles
+// would leave most SMs of the tile GEMMs idle, and up to 192 rows of x, in blocks of 32.  us with the quantization, the tile
+// GEMM that policy took / this kernel: M = 65 (gemm_chunk.cu) 1536 -> 1536 13.3 / 7.8, 8960 -> 1536 50.1 / 19.6, 4864 -> 896
+// 30.0 / 12.7; M = 127 14.7 / 9.2, 54.0 / 26.9, 32.1 / 14.3; M = 192 (gemm_tcf16.cu) 15.6 / 11.5, 33.7 / 33.0, 23.4 / 17.3;
+// M = 256 16.8 / 13.5, 35.2 / 43.5, 24.4 / 20.6; more weight rows: 896 -> 9728, M = 128 10.8 / 19.7.  Error against 64 bits, the
+// same: K = 8960 9.7e-8 / 6.9e-8 (M = 65) and 4.3e-7 / 6.9e-8 (M = 192), K = 1536 5.2e-8 / 5.1e-8 and 7.8e-8 / 5.2e-8, K = 896
+// 4.3e-8 / 4.5e-8 and 9.5e-8 / 4.6e-8: short K below 128 rows stays where it was.
+bool w4a32_gemm_stream_preferred(int m, int k, int count, const int* n) {
+  MsPlan plan;
+  return m > kMsNamedMaxM && (m >= 128 || k >= 1024) && ms_shape_plan(m, k, count, n, &plan) && plan.total_panels <= 4096 / kPanelRows;
 }
 
 // bytes of the activation blocks for m rows of k values (rows padded to a multiple of 8; what workspaces are made for)

@@ -28,7 +28,7 @@ def _group_magnitudes(orc, x, w64):
     return total * recip
 
 
-def _case(m, k, ns, mode=mb.SCALE_BF16_TRUNC, odd=False):
+def _case(m, k, ns, mode=mb.SCALE_BF16_TRUNC, odd=False, policy=mb.KERNEL_AUTO):
     orc, rng = Oracle(), np.random.default_rng(m + 7 * k + sum(ns))
     x = rng.standard_normal((m, k)).astype(np.float32)
     x[-1], x[1] = np.abs(x[-1]) + 1, 0
@@ -39,7 +39,7 @@ def _case(m, k, ns, mode=mb.SCALE_BF16_TRUNC, odd=False):
         bias = (rng.standard_normal(n) * 0.1).astype(np.float32)
         blob = mb.quant_prepack((rng.standard_normal((n, k)) * 0.02).astype(np.float32), bias, scale_mode=mode)
         wts.append((mb.W4A32Weights.from_blob(blob), *_weights64(blob, mode)))
-    outs = mb.linear_forward_grouped(xd, [w for w, _, _ in wts], pdl=True)
+    outs = mb.linear_forward_grouped(xd, [w for w, _, _ in wts], pdl=True, policy=policy)
     mb.check_device_status()
     rounds = ((k + 31) // 32 + 7) // 8 + 3 + 7 + 2
     for (wt, w64, bias), y in zip(wts, outs):
@@ -47,7 +47,7 @@ def _case(m, k, ns, mode=mb.SCALE_BF16_TRUNC, odd=False):
         bar = rounds * 2.0 ** -24 * (_group_magnitudes(orc, x, w64) + np.abs(bias) + np.abs(want)) + 1e-30
         assert (np.abs(y.cpu().numpy() - want) <= bar).all(), (wt.n, np.max(np.abs(y.cpu().numpy() - want) / bar))
         buf = torch.full((m, wt.n + (21 if odd else 24)), float("nan"), device="cuda")
-        mb.linear_forward(xd, wt, out=buf[:, :wt.n])  # the same bits by itself, and nothing outside of its columns
+        mb.linear_forward(xd, wt, out=buf[:, :wt.n], kernel=policy)  # the same bits by itself, and nothing outside of its columns
         mb.check_device_status()
         assert torch.equal(buf[:, :wt.n], y) and bool(torch.isnan(buf[:, wt.n:]).all())
 
@@ -70,6 +70,13 @@ def test_fp16_scales(m, k, ns):
 @pytest.mark.parametrize("m,k,ns", [(7, 1537, (129,)), (64, 1001, (4803, 31)), (20, 13000, (35,))])
 def test_rows_and_outputs_off_16_bytes(m, k, ns):
     _case(m, k, ns, odd=True)
+
+
+# above 64 rows, where the fastest policy takes the kernel: three to six blocks, the borders of its rows, columns and K
+@pytest.mark.parametrize("m,k,ns", [(65, 1024, (31,)), (80, 1536, (1536, 256)), (97, 8960, (1536,)), (127, 4448, (4096,)), (128, 896, (896, 128, 128)),
+                                    (161, 4864, (896,)), (192, 2048, (2048, 1024))])
+def test_fastest_above_64_rows(m, k, ns):
+    _case(m, k, ns, policy=mb.KERNEL_FASTEST)
 
 
 @pytest.mark.parametrize("scale", [2.0 ** -120, 2.0 ** 100])
