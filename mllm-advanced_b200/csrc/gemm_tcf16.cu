@@ -635,13 +635,17 @@ static TfTile tf_tile_for(int m, int count, const int* n) {
     wide = wide && n[i] >= 4096;
   }
   TfTile t;
-  if (MLLMB200_TF_WIDE && wide && m >= 256 && t256 * ((m + 255) / 256) >= 100) {  // (256 rows x 128: measured slower than 128 x 256, 31 vs 24 us)
+  // One tile of x as wide as the rows need, where the weight tiles alone give most SMs one: the weights are dequantized once
+  // a tile, which costs more than the columns of padding (us with the quantization, 1536 -> 17920 in narrower / one tile:
+  // M = 65 23.6 / 14.1, M = 127 24.3 / 15.3, M = 129 27.4 / 19.6, M = 255 28.0 / 21.6; 896 -> 9728, 76 weight tiles, M = 65
+  // 15.6 / 9.9, but M = 160 18.6 / 20.5; 8192 -> 28672 M = 160, 128 / 256 / 256 with 256 weight rows 154 / 127 / 117).
+  if (MLLMB200_TF_WIDE && wide && m > 128 && t256 * ((m + 255) / 256) >= 100) {  // (256 rows x 128: measured slower than 128 x 256, 31 vs 24 us)
     t.rows = 256;
     t.nt = 256;
     return t;
   }
   t.rows = 128;
-  t.nt = (m >= 256 && t128 * ((m + 255) / 256) >= 100) ? 256 : (m >= 128 ? 128 : 64);
+  t.nt = (m > 128 && t128 * ((m + 255) / 256) >= 100) ? 256 : (m >= 128 || (m > 64 && t128 >= 64) ? 128 : 64);
   return t;
 }
 int w4a32_gemm_tcf16_tile(int m, int n) { return tf_tile_for(m, 1, &n).nt; }

@@ -79,6 +79,24 @@ def test_fastest_above_64_rows(m, k, ns):
     _case(m, k, ns, policy=mb.KERNEL_FASTEST)
 
 
+# one tile of x where the weight tiles fill the SMs: columns of padding up to half a tile, 256 weight rows, the last panel short
+@pytest.mark.parametrize("m,k,ns", [(65, 896, (8192,)), (127, 96, (4864, 4864)), (129, 512, (12900,)), (200, 224, (28672,)), (255, 1536, (8960, 8960))])
+def test_fastest_tiles_of_uneven_rows(m, k, ns):
+    """The fp16 tile GEMM: one truncated sum over K, K / 16 additions as in test_chunk_gemm's bar."""
+    orc, rng = Oracle(), np.random.default_rng(m + k)
+    x = rng.standard_normal((m, k)).astype(np.float32)
+    wts = []
+    for n in ns:
+        blob = mb.quant_prepack((rng.standard_normal((n, k)) * 0.02).astype(np.float32))
+        wts.append((mb.W4A32Weights.from_blob(blob), _weights64(blob, mb.SCALE_BF16_TRUNC)[0]))
+    outs = mb.linear_forward_grouped(torch.from_numpy(x).cuda(), [w for w, _ in wts], pdl=True, policy=mb.KERNEL_FASTEST)
+    mb.check_device_status()
+    a = _acts64(orc, x)
+    for (_, w64), y in zip(wts, outs):
+        want = a @ w64.T
+        assert np.linalg.norm(y.cpu().numpy() - want) <= (k / 16 / 3 + 2) * 2.0 ** -23 * np.linalg.norm(want)
+
+
 @pytest.mark.parametrize("scale", [2.0 ** -120, 2.0 ** 100])
 def test_far_scales(scale):
     """Group sums up to 2^15 times scales near the ends of bf16: the sixteenfold integers of the tensor cores leave no trace."""
