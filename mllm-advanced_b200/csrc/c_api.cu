@@ -4,6 +4,7 @@
 
 #include "../../include/mllmb200.h"
 #include "device_common.cuh"
+#include "linear_blocks.h"
 
 namespace mllmb200 {
 // repack.cu
@@ -36,8 +37,6 @@ bool w4a32_gemm_tcf16_supported(int m, int k, int n);
 bool w4a32_gemm_tcf16_preferred(int m, int k, int n);
 int w4a32_gemm_tcf16_m_pad(int m, int n);
 int w4a32_gemm_tcf16_m_pad_max(int m);
-cudaError_t launch_w4a32_gemm_tcf16(const uint8_t*, const float2*, const void*, float*, int, int, int, int, cudaStream_t, int use_pdl,
-                                    int* split_sync, int split_sync_ints);
 cudaError_t launch_act_quant_blocks_f16(const float*, int, int, int, int, uint8_t*, float2*, cudaStream_t, int use_pdl = 0,
                                         int* clear_ints = nullptr, int clear_count = 0);
 int w4a32_gemm_tcf16_tile_grouped(int m, int count, const int* n);
@@ -50,6 +49,7 @@ constexpr int kSplitSyncInts = 1024;  // K-split counters of the fp16 tile GEMM 
 bool w4a32_gemm_stream_supported(int m, int k, int count, const int* n);
 bool w4a32_gemm_stream_preferred(int m, int k, int count, const int* n);
 size_t w4a32_gemm_stream_act_bytes(int m, int k);
+int w4a32_gemm_stream_block_rows(int m);
 cudaError_t launch_act_quant_mma(const float*, int, int, int, uint8_t*, float2*, int, cudaStream_t);
 cudaError_t launch_w4a32_gemm_stream(const uint8_t*, const float2*, int, int, int, const void* const*, float* const*,
                                      const int*, const int*, int, cudaStream_t);
@@ -96,6 +96,44 @@ int* w4a32_ws_split_sync(void* ws_dev, int m, int k) {
   return reinterpret_cast<int*>(static_cast<uint8_t*>(ws_dev) + ws_rec_bytes(m, k) + align_up((size_t)m * sizeof(float2), 256));
 }
 int w4a32_ws_split_sync_ints() { return kSplitSyncInts; }
+
+static W4Blocks blocks_at(W4Form form, int M, int K, int m_pad, void* ws) {
+  W4Blocks b = {};
+  b.form = form;
+  b.m_pad = form == kW4Tile ? m_pad : (M + 7) / 8 * 8;
+  if (form == kW4Stream) b.block_rows = w4a32_gemm_stream_block_rows(M);
+  b.blocks = static_cast<uint8_t*>(ws);
+  if (!ws) return b;
+  b.hdr = reinterpret_cast<float2*>(b.blocks + ws_rec_bytes(M, K));
+  if (form == kW4Tile) b.clear = w4a32_ws_split_sync(ws, M, K), b.clear_count = kSplitSyncInts;
+  return b;
+}
+W4Blocks w4a32_blocks_for(int M, int K, int count, const int* N, int policy_and_flags, void* ws) {
+  const bool fastest = (policy_and_flags & 0xFF) == 5, fp16_scales = (policy_and_flags & kFlagFp16Scales) != 0;
+  W4Blocks none = {};
+  int ks[4], n_sum = 0;
+  for (int i = 0; i < count; ++i) ks[i] = K, n_sum += N[i];
+  if (w4a32_gemv_stream_supported(M, count, ks, N)) return none;
+  if (fastest && w4a32_gemm_stream_preferred(M, K, count, N)) return blocks_at(kW4Stream, M, K, 0, ws);
+  // (a group's weight tiles ride in one grid)
+  if (fastest && w4a32_gemm_tcf16_preferred(M, K, n_sum)) {
+    const int nt = w4a32_gemm_tcf16_tile_grouped(M, count, N);
+    return blocks_at(kW4Tile, M, K, (M + nt - 1) / nt * nt, ws);
+  }
+  if (M >= kStreamGemmMinM && M <= kStreamGemmMaxM && w4a32_gemm_stream_supported(M, K, count, N)) return blocks_at(kW4Stream, M, K, 0, ws);
+  bool tiles = M >= kChunkMinM && !(count == 1 && fp16_scales && int8_suits_fp16_scales(M, N[0]));
+  for (int i = 0; i < count && tiles; ++i) tiles = mllmb200_w4a32_select_kernel(M, K, N[i]) == 3;
+  return tiles ? blocks_at(kW4Chunk, M, K, 0, ws) : none;
+}
+cudaError_t w4a32_forward_blocks(const W4Blocks& b, int M, int K, int count, const void* const* tiled, float* const* y, const int* N,
+                                 const int* ldy, int use_pdl, cudaStream_t stream) {
+  switch (b.form) {
+    case kW4Stream: return launch_w4a32_gemm_stream(b.blocks, b.hdr, M, K, count, tiled, y, N, ldy, use_pdl, stream);
+    case kW4Tile: return launch_w4a32_gemm_tcf16_grouped(b.blocks, b.hdr, M, K, count, tiled, y, N, ldy, stream, 0, nullptr, use_pdl, b.clear, b.clear_count);
+    case kW4Chunk: return launch_w4a32_gemm_chunk(b.blocks, b.hdr, M, K, count, tiled, y, N, ldy, use_pdl, stream);
+    default: return cudaErrorInvalidValue;
+  }
+}
 }  // namespace mllmb200
 
 using namespace mllmb200;
@@ -219,25 +257,13 @@ static int quantize_into_ws(const float* x_dev, void* ws_dev, int M, int K, int 
   return e == cudaSuccess ? MLLMB200_OK : cuda_fail(e);
 }
 
-// One quantization and one launch of the streaming tensor-core GEMM for up to four matrices that share x.
-static int stream_forward(const float* x_dev, int M, int K, int ldx, int count, const void* const* tiled_dev, float* const* y_dev,
-                          const int* N, const int* ldy, void* ws_dev, int use_pdl, cudaStream_t st) {
-  if (!ws_dev || (reinterpret_cast<uintptr_t>(ws_dev) & 255u)) return MLLMB200_INVALID_ARG;
-  uint8_t* acts = static_cast<uint8_t*>(ws_dev);
-  float2* hdr = reinterpret_cast<float2*>(acts + ws_rec_bytes(M, K));
-  cudaError_t e = launch_act_quant_mma(x_dev, M, K, ldx, acts, hdr, use_pdl, st);
-  if (e == cudaSuccess) e = launch_w4a32_gemm_stream(acts, hdr, M, K, count, tiled_dev, y_dev, N, ldy, use_pdl, st);
-  return e == cudaSuccess ? MLLMB200_OK : cuda_fail(e);
-}
-
-// One quantization and one launch of the chunked tile GEMM for up to four matrices that share x.
-static int chunk_forward(const float* x_dev, int M, int K, int ldx, int count, const void* const* tiled_dev, float* const* y_dev,
-                         const int* N, const int* ldy, void* ws_dev, int use_pdl, cudaStream_t st) {
-  if (!ws_dev || (reinterpret_cast<uintptr_t>(ws_dev) & 255u)) return MLLMB200_INVALID_ARG;
-  uint8_t* blocks = static_cast<uint8_t*>(ws_dev);
-  float2* hdr = reinterpret_cast<float2*>(blocks + ws_rec_bytes(M, K));
-  cudaError_t e = launch_act_quant_blocks_f16(x_dev, M, (M + 7) / 8 * 8, K, ldx, blocks, hdr, st, use_pdl);
-  if (e == cudaSuccess) e = launch_w4a32_gemm_chunk(blocks, hdr, M, K, count, tiled_dev, y_dev, N, ldy, use_pdl, st);
+// One quantization and one launch for up to four matrices that share x.
+static int forward_through_blocks(const W4Blocks& b, const float* x_dev, int M, int K, int ldx, int count, const void* const* tiled_dev,
+                                  float* const* y_dev, const int* N, const int* ldy, int use_pdl, cudaStream_t st) {
+  if (!b.blocks || (reinterpret_cast<uintptr_t>(b.blocks) & 255u)) return MLLMB200_INVALID_ARG;
+  cudaError_t e = b.form == kW4Stream ? launch_act_quant_mma(x_dev, M, K, ldx, b.blocks, b.hdr, use_pdl, st)
+                                      : launch_act_quant_blocks_f16(x_dev, M, b.m_pad, K, ldx, b.blocks, b.hdr, st, use_pdl, b.clear, b.clear_count);
+  if (e == cudaSuccess) e = w4a32_forward_blocks(b, M, K, count, tiled_dev, y_dev, N, ldy, use_pdl, st);
   return e == cudaSuccess ? MLLMB200_OK : cuda_fail(e);
 }
 
@@ -252,13 +278,11 @@ int mllmb200_w4a32_linear_forward_ex(const float* x_dev, const void* tiled_dev, 
   const bool fp16_scales = (kernel & kFlagFp16Scales) != 0;
   kernel &= 0xFF;
   if (kernel < 0 || kernel > 7) return MLLMB200_INVALID_ARG;
-  if (kernel == 5) {  // "fastest": the fp16 path or, above the rows of the default, the streaming kernel where they win
-    kernel = w4a32_gemm_tcf16_preferred(M, K, N) ? 4 : 0;
-    if (w4a32_gemm_stream_preferred(M, K, 1, &N))
-      return stream_forward(x_dev, M, K, ldx, 1, &tiled_dev, &y_dev, &N, &ldy, ws_dev, use_pdl, st);
+  if (kernel == 0 || kernel == 5) {
+    const W4Blocks b = w4a32_blocks_for(M, K, 1, &N, kernel | (fp16_scales ? kFlagFp16Scales : 0), ws_dev);
+    if (b.form != kW4None) return forward_through_blocks(b, x_dev, M, K, ldx, 1, &tiled_dev, &y_dev, &N, &ldy, use_pdl, st);
+    kernel = mllmb200_w4a32_select_kernel(M, K, N);
   }
-  const bool by_default = kernel == 0;
-  if (by_default) kernel = mllmb200_w4a32_select_kernel(M, K, N);
   if (kernel == 1) {  // single launch: x is quantized inside the GEMV, no workspace
     if (!w4a32_gemv_stream_supported(M, 1, &K, &N)) return MLLMB200_UNSUPPORTED;
     const cudaError_t e1 =
@@ -267,23 +291,14 @@ int mllmb200_w4a32_linear_forward_ex(const float* x_dev, const void* tiled_dev, 
   }
   if (kernel == 7) {  // streaming tensor-core GEMM for small batches: its own activation layout
     if (!w4a32_gemm_stream_supported(M, K, 1, &N)) return MLLMB200_UNSUPPORTED;
-    return stream_forward(x_dev, M, K, ldx, 1, &tiled_dev, &y_dev, &N, &ldy, ws_dev, use_pdl, st);
+    return forward_through_blocks(blocks_at(kW4Stream, M, K, 0, ws_dev), x_dev, M, K, ldx, 1, &tiled_dev, &y_dev, &N, &ldy, use_pdl, st);
   }
   if (kernel == 6 && !w4a32_gemv_supported(M, K, N)) return MLLMB200_UNSUPPORTED;
   if (kernel == 3 && !w4a32_gemm_tc_supported(M, K, N)) return MLLMB200_UNSUPPORTED;
-  if (kernel == 3 && by_default && M >= kChunkMinM && !(fp16_scales && int8_suits_fp16_scales(M, N)))
-    return chunk_forward(x_dev, M, K, ldx, 1, &tiled_dev, &y_dev, &N, &ldy, ws_dev, use_pdl, st);
   if (kernel == 4) {  // fp16 tensor-core path: its own activation layout
     if (!w4a32_gemm_tcf16_supported(M, K, N)) return MLLMB200_UNSUPPORTED;
-    if (!ws_dev || (reinterpret_cast<uintptr_t>(ws_dev) & 255u)) return MLLMB200_INVALID_ARG;
-    uint8_t* blocks = static_cast<uint8_t*>(ws_dev);
-    float2* hdr16 = reinterpret_cast<float2*>(blocks + ws_rec_bytes(M, K));
-    int* sync16 = reinterpret_cast<int*>(reinterpret_cast<uint8_t*>(hdr16) + align_up((size_t)M * sizeof(float2), 256));
-    cudaError_t e16 = launch_act_quant_blocks_f16(x_dev, M, w4a32_gemm_tcf16_m_pad(M, N), K, ldx, blocks, hdr16, st, use_pdl,
-                                                  sync16, kSplitSyncInts);
-    if (e16 == cudaSuccess)
-      e16 = launch_w4a32_gemm_tcf16(blocks, hdr16, tiled_dev, y_dev, M, K, N, ldy, st, use_pdl, sync16, kSplitSyncInts);
-    return e16 == cudaSuccess ? MLLMB200_OK : cuda_fail(e16);
+    return forward_through_blocks(blocks_at(kW4Tile, M, K, w4a32_gemm_tcf16_m_pad(M, N), ws_dev), x_dev, M, K, ldx, 1, &tiled_dev, &y_dev, &N, &ldy,
+                                  use_pdl, st);
   }
   uint8_t* a_rec;
   float2* a_hdr;
@@ -320,16 +335,13 @@ int mllmb200_w4a32_linear_forward_grouped(const float* x_dev, int M, int K, int 
                                                    (flags >> 8) & 1, static_cast<cudaStream_t>(stream));
     return e == cudaSuccess ? MLLMB200_OK : cuda_fail(e);
   }
-  int n_group = 0;
-  for (int i = 0; i < count; ++i) n_group += N[i];
-  // ("fastest" at 64 <= M: wide groups with a short K go to the fp16 tile GEMM further down)
-  const bool stream_fastest = (flags & 0xFF) == 5 && w4a32_gemm_stream_preferred(M, K, count, N);
-  const bool tile16_first = (flags & 0xFF) == 5 && count > 1 && w4a32_gemm_tcf16_preferred(M, K, n_group);
-  // small batch: one quantization, ONE streaming tensor-core launch
-  const bool stream_default = ((flags & 0xFF) == 0 || (flags & 0xFF) == 5) && M >= kStreamGemmMinM && M <= kStreamGemmMaxM &&
-                              w4a32_gemm_stream_supported(M, K, count, N);
-  if (stream_fastest || (stream_default && !tile16_first))
-    return stream_forward(x_dev, M, K, ldx, count, tiled_dev, y_dev, N, ldy, ws_dev, (flags >> 8) & 1, static_cast<cudaStream_t>(stream));
+  // Larger M: the matrices share ONE quantization of x and ONE launch, their panels or tiles side by side in the grid (q, k, v alone
+  // fill 16 + 2 + 2 tiles): of the streaming kernel, of gemm_tcf16.cu where the "fastest" policy (5) takes it, else of gemm_chunk.cu.
+  if ((flags & 0xFF) == 0 || (flags & 0xFF) == 5) {
+    const W4Blocks b = w4a32_blocks_for(M, K, count, N, flags & (0xFF | kFlagFp16Scales), ws_dev);
+    if (b.form != kW4None)
+      return forward_through_blocks(b, x_dev, M, K, ldx, count, tiled_dev, y_dev, N, ldy, (flags >> 8) & 1, static_cast<cudaStream_t>(stream));
+  }
   bool gemv = (flags & 0xFF) == 6;  // the two-launch path (quantization kernel + one-shot GEMV), kept for comparison
   for (int i = 0; i < count && gemv; ++i) gemv = w4a32_gemv_supported(M, K, N[i]);
   if ((flags & 0xFF) == 6 && !gemv) return MLLMB200_UNSUPPORTED;
@@ -341,39 +353,12 @@ int mllmb200_w4a32_linear_forward_grouped(const float* x_dev, int M, int K, int 
     cudaError_t e = launch_w4a32_gemv_grouped(a_rec, a_hdr, M, K, count, tiled_dev, y_dev, N, ldy, (flags >> 8) & 1, st);
     return e == cudaSuccess ? MLLMB200_OK : cuda_fail(e);
   }
-  // Larger M: the matrices share ONE quantization of x.  From M = 65 they also share ONE launch, their tiles side by
-  // side in the grid (q, k, v alone fill 16 + 2 + 2): of gemm_tcf16.cu where the "fastest" policy (5) takes it, else of
-  // gemm_chunk.cu.  Below, what the streaming kernel does not take runs as separate int8 tensor-core launches behind one
-  // quantization, or as ordinary forwards.
+  // What neither takes runs as separate int8 tensor-core launches behind one quantization, or as ordinary forwards.
   const int policy = flags & 0xFF;  // 0 auto, 5 fastest (as the kernel argument of linear_forward_ex)
   if (policy != 0 && policy != 5) return MLLMB200_INVALID_ARG;
   cudaStream_t st_grp = static_cast<cudaStream_t>(stream);
-  if (count > 1 && policy == 5 && M >= 64) {
-    bool all16 = true;
-    int n_sum = 0;
-    for (int i = 0; i < count; ++i) {
-      all16 = all16 && w4a32_gemm_tcf16_supported(M, K, N[i]);
-      n_sum += N[i];
-    }
-    all16 = all16 && w4a32_gemm_tcf16_preferred(M, K, n_sum);  // (the group's weight tiles ride in one grid)
-    if (all16) {
-      if (!ws_dev || (reinterpret_cast<uintptr_t>(ws_dev) & 255u)) return MLLMB200_INVALID_ARG;
-      uint8_t* blocks = static_cast<uint8_t*>(ws_dev);
-      float2* hdr = reinterpret_cast<float2*>(blocks + ws_rec_bytes(M, K));
-      const int nt = w4a32_gemm_tcf16_tile_grouped(M, count, N);
-      const int pdl = (flags >> 8) & 1;
-      int* sync = reinterpret_cast<int*>(reinterpret_cast<uint8_t*>(hdr) + align_up((size_t)M * sizeof(float2), 256));
-      cudaError_t e = launch_act_quant_blocks_f16(x_dev, M, (M + nt - 1) / nt * nt, K, ldx, blocks, hdr, st_grp, pdl, sync, kSplitSyncInts);
-      if (e == cudaSuccess)
-        e = launch_w4a32_gemm_tcf16_grouped(blocks, hdr, M, K, count, tiled_dev, y_dev, N, ldy, st_grp, 0, nullptr, pdl, sync,
-                                            kSplitSyncInts);
-      return e == cudaSuccess ? MLLMB200_OK : cuda_fail(e);
-    }
-  }
   bool all8 = count > 1;
   for (int i = 0; i < count; ++i) all8 = all8 && mllmb200_w4a32_select_kernel(M, K, N[i]) == 3;
-  if (all8 && M >= kChunkMinM)
-    return chunk_forward(x_dev, M, K, ldx, count, tiled_dev, y_dev, N, ldy, ws_dev, (flags >> 8) & 1, st_grp);
   if (all8) {
     if (!ws_dev || (reinterpret_cast<uintptr_t>(ws_dev) & 255u)) return MLLMB200_INVALID_ARG;
     uint8_t* blocks = static_cast<uint8_t*>(ws_dev);

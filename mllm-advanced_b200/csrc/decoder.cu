@@ -18,6 +18,7 @@
 #include "../../include/mllmb200.h"
 #include "decoder_state.h"
 #include "device_common.cuh"
+#include "linear_blocks.h"
 
 namespace mllmb200 {
 // persistent decode kernel (decoder_persistent.cu)
@@ -30,6 +31,8 @@ int persistent_phase_cycles(Decoder* d, long long* out, int capacity, int* nctas
 __global__ void add_rmsnorm_quant_kernel(const float*, const float*, const float*, float, int, float*, float*, uint8_t*,
                                          float2*, int);
 __global__ void silu_mul_quant_kernel(const float*, const float*, int, float*, uint8_t*, float2*, int);
+cudaError_t launch_add_rmsnorm_blocks(const float*, const float*, const float*, float, int, float*, int, const W4Blocks&, int, cudaStream_t);
+cudaError_t launch_silu_mul_blocks(const float*, const float*, int, int, const W4Blocks&, int, cudaStream_t);
 __global__ void embedding_kernel(const int*, const float*, int, float*);
 __global__ void rope_tables_kernel(float*, float*, int, int, float);
 template <int D>
@@ -194,6 +197,20 @@ static cudaError_t prompt_attention(bool tensor_cores, const float* q, const flo
                                       cache_k, cache_v, out, QD);
 }
 
+// h += delta, and the linears of the normalized rows of a prompt
+static int norm_linears(Decoder* d, const float* delta, const float* w, int n, int count, const void* const* tiled, float* const* y,
+                        const int* rows) {
+  const auto& c = d->cfg;
+  const W4Blocks b = w4a32_blocks_for(n, c.hidden, count, rows, 5, d->ws);
+  if (b.form == kW4None) {
+    DEC_CHECK(launch_pdl(add_rmsnorm_quant_kernel, dim3(n), dim3(256), 0, d->stream, d->h, delta, w, c.eps, c.hidden, d->h, d->xn, nullptr, nullptr, 1));
+    return mllmb200_w4a32_linear_forward_grouped(d->xn, n, c.hidden, c.hidden, count, tiled, y, rows, rows, d->ws, 5 | 0x100, d->stream);
+  }
+  DEC_CHECK(launch_add_rmsnorm_blocks(d->h, delta, w, c.eps, c.hidden, d->h, n, b, 1, d->stream));
+  DEC_CHECK(w4a32_forward_blocks(b, n, c.hidden, count, tiled, y, rows, rows, 1, d->stream));
+  return MLLMB200_OK;
+}
+
 // The prompt pass of the batch-1 decoder, writing keys / values into the given per-layer caches
 // ([kv_heads][max_ctx][D] each) and the sampled token and position into the given words: the decoder's own for
 // mllmb200_qwen2_prefill, a sequence's for the batched decoder (decoder_batch.cu).  Exactly one of tokens_dev
@@ -211,27 +228,31 @@ int prefill_into(Decoder* d, const int* tokens_dev, const float* embeds_dev, int
     DEC_CHECK(cudaMemcpyAsync(d->h, embeds_dev, (size_t)n * H * sizeof(float), cudaMemcpyDeviceToDevice, s));
   for (int l = 0; l < c.layers; ++l) {
     const Layer& L = d->layers[l];
-    DEC_CHECK(launch_pdl(add_rmsnorm_quant_kernel, dim3(n), dim3(256), 0, s, d->h, l == 0 ? nullptr : d->down, L.ln1, c.eps, H, d->h,
-                         d->xn, nullptr, nullptr, 1));
     {  // q, k, v share one quantization of the normalized rows
       const void* tw[3] = {L.w[kQ], L.w[kK], L.w[kV]};
       float* ty[3] = {d->q, d->k, d->v};
       const int tn[3] = {QD, KD, KD};
-      DEC_ST(mllmb200_w4a32_linear_forward_grouped(d->xn, n, H, H, 3, tw, ty, tn, tn, d->ws, 5 | 0x100, s));
+      DEC_ST(norm_linears(d, l == 0 ? nullptr : d->down, L.ln1, n, 3, tw, ty, tn));
     }
     DEC_CHECK(prompt_attention(n > kShortPrompt, d->q, d->k, d->v, n, c.q_heads, c.kv_heads, c.head_dim, d->sin_t, d->cos_t, d->zero, c.max_ctx,
                                cache_k[l], cache_v[l], d->kv_split, d->attn, s));
     DEC_ST(mllmb200_w4a32_linear_forward_ex(d->attn, L.w[kO], d->o, d->ws, n, QD, H, QD, H, 5 | 0x100 | L.flags[kO], s));
-    DEC_CHECK(launch_pdl(add_rmsnorm_quant_kernel, dim3(n), dim3(256), 0, s, d->h, d->o, L.ln2, c.eps, H, d->h, d->xn, nullptr, nullptr, 1));
     {  // gate and up likewise
       const void* tw[2] = {L.w[kGate], L.w[kUp]};
       float* ty[2] = {d->gate, d->up};
       const int tn[2] = {I, I};
-      DEC_ST(mllmb200_w4a32_linear_forward_grouped(d->xn, n, H, H, 2, tw, ty, tn, tn, d->ws, 5 | 0x100, s));
+      DEC_ST(norm_linears(d, d->o, L.ln2, n, 2, tw, ty, tn));
     }
-    DEC_CHECK(launch_pdl(silu_mul_quant_kernel, dim3(n), dim3(512), (size_t)I * sizeof(float), s, d->gate, d->up, I, d->act, nullptr,
-                         nullptr, 1));
-    DEC_ST(mllmb200_w4a32_linear_forward_ex(d->act, L.w[kDown], d->down, d->ws, n, I, H, I, H, 5 | 0x100 | L.flags[kDown], s));
+    const W4Blocks act = w4a32_blocks_for(n, I, 1, &H, 5 | L.flags[kDown], d->ws);
+    if (act.form != kW4None) {
+      const void* tw[1] = {L.w[kDown]};
+      DEC_CHECK(launch_silu_mul_blocks(d->gate, d->up, I, n, act, 1, s));
+      DEC_CHECK(w4a32_forward_blocks(act, n, I, 1, tw, &d->down, &H, &H, 1, s));
+    } else {
+      DEC_CHECK(launch_pdl(silu_mul_quant_kernel, dim3(n), dim3(512), (size_t)I * sizeof(float), s, d->gate, d->up, I, d->act, nullptr,
+                           nullptr, 1));
+      DEC_ST(mllmb200_w4a32_linear_forward_ex(d->act, L.w[kDown], d->down, d->ws, n, I, H, I, H, 5 | 0x100 | L.flags[kDown], s));
+    }
   }
   // only the last position feeds the sampler (the reference computes all rows and reads the last)
   const size_t last = (size_t)(n - 1) * H;

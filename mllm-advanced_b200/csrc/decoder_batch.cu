@@ -27,6 +27,7 @@
 #include "decoder_attn_body.cuh"
 #include "decoder_state.h"
 #include "device_common.cuh"
+#include "linear_blocks.h"
 
 #ifndef MLLMB200_BATCH_ATTN_CTAS_PER_SM
 #define MLLMB200_BATCH_ATTN_CTAS_PER_SM 4
@@ -40,6 +41,8 @@ namespace mllmb200 {
 __global__ void add_rmsnorm_quant_kernel(const float*, const float*, const float*, float, int, float*, float*, uint8_t*,
                                          float2*, int);
 __global__ void silu_mul_quant_kernel(const float*, const float*, int, float*, uint8_t*, float2*, int);
+cudaError_t launch_add_rmsnorm_blocks(const float*, const float*, const float*, float, int, float*, int, const W4Blocks&, int, cudaStream_t);
+cudaError_t launch_silu_mul_blocks(const float*, const float*, int, int, const W4Blocks&, int, cudaStream_t);
 __global__ void embedding_kernel(const int*, const float*, int, float*);
 __global__ void sample_advance_batched_kernel(const float2*, int, int*, int*, int*, int, const int*, int*);
 
@@ -486,6 +489,20 @@ bool balloc(BatchDecoder* b, T** p, size_t count) {
     if (s__ != MLLMB200_OK) return s__;     \
   } while (0)
 
+// h += delta, and the linears of the normalized rows
+int norm_linears(BatchDecoder* b, const float* delta, const float* w, int count, const void* const* tiled, float* const* y, const int* rows) {
+  const auto& c = b->base->cfg;
+  cudaStream_t s = b->base->stream;
+  const W4Blocks blocks = b->policy == 4 ? W4Blocks{} : w4a32_blocks_for(b->batch, c.hidden, count, rows, b->policy, b->ws);
+  if (blocks.form == kW4None) {
+    add_rmsnorm_quant_kernel<<<b->batch, 256, 0, s>>>(b->h, delta, w, c.eps, c.hidden, b->h, b->xn, nullptr, nullptr, 0);
+    return mllmb200_w4a32_linear_forward_grouped(b->xn, b->batch, c.hidden, c.hidden, count, tiled, y, rows, rows, b->ws, b->policy | 0x100, s);
+  }
+  BD_CHECK(launch_add_rmsnorm_blocks(b->h, delta, w, c.eps, c.hidden, b->h, b->batch, blocks, 1, s));
+  BD_CHECK(w4a32_forward_blocks(blocks, b->batch, c.hidden, count, tiled, y, rows, rows, 1, s));
+  return MLLMB200_OK;
+}
+
 int enqueue_batched_step(BatchDecoder* b) {
   Decoder* d = b->base;
   const auto& c = d->cfg;
@@ -495,13 +512,11 @@ int enqueue_batched_step(BatchDecoder* b) {
   embedding_kernel<<<B, 256, 0, s>>>(b->token, d->embedding, H, b->h);
   for (int l = 0; l < c.layers; ++l) {
     const Layer& L = d->layers[l];
-    add_rmsnorm_quant_kernel<<<B, 256, 0, s>>>(b->h, l == 0 ? nullptr : b->down, L.ln1, c.eps, H, b->h, b->xn, nullptr,
-                                               nullptr, 0);
     {
       const void* tw[3] = {L.w[kQ], L.w[kK], L.w[kV]};
       float* ty[3] = {b->q, b->k, b->v};
       const int tn[3] = {QD, KD, KD};
-      BD_ST(mllmb200_w4a32_linear_forward_grouped(b->xn, B, H, H, 3, tw, ty, tn, tn, b->ws, b->policy | 0x100, s));
+      BD_ST(norm_linears(b, l == 0 ? nullptr : b->down, L.ln1, 3, tw, ty, tn));
     }
     {
       const dim3 grid(b->attn_splits, c.kv_heads, B);
@@ -521,15 +536,21 @@ int enqueue_batched_step(BatchDecoder* b) {
           b->part_o, b->part_ml, b->pos, c.max_ctx, b->attn_chunk, b->attn_splits, c.q_heads, c.head_dim, b->attn);
     }
     BD_ST(mllmb200_w4a32_linear_forward_ex(b->attn, L.w[kO], b->o, b->ws, B, QD, H, QD, H, b->policy | 0x100 | L.flags[kO], s));
-    add_rmsnorm_quant_kernel<<<B, 256, 0, s>>>(b->h, b->o, L.ln2, c.eps, H, b->h, b->xn, nullptr, nullptr, 0);
     {
       const void* tw[2] = {L.w[kGate], L.w[kUp]};
       float* ty[2] = {b->gate, b->up};
       const int tn[2] = {I, I};
-      BD_ST(mllmb200_w4a32_linear_forward_grouped(b->xn, B, H, H, 2, tw, ty, tn, tn, b->ws, b->policy | 0x100, s));
+      BD_ST(norm_linears(b, b->o, L.ln2, 2, tw, ty, tn));
     }
-    silu_mul_quant_kernel<<<B, 512, (size_t)I * sizeof(float), s>>>(b->gate, b->up, I, b->act, nullptr, nullptr, 0);
-    BD_ST(mllmb200_w4a32_linear_forward_ex(b->act, L.w[kDown], b->down, b->ws, B, I, H, I, H, b->policy | 0x100 | L.flags[kDown], s));
+    const W4Blocks act = b->policy == 4 ? W4Blocks{} : w4a32_blocks_for(B, I, 1, &H, b->policy | L.flags[kDown], b->ws);
+    if (act.form != kW4None) {
+      const void* tw[1] = {L.w[kDown]};
+      BD_CHECK(launch_silu_mul_blocks(b->gate, b->up, I, B, act, 1, s));
+      BD_CHECK(w4a32_forward_blocks(act, B, I, 1, tw, &b->down, &H, &H, 1, s));
+    } else {
+      silu_mul_quant_kernel<<<B, 512, (size_t)I * sizeof(float), s>>>(b->gate, b->up, I, b->act, nullptr, nullptr, 0);
+      BD_ST(mllmb200_w4a32_linear_forward_ex(b->act, L.w[kDown], b->down, b->ws, B, I, H, I, H, b->policy | 0x100 | L.flags[kDown], s));
+    }
   }
   add_rmsnorm_quant_kernel<<<B, 256, 0, s>>>(b->h, b->down, d->final_norm, c.eps, H, nullptr, b->xn, nullptr, nullptr, 0);
   {

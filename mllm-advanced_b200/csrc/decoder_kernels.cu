@@ -4,6 +4,7 @@
 // also emit that linear's quantized activations (the records / blocks of act_quant.cu), so that in
 // decode the linears launch without a separate quantization kernel in front of them.
 #include "device_common.cuh"
+#include "linear_blocks.h"
 
 namespace mllmb200 {
 
@@ -241,6 +242,194 @@ __global__ void __launch_bounds__(kCombineThreads) attn_combine_quant_kernel(
   if (tid == 0) hdr[0] = make_float2(p.recip_scale, __int_as_float(-p.nzp));
   const int num_groups = (width + kGroup - 1) / kGroup;
   emit_records([&](int k) { return s_y[k]; }, width, num_groups, p, records);
+}
+
+// ---------------------------------------------------------------------------------------------
+// The same two operators in front of a linear of several rows: their values go straight into the operand blocks that the linear reads
+// (linear_blocks.h), the bits are those of the operator followed by the linear's own quantization.  One CTA per row of the
+// padded blocks; a row's pieces of 16 bytes are half sectors, the neighbouring row's CTA writes the other half.
+// Bound: the chain of loads, reductions and stores on short prompts, memory on documents: gate and up of 1900 tokens are 136 MB,
+// which L2 is still writing back (50 us for 306 MB).  us, width 1536 and feed-forward 8960, from the end of the GEMM before to
+// the last block, operator + quantization / here: silu, 1900 tokens 50 + 34.5 / 50, 512 10.2 + 9.5 / 15.7, 64 rows 4.3 + 3.4 / 7.6
+// (one launch less); norm 13 + 6.5 / 18, 4.6 + 3.9 / 6.6, 3.6 + 2.1 / 4.7.
+// ---------------------------------------------------------------------------------------------
+// eight values of K (left of them exist) of row m
+template <int FORM>
+__device__ __forceinline__ void put_item(const W4Blocks& o, int num_groups, int m, int item, const float (&f)[8], int left,
+                                         const ActQuantParams& p) {
+  if (FORM == kW4Stream) {
+    const int first = m / o.block_rows * o.block_rows, rows = min(o.block_rows, o.m_pad - first);
+    uint32_t lo = 0, hi = 0;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const uint32_t q = i < left ? (uint32_t)act_quant_value(f[i], p) & 0xFFu : 0u;
+      if (i & 1) hi |= q << (4 * (i - 1));
+      else lo |= q << (4 * i);
+    }
+    uint8_t* at = o.blocks + ((size_t)num_groups * first + (size_t)(item >> 2) * rows) * 32 + (size_t)(m - first) * 16 + (item & 3) * 4;
+    *reinterpret_cast<uint32_t*>(at) = lo;
+    *reinterpret_cast<uint32_t*>(at + (size_t)rows * 16) = hi;
+  } else {
+    __align__(16) __half h[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const int q = j < left ? act_quant_value(f[j], p) - p.nzp : 0;
+      h[(j < 4) ? 2 * j : 2 * (j - 4) + 1] = __int2half_rn(q);  // chunk order {0,4,1,5,2,6,3,7}
+    }
+    uint8_t* at = o.blocks + ((size_t)(item >> 2) * (o.m_pad >> 3) + (m >> 3)) * 512 + (m & 7) * 16 + (item & 3) * 128;
+    *reinterpret_cast<uint4*>(at) = *reinterpret_cast<const uint4*>(h);
+  }
+}
+// what the CTAs of either kernel do before and beside their row: the K-split counters, rows of padding
+template <int FORM>
+__device__ __forceinline__ bool blocks_row_is_padding(const W4Blocks& o, int num_groups, int m, int m_total) {
+  if (m == 0)
+    for (int i = threadIdx.x; i < o.clear_count; i += blockDim.x) o.clear[i] = 0;
+  if (m < m_total) return false;
+  const float zeros[8] = {};
+  for (int item = threadIdx.x; item < num_groups * 4; item += blockDim.x) put_item<FORM>(o, num_groups, m, item, zeros, 0, ActQuantParams{});
+  return true;
+}
+
+template <int FORM>
+__global__ void __launch_bounds__(kNormThreads) add_rmsnorm_blocks_kernel(const float* __restrict__ h_in, const float* __restrict__ delta,
+                                                                          const float* __restrict__ w, float eps, int hidden,
+                                                                          float* __restrict__ h_out, int m_total, W4Blocks out, int use_pdl) {
+  __shared__ float scratch[64];
+  __shared__ __align__(16) float s_y[kNormThreads * kNormMaxPerThread];
+  const int m = blockIdx.x, tid = threadIdx.x, num_groups = (hidden + kGroup - 1) / kGroup;
+  float v[kNormMaxPerThread], wv[kNormMaxPerThread];
+#pragma unroll
+  for (int i = 0; i < kNormMaxPerThread; ++i) {
+    const int k = tid + i * kNormThreads;
+    wv[i] = k < hidden ? w[k] : 0.0f;
+  }
+  if (use_pdl) {
+    pdl_launch_dependents();
+    pdl_wait_prior();
+  }
+  if (blocks_row_is_padding<FORM>(out, num_groups, m, m_total)) return;
+  const float* hi = h_in + (size_t)m * hidden;
+  float ss = 0.0f;
+#pragma unroll
+  for (int i = 0; i < kNormMaxPerThread; ++i) {
+    const int k = tid + i * kNormThreads;
+    v[i] = 0.0f;
+    if (k < hidden) {
+      v[i] = hi[k] + (delta ? delta[(size_t)m * hidden + k] : 0.0f);
+      if (h_out) h_out[(size_t)m * hidden + k] = v[i];
+      ss += v[i] * v[i];
+    }
+  }
+  const float rms = 1.0f / sqrtf(block_sum(ss, scratch) / (float)hidden + eps);
+  float mn = 3.402823466e+38f, mx = -3.402823466e+38f;
+#pragma unroll
+  for (int i = 0; i < kNormMaxPerThread; ++i) {
+    const int k = tid + i * kNormThreads;
+    if (k < hidden) {
+      const float y = v[i] * (wv[i] * rms);
+      s_y[k] = y;
+      mn = fminf(mn, y);
+      mx = fmaxf(mx, y);
+    }
+  }
+  block_minmax(mn, mx, scratch);  // contains the __syncthreads that publishes s_y
+  const ActQuantParams p = act_quant_params(mn, mx);
+  if (tid == 0) out.hdr[m] = make_float2(p.recip_scale, __int_as_float(-p.nzp));
+  for (int item = tid; item < num_groups * 4; item += kNormThreads) {
+    float f[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) f[j] = item * 8 + j < hidden ? s_y[item * 8 + j] : 0.0f;
+    put_item<FORM>(out, num_groups, m, item, f, hidden - item * 8, p);
+  }
+}
+
+// A thread keeps its ITEMS items of 8 products in registers between the minimum / maximum and the blocks.
+constexpr int kSiluBlockThreads = 384;
+template <int FORM, int ITEMS>
+__global__ void __launch_bounds__(kSiluBlockThreads) silu_mul_blocks_kernel(const float* __restrict__ gate, const float* __restrict__ up,
+                                                                            int inter, int m_total, W4Blocks out, int use_pdl) {
+  __shared__ float scratch[64];
+  if (use_pdl) {
+    pdl_launch_dependents();
+    pdl_wait_prior();
+  }
+  const int m = blockIdx.x, tid = threadIdx.x, num_groups = (inter + kGroup - 1) / kGroup;
+  if (blocks_row_is_padding<FORM>(out, num_groups, m, m_total)) return;
+  const float *g_row = gate + (size_t)m * inter, *u_row = up + (size_t)m * inter;
+  const bool vec = (inter & 3) == 0;  // (the rows start on 16 bytes)
+  float a[ITEMS][8], u[ITEMS][8];
+#pragma unroll
+  for (int i = 0; i < ITEMS; ++i) {
+    const int k0 = (tid + i * kSiluBlockThreads) * 8;
+    if (vec && k0 + 8 <= inter) {
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const float4 x = __ldcs(reinterpret_cast<const float4*>(g_row + k0) + h), y = __ldcs(reinterpret_cast<const float4*>(u_row + k0) + h);
+        a[i][4 * h] = x.x, a[i][4 * h + 1] = x.y, a[i][4 * h + 2] = x.z, a[i][4 * h + 3] = x.w;
+        u[i][4 * h] = y.x, u[i][4 * h + 1] = y.y, u[i][4 * h + 2] = y.z, u[i][4 * h + 3] = y.w;
+      }
+    } else {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        a[i][j] = k0 + j < inter ? g_row[k0 + j] : 0.0f;
+        u[i][j] = k0 + j < inter ? u_row[k0 + j] : 0.0f;
+      }
+    }
+  }
+  float mn = 3.402823466e+38f, mx = -3.402823466e+38f;
+#pragma unroll
+  for (int i = 0; i < ITEMS; ++i)
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      a[i][j] = (a[i][j] / (1.0f + expf(-a[i][j]))) * u[i][j];
+      if ((tid + i * kSiluBlockThreads) * 8 + j < inter) {
+        mn = fminf(mn, a[i][j]);
+        mx = fmaxf(mx, a[i][j]);
+      }
+    }
+  block_minmax(mn, mx, scratch);
+  const ActQuantParams p = act_quant_params(mn, mx);
+  if (tid == 0) out.hdr[m] = make_float2(p.recip_scale, __int_as_float(-p.nzp));
+#pragma unroll
+  for (int i = 0; i < ITEMS; ++i) {
+    const int item = tid + i * kSiluBlockThreads;
+    if (item < num_groups * 4) put_item<FORM>(out, num_groups, m, item, a[i], inter - item * 8, p);
+  }
+}
+
+template <class K, class... A>
+static cudaError_t launch_blocks_op(K kernel, int rows, int threads, int use_pdl, cudaStream_t s, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)rows, 1, 1);
+  cfg.blockDim = dim3((unsigned)threads, 1, 1);
+  cfg.stream = s;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = use_pdl ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, args..., use_pdl);
+}
+cudaError_t launch_add_rmsnorm_blocks(const float* h_in, const float* delta, const float* w, float eps, int hidden, float* h_out, int m,
+                                      const W4Blocks& out, int use_pdl, cudaStream_t s) {
+  return out.form == kW4Stream
+             ? launch_blocks_op(add_rmsnorm_blocks_kernel<kW4Stream>, out.m_pad, kNormThreads, use_pdl, s, h_in, delta, w, eps, hidden, h_out, m, out)
+             : launch_blocks_op(add_rmsnorm_blocks_kernel<kW4Tile>, out.m_pad, kNormThreads, use_pdl, s, h_in, delta, w, eps, hidden, h_out, m, out);
+}
+template <int FORM>
+static cudaError_t launch_silu_form(const float* gate, const float* up, int inter, int m, const W4Blocks& out, int use_pdl, cudaStream_t s) {
+  switch ((inter + 8 * kSiluBlockThreads - 1) / (8 * kSiluBlockThreads)) {
+    case 1: return launch_blocks_op(silu_mul_blocks_kernel<FORM, 1>, out.m_pad, kSiluBlockThreads, use_pdl, s, gate, up, inter, m, out);
+    case 2: return launch_blocks_op(silu_mul_blocks_kernel<FORM, 2>, out.m_pad, kSiluBlockThreads, use_pdl, s, gate, up, inter, m, out);
+    case 3: return launch_blocks_op(silu_mul_blocks_kernel<FORM, 3>, out.m_pad, kSiluBlockThreads, use_pdl, s, gate, up, inter, m, out);
+    case 4: return launch_blocks_op(silu_mul_blocks_kernel<FORM, 4>, out.m_pad, kSiluBlockThreads, use_pdl, s, gate, up, inter, m, out);
+    default: return cudaErrorInvalidValue;  // (the decoder takes widths up to 12000)
+  }
+}
+cudaError_t launch_silu_mul_blocks(const float* gate, const float* up, int inter, int m, const W4Blocks& out, int use_pdl, cudaStream_t s) {
+  return out.form == kW4Stream ? launch_silu_form<kW4Stream>(gate, up, inter, m, out, use_pdl, s)
+                               : launch_silu_form<kW4Tile>(gate, up, inter, m, out, use_pdl, s);
 }
 
 // Embedding lookup: row gather (mllm/Backends/Arm/Ops/LLMEmbeddingTokenOp.cpp:23-52).

@@ -532,6 +532,8 @@ static int ms_block_tiles(int m) {
   return (tiles + blocks - 1) / blocks;
 }
 
+int w4a32_gemm_stream_block_rows(int m) { return ms_block_tiles(m) * 8; }
+
 // ------------------------------------------------------------------------------------------------ activations
 // Per-row int8 quantization (the arithmetic of act_quant_records_kernel) into the layout above: for K-group g
 // and row m the four low words (even k of each 8-value item) at [g][m][0..16), the four high words (odd k) at

@@ -773,10 +773,4 @@ cudaError_t launch_w4a16_gemm_tcf16(const uint8_t* a_blocks, const void* tiled, 
   return launch_w4a16_gemm_tcf16_grouped(a_blocks, m, k, 1, &tiled, &y_f16, &n, &ldy, stream);
 }
 
-cudaError_t launch_w4a32_gemm_tcf16(const uint8_t* a_blocks, const float2* a_hdr, const void* tiled, float* y, int m, int k,
-                                    int n, int ldy, cudaStream_t stream, int use_pdl, int* split_sync, int split_sync_ints) {
-  return launch_w4a32_gemm_tcf16_grouped(a_blocks, a_hdr, m, k, 1, &tiled, &y, &n, &ldy, stream, 0, nullptr, use_pdl,
-                                         split_sync, split_sync_ints);
-}
-
 }  // namespace mllmb200

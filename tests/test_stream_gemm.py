@@ -110,3 +110,38 @@ def test_far_scales(scale):
     y = mb.linear_forward(torch.from_numpy(x).cuda(), mb.W4A32Weights.from_blob(blob)).cpu().numpy().astype(np.float64)
     mb.check_device_status()
     assert np.linalg.norm((y - want) / scale) <= 1e-6 * np.linalg.norm(want / scale)
+
+
+@pytest.mark.parametrize("m,policy", [(24, mb.KERNEL_AUTO), (70, mb.KERNEL_AUTO), (200, mb.KERNEL_FASTEST)])
+def test_halves_round_away_from_zero(m, policy):
+    """Rows with range -128 .. 127 (a scale of one) or half of it and zero points at either end: every x is an integer, a half or
+    next to one.  One quantum too far would be off by a hundred times the bar."""
+    orc, rng = Oracle(), np.random.default_rng(m)
+    k, n = 544, 64
+    x = rng.integers(-256, 255, (m, k)).astype(np.float32) / 2
+    x[1::4] = np.abs(x[1::4]) * np.float32(255 / 128)
+    x[2::4] = -np.abs(x[2::4])
+    x[3::4] = np.nextafter(x[3::4], np.float32(0) if m & 2 else np.float32(1e9), dtype=np.float32)
+    x[0::2, 5], x[0::4, 7], x[0::4, 9] = 0.5, -128, 127
+    blob = mb.quant_prepack((rng.standard_normal((n, k)) * 0.02).astype(np.float32))
+    w64 = _weights64(blob, mb.SCALE_BF16_TRUNC)[0]
+    y = mb.linear_forward(torch.from_numpy(x).cuda(), mb.W4A32Weights.from_blob(blob), kernel=policy).cpu().numpy()
+    mb.check_device_status()
+    bar = 40 * 2.0 ** -23 * _group_magnitudes(orc, x, w64)
+    assert (np.abs(y - _acts64(orc, x) @ w64.T) <= bar).all()
+
+
+def test_infinities_and_nan_in_a_row():
+    """A row's infinity takes its scale to zero, a NaN counts as zero; other rows do not notice."""
+    rng = np.random.default_rng(8)
+    wt = mb.W4A32Weights.from_blob(mb.quant_prepack((rng.standard_normal((64, 512)) * 0.02).astype(np.float32), np.ones(64, np.float32)))
+    for m, policy in ((24, mb.KERNEL_AUTO), (70, mb.KERNEL_AUTO), (200, mb.KERNEL_FASTEST)):
+        x = rng.standard_normal((m, 512)).astype(np.float32)
+        x[3, 17], x[5, 100] = np.inf, np.nan
+        zeroed = x.copy()
+        zeroed[5, 100] = 0
+        run = lambda v: mb.linear_forward(torch.from_numpy(v).cuda(), wt, kernel=policy).cpu().numpy()  # noqa: E731
+        got, want = run(x), run(zeroed)
+        mb.check_device_status()
+        rest = np.arange(m) != 3
+        assert np.array_equal(got[rest], want[rest]) and np.array_equal(got[3], np.ones(64, np.float32))
