@@ -262,14 +262,12 @@ __global__ void __launch_bounds__(256) act_quant_reflayout_kernel(const float* _
 template <int ROWS, int WARPS, int ITEMS>
 __global__ void __launch_bounds__(ROWS * WARPS * 32) act_quant_blocks_f16_kernel(
     const float* __restrict__ x, int m_total, int k, int ldx, int num_groups, int m8_pad, uint8_t* __restrict__ blocks,
-    float2* __restrict__ hdr, int use_pdl, int* __restrict__ clear_ints, int clear_count) {
+    float2* __restrict__ hdr, int* __restrict__ clear_ints, int clear_count) {
   __shared__ float s_mm[ROWS][WARPS][2];
-  if (use_pdl) {
-    // x may be the previous kernel's output, and that kernel may still be reading the blocks this one overwrites:
-    // nothing happens before it has finished; the kernel behind this one may set itself up meanwhile
-    pdl_launch_dependents();
-    pdl_wait_prior();
-  }
+  // x may be the previous kernel's output, and that kernel may still be reading the blocks this one overwrites:
+  // nothing happens before it has finished; the GEMM behind this kernel, a dependent launch, may set itself up meanwhile
+  pdl_launch_dependents();
+  pdl_wait_prior();
   // the K-split counters of the GEMM behind this kernel (it reads them only after this grid has finished)
   if (blockIdx.x == 0)
     for (int i = threadIdx.x; i < clear_count; i += blockDim.x) clear_ints[i] = 0;
@@ -372,7 +370,7 @@ static cudaError_t launch_blocks_f16_t(const float* x, int m, int m_pad, int k, 
     cfg.numAttrs = 1;
   }
   return cudaLaunchKernelEx(&cfg, act_quant_blocks_f16_kernel<ROWS, WARPS, ITEMS>, x, m, k, ldx, (k + kGroup - 1) / kGroup, m_pad / 8, blocks,
-                            hdr, use_pdl, clear_ints, clear_ints != nullptr ? clear_count : 0);
+                            hdr, clear_ints, clear_ints != nullptr ? clear_count : 0);
 }
 // m_pad: a multiple of 8
 cudaError_t launch_act_quant_blocks_f16(const float* x, int m, int m_pad, int k, int ldx, uint8_t* blocks, float2* hdr,

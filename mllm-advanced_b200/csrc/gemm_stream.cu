@@ -544,13 +544,10 @@ constexpr int kMsQuantThreads = 512;
 template <int ITEMS>
 __global__ void __launch_bounds__(kMsQuantThreads) act_quant_mma_kernel(const float* __restrict__ x, int m_total, int m_pad, int block_rows,
                                                                         int k, int ldx, int num_groups,
-                                                                        uint8_t* __restrict__ acts, float2* __restrict__ hdr,
-                                                                        int use_pdl) {
+                                                                        uint8_t* __restrict__ acts, float2* __restrict__ hdr) {
   __shared__ float scratch[64];
-  if (use_pdl) {
-    pdl_launch_dependents();
-    pdl_wait_prior();  // x may be the previous kernel's output, and that kernel may still read the blocks we overwrite
-  }
+  pdl_launch_dependents();  // the GEMM behind this kernel is always a dependent launch
+  pdl_wait_prior();  // x may be the previous kernel's output, and that kernel may still read the blocks we overwrite
   const int m = blockIdx.x, tid = threadIdx.x;
   const bool live = m < m_total;
   const float* row = x + (size_t)(live ? m : 0) * ldx;
@@ -751,8 +748,8 @@ cudaError_t launch_act_quant_mma(const float* x, int m, int k, int ldx, uint8_t*
     cfg.numAttrs = 1;
   }
   return num_groups * 4 <= kMsQuantThreads
-             ? cudaLaunchKernelEx(&cfg, act_quant_mma_kernel<1>, x, m, m_pad, ms_block_tiles(m) * 8, k, ldx, num_groups, acts, hdr, use_pdl)
-             : cudaLaunchKernelEx(&cfg, act_quant_mma_kernel<3>, x, m, m_pad, ms_block_tiles(m) * 8, k, ldx, num_groups, acts, hdr, use_pdl);
+             ? cudaLaunchKernelEx(&cfg, act_quant_mma_kernel<1>, x, m, m_pad, ms_block_tiles(m) * 8, k, ldx, num_groups, acts, hdr)
+             : cudaLaunchKernelEx(&cfg, act_quant_mma_kernel<3>, x, m, m_pad, ms_block_tiles(m) * 8, k, ldx, num_groups, acts, hdr);
 }
 
 template <int NT>

@@ -734,7 +734,7 @@ cudaError_t launch_w4a32_gemm_tcf16_grouped(const uint8_t* a_blocks, const float
 int w4a16_gemm_tcf16_tile_grouped(int m, int count, const int* n) {
   long long t128 = 0;
   for (int i = 0; i < count; ++i) t128 += (n[i] + 127) / 128;
-  return (m >= 256 && t128 * ((m + 255) / 256) >= 100) ? 256 : (m >= 128 ? 128 : 64);
+  return (m > 128 && t128 * ((m + 255) / 256) >= 100) ? 256 : (m >= 128 || (m > 64 && t128 >= 64) ? 128 : 64);  // as tf_tile_for
 }
 int w4a16_gemm_tcf16_tile(int m, int n) { return w4a16_gemm_tcf16_tile_grouped(m, 1, &n); }
 cudaError_t launch_w4a16_gemm_tcf16_grouped(const uint8_t* a_blocks, int m, int k, int count, const void* const* tiled,
@@ -744,6 +744,7 @@ cudaError_t launch_w4a16_gemm_tcf16_grouped(const uint8_t* a_blocks, int m, int 
   TfParams prm = {};
   prm.a_blocks = a_blocks;
   prm.a_hdr = nullptr;
+  prm.use_pdl = 1;  // (behind its quantization, which is launched in order)
   prm.m = m, prm.k = k;
   prm.num_groups = (k + kGroup - 1) / kGroup;
   prm.m8_pad = (m + nt - 1) / nt * nt / 8;

@@ -135,6 +135,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) a16_act_quant_blocks_f16_kernel(const T* __restrict__ x, int m_total, int k,
                                                                        int ldx, int num_groups, int m8_pad,
                                                                        uint8_t* __restrict__ blocks) {
+  pdl_launch_dependents();  // the GEMM behind this kernel is a dependent launch
   const int m = blockIdx.x;
   const bool live = m < m_total;
   const T* row = x + (size_t)(live ? m : 0) * ldx;
