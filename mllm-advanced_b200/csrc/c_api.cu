@@ -280,13 +280,14 @@ int mllmb200_w4a32_linear_forward_ex(const float* x_dev, const void* tiled_dev, 
   const bool fp16_scales = (kernel & kFlagFp16Scales) != 0;
   kernel &= 0xFF;
   if (kernel < 0 || kernel > 7) return MLLMB200_INVALID_ARG;
-  if (kernel == 0 || kernel == 5) {
+  const bool by_default = kernel == 0 || kernel == 5;
+  if (by_default) {
     const W4Blocks b = w4a32_blocks_for(M, K, 1, &N, kernel | (fp16_scales ? kFlagFp16Scales : 0), ws_dev);
     if (b.form != kW4None) return forward_through_blocks(b, x_dev, M, K, ldx, 1, &tiled_dev, &y_dev, &N, &ldy, use_pdl, st);
     kernel = mllmb200_w4a32_select_kernel(M, K, N);
   }
   if (kernel == 1) {  // single launch: x is quantized inside the GEMV, no workspace
-    if (!w4a32_gemv_stream_supported(M, 1, &K, &N)) return MLLMB200_UNSUPPORTED;
+    if (!by_default && !w4a32_gemv_stream_supported(M, 1, &K, &N)) return MLLMB200_UNSUPPORTED;
     const cudaError_t e1 =
         launch_w4a32_gemv_stream(1, &x_dev, &ldx, nullptr, nullptr, M, &K, &tiled_dev, &y_dev, &N, &ldy, use_pdl, st);
     return e1 == cudaSuccess ? MLLMB200_OK : cuda_fail(e1);

@@ -1,4 +1,5 @@
 import ctypes as C
+import functools
 import os
 
 import numpy as np
@@ -110,6 +111,7 @@ def tiled_size(n, k):
     return out.value
 
 
+@functools.lru_cache(maxsize=4096)  # a function of two numbers
 def workspace_size(m, k):
     out = C.c_size_t()
     _check(lib().mllmb200_w4a32_workspace_size(m, k, C.byref(out)), "workspace_size")
@@ -160,8 +162,10 @@ def blob_sections(blob):
 
 def _stream_ptr(stream):
     import torch
-    s = torch.cuda.current_stream() if stream is None else stream
-    return C.c_void_p(s.cuda_stream)
+    if stream is not None:
+        return C.c_void_p(stream.cuda_stream)
+    # torch.cuda.current_stream().cuda_stream without the Python objects around it (3.6 us of a call that takes 18 in all)
+    return C.c_void_p(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))
 
 
 class W4A32Weights:
@@ -201,7 +205,7 @@ def _workspace_for(m, k, device):
     """One cached workspace per device, grown on demand (the op keeps its own in the C++ backend)."""
     import torch
     need = workspace_size(m, k)
-    key = str(device)
+    key = device.index
     ws = _ws_cache.get(key)
     if ws is None or ws.numel() < need:
         ws = torch.empty(need, dtype=torch.uint8, device=device)
@@ -216,7 +220,7 @@ def linear_forward(x, weights, out=None, workspace=None, kernel=KERNEL_AUTO, str
     m, k = x.shape
     assert k == weights.k
     if out is None:
-        out = torch.empty((m, weights.n), dtype=torch.float32, device=x.device)
+        out = x.new_empty((m, weights.n))
     if workspace is None:
         workspace = _workspace_for(m, k, x.device)
     _check(lib().mllmb200_w4a32_linear_forward_ex(x.data_ptr(), weights.tiled.data_ptr(), out.data_ptr(),

@@ -2,6 +2,7 @@
 fp32 scale and zero term per group of 32, per-block int8 activations, fp16 output
 (reference project: KaiLinear_f16_qsi8d32p_qai4c32p_mxk_nxk, mllm/Backends/Arm/Kernels/kai_linear.cpp:680-951)."""
 import ctypes as C
+import functools
 
 import numpy as np
 
@@ -52,6 +53,7 @@ def tiled_size(n, k):
     return out.value
 
 
+@functools.lru_cache(maxsize=4096)  # a function of three numbers
 def workspace_size(m, k, n):
     out = C.c_size_t()
     _check(lib().mllmb200_w4a16_workspace_size(m, k, n, C.byref(out)), "w4a16_workspace_size")
@@ -89,9 +91,9 @@ def linear_forward(x, weights, out=None, workspace=None, stream=None, kernel=KER
     m, k = x.shape
     assert k == weights.k
     if out is None:
-        out = torch.empty((m, weights.n), dtype=torch.float16, device=x.device)
+        out = x.new_empty((m, weights.n), dtype=torch.float16)
     if workspace is None:
-        workspace = torch.empty(workspace_size(m, k, weights.n), dtype=torch.uint8, device=x.device)
+        workspace = x.new_empty((workspace_size(m, k, weights.n),), dtype=torch.uint8)
     _check(lib().mllmb200_w4a16_linear_forward_ex(x.data_ptr(), 1 if x.dtype == torch.float16 else 0,
                                                   weights.tiled.data_ptr(), out.data_ptr(), workspace.data_ptr(), m, k,
                                                   weights.n, x.stride(0), out.stride(0), kernel | (0x100 if pdl else 0),
