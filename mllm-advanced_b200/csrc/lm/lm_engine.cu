@@ -240,7 +240,7 @@ int create(Engine* e, const mllmb200_lm_layer* descs) {
   LM_CUDA(retention_configure());
   LM_CUDA(latent_configure());
   const size_t rows = c.max_rows, slots = c.max_seqs;
-  e->plane_rows = std::max(c.max_rows, 1024);
+  e->plane_rows = std::max(2 * c.max_rows, 1024);  // (a whole step of prompts can still split K in two)
   e->logit_rows = std::max(std::min(c.max_rows, 128), c.max_seqs);
   e->max_splits_ctx = (c.max_ctx + kMinDecodeChunk - 1) / kMinDecodeChunk;
   LM_OK(dalloc(e, &e->embed, (size_t)c.vocab * c.width));

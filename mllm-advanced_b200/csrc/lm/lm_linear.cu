@@ -85,14 +85,36 @@ __device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
   return *reinterpret_cast<const uint32_t*>(&h);
 }
 
-// eight gated pairs, the first of them columns (n, n + 1); pairs past N write zeros into the padding of the row
+// A whole sector: the lanes of an epilogue warp hold different rows, and two stores of 16 bytes would move it twice.
+// (p: 16-byte aligned at least)
+__device__ __forceinline__ void store_sector(void* p, const uint4& a, const uint4& b) {
+  if (reinterpret_cast<uintptr_t>(p) & 31u) {
+    static_cast<uint4*>(p)[0] = a;
+    static_cast<uint4*>(p)[1] = b;
+    return;
+  }
+  asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w), "r"(b.x), "r"(b.y),
+               "r"(b.z), "r"(b.w)
+               : "memory");
+}
+__device__ __forceinline__ uint4 words(float a, float b, float c, float d) {
+  return make_uint4(__float_as_uint(a), __float_as_uint(b), __float_as_uint(c), __float_as_uint(d));
+}
+
+// eight gated pairs, the first of them columns (n, n + 1); pairs past N are zeros (the padding of the row)
 template <int ACT>
-__device__ __forceinline__ void gate8(const Epi& e, int m, int n, int N, const float (&v)[16]) {
+__device__ __forceinline__ uint4 gate8(const Epi& e, int n, int N, const float (&v)[16]) {
   float a[8];
 #pragma unroll
   for (int i = 0; i < 8; ++i) a[i] = n + 2 * i < N ? gated_as<ACT>(e.limit, v[2 * i], v[2 * i + 1]) : 0.0f;
-  *reinterpret_cast<uint4*>(static_cast<__nv_bfloat16*>(e.act) + (size_t)m * e.ld_act + (n >> 1)) =
-      make_uint4(pack_bf16(a[0], a[1]), pack_bf16(a[2], a[3]), pack_bf16(a[4], a[5]), pack_bf16(a[6], a[7]));
+  return make_uint4(pack_bf16(a[0], a[1]), pack_bf16(a[2], a[3]), pack_bf16(a[4], a[5]), pack_bf16(a[6], a[7]));
+}
+template <int ACT>
+__device__ __forceinline__ void gate16(const Epi& e, int m, int n, int N, const float (&v0)[16], const float (&v1)[16]) {
+  __nv_bfloat16* to = static_cast<__nv_bfloat16*>(e.act) + (size_t)m * e.ld_act + (n >> 1);
+  const uint4 a = gate8<ACT>(e, n, N, v0);
+  if (n + 16 < N) store_sector(to, a, gate8<ACT>(e, n + 16, N, v1));  // (rows of act are multiples of 128 bytes, n of 32)
+  else *reinterpret_cast<uint4*>(to) = a;
 }
 
 // columns [n, n + 16) of row m (n a multiple of 16), bf16 outputs; FORM: see form_of
@@ -103,30 +125,39 @@ __device__ __forceinline__ void store16(const Epi& e, int m, int n, int N, const
     float* y = e.y + (size_t)split * e.plane + (size_t)m * e.ldy + n;
     if (n + 16 <= N && (e.ldy & 3) == 0) {
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
-        reinterpret_cast<float4*>(y)[i] =
-            make_float4(v[4 * i] * e.scale, v[4 * i + 1] * e.scale, v[4 * i + 2] * e.scale, v[4 * i + 3] * e.scale);
+      for (int i = 0; i < 2; ++i)
+        store_sector(y + 8 * i, words(v[8 * i] * e.scale, v[8 * i + 1] * e.scale, v[8 * i + 2] * e.scale, v[8 * i + 3] * e.scale),
+                     words(v[8 * i + 4] * e.scale, v[8 * i + 5] * e.scale, v[8 * i + 6] * e.scale, v[8 * i + 7] * e.scale));
     } else {
 #pragma unroll
       for (int i = 0; i < 16; ++i)
         if (n + i < N) y[i] = v[i] * e.scale;
     }
-  } else if (FORM == kFormScatter) {
+  } else {
     if (e.kind == kEpiQLatent && n >= e.q_end) {
       float4* y = reinterpret_cast<float4*>(e.y + (size_t)m * e.ldy + (n - e.q_end));
 #pragma unroll
       for (int i = 0; i < 4; ++i) y[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
-    } else {  // head sizes are multiples of 16: the chunk lies in one head
-      uint4* p = reinterpret_cast<uint4*>(qkv_ptr<__nv_bfloat16>(e, m, n));
-      p[0] = make_uint4(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]), pack_bf16(v[4], v[5]), pack_bf16(v[6], v[7]));
-      p[1] = make_uint4(pack_bf16(v[8], v[9]), pack_bf16(v[10], v[11]), pack_bf16(v[12], v[13]), pack_bf16(v[14], v[15]));
+    } else {  // head sizes are multiples of 16: the chunk lies in one head, and every head starts on 32 bytes
+      store_sector(qkv_ptr<__nv_bfloat16>(e, m, n),
+                   make_uint4(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]), pack_bf16(v[4], v[5]), pack_bf16(v[6], v[7])),
+                   make_uint4(pack_bf16(v[8], v[9]), pack_bf16(v[10], v[11]), pack_bf16(v[12], v[13]), pack_bf16(v[14], v[15])));
     }
-  } else if (e.act_kind == MLLMB200_LM_ACT_GELU) {
-    gate8<MLLMB200_LM_ACT_GELU>(e, m, n, N, v);
-  } else if (e.act_kind == MLLMB200_LM_ACT_SILU) {
-    gate8<MLLMB200_LM_ACT_SILU>(e, m, n, N, v);
+  }
+}
+// columns [n, n + 32) of row m (n a multiple of 32) from two halves of tensor memory
+template <int FORM>
+__device__ __forceinline__ void store32(const Epi& e, int m, int n, int N, const uint32_t (&r0)[16], const uint32_t (&r1)[16], int split) {
+  float v0[16], v1[16];
+#pragma unroll
+  for (int i = 0; i < 16; ++i) v0[i] = __uint_as_float(r0[i]), v1[i] = __uint_as_float(r1[i]);
+  if (FORM == kFormGate) {
+    if (e.act_kind == MLLMB200_LM_ACT_GELU) gate16<MLLMB200_LM_ACT_GELU>(e, m, n, N, v0, v1);
+    else if (e.act_kind == MLLMB200_LM_ACT_SILU) gate16<MLLMB200_LM_ACT_SILU>(e, m, n, N, v0, v1);
+    else gate16<MLLMB200_LM_ACT_CLAMPED>(e, m, n, N, v0, v1);
   } else {
-    gate8<MLLMB200_LM_ACT_CLAMPED>(e, m, n, N, v);
+    store16<FORM>(e, m, n, N, v0, split);
+    if (n + 16 < N) store16<FORM>(e, m, n + 16, N, v1, split);
   }
 }
 Form form_of(const Epi& e) { return e.kind == kEpiPlanes ? kFormPlanes : e.kind == kEpiGate ? kFormGate : kFormScatter; }
@@ -292,7 +323,6 @@ __global__ void __launch_bounds__(256) lm_gemm_f32_kernel(const float* __restric
 }
 
 // ------------------------------------------------------------------------------------------ tcgen05 GEMM
-constexpr int kTcThreads = 192;  // copy warp, MMA warp, four epilogue warps
 constexpr int kTileM = 128, kTileK = 64;
 constexpr int kABytes = kTileM * kTileK * 2;
 
@@ -302,6 +332,9 @@ struct TcShape {
   static constexpr int kStageBytes = kABytes + BN * kTileK * 2;
   static constexpr int kSmem = kStages * kStageBytes + 1024;
   static constexpr int kTmemCols = 2 * BN;
+  // two epilogue warps for 32 rows where the tile is wide enough: a warp's gated products and stores take longer than a short K loop
+  static constexpr int kEpiWarps = BN >= 64 ? 8 : 4, kEpiCols = BN / (kEpiWarps / 4);
+  static constexpr int kThreads = 64 + 32 * kEpiWarps;  // copy warp, MMA warp, epilogue
 };
 
 __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
@@ -319,7 +352,7 @@ __device__ __forceinline__ uint64_t swizzled_desc(uint32_t addr) {
 // GROUPED: the row tiles are those of `tiles`; whole tiles are copied through amap (boxes of 128 rows), the others through
 // amap16 (16 rows).  Weight tiles and boxes may reach into the next group: those sums are not stored.
 template <int BN, bool GROUPED, int FORM>
-__global__ void __launch_bounds__(kTcThreads, 1) lm_gemm_tc_kernel(const __grid_constant__ CUtensorMap amap,
+__global__ void __launch_bounds__(TcShape<BN>::kThreads, 1) lm_gemm_tc_kernel(const __grid_constant__ CUtensorMap amap,
                                                                    const __grid_constant__ CUtensorMap amap16,
                                                                    const __grid_constant__ CUtensorMap wmap, int a_box, int M, int N,
                                                                    int K, int splits, const int4* __restrict__ tiles,
@@ -342,7 +375,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) lm_gemm_tc_kernel(const __grid_
   constexpr int kWBox = BN < 128 ? 32 : 128;
   if (tid == 0) {
     for (int i = 0; i < S::kStages; ++i) mbar_init(&full[i], 1), mbar_init(&empty[i], 1);
-    for (int i = 0; i < 2; ++i) mbar_init(&acc_full[i], 1), mbar_init(&acc_empty[i], 4);
+    for (int i = 0; i < 2; ++i) mbar_init(&acc_full[i], 1), mbar_init(&acc_empty[i], S::kEpiWarps);
     gave_up = 0;
     mbar_fence_init();
   }
@@ -442,7 +475,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) lm_gemm_tc_kernel(const __grid_
   } else {
     if (GROUPED) grouped_start();
     else pdl_wait_prior();  // outputs may still be read by the kernel before
-    const int quarter = warp & 3;
+    const int quarter = warp & 3, c_begin = (warp - 2) / 4 * S::kEpiCols;
     int t = 0;
     for (int item = blockIdx.x; item < mt * nt * splits; item += gridDim.x, ++t) {
       const int buf = t & 1;
@@ -462,23 +495,13 @@ __global__ void __launch_bounds__(kTcThreads, 1) lm_gemm_tc_kernel(const __grid_
       if (m0 + quarter * 32 < m_end) {
         const uint32_t base = tmem + ((uint32_t)(quarter * 32) << 16) + buf * BN;
 #pragma unroll 1  // a kernel starts with a cold instruction cache: short code
-        for (int c = 0; c < BN; c += 32) {
+        for (int c = c_begin; c < c_begin + S::kEpiCols; c += 32) {
           if (n0 + c >= N) break;
           uint32_t r0[16], r1[16];
           tmem_ld16(base + c, r0);
           tmem_ld16(base + c + 16, r1);
           tmem_ld_wait();
-          float v[16];
-          if (m < m_end) {
-#pragma unroll
-            for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r0[i]);
-            store16<FORM>(e, m, n0 + c, N, v, split);
-            if (n0 + c + 16 < N) {
-#pragma unroll
-              for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r1[i]);
-              store16<FORM>(e, m, n0 + c + 16, N, v, split);
-            }
-          }
+          if (m < m_end) store32<FORM>(e, m, n0 + c, N, r0, r1, split);
           __syncwarp();
         }
       }
@@ -491,6 +514,186 @@ __global__ void __launch_bounds__(kTcThreads, 1) lm_gemm_tc_kernel(const __grid_
   __syncthreads();
   tc_fence_after();
   if (warp == 1) tmem_dealloc(tmem, S::kTmemCols);
+}
+
+// ------------------------------------------------------------------------------------------ tcgen05 GEMM of CTA pairs
+// 256 rows of x x 256 weight rows by two CTAs (cta_group::2): each loads its 128 rows of x and its 128 weight rows, one instruction
+// of CTA 0 multiplies what lies in both shared memories, and each CTA's tensor memory gets its 128 rows of the result.  What
+// bounds the kernel above with prompts is the way from L2: 48 KB a K tile of 64 for 128 x 256 sums at about 40 bytes a cycle
+// (1230 cycles; the tensor pipe needs 512).  A CTA of a pair loads 32 KB for as many.  us of a prompt of 1500 rows, single CTAs with
+// four epilogue warps and stores of 16 bytes / pairs with eight and of 32: 1536 -> 17920 gated 96 / 78 (pairs with the old
+// epilogue 97, with eight warps 79.5), 8960 -> 1536 48 / 38 (K in two), 1536 -> 6144 35 / 30, 1536 -> 2048 15.5 / 15.2,
+// 1536 -> 1536 14.6 / 13.  Now 1000 cycles a K tile.
+// Barriers: a CTA's own loads complete on its `full`; in CTA 1 the MMA warp hands that on to `peer_full` of CTA 0; commits arrive
+// in both CTAs; the epilogue warps of both free an accumulator in CTA 0.
+constexpr int kPairN = 256, kPairStages = 6, kPairStageBytes = 2 * kABytes;
+constexpr int kPairSmem = kPairStages * kPairStageBytes + 1024;
+constexpr int kPairEpiWarps = 8, kPairEpiCols = kPairN / (kPairEpiWarps / 4);  // epilogue warps, columns of one (and 32 rows)
+constexpr int kPairThreads = 64 + 32 * kPairEpiWarps;  // copy warp, MMA warp, epilogue
+
+// (The arrival hands on completed copies and tensor-memory reads, no stores: at cluster scope, with the memory barrier that
+// brings, it would cost more than it orders.)
+__device__ __forceinline__ void arrive_at_cta0(uint64_t* bar) {
+  asm volatile(
+      "{\n\t.reg .b32 r;\n\t"
+      "mapa.shared::cluster.u32 r, %0, 0;\n\t"
+      "mbarrier.arrive.shared::cluster.b64 _, [r];\n\t}" ::"r"(smem_u32(bar))
+      : "memory");
+}
+__device__ __forceinline__ void pair_commit(uint64_t* bar) {
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(smem_u32(bar)),
+               "h"((uint16_t)3)
+               : "memory");
+}
+__device__ __forceinline__ void pair_mma_f16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+
+// Work items as above, a row tile is 256 rows; pair c takes items c, c + pairs, ...
+template <int FORM>
+__global__ void __launch_bounds__(kPairThreads, 1) lm_gemm_pair_kernel(const __grid_constant__ CUtensorMap amap,
+                                                                     const __grid_constant__ CUtensorMap wmap, int M, int N, int K, int splits,
+                                                                     Epi e) {
+  extern __shared__ uint8_t tc_smem_raw[];
+  __shared__ uint64_t full[kPairStages], empty[kPairStages], peer_full[kPairStages], acc_full[2], acc_empty[2];
+  __shared__ uint32_t tmem_slot;
+  __shared__ volatile int gave_up;
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(tc_smem_raw) + 1023) & ~(uintptr_t)1023);
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
+  const int rank = (int)(blockIdx.x & 1), pair = (int)(blockIdx.x >> 1), pairs = (int)(gridDim.x >> 1);
+  const int mt = (M + 2 * kTileM - 1) / (2 * kTileM), nt = (N + kPairN - 1) / kPairN, kt = K / kTileK, items = mt * nt * splits;
+  if (tid == 0) {
+    for (int i = 0; i < kPairStages; ++i) mbar_init(&full[i], 1), mbar_init(&empty[i], 1), mbar_init(&peer_full[i], 1);
+    for (int i = 0; i < 2; ++i) mbar_init(&acc_full[i], 1), mbar_init(&acc_empty[i], 2 * kPairEpiWarps);
+    gave_up = 0;
+    mbar_fence_init();
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)), "r"(512u) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+  }
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync_all();  // the other CTA's barriers and tensor memory exist
+  tc_fence_after();
+  const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_slot, 0);
+  pdl_launch_dependents();
+  auto k_range = [&](int item, int& k0, int& k1) {
+    const int split = item / (mt * nt);
+    k0 = (int)((long long)kt * split / splits);
+    k1 = (int)((long long)kt * (split + 1) / splits);
+  };
+  if (warp == 0) {
+    if (elect_one_sync()) {
+      int it = 0, ahead = 0, st = 0;
+      uint32_t ph = 0;
+      bool ok = true;
+      auto load_w = [&](int stage, int k, int item) {
+        mbar_arrive_expect_tx(&full[stage], (uint32_t)kPairStageBytes);
+        tma_load_2d(smem + stage * kPairStageBytes + kABytes, &wmap, k * kTileK, (item / mt % nt) * kPairN + rank * 128, &full[stage]);
+      };
+      {  // the weights do not depend on the previous kernel, the activations do: fill the ring with weights first
+        int k0, k1;
+        k_range(pair, k0, k1);
+        for (; ahead < kPairStages && ahead < k1 - k0; ++ahead) load_w(ahead, k0 + ahead, pair);
+        pdl_wait_prior();
+      }
+      for (int item = pair; item < items && ok; item += pairs) {
+        int k0, k1;
+        k_range(item, k0, k1);
+        for (int k = k0; k < k1; ++k, ++it) {
+          if (it >= kPairStages && (gave_up || !mbar_wait_bounded(&empty[st], ph ^ 1u))) {
+            ok = false;
+            break;
+          }
+          if (it >= ahead) load_w(st, k, item);
+          tma_load_2d(smem + st * kPairStageBytes, &amap, k * kTileK, (item % mt) * 2 * kTileM + rank * kTileM, &full[st]);
+          if (++st == kPairStages) st = 0, ph ^= 1u;
+        }
+      }
+      if (!ok) gave_up = 1;
+      // nothing in flight when the CTA leaves: the last copies of every stage have landed
+      for (int i = it > kPairStages ? it - kPairStages : 0; !ok && i < it; ++i) mbar_wait_bounded(&full[i % kPairStages], (i / kPairStages) & 1);
+    }
+  } else if (warp == 1) {
+    const bool leader = elect_one_sync();
+    const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kPairN >> 3) << 17) | ((uint32_t)(2 * kTileM >> 4) << 24);
+    const uint32_t smem0 = (smem_u32(tc_smem_raw) + 1023u) & ~1023u;
+    int st = 0, t = 0;
+    uint32_t ph = 0;
+    bool ok = true;
+    for (int item = pair; item < items && ok; item += pairs, ++t) {
+      int k0, k1;
+      k_range(item, k0, k1);
+      const int buf = t & 1;
+      if (rank == 0 && t >= 2) ok = __all_sync(0xffffffffu, !gave_up && mbar_wait_bounded(&acc_empty[buf], ((t >> 1) & 1) ^ 1));
+      tc_fence_after();
+      for (int k = k0; k < k1 && ok; ++k) {
+        ok = __all_sync(0xffffffffu, !gave_up && mbar_wait_bounded(&full[st], ph));
+        if (!ok) break;
+        if (rank == 0) {
+          ok = __all_sync(0xffffffffu, !gave_up && mbar_wait_bounded(&peer_full[st], ph));
+          if (!ok) break;
+          tc_fence_after();
+          // (operands are values of the whole warp, outside of the elected lane's branch: see above)
+          const uint32_t a = smem0 + (uint32_t)(st * kPairStageBytes);
+          const uint64_t ad = swizzled_desc(a), bd = swizzled_desc(a + kABytes);
+          if (leader) {
+#pragma unroll
+            for (int j = 0; j < kTileK / 16; ++j)
+              pair_mma_f16(tmem + buf * kPairN, ad + j * 2, bd + j * 2, idesc, (k > k0 || j > 0) ? 1u : 0u);
+            pair_commit(&empty[st]);
+          }
+        } else if (leader) {
+          arrive_at_cta0(&peer_full[st]);
+        }
+        __syncwarp();
+        if (++st == kPairStages) st = 0, ph ^= 1u;
+      }
+      if (ok && rank == 0 && leader) pair_commit(&acc_full[buf]);
+      __syncwarp();
+    }
+    if (!ok) gave_up = 1;
+  } else {
+    pdl_wait_prior();  // outputs may still be read by the kernel before
+    const int quarter = warp & 3, c_begin = (warp - 2) / 4 * kPairEpiCols;
+    int t = 0;
+    for (int item = pair; item < items; item += pairs, ++t) {
+      const int buf = t & 1;
+      if (gave_up || !mbar_wait_bounded(&acc_full[buf], (t >> 1) & 1)) {
+        gave_up = 1;
+        break;
+      }
+      tc_fence_after();
+      const int n0 = (item / mt % nt) * kPairN, split = item / (mt * nt);
+      const int m0 = (item % mt) * 2 * kTileM + rank * kTileM + quarter * 32, m = m0 + lane;
+      if (m0 < M) {
+        const uint32_t base = tmem + ((uint32_t)(quarter * 32) << 16) + buf * kPairN;
+#pragma unroll 1
+        for (int c = c_begin; c < c_begin + kPairEpiCols; c += 32) {
+          if (n0 + c >= N) break;
+          uint32_t r0[16], r1[16];
+          tmem_ld16(base + c, r0);
+          tmem_ld16(base + c + 16, r1);
+          tmem_ld_wait();
+          if (m < M) store32<FORM>(e, m, n0 + c, N, r0, r1, split);
+          __syncwarp();
+        }
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) arrive_at_cta0(&acc_empty[buf]);
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync_all();  // nobody frees tensor memory or leaves while the other still uses it
+  tc_fence_after();
+  if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
 }
 
 // ------------------------------------------------------------------------------------------ packing
@@ -532,10 +735,18 @@ int encode(CUtensorMap* map, const void* base, int rows, int k, int box_rows) {
              : MLLMB200_CUDA_ERROR;
 }
 
-// Tile width and K splits with the smallest estimated time: waves x (K tiles x cycles per K tile + fixed cost).
-void choose_tile(int M, int mt, int a_rows, int N, int K, int max_splits, int* bn_out, int* splits_out) {
+// Tile width (kPairTile: 256 x 256 by pairs of CTAs) and K splits with the smallest estimated time: waves x (K tiles x cycles per
+// K tile + fixed cost).
+constexpr int kPairTile = 512;
+void choose_tile(int M, int mt, int a_rows, int N, int K, int max_splits, bool pairs, int* bn_out, int* splits_out) {
   const int kt = K / kTileK;
   double best = 1e30;
+  for (int s = 1; pairs && s <= max_splits && s <= kt; ++s) {
+    const long long items = (long long)((M + 255) / 256) * ((N + 255) / 256) * s;
+    const double waves = (double)((items + kSms / 2 - 1) / (kSms / 2));
+    const double t = waves * (((kt + s - 1) / s) * 820.0 + 600.0 + 6.0 * 256) + 1200.0 + (s - 1) * (150.0 + 8.0 * M * N / 2600.0);
+    if (t < best) best = t, *bn_out = kPairTile, *splits_out = s;
+  }
   for (int bn : {256, 128, 64, 32}) {
     const int nt = (N + bn - 1) / bn;
     for (int s = 1; s <= max_splits && s <= kt; ++s) {
@@ -554,10 +765,10 @@ cudaError_t launch_tc_form(cudaStream_t s, const Linear& w, const ActMap& am, in
   const int nt = (w.n + BN - 1) / BN;
   const CUtensorMap& wmap = BN < 128 ? w.map32 : w.map128;
   if (g)
-    return launch_pdl(lm_gemm_tc_kernel<BN, true, FORM>, dim3(std::min(g->max_tiles * nt * splits, kSms)), dim3(kTcThreads), TcShape<BN>::kSmem,
+    return launch_pdl(lm_gemm_tc_kernel<BN, true, FORM>, dim3(std::min(g->max_tiles * nt * splits, kSms)), dim3(TcShape<BN>::kThreads), TcShape<BN>::kSmem,
                       s, am.map128, am.map16, wmap, 128, M, w.n, w.k, splits, g->tiles, g->n_tiles, g->max_tiles, e);
   const int mt = (M + kTileM - 1) / kTileM;
-  return launch_pdl(lm_gemm_tc_kernel<BN, false, FORM>, dim3(std::min(mt * nt * splits, kSms)), dim3(kTcThreads), TcShape<BN>::kSmem, s,
+  return launch_pdl(lm_gemm_tc_kernel<BN, false, FORM>, dim3(std::min(mt * nt * splits, kSms)), dim3(TcShape<BN>::kThreads), TcShape<BN>::kSmem, s,
                     M >= kTileM ? am.map128 : am.map16, am.map16, wmap, M >= kTileM ? 128 : 16, M, w.n, w.k, splits, nullptr, nullptr, 0, e);
 }
 template <int BN>
@@ -566,6 +777,36 @@ cudaError_t launch_tc(cudaStream_t s, const Linear& w, const ActMap& am, int M, 
   return f == kFormPlanes ? launch_tc_form<BN, kFormPlanes>(s, w, am, M, splits, g, e)
          : f == kFormGate ? launch_tc_form<BN, kFormGate>(s, w, am, M, splits, g, e)
                           : launch_tc_form<BN, kFormScatter>(s, w, am, M, splits, g, e);
+}
+template <int FORM>
+cudaError_t launch_pair_form(cudaStream_t s, const Linear& w, const ActMap& am, int M, int splits, const Epi& e) {
+  const int items = (M + 255) / 256 * ((w.n + 255) / 256) * splits;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)std::min(2 * items, kSms), 1, 1);
+  cfg.blockDim = dim3(kPairThreads, 1, 1);
+  cfg.dynamicSmemBytes = kPairSmem;
+  cfg.stream = s;
+  cudaLaunchAttribute attrs[2];
+  attrs[0].id = cudaLaunchAttributeClusterDimension;
+  attrs[0].val.clusterDim.x = 2;
+  attrs[0].val.clusterDim.y = attrs[0].val.clusterDim.z = 1;
+  attrs[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attrs[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attrs;
+  cfg.numAttrs = 2;
+  ++g_launches;
+  return cudaLaunchKernelEx(&cfg, lm_gemm_pair_kernel<FORM>, am.map128, w.map128, M, w.n, w.k, splits, e);
+}
+cudaError_t launch_pair(cudaStream_t s, const Linear& w, const ActMap& am, int M, int splits, const Epi& e) {
+  const Form f = form_of(e);
+  return f == kFormPlanes ? launch_pair_form<kFormPlanes>(s, w, am, M, splits, e)
+         : f == kFormGate ? launch_pair_form<kFormGate>(s, w, am, M, splits, e)
+                          : launch_pair_form<kFormScatter>(s, w, am, M, splits, e);
+}
+cudaError_t configure_pair() {
+  cudaError_t r = cudaFuncSetAttribute(lm_gemm_pair_kernel<kFormPlanes>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmem);
+  if (r == cudaSuccess) r = cudaFuncSetAttribute(lm_gemm_pair_kernel<kFormScatter>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmem);
+  return r != cudaSuccess ? r : cudaFuncSetAttribute(lm_gemm_pair_kernel<kFormGate>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmem);
 }
 template <int BN, int FORM>
 cudaError_t configure_tc() {
@@ -618,6 +859,7 @@ cudaError_t linear_configure() {
   if (r == cudaSuccess) r = configure_tc_forms<128>();
   if (r == cudaSuccess) r = configure_tc_forms<64>();
   if (r == cudaSuccess) r = configure_tc_forms<32>();
+  if (r == cudaSuccess) r = configure_pair();
   if (r == cudaSuccess) r = configure_gemv<float>();
   if (r == cudaSuccess) r = configure_gemv<__nv_bfloat16>();
   return r;
@@ -654,8 +896,9 @@ int launch_linear(cudaStream_t s, bool f32, const Linear& w, const ActMap& am, c
                    static_cast<const float*>(x), w.w, M, w.n, w.k, nullptr, nullptr, e);
   } else {
     int bn = 32;
-    choose_tile(M, (M + kTileM - 1) / kTileM, M >= kTileM ? kTileM : pad_to(M, 16), w.n, w.k, e.kind == kEpiPlanes ? max_splits : 1, &bn, &splits);
-    r = launch_tc_any(s, bn, w, am, M, splits, nullptr, e);
+    choose_tile(M, (M + kTileM - 1) / kTileM, M >= kTileM ? kTileM : pad_to(M, 16), w.n, w.k, e.kind == kEpiPlanes ? max_splits : 1,
+                M >= 2 * kTileM, &bn, &splits);
+    r = bn == kPairTile ? launch_pair(s, w, am, M, splits, e) : launch_tc_any(s, bn, w, am, M, splits, nullptr, e);
   }
   return r == cudaSuccess ? splits : -1;
 }
@@ -671,7 +914,8 @@ int launch_linear_groups(cudaStream_t s, bool f32, const Linear& w, const ActMap
   } else {
     int bn = 32;
     const int per = (g.rows + g.likely_tiles - 1) / g.likely_tiles;
-    choose_tile(g.rows, g.likely_tiles, std::min(kTileM, pad_to(per, 16)), w.n, w.k, e.kind == kEpiPlanes ? max_splits : 1, &bn, &splits);
+    choose_tile(g.rows, g.likely_tiles, std::min(kTileM, pad_to(per, 16)), w.n, w.k, e.kind == kEpiPlanes ? max_splits : 1,
+                false, &bn, &splits);
     r = launch_tc_any(s, bn, w, am, g.rows, splits, &g, e);
   }
   return r == cudaSuccess ? splits : -1;
