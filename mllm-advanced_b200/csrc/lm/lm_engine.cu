@@ -660,6 +660,7 @@ NormArgs norm_args(Engine* e, const StepCtx& t, const Stream& r, const float* g_
   a.entries = t.entry;
   a.row_entry = t.row_entry;
   a.rows_per_cta = 1;
+  a.single = t.single;
   return a;
 }
 

@@ -37,21 +37,49 @@ __device__ __forceinline__ void store4(__nv_bfloat16* p, const float4& v) {
   *reinterpret_cast<uint2*>(p) = make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
 }
 
-// columns [c, c + 4) of a row of the sublayer output
-__device__ __forceinline__ float4 load_delta(const Delta& d, int row, int c) {
-  if (!d.mix_w) {
-    const float* p = d.p + (size_t)row * d.ldx + c;
-    float4 v = *reinterpret_cast<const float4*>(p);
-    for (int i = 1; i < d.planes; ++i) v = fma4(1.0f, *reinterpret_cast<const float4*>(p + i * d.plane), v);
-    return v;
-  }
+// columns [c, c + 4) of a row of the sublayer output.  Four planes, or the rows of four experts, are requested before the first is
+// added (in order): a row by itself is a chain of latencies.
+__device__ __forceinline__ float4 load_planes(const Delta& d, const float* p) {
   float4 v = make_float4(0, 0, 0, 0);
-  for (int k = 0; k < d.top; ++k) {
-    const int pair = row * d.top + k;
-    const float* p = d.p + (size_t)(d.mix_row ? d.mix_row[pair] : pair) * d.ldx + c;
-    float4 y = *reinterpret_cast<const float4*>(p);
-    for (int i = 1; i < d.planes; ++i) y = fma4(1.0f, *reinterpret_cast<const float4*>(p + i * d.plane), y);
-    v = fma4(d.mix_w[pair], y, v);
+  for (int i0 = 0; i0 < d.planes; i0 += 4) {
+    float4 q[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (i0 + j < d.planes) q[j] = *reinterpret_cast<const float4*>(p + (i0 + j) * d.plane);
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (i0 + j < d.planes) v = i0 + j == 0 ? q[j] : fma4(1.0f, q[j], v);
+  }
+  return v;
+}
+__device__ __forceinline__ float4 load_delta(const Delta& d, int row, int c) {
+  if (!d.mix_w) return load_planes(d, d.p + (size_t)row * d.ldx + c);
+  float4 v = make_float4(0, 0, 0, 0);
+  for (int k0 = 0; k0 < d.top; k0 += 4) {
+    float w[4];
+    const float* p[4];
+    float4 y[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int pair = row * d.top + min(k0 + j, d.top - 1);
+      w[j] = d.mix_w[pair];
+      p[j] = d.p + (size_t)(d.mix_row ? d.mix_row[pair] : pair) * d.ldx + c;
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (k0 + j < d.top) y[j] = *reinterpret_cast<const float4*>(p[j]);
+    for (int i = 1; i < d.planes; ++i) {
+      float4 q[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (k0 + j < d.top) q[j] = *reinterpret_cast<const float4*>(p[j] + i * d.plane);
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (k0 + j < d.top) y[j] = fma4(1.0f, q[j], y[j]);
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (k0 + j < d.top) v = fma4(w[j], y[j], v);
   }
   return v;
 }
@@ -146,6 +174,76 @@ __global__ void __launch_bounds__(kNormThreads) lm_norm_kernel(NormArgs a) {
         for (int j = 0; j + e.count < keep; ++j)
           store4(new_tail + (size_t)j * a.ldx + c * 4, *reinterpret_cast<const float4*>(old_tail + (size_t)(j + e.count) * a.ldx + c * 4));
     }
+  }
+}
+
+// The same for a decode step: every row is one token of a sequence of its own, so the rows in front of it come from the tail.  Bound
+// by the chain of what has to be read; everything is requested as soon as its address is known, the weights before
+// griddepcontrol.wait.  Batch of 32, width 2048, behind the planes of a linear, from the end of the kernel before: 5.1 us with a
+// convolution, where the kernel above takes 10.3.
+constexpr int kSingleTaps = 4;
+template <class T, int NV>
+__global__ void __launch_bounds__(kNormThreads) lm_norm_single_kernel(NormArgs a) {
+  __shared__ float scratch[32];
+  pdl_launch_dependents();
+  const int tid = threadIdx.x, nv = a.ldx >> 2, t = blockIdx.x, keep = a.taps - 1;
+  const float4 zero = make_float4(0, 0, 0, 0);
+  const float g_pre = *a.g_pre, g_post = a.delta.p ? *a.g_post : 0.0f, inv_w = 1.0f / (float)a.width;
+  float4 w[kSingleTaps][NV];  // w[s]: of the row s rows ago
+#pragma unroll
+  for (int s = 0; s < kSingleTaps; ++s)
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+      const int c = tid + i * kNormThreads;
+      w[s][i] = s < a.taps && c < nv ? __ldg(reinterpret_cast<const float4*>(a.conv_w + (size_t)(keep - s) * a.ldx) + c) : zero;
+    }
+  pdl_wait_prior();
+  Entry e{};
+  if (a.taps) e = a.entries[a.row_entry[t]];
+  const int src = a.gather ? a.gather[t] : t;
+  float4 x[NV], d[NV], h[kSingleTaps][NV];  // h[s]: the normed row s rows ago
+#pragma unroll
+  for (int i = 0; i < NV; ++i) {
+    const int c = tid + i * kNormThreads;
+    x[i] = c < nv ? reinterpret_cast<const float4*>(a.x_in + (size_t)src * a.ldx)[c] : zero;
+    d[i] = a.delta.p && c < nv ? load_delta(a.delta, src, c * 4) : zero;
+  }
+  const float* old_tail = a.tail + ((size_t)e.slot * 2 + e.tail) * keep * a.ldx;
+  float* new_tail = a.tail + ((size_t)e.slot * 2 + (e.tail ^ 1)) * keep * a.ldx;
+#pragma unroll
+  for (int s = 1; s < kSingleTaps; ++s)
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+      const int c = tid + i * kNormThreads;
+      h[s][i] = s <= keep && c < nv ? *reinterpret_cast<const float4*>(old_tail + (size_t)(keep - s) * a.ldx + c * 4) : zero;
+    }
+  if (a.delta.p) {
+    float ss = 0.0f;
+#pragma unroll
+    for (int i = 0; i < NV; ++i) ss += dot4(d[i]);
+    const float r = g_post / sqrtf(block_sum(ss, scratch) * inv_w + a.eps);
+#pragma unroll
+    for (int i = 0; i < NV; ++i) x[i] = fma4(r, d[i], x[i]);
+  }
+  float ss = 0.0f;
+#pragma unroll
+  for (int i = 0; i < NV; ++i) ss += dot4(x[i]);
+  const float r = g_pre / sqrtf(block_sum(ss, scratch) * inv_w + a.eps);
+#pragma unroll
+  for (int i = 0; i < NV; ++i) {
+    const int c = tid + i * kNormThreads;
+    if (c >= nv) continue;
+    if (a.x_out) store4(a.x_out + (size_t)t * a.ldx + c * 4, x[i]);
+    h[0][i] = fma4(r, x[i], zero);
+    float4 y = h[0][i];
+#pragma unroll
+    for (int s = 0; s < kSingleTaps; ++s)
+      if (s < a.taps && s <= e.pos0)  // not before the start of the sequence
+        y = make_float4(fmaf(w[s][i].x, h[s][i].x, y.x), fmaf(w[s][i].y, h[s][i].y, y.y), fmaf(w[s][i].z, h[s][i].z, y.z), fmaf(w[s][i].w, h[s][i].w, y.w));
+    store4(static_cast<T*>(a.out) + (size_t)t * a.ldx + c * 4, y);
+#pragma unroll
+    for (int s = 0; s < kSingleTaps - 1; ++s)  // the newest row behind the ones that stay
+      if (s < keep) store4(new_tail + (size_t)(keep - 1 - s) * a.ldx + c * 4, h[s][i]);
   }
 }
 
@@ -314,6 +412,10 @@ cudaError_t launch_norm_t(cudaStream_t s, const NormArgs& a) {
     return launch_norm_rows<T, 32>(s, a);
   }
   const int per = (a.ldx / 4 + kNormThreads - 1) / kNormThreads;
+  // (two float4 columns a thread: more do not fit the registers with all that is in flight)
+  if (a.single && per <= 2 && a.taps <= kSingleTaps && a.taps != 1)
+    return per <= 1 ? launch_pdl(lm_norm_single_kernel<T, 1>, dim3(a.rows), dim3(kNormThreads), 0, s, a)
+                    : launch_pdl(lm_norm_single_kernel<T, 2>, dim3(a.rows), dim3(kNormThreads), 0, s, a);
   if (per <= 1) return launch_norm_nv<T, 1>(s, a);
   if (per <= 2) return launch_norm_nv<T, 2>(s, a);
   if (per <= 4) return launch_norm_nv<T, 4>(s, a);

@@ -160,6 +160,7 @@ struct NormArgs {
   const Entry* entries;
   const int* row_entry;
   int rows_per_cta;
+  bool single;  // every row is the only one of its sequence
 };
 
 // launchers -----------------------------------------------------------------------------------

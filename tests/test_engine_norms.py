@@ -1,0 +1,37 @@
+"""The engine's norms with an input convolution: many rows a step (shared memory's rows, shares of one and two tokens, the rows in front
+of a block recomputed) and one token a sequence, over taps and widths at the edges of what a thread and a warp hold."""
+import os
+import sys
+
+import numpy as np
+import pytest
+
+pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+sys.path.insert(0, os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "oracle"))
+import lm_models as M  # noqa: E402
+import vupuzen_oracle as V  # noqa: E402
+from lm_case import Case  # noqa: E402
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("width,taps", [(72, 4), (1024, 2), (1032, 3), (1536, 4), (2048, 3), (2056, 4), (2560, 1)])
+def test_convolution_in_steps(width, taps, dtype, tmp_path):
+    cfg = M.config(width, 120, [M.layer("attention", M.attention(2, 1, 32, 32, 25), 64), M.layer("attention", M.attention(2, 2, 32, 16, 30))], taps=taps)
+    w = M.weights(cfg, 5)
+    c = Case(M.write(tmp_path / "m", cfg, w), V, cfg, w, dtype, max_seqs=6, max_ctx=400, max_rows=720)
+    toks = [c.tokens(400, seed=i) for i in range(6)]
+    want = [c.oracle(t) for t in toks]
+    at, slots = [0] * 6, [c.model.acquire() for _ in toks]
+    got = [[] for _ in toks]
+    # shares of a step: many rows (and a new sequence of one), short ones in front of and behind long ones, decode, and so on
+    for counts in ([1, 300, 2, 1, 60, 3], [1] * 6, [1] * 6, [1, 1, 330, 2, 1, 13], [1] * 6, [31, 7, 1, 300, 1, 300], [1] * 6):
+        part = [(s, t[a:a + n]) for s, t, a, n in zip(slots, toks, at, counts)]
+        rows = c.model.step(part, list(range(sum(counts))))
+        for i, n in enumerate(counts):
+            got[i].append(rows[sum(counts[:i]):sum(counts[:i + 1])])
+            at[i] += n
+    c.model.check_device_status()
+    for g, o, a in zip(got, want, at):
+        c.check(np.concatenate(g), o[:a])
+    c.model.close()
