@@ -267,33 +267,46 @@ __device__ __forceinline__ void warp_delta(const Delta& d, int row, int lane, in
 }
 
 // The same for many rows: a warp per row for the sums (no block barrier inside), then - with a convolution - the threads
-// sweep the CTA's rows column by column with the last TW - 1 rows of h in registers.  x' of the CTA's own rows is read
-// back from x_out (or x_in when there is nothing to fold in), that of the rows in front of them from shared memory.
-constexpr int kRowsThreads = 384, kRowsWarps = kRowsThreads / 32;  // rows a CTA handles at once, the recomputed ones included
+// sweep the CTA's rows column by column with the last three rows of h in registers.  All rows of h, the recomputed ones in
+// front of the CTA's own included, wait in shared memory.  A row is its warp's latency, so that of the stream is requested
+// along with the sublayer's where the registers hold both, and the rows are dealt out so that no SM gets a second
+// block before each has one.  1500 rows x 1536 behind two planes: 7.2 us alone and 11.5 in a layer, where reading the rows back
+// from memory for the convolution, in blocks of 12, took 13.9 and 22.8; 2048 wide, 1000 rows: 7.2 and 11.8.  (Above 2048 columns
+// the rows in front weigh more: from 7000 rows on 8% slower than blocks of two passes, 10 to 30% faster below.)
+template <int NVW>
+constexpr int kRowsWarps = NVW <= 16 ? 16 : 12;  // rows of a CTA, and what leaves a warp enough registers
 
-template <class T, int NVW, int TW>
-__global__ void __launch_bounds__(kRowsThreads) lm_norm_rows_kernel(NormArgs a) {
-  extern __shared__ __align__(16) float halo[];  // [TW - 1][ldx]
-  __shared__ float s_r[2 * kRowsWarps];
-  __shared__ Entry s_e[2 * kRowsWarps];
+template <class T, int NVW, bool CONV>
+__global__ void __launch_bounds__(kRowsWarps<NVW> * 32) lm_norm_rows_kernel(NormArgs a) {
+  constexpr int kWarps = kRowsWarps<NVW>, kThreads = kWarps * 32, kTaps = CONV ? 4 : 1;
+  constexpr bool kAhead = NVW <= 12;
+  extern __shared__ __align__(16) float rows_h[];  // [kWarps][ldx]
+  __shared__ Entry s_e[kWarps];
   pdl_launch_dependents();
-  pdl_wait_prior();
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nv = a.ldx >> 2;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nv = a.ldx >> 2, keep = a.taps - 1;
   const float g_pre = *a.g_pre, g_post = a.delta.p ? *a.g_post : 0.0f, inv_w = 1.0f / (float)a.width;
+  const float4 zero = make_float4(0, 0, 0, 0);
+  pdl_wait_prior();
   const int r_begin = blockIdx.x * a.rows_per_cta, r_end = min(r_begin + a.rows_per_cta, a.rows);
   int t0 = r_begin;
-  if (TW > 1) t0 = max(r_begin - (a.taps - 1), a.entries[a.row_entry[r_begin]].row0);
+  if (CONV) {
+    t0 = max(r_begin - keep, a.entries[a.row_entry[r_begin]].row0);
+    if (tid < r_end - t0) s_e[tid] = a.entries[a.row_entry[t0 + tid]];
+  }
   auto warp_sum = [](float v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     return v;
   };
-  if (TW > 1 && tid < r_end - t0) s_e[tid] = a.entries[a.row_entry[t0 + tid]];
-  for (int t = t0 + warp; t < r_end; t += kRowsWarps) {
+  const int t = t0 + warp;
+  if (t < r_end) {
     const float4* xr = reinterpret_cast<const float4*>(a.x_in + (size_t)t * a.ldx);
-    float4 x[NVW];
+    float4 x[NVW], ahead[kAhead ? NVW : 1];
     float ss = 0.0f;
     if (a.delta.p) {
+      if (kAhead)
+#pragma unroll
+        for (int i = 0; i < NVW; ++i) ahead[i] = lane + i * 32 < nv ? xr[lane + i * 32] : zero;
       warp_delta<NVW>(a.delta, t, lane, nv, x);
 #pragma unroll
       for (int i = 0; i < NVW; ++i) ss += dot4(x[i]);
@@ -302,79 +315,64 @@ __global__ void __launch_bounds__(kRowsThreads) lm_norm_rows_kernel(NormArgs a) 
 #pragma unroll
       for (int i = 0; i < NVW; ++i) {
         const int c = lane + i * 32;
-        if (c < nv) x[i] = fma4(r, x[i], xr[c]);
+        if (c < nv) x[i] = fma4(r, x[i], kAhead ? ahead[i] : xr[c]);
         ss += dot4(x[i]);
       }
     } else {
 #pragma unroll
       for (int i = 0; i < NVW; ++i) {
         const int c = lane + i * 32;
-        x[i] = c < nv ? xr[c] : make_float4(0, 0, 0, 0);
+        x[i] = c < nv ? xr[c] : zero;
         ss += dot4(x[i]);
       }
     }
     const float r = g_pre / sqrtf(warp_sum(ss) * inv_w + a.eps);
-    float* keep = t < r_begin ? halo + (size_t)(t - t0) * a.ldx : (a.x_out ? a.x_out + (size_t)t * a.ldx : nullptr);
-    T* out = static_cast<T*>(a.out) + (size_t)t * a.ldx;
-    if (lane == 0) s_r[t - t0] = r;
+    const bool out_x = t >= r_begin && a.x_out;
 #pragma unroll
     for (int i = 0; i < NVW; ++i) {
       const int c = lane + i * 32;
       if (c >= nv) continue;
-      if (keep) store4(keep + c * 4, x[i]);
-      if (TW == 1) store4(out + c * 4, fma4(r, x[i], make_float4(0, 0, 0, 0)));
+      if (out_x) store4(a.x_out + (size_t)t * a.ldx + c * 4, x[i]);
+      const float4 h = fma4(r, x[i], zero);
+      if (CONV) store4(rows_h + (size_t)warp * a.ldx + c * 4, h);
+      else store4(static_cast<T*>(a.out) + (size_t)t * a.ldx + c * 4, h);
     }
   }
-  if (TW == 1) return;
+  if (!CONV) return;
   __syncthreads();
-  const int keep = a.taps - 1;
-  const float* own_x = a.delta.p ? a.x_out : a.x_in;
-  for (int c = tid * 4; c < a.ldx; c += kRowsThreads * 4) {
-    float4 w[TW], hist[TW];  // hist[s]: h of s rows ago
+  for (int c = tid * 4; c < a.ldx; c += kThreads * 4) {
+    float4 w[kTaps], hist[kTaps];  // hist[s]: h of s rows ago
 #pragma unroll
-    for (int s = 0; s < TW; ++s) {
-      w[s] = s <= keep ? *reinterpret_cast<const float4*>(a.conv_w + (size_t)(keep - s) * a.ldx + c) : make_float4(0, 0, 0, 0);
-      hist[s] = make_float4(0, 0, 0, 0);
+    for (int s = 0; s < kTaps; ++s) {
+      w[s] = s <= keep ? __ldg(reinterpret_cast<const float4*>(a.conv_w + (size_t)(keep - s) * a.ldx + c)) : zero;
+      hist[s] = zero;
     }
-    for (int tb = t0; tb < r_end; tb += kRowsWarps) {
-      float4 x[kRowsWarps];
+#pragma unroll 4
+    for (int u = 0; u < r_end - t0; ++u) {
+      const Entry e = s_e[u];
+      const int off = t0 + u - e.row0;
+      const float* old_tail = a.tail + ((size_t)e.slot * 2 + e.tail) * keep * a.ldx + c;
+      if (off == 0)  // a sequence's share starts: the rows before it come from its tail, or are zero
 #pragma unroll
-      for (int u = 0; u < kRowsWarps; ++u) {
-        const int t = tb + u;
-        if (t < r_end) x[u] = *reinterpret_cast<const float4*>(t >= r_begin ? own_x + (size_t)t * a.ldx + c : halo + (size_t)(t - t0) * a.ldx + c);
+        for (int s = 1; s < kTaps; ++s) hist[s] = s <= keep && s <= e.pos0 ? *reinterpret_cast<const float4*>(old_tail + (size_t)(keep - s) * a.ldx) : zero;
+      hist[0] = *reinterpret_cast<const float4*>(rows_h + (size_t)u * a.ldx + c);
+      if (t0 + u >= r_begin) {
+        float4 y = hist[0];
+#pragma unroll
+        for (int s = 0; s < kTaps; ++s)
+          y = make_float4(fmaf(w[s].x, hist[s].x, y.x), fmaf(w[s].y, hist[s].y, y.y), fmaf(w[s].z, hist[s].z, y.z), fmaf(w[s].w, hist[s].w, y.w));
+        store4(static_cast<T*>(a.out) + (size_t)(t0 + u) * a.ldx + c, y);
+        const int at = keep - (e.count - off);
+        if (at >= 0) {  // among the last rows of its sequence's share: the new tail
+          float* new_tail = a.tail + ((size_t)e.slot * 2 + (e.tail ^ 1)) * keep * a.ldx + c;
+          store4(new_tail + (size_t)at * a.ldx, hist[0]);
+          if (off == e.count - 1)  // a short step: older rows move down
+            for (int j = 0; j + e.count < keep; ++j)
+              store4(new_tail + (size_t)j * a.ldx, *reinterpret_cast<const float4*>(old_tail + (size_t)(j + e.count) * a.ldx));
+        }
       }
 #pragma unroll
-      for (int u = 0; u < kRowsWarps; ++u) {
-        const int t = tb + u;
-        if (t >= r_end) break;
-        const Entry e = s_e[t - t0];
-        const int off = t - e.row0;
-        if (off == 0) {  // a sequence's share starts: the rows before it come from its tail, or are zero
-          const float* old_tail = a.tail + ((size_t)e.slot * 2 + e.tail) * keep * a.ldx + c;
-#pragma unroll
-          for (int s = 1; s < TW; ++s)
-            hist[s] = s <= keep && s <= e.pos0 ? *reinterpret_cast<const float4*>(old_tail + (size_t)(keep - s) * a.ldx) : make_float4(0, 0, 0, 0);
-        }
-        hist[0] = fma4(s_r[t - t0], x[u], make_float4(0, 0, 0, 0));
-        if (t >= r_begin) {
-          float4 y = hist[0];
-#pragma unroll
-          for (int s = 0; s < TW; ++s)
-            y = make_float4(fmaf(w[s].x, hist[s].x, y.x), fmaf(w[s].y, hist[s].y, y.y), fmaf(w[s].z, hist[s].z, y.z), fmaf(w[s].w, hist[s].w, y.w));
-          store4(static_cast<T*>(a.out) + (size_t)t * a.ldx + c, y);
-          const int at = keep - (e.count - off);
-          if (at >= 0) {  // among the last rows of its sequence's share: the new tail
-            const float* old_tail = a.tail + ((size_t)e.slot * 2 + e.tail) * keep * a.ldx + c;
-            float* new_tail = a.tail + ((size_t)e.slot * 2 + (e.tail ^ 1)) * keep * a.ldx + c;
-            store4(new_tail + (size_t)at * a.ldx, hist[0]);
-            if (off == e.count - 1)  // a short step: older rows move down
-              for (int j = 0; j + e.count < keep; ++j)
-                store4(new_tail + (size_t)j * a.ldx, *reinterpret_cast<const float4*>(old_tail + (size_t)(j + e.count) * a.ldx));
-          }
-        }
-#pragma unroll
-        for (int s = TW - 1; s > 0; --s) hist[s] = hist[s - 1];
-      }
+      for (int s = kTaps - 1; s > 0; --s) hist[s] = hist[s - 1];
     }
   }
 }
@@ -382,15 +380,15 @@ __global__ void __launch_bounds__(kRowsThreads) lm_norm_rows_kernel(NormArgs a) 
 template <class T, int NVW>
 cudaError_t launch_norm_rows(cudaStream_t s, NormArgs a) {
   const int halo = a.taps ? a.taps - 1 : 0;
-  a.rows_per_cta = (a.rows >= 4 * kSms * kRowsWarps ? 2 : 1) * kRowsWarps - halo;
-  const dim3 grid((a.rows + a.rows_per_cta - 1) / a.rows_per_cta);
-  if (a.taps == 0) return launch_pdl(lm_norm_rows_kernel<T, NVW, 1>, grid, dim3(kRowsThreads), 0, s, a);
-  const size_t smem = (size_t)halo * a.ldx * sizeof(float);
+  a.rows_per_cta = std::min(std::max(4, (a.rows + kSms - 1) / kSms), kRowsWarps<NVW> - halo);
+  const dim3 grid((a.rows + a.rows_per_cta - 1) / a.rows_per_cta), block(kRowsWarps<NVW> * 32);
+  if (a.taps == 0) return launch_pdl(lm_norm_rows_kernel<T, NVW, false>, grid, block, 0, s, a);
+  const size_t smem = (size_t)kRowsWarps<NVW> * a.ldx * sizeof(float);  // 192 KB at the widest, 4096
   if (smem > 40 * 1024) {
-    const cudaError_t r = cudaFuncSetAttribute(lm_norm_rows_kernel<T, NVW, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const cudaError_t r = cudaFuncSetAttribute(lm_norm_rows_kernel<T, NVW, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (r != cudaSuccess) return r;
   }
-  return launch_pdl(lm_norm_rows_kernel<T, NVW, 4>, grid, dim3(kRowsThreads), smem, s, a);
+  return launch_pdl(lm_norm_rows_kernel<T, NVW, true>, grid, block, smem, s, a);
 }
 
 template <class T, int NV>
@@ -408,6 +406,7 @@ cudaError_t launch_norm_t(cudaStream_t s, const NormArgs& a) {
   if (a.rows >= 2 * kSms && !a.gather && (a.taps == 0 || (a.taps >= 2 && a.taps <= 4)) && a.ldx <= 4096) {
     const int w = (a.ldx / 4 + 31) / 32;
     if (w <= 8) return launch_norm_rows<T, 8>(s, a);
+    if (w <= 12) return launch_norm_rows<T, 12>(s, a);
     if (w <= 16) return launch_norm_rows<T, 16>(s, a);
     return launch_norm_rows<T, 32>(s, a);
   }
