@@ -313,20 +313,27 @@ __global__ void __launch_bounds__(kBatchCombineThreads) attn_combine_batched_ker
   }
 }
 
-// logits[b][v] = sum_k x[b][k] * W[v][k] for a tile of kLmRows activation rows (blockIdx.y), W fp16 [V, hidden], on
+// logits[b][v] = sum_k x[b][k] * W[v][k] for a tile of kLmRows activation rows (blockIdx.x), W fp16 [V, hidden], on
 // the tensor cores without giving up the fp32 activations: x = hi + lo with hi = fp16(x), lo = fp16(x - hi) (error
 // 2^-22 |x|), both halves in shared memory, every product w * hi and w * lo exact in the fp32 accumulator of
-// mma.sync.m16n8k16.  A warp owns tiles of 16 vocabulary rows; per 32 values of k a lane loads 16 bytes of W rows
-// g and g + 8 straight from global memory (k = 8 c .. 8 c + 7 of the step; the contraction index may be permuted
-// freely as long as both operands agree, so two instructions use the words {0, 1} and {2, 3} of what was loaded)
-// and, per 8 activation rows, 16 bytes of hi and of lo from shared memory for the same k.  Rows of the activation
-// tile are padded to 64 bytes past a multiple of 128, which makes those 16-byte loads conflict-free.
+// mma.sync.m16n8k16.  A warp owns tiles of 32 vocabulary rows; per 64 values of k a lane loads 32 bytes of W rows
+// g, g + 8, g + 16 and g + 24 straight from global memory (k = 16 c .. 16 c + 15 of the step, whole lines of 128 bytes; the
+// contraction index may be permuted freely as long as both operands agree, so four instructions use the words {0, 1}, {2, 3},
+// {4, 5} and {6, 7} of what was loaded) and, per 8 activation rows, 32 bytes of hi and of lo from shared memory for the same k.  Rows
+// of the activation tile are padded to 16 bytes past a multiple of 128, which makes those 16-byte loads conflict-free.
 // Each CTA also leaves, per activation row, its largest logit and the index (lowest index on ties) in
-// best[b][blockIdx.x].  hidden must be a multiple of 32.
+// best[b][blockIdx.y].  hidden must be a multiple of 32.
+// What it cannot do without, 151936 x 1536: 71 us of memory, and 57 us of the tensor cores per tile of x.  Bound by the way of W: with
+// 16-byte words and 16 vocabulary rows a warp the loads of either operand were 74% of what the L1 pipe can do, hence whole lines, twice
+// the rows behind each word of x, and words that are always kLmAhead steps ahead.  The tiles of x that read the same part of the
+// vocabulary run side by side, so that memory is read once for all of them.  us before / now, batch 8, 32, 64, 96: width 896
+// 100 / 76, 104 / 80, 189 / 148, 273 / 215; width 1536 180 / 127, 188 / 133, 339 / 239, 487 / 348.  (8 warps of three or four steps
+// ahead: 252 to 277 us at 64 rows; 16-byte words, six steps ahead: 260.)
 constexpr int kLmRows = 32;     // activation rows per CTA tile (4 column tiles of the instruction)
-constexpr int kLmWarps = 16;
+constexpr int kLmWarps = 12;
+constexpr int kLmAhead = 2;     // steps of W on their way: 12 warps x 2 x 4 KB
 constexpr int kLmThreads = kLmWarps * 32;
-__host__ __device__ inline size_t lm_row_bytes(int hidden) { return (size_t)hidden * 2 + 64; }
+__host__ __device__ inline size_t lm_row_bytes(int hidden) { return (((size_t)hidden * 2 + 127) & ~(size_t)127) + 16; }
 __host__ __device__ inline size_t lm_smem_bytes(int hidden) { return 2 * (size_t)kLmRows * lm_row_bytes(hidden); }
 
 __device__ __forceinline__ void lm_mma_f16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
@@ -334,6 +341,22 @@ __device__ __forceinline__ void lm_mma_f16(float (&d)[4], uint32_t a0, uint32_t 
   asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
       : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+struct alignas(32) LmWords {
+  uint4 lo, hi;
+};
+// 32 bytes of W (`wide`: at once), in program order with the loads from shared memory, so that the words stay as far ahead as they are
+// written here
+__device__ __forceinline__ LmWords lm_load_w(const __half* p, bool wide) {
+  LmWords v;
+  if (wide)
+    asm volatile("ld.global.nc.L1::no_allocate.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(v.lo.x), "=r"(v.lo.y), "=r"(v.lo.z), "=r"(v.lo.w), "=r"(v.hi.x), "=r"(v.hi.y), "=r"(v.hi.z), "=r"(v.hi.w)
+                 : "l"(p));
+  else
+    v.lo = __ldg(reinterpret_cast<const uint4*>(p)), v.hi = __ldg(reinterpret_cast<const uint4*>(p) + 1);
+  return v;
 }
 
 __global__ void __launch_bounds__(kLmThreads, 1) lm_head_f16_batched_kernel(const float* __restrict__ x, int batch,
@@ -344,59 +367,106 @@ __global__ void __launch_bounds__(kLmThreads, 1) lm_head_f16_batched_kernel(cons
   __shared__ float s_bv[kLmRows][kLmWarps];
   __shared__ int s_bi[kLmRows][kLmWarps];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, c = lane & 3;
-  const int b0 = blockIdx.y * kLmRows;
+  const int b0 = blockIdx.x * kLmRows;
   const int nb = min(kLmRows, batch - b0);
   const size_t row_bytes = lm_row_bytes(hidden);
   uint8_t* s_hi = lm_smem;
   uint8_t* s_lo = lm_smem + (size_t)kLmRows * row_bytes;
-  for (int i = tid; i < kLmRows * (hidden >> 1); i += kLmThreads) {  // two values per thread and trip
-    const int r = i / (hidden >> 1), k = (i - r * (hidden >> 1)) * 2;
-    float2 v = make_float2(0.0f, 0.0f);
-    if (r < nb) v = *reinterpret_cast<const float2*>(x + (size_t)(b0 + r) * hidden + k);
-    const __half2 hi = __floats2half2_rn(v.x, v.y);
-    const float2 hf = __half22float2(hi);
-    const __half2 lo = __floats2half2_rn(v.x - hf.x, v.y - hf.y);
-    *reinterpret_cast<__half2*>(s_hi + (size_t)r * row_bytes + (size_t)k * 2) = hi;
-    *reinterpret_cast<__half2*>(s_lo + (size_t)r * row_bytes + (size_t)k * 2) = lo;
-  }
+  // tiles dealt out warp by warp: those of an incomplete last round land on as many SMs as there are
+  const int stride = kLmWarps * gridDim.y, tiles = (vocab + 31) >> 5, steps = (hidden + 63) >> 6;  // 64 values of k per step
+  int tile = warp * gridDim.y + blockIdx.y;
+  const bool wide = (reinterpret_cast<uintptr_t>(w) & 31) == 0;  // (the rows are multiples of 64 bytes)
+  const __half* wr[4];          // rows g, g + 8, g + 16 and g + 24 of the tile
+  LmWords ring[kLmAhead][4];    // 32 bytes of each: k = 64 step + 16 c ..
+  auto load_step = [&](int j, int ss) {
+    const bool some = 64 * ss + 16 * c < hidden;  // (an odd multiple of 32: the last step is half a step)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      if (some) ring[j][i] = lm_load_w(wr[i] + 64 * ss, wide);
+      else ring[j][i].lo = ring[j][i].hi = make_uint4(0, 0, 0, 0);
+    }
+  };
+  auto start_tile = [&]() {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) wr[i] = w + (size_t)min(32 * tile + g + 8 * i, vocab - 1) * hidden + 16 * c;  // (past the end: the last row again, dropped below)
+#pragma unroll
+    for (int j = 0; j < kLmAhead; ++j) load_step(j, j);
+  };
+  start_tile();
+  for (int r = warp; r < kLmRows; r += kLmWarps)
+#pragma unroll 4
+    for (int k = lane * 4; k < steps * 64; k += 128) {
+      float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      if (r < nb && k < hidden) v = *reinterpret_cast<const float4*>(x + (size_t)(b0 + r) * hidden + k);
+      const __half2 h0 = __floats2half2_rn(v.x, v.y), h1 = __floats2half2_rn(v.z, v.w);
+      const float2 f0 = __half22float2(h0), f1 = __half22float2(h1);
+      const __half2 l0 = __floats2half2_rn(v.x - f0.x, v.y - f0.y), l1 = __floats2half2_rn(v.z - f1.x, v.w - f1.y);
+      __half2* hi = reinterpret_cast<__half2*>(s_hi + (size_t)r * row_bytes + (size_t)k * 2);
+      __half2* lo = reinterpret_cast<__half2*>(s_lo + (size_t)r * row_bytes + (size_t)k * 2);
+      hi[0] = h0, hi[1] = h1, lo[0] = l0, lo[1] = l1;
+    }
   __syncthreads();
   float bv[8];
   int bi[8];
 #pragma unroll
   for (int i = 0; i < 8; ++i) bv[i] = -3.402823466e+38f, bi[i] = 0x7fffffff;
-  const int steps = hidden >> 5;  // 32 values of k per step
-  const uint32_t hi_s = (uint32_t)__cvta_generic_to_shared(s_hi) + (uint32_t)g * (uint32_t)row_bytes + (uint32_t)c * 16;
-  const uint32_t lo_s = hi_s + (uint32_t)((size_t)kLmRows * row_bytes);
-  for (int v0 = 16 * (blockIdx.x * kLmWarps + warp); v0 < vocab; v0 += 16 * kLmWarps * gridDim.x) {
-    float acc[4][4];
+  const uint32_t hi_s = (uint32_t)__cvta_generic_to_shared(s_hi) + (uint32_t)g * (uint32_t)row_bytes + (uint32_t)c * 32;
+  const uint32_t lo_off = (uint32_t)((size_t)kLmRows * row_bytes);
+  while (tile < tiles) {
+    const int v0 = 32 * tile;
+    float acc[2][4][4];
 #pragma unroll
-    for (int t = 0; t < 4; ++t) acc[t][0] = acc[t][1] = acc[t][2] = acc[t][3] = 0.0f;
-    // rows past the end of the vocabulary repeat its last row (their results are dropped)
-    const uint4* wa = reinterpret_cast<const uint4*>(w + (size_t)min(v0 + g, vocab - 1) * hidden) + c;
-    const uint4* wb = reinterpret_cast<const uint4*>(w + (size_t)min(v0 + g + 8, vocab - 1) * hidden) + c;
-#pragma unroll 4
-    for (int ss = 0; ss < steps; ++ss) {
-      const uint4 ra = wa[ss * 4], rb = wb[ss * 4];  // 16 bytes of either row: k = 32 ss + 8 c ..
+    for (int h = 0; h < 2; ++h)
 #pragma unroll
-      for (int t = 0; t < 4; ++t) {
-        uint4 xh, xl;
-        const uint32_t off = (uint32_t)t * 8 * (uint32_t)row_bytes + (uint32_t)ss * 64;
-        asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(xh.x), "=r"(xh.y), "=r"(xh.z), "=r"(xh.w) : "r"(hi_s + off));
-        asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(xl.x), "=r"(xl.y), "=r"(xl.z), "=r"(xl.w) : "r"(lo_s + off));
-        lm_mma_f16(acc[t], ra.x, rb.x, ra.y, rb.y, xh.x, xh.y);
-        lm_mma_f16(acc[t], ra.x, rb.x, ra.y, rb.y, xl.x, xl.y);
-        lm_mma_f16(acc[t], ra.z, rb.z, ra.w, rb.w, xh.z, xh.w);
-        lm_mma_f16(acc[t], ra.z, rb.z, ra.w, rb.w, xl.z, xl.w);
+      for (int t = 0; t < 4; ++t) acc[h][t][0] = acc[h][t][1] = acc[h][t][2] = acc[h][t][3] = 0.0f;
+#pragma unroll 1
+    for (int s0 = 0; s0 < steps; s0 += kLmAhead) {
+#pragma unroll
+      for (int j = 0; j < kLmAhead; ++j) {
+        const int ss = s0 + j;
+        if (ss >= steps) break;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {  // tiles of x {0, 1} and {2, 3}, either half of the 32 bytes: four sums at a time, each is a chain
+          const int t = q >> 1 << 1;
+          uint4 a[4], xh[2], xl[2];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) a[i] = q & 1 ? ring[j][i].hi : ring[j][i].lo;
+#pragma unroll
+          for (int u = 0; u < 2; ++u) {
+            const uint32_t at = hi_s + (uint32_t)(t + u) * 8 * (uint32_t)row_bytes + (uint32_t)(ss * 128 + (q & 1) * 16);
+            asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(xh[u].x), "=r"(xh[u].y), "=r"(xh[u].z), "=r"(xh[u].w) : "r"(at));
+            asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(xl[u].x), "=r"(xl[u].y), "=r"(xl[u].z), "=r"(xl[u].w) : "r"(at + lo_off));
+          }
+#pragma unroll
+          for (int u = 0; u < 2; ++u)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) lm_mma_f16(acc[h][t + u], a[2 * h].x, a[2 * h + 1].x, a[2 * h].y, a[2 * h + 1].y, xh[u].x, xh[u].y);
+#pragma unroll
+          for (int u = 0; u < 2; ++u)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) lm_mma_f16(acc[h][t + u], a[2 * h].x, a[2 * h + 1].x, a[2 * h].y, a[2 * h + 1].y, xl[u].x, xl[u].y);
+#pragma unroll
+          for (int u = 0; u < 2; ++u)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) lm_mma_f16(acc[h][t + u], a[2 * h].z, a[2 * h + 1].z, a[2 * h].w, a[2 * h + 1].w, xh[u].z, xh[u].w);
+#pragma unroll
+          for (int u = 0; u < 2; ++u)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) lm_mma_f16(acc[h][t + u], a[2 * h].z, a[2 * h + 1].z, a[2 * h].w, a[2 * h + 1].w, xl[u].z, xl[u].w);
+        }
+        load_step(j, ss + kLmAhead);
       }
     }
-    // lane (g, c): rows v0 + g and v0 + g + 8, activation rows 8 t + 2 c and 8 t + 2 c + 1
+    tile += stride;
+    if (tile < tiles) start_tile();
+    // lane (g, c): rows v0 + g + 8 i, activation rows 8 t + 2 c and 8 t + 2 c + 1
 #pragma unroll
     for (int t = 0; t < 4; ++t)
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
+      for (int i = 0; i < 8; ++i) {
         const int v = v0 + g + (i >> 1) * 8, r = 8 * t + 2 * c + (i & 1);
         if (v < vocab && r < nb) {
-          const float a = acc[t][i];
+          const float a = acc[i >> 2][t][i & 3];
           if (logits) logits[(size_t)(b0 + r) * vocab + v] = a;
           const int slot = 2 * t + (i & 1);
           if (a > bv[slot]) {  // this lane meets the rows of a column in increasing order: a strict test keeps the lowest index
@@ -436,7 +506,7 @@ __global__ void __launch_bounds__(kLmThreads, 1) lm_head_f16_batched_kernel(cons
         v = s_bv[r][k];
         i = s_bi[r][k];
       }
-    best[(size_t)(b0 + r) * gridDim.x + blockIdx.x] = make_float2(v, __int_as_float(i));
+    best[(size_t)(b0 + r) * gridDim.y + blockIdx.y] = make_float2(v, __int_as_float(i));
   }
 }
 
@@ -554,7 +624,7 @@ int enqueue_batched_step(BatchDecoder* b) {
   }
   add_rmsnorm_quant_kernel<<<B, 256, 0, s>>>(b->h, b->down, d->final_norm, c.eps, H, nullptr, b->xn, nullptr, nullptr, 0);
   {
-    const dim3 grid(kLmCtas, (B + kLmRows - 1) / kLmRows);
+    const dim3 grid((B + kLmRows - 1) / kLmRows, kLmCtas);
     lm_head_f16_batched_kernel<<<grid, kLmThreads, lm_smem_bytes(H), s>>>(b->xn, B, d->lm_head, H, c.vocab,
                                                                                       b->logits, b->best);
   }
