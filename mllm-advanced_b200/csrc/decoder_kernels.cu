@@ -250,7 +250,7 @@ __global__ void __launch_bounds__(kCombineThreads) attn_combine_quant_kernel(
 // padded blocks; a row's pieces of 16 bytes are half sectors, the neighbouring row's CTA writes the other half.
 // Bound: the chain of loads, reductions and stores on short prompts, memory on documents: gate and up of 1900 tokens are 136 MB,
 // which L2 is still writing back (50 us for 306 MB).  us, width 1536 and feed-forward 8960, from the end of the GEMM before to
-// the last block, operator + quantization / here: silu, 1900 tokens 50 + 34.5 / 50, 512 10.2 + 9.5 / 15.7, 64 rows 4.3 + 3.4 / 7.6
+// the last block, operator + quantization / here: silu, 1900 tokens 50 + 34.5 / 50, 512 10.2 + 9.5 / 15.7, 64 rows 4.3 + 3.4 / 5.9
 // (one launch less); norm 13 + 6.5 / 18, 4.6 + 3.9 / 6.6, 3.6 + 2.1 / 4.7.
 // ---------------------------------------------------------------------------------------------
 // eight values of K (left of them exist) of row m
@@ -344,17 +344,24 @@ __global__ void __launch_bounds__(kNormThreads) add_rmsnorm_blocks_kernel(const 
   }
 }
 
-// A thread keeps its ITEMS items of 8 products in registers between the minimum / maximum and the blocks.
-constexpr int kSiluBlockThreads = 384;
-template <int FORM, int ITEMS>
+// A thread keeps its ITEMS items of 8 products in registers between the minimum / maximum and the blocks.  A row is one CTA, or a
+// cluster of SPLIT that exchanges minima and maxima (the order of those does not matter: same bits): a row is 72 KB of gate and up and
+// three items a thread at a width of 8960, and short prompts leave SMs idle.  us from the end of the GEMM before, width 8960, one CTA /
+// four: 8 rows 6.4 / 4.8, 48 7.9 / 5.9, 128 8.4 / 6.0, 192 8.5 / 10.2 (no longer all at once); 4864: 24 rows 7.6 / 4.0, 128 7.7 / 6.4.
+constexpr int kSiluBlockThreads = 384, kSiluSplit = 4, kSiluSplitRows = 128;
+template <int FORM, int ITEMS, int SPLIT>
 __global__ void __launch_bounds__(kSiluBlockThreads) silu_mul_blocks_kernel(const float* __restrict__ gate, const float* __restrict__ up,
                                                                             int inter, int m_total, W4Blocks out, int use_pdl) {
-  __shared__ float scratch[64];
+  static_assert(SPLIT == 1 || (ITEMS == 1 && SPLIT * kSiluBlockThreads / 32 <= 64), "");
+  __shared__ float scratch[64], s_mn[64], s_mx[64];
+  const int num_groups = (inter + kGroup - 1) / kGroup, m = blockIdx.x / SPLIT, rank = SPLIT > 1 ? cluster_ctarank() : 0;
+  const int tid = rank * blockDim.x + threadIdx.x;  // of the row's
+  if (SPLIT > 1) cluster_arrive_relaxed();          // (every CTA of the cluster runs when the peers write into it)
   if (use_pdl) {
     pdl_launch_dependents();
     pdl_wait_prior();
   }
-  const int m = blockIdx.x, tid = threadIdx.x, num_groups = (inter + kGroup - 1) / kGroup;
+  if (SPLIT > 1) cluster_wait();
   if (blocks_row_is_padding<FORM>(out, num_groups, m, m_total)) return;
   const float *g_row = gate + (size_t)m * inter, *u_row = up + (size_t)m * inter;
   const bool vec = (inter & 3) == 0;  // (the rows start on 16 bytes)
@@ -388,7 +395,30 @@ __global__ void __launch_bounds__(kSiluBlockThreads) silu_mul_blocks_kernel(cons
         mx = fmaxf(mx, a[i][j]);
       }
     }
-  block_minmax(mn, mx, scratch);
+  if (SPLIT == 1) {
+    block_minmax(mn, mx, scratch);
+  } else {
+    const int lane = threadIdx.x & 31, nw = blockDim.x >> 5, all = SPLIT * nw;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      mn = fminf(mn, __shfl_xor_sync(0xffffffffu, mn, o));
+      mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    }
+    if (lane < SPLIT) {  // each warp to every CTA of the row
+      st_cluster_f32(map_to_cta(s_mn + rank * nw + (threadIdx.x >> 5), lane), mn);
+      st_cluster_f32(map_to_cta(s_mx + rank * nw + (threadIdx.x >> 5), lane), mx);
+    }
+    cluster_sync_all();
+    for (int i = lane; i < all; i += 32) {
+      mn = fminf(mn, s_mn[i]);
+      mx = fmaxf(mx, s_mx[i]);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      mn = fminf(mn, __shfl_xor_sync(0xffffffffu, mn, o));
+      mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    }
+  }
   const ActQuantParams p = act_quant_params(mn, mx);
   if (tid == 0) out.hdr[m] = make_float2(p.recip_scale, __int_as_float(-p.nzp));
 #pragma unroll
@@ -399,31 +429,43 @@ __global__ void __launch_bounds__(kSiluBlockThreads) silu_mul_blocks_kernel(cons
 }
 
 template <class K, class... A>
-static cudaError_t launch_blocks_op(K kernel, int rows, int threads, int use_pdl, cudaStream_t s, A... args) {
+static cudaError_t launch_blocks_op(K kernel, int rows, int split, int threads, int use_pdl, cudaStream_t s, A... args) {
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)rows, 1, 1);
+  cfg.gridDim = dim3((unsigned)(rows * split), 1, 1);
   cfg.blockDim = dim3((unsigned)threads, 1, 1);
   cfg.stream = s;
-  cudaLaunchAttribute attr;
-  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr.val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = &attr;
-  cfg.numAttrs = use_pdl ? 1 : 0;
+  cudaLaunchAttribute attr[2];
+  cfg.attrs = attr;
+  if (split > 1) {
+    attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+    attr[cfg.numAttrs].val.clusterDim.x = (unsigned)split;
+    attr[cfg.numAttrs].val.clusterDim.y = attr[cfg.numAttrs].val.clusterDim.z = 1;
+    ++cfg.numAttrs;
+  }
+  if (use_pdl) {
+    attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[cfg.numAttrs].val.programmaticStreamSerializationAllowed = 1;
+    ++cfg.numAttrs;
+  }
   return cudaLaunchKernelEx(&cfg, kernel, args..., use_pdl);
 }
 cudaError_t launch_add_rmsnorm_blocks(const float* h_in, const float* delta, const float* w, float eps, int hidden, float* h_out, int m,
                                       const W4Blocks& out, int use_pdl, cudaStream_t s) {
   return out.form == kW4Stream
-             ? launch_blocks_op(add_rmsnorm_blocks_kernel<kW4Stream>, out.m_pad, kNormThreads, use_pdl, s, h_in, delta, w, eps, hidden, h_out, m, out)
-             : launch_blocks_op(add_rmsnorm_blocks_kernel<kW4Tile>, out.m_pad, kNormThreads, use_pdl, s, h_in, delta, w, eps, hidden, h_out, m, out);
+             ? launch_blocks_op(add_rmsnorm_blocks_kernel<kW4Stream>, out.m_pad, 1, kNormThreads, use_pdl, s, h_in, delta, w, eps, hidden, h_out, m, out)
+             : launch_blocks_op(add_rmsnorm_blocks_kernel<kW4Tile>, out.m_pad, 1, kNormThreads, use_pdl, s, h_in, delta, w, eps, hidden, h_out, m, out);
 }
 template <int FORM>
 static cudaError_t launch_silu_form(const float* gate, const float* up, int inter, int m, const W4Blocks& out, int use_pdl, cudaStream_t s) {
+  const int items = ((inter + kGroup - 1) / kGroup) * 4;
+  if (out.m_pad <= kSiluSplitRows && items > kSiluBlockThreads && items <= kSiluSplit * kSiluBlockThreads)
+    return launch_blocks_op(silu_mul_blocks_kernel<FORM, 1, kSiluSplit>, out.m_pad, kSiluSplit, (items + 32 * kSiluSplit - 1) / (32 * kSiluSplit) * 32,
+                            use_pdl, s, gate, up, inter, m, out);
   switch ((inter + 8 * kSiluBlockThreads - 1) / (8 * kSiluBlockThreads)) {
-    case 1: return launch_blocks_op(silu_mul_blocks_kernel<FORM, 1>, out.m_pad, kSiluBlockThreads, use_pdl, s, gate, up, inter, m, out);
-    case 2: return launch_blocks_op(silu_mul_blocks_kernel<FORM, 2>, out.m_pad, kSiluBlockThreads, use_pdl, s, gate, up, inter, m, out);
-    case 3: return launch_blocks_op(silu_mul_blocks_kernel<FORM, 3>, out.m_pad, kSiluBlockThreads, use_pdl, s, gate, up, inter, m, out);
-    case 4: return launch_blocks_op(silu_mul_blocks_kernel<FORM, 4>, out.m_pad, kSiluBlockThreads, use_pdl, s, gate, up, inter, m, out);
+    case 1: return launch_blocks_op(silu_mul_blocks_kernel<FORM, 1, 1>, out.m_pad, 1, kSiluBlockThreads, use_pdl, s, gate, up, inter, m, out);
+    case 2: return launch_blocks_op(silu_mul_blocks_kernel<FORM, 2, 1>, out.m_pad, 1, kSiluBlockThreads, use_pdl, s, gate, up, inter, m, out);
+    case 3: return launch_blocks_op(silu_mul_blocks_kernel<FORM, 3, 1>, out.m_pad, 1, kSiluBlockThreads, use_pdl, s, gate, up, inter, m, out);
+    case 4: return launch_blocks_op(silu_mul_blocks_kernel<FORM, 4, 1>, out.m_pad, 1, kSiluBlockThreads, use_pdl, s, gate, up, inter, m, out);
     default: return cudaErrorInvalidValue;  // (the decoder takes widths up to 12000)
   }
 }
