@@ -34,7 +34,7 @@
 // error against 64 bits (2-norm) 6.0e-8 / 5.3e-8 at K = 1536, 1.29e-7 / 9.4e-8 at K = 8192; where weights and activations
 // are of one sign throughout, 1.3e-7 / 1.0e-7 at K = 1536, 3.9e-7 / 5.3e-7 at K = 8960.  M = 65, 17920 x 1536
 // 33 / 24 us; the three matrices of q, k, v, M = 65 (one launch instead of three) 47 / 14 us.  At M <= 64 the streaming
-// kernel (gemm_stream.cu) mostly stays ahead: it needs no 128-row tiles (1536 x 1536, M = 48: 8 us, here 14).
+// kernel (gemm_stream.cu) mostly stays ahead: it needs no 128-row tiles (1536 x 1536, M = 64: 6.2 us; here, M = 65, 13.3).
 // fp16-encoded scales, us: 1536 x 1536, M = 65 19.4, 1536 x 8960, M = 512 87, 8960 x 1536, M = 512 38 (27, 110 and 47 with
 // finished chunks fetched in front of every turn and a wait of the MMA issuer for either part).
 #include <cuda_fp16.h>

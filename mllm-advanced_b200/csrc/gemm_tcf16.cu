@@ -659,8 +659,8 @@ bool w4a32_gemm_tcf16_supported(int m, int k, int n) { return m >= 64 && k >= 1 
 // Where the "fastest" policy (5) takes this kernel: from 128 rows on (1.5B layer shapes, M = 512, against the default, which is
 // gemm_chunk.cu: 8960 x 1536 26 vs 29 us, 17920 x 1536 39 vs 50, 1536 x 8960 42 vs 63; 1536 x 1536 20 vs 19); below that only
 // where the weight tiles alone fill the GPU and K is short (gate / up of the 1.5B model, alone or grouped: M = 64 17 vs 30 us
-// against the streaming small-batch GEMM, M = 65 to 127 15 vs 16 to 17 us against gemm_chunk.cu).  Narrow or long-K matrices
-// stay with the default there: ONE truncated fp32 sum over a long K is off by 4.3e-7 at K = 8960 (gemm_chunk.cu 9.6e-8, int32
+// against the streaming small-batch GEMM as it was, now 21.9; M = 65 to 127 15 vs 16 to 17 us against gemm_chunk.cu).  Narrow
+// matrices go to gemm_stream.cu before this rule is asked; other long-K matrices stay with the default there: ONE truncated fp32 sum over a long K is off by 4.3e-7 at K = 8960 (gemm_chunk.cu 9.6e-8, int32
 // group sums 1.4e-7), and fp16-encoded scales are rounded here, not there.
 bool w4a32_gemm_tcf16_preferred(int m, int k, int n) {
   if (!w4a32_gemm_tcf16_supported(m, k, n)) return false;
@@ -744,7 +744,9 @@ cudaError_t launch_w4a16_gemm_tcf16_grouped(const uint8_t* a_blocks, int m, int 
   TfParams prm = {};
   prm.a_blocks = a_blocks;
   prm.a_hdr = nullptr;
-  prm.use_pdl = 1;  // (behind its quantization, which is launched in order)
+  long long t256 = 0;
+  for (int i = 0; i < count; ++i) t256 += (long long)((n[i] + 127) / 128) * ((m + 255) / 256);
+  prm.use_pdl = t256 <= 148;  // (behind its quantization, which is launched in order; not for more than a wave, as in c_api.cu)
   prm.m = m, prm.k = k;
   prm.num_groups = (k + kGroup - 1) / kGroup;
   prm.m8_pad = (m + nt - 1) / nt * nt / 8;
