@@ -136,10 +136,11 @@ MLLMB200_API int mllmb200_w4a32_linear_forward(const float* x_dev, const void* t
  * tensor memory; same 1e-3*rms bound; auto never picks it; launches that would fill less than half of the SMs
  * split K between two CTAs per output tile, and y holds one half's partial sums for a moment during the
  * call - deterministic, but y is scratch until the call's work on the stream has finished), 5 fastest: kernel 4
- * for M >= 128 and, at 64 <= M < 128, for matrices (or groups) of at least 8192 rows with K <= 4096; else auto,
+ * for M >= 128 and, at 64 <= M < 128, for matrices (or groups) of at least 8192 rows with K <= 4096; kernel 7's code for
+ * 65 <= M <= 192 and matrices (or groups) of at most 4096 rows (below M = 128: K >= 1024); else auto,
  * 6 the two-launch GEMV (activation-quantization kernel + one-shot GEMV), kept for comparison,
  * 7 streaming tensor-core GEMM for small batches (M <= 64; what auto picks for 5 <= M <= 64): the weight cells are
- * spread over all SMs as in the GEMV, the per-group integer products run as mma.sync u8 x s8 (exact int32 group
+ * spread over all SMs as in the GEMV, the per-group integer products run as mma.sync s8 x s8 (exact int32 group
  * sums, as the reference), clusters split K where the quantized activations of a whole row do not fit one CTA.
  * OR 0x100 into `kernel` to allow programmatic dependent launch (kernels 1, 4, 5, 6, 7 and the default from 65 rows
  * on): the kernel then requests its (constant) weights while the previous kernel of the stream still runs and reads x
