@@ -524,21 +524,46 @@ __global__ void __launch_bounds__(TcShape<BN>::kThreads, 1) lm_gemm_tc_kernel(co
 // four epilogue warps and stores of 16 bytes / pairs with eight and of 32: 1536 -> 17920 gated 96 / 78 (pairs with the old
 // epilogue 97, with eight warps 79.5), 8960 -> 1536 48 / 38 (K in two), 1536 -> 6144 35 / 30, 1536 -> 2048 15.5 / 15.2,
 // 1536 -> 1536 14.6 / 13.  Now 1000 cycles a K tile.
-// Barriers: a CTA's own loads complete on its `full`; in CTA 1 the MMA warp hands that on to `peer_full` of CTA 0; commits arrive
-// in both CTAs; the epilogue warps of both free an accumulator in CTA 0.
+// Barriers: the loads of both CTAs complete on `full` of CTA 0, whose MMA warp is the one that waits for them; commits arrive in
+// both CTAs; the epilogue warps of both free an accumulator in CTA 0.
 constexpr int kPairN = 256, kPairStages = 6, kPairStageBytes = 2 * kABytes;
 constexpr int kPairSmem = kPairStages * kPairStageBytes + 1024;
 constexpr int kPairEpiWarps = 8, kPairEpiCols = kPairN / (kPairEpiWarps / 4);  // epilogue warps, columns of one (and 32 rows)
 constexpr int kPairThreads = 64 + 32 * kPairEpiWarps;  // copy warp, MMA warp, epilogue
 
-// (The arrival hands on completed copies and tensor-memory reads, no stores: at cluster scope, with the memory barrier that
-// brings, it would cost more than it orders.)
-__device__ __forceinline__ void arrive_at_cta0(uint64_t* bar) {
+// The box goes into this CTA's shared memory, its bytes are counted on a barrier of CTA 0 (bar: an address of the cluster).
+__device__ __forceinline__ void pair_load_2d(void* dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
+  asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
+                   smem_u32(dst)),
+               "l"(map), "r"(x), "r"(y), "r"(bar)
+               : "memory");
+}
+// Hands on tensor-memory reads that tcgen05.wait::ld and a tcgen05 fence have closed: those two and a relaxed arrival order tensor
+// memory between threads of a cluster, stores would need a release.
+__device__ __forceinline__ void arrive_at_cta0(uint32_t bar) {
+  asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+// mbar_wait_bounded for those arrivals
+__device__ __forceinline__ bool pair_try_wait(uint64_t* bar, uint32_t parity) {
+  uint32_t ok;
   asm volatile(
-      "{\n\t.reg .b32 r;\n\t"
-      "mapa.shared::cluster.u32 r, %0, 0;\n\t"
-      "mbarrier.arrive.shared::cluster.b64 _, [r];\n\t}" ::"r"(smem_u32(bar))
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.try_wait.parity.relaxed.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(smem_u32(bar)), "r"(parity)
       : "memory");
+  return ok != 0;
+}
+__device__ __forceinline__ bool pair_wait_bounded(uint64_t* bar, uint32_t parity) {
+  if (pair_try_wait(bar, parity)) return true;
+  const long long t0 = clock64();
+  while (!pair_try_wait(bar, parity))
+    if (clock64() - t0 > (1ll << 31)) {
+      atomicOr(&g_device_status, kDevStatusTimeout);
+      return false;
+    }
+  return true;
 }
 __device__ __forceinline__ void pair_commit(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(smem_u32(bar)),
@@ -559,7 +584,7 @@ __global__ void __launch_bounds__(kPairThreads, 1) lm_gemm_pair_kernel(const __g
                                                                      const __grid_constant__ CUtensorMap wmap, int M, int N, int K, int splits,
                                                                      Epi e) {
   extern __shared__ uint8_t tc_smem_raw[];
-  __shared__ uint64_t full[kPairStages], empty[kPairStages], peer_full[kPairStages], acc_full[2], acc_empty[2];
+  __shared__ uint64_t full[kPairStages], empty[kPairStages], acc_full[2], acc_empty[2];  // (full and acc_empty: those of CTA 0 are used)
   __shared__ uint32_t tmem_slot;
   __shared__ volatile int gave_up;
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(tc_smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -567,7 +592,7 @@ __global__ void __launch_bounds__(kPairThreads, 1) lm_gemm_pair_kernel(const __g
   const int rank = (int)(blockIdx.x & 1), pair = (int)(blockIdx.x >> 1), pairs = (int)(gridDim.x >> 1);
   const int mt = (M + 2 * kTileM - 1) / (2 * kTileM), nt = (N + kPairN - 1) / kPairN, kt = K / kTileK, items = mt * nt * splits;
   if (tid == 0) {
-    for (int i = 0; i < kPairStages; ++i) mbar_init(&full[i], 1), mbar_init(&empty[i], 1), mbar_init(&peer_full[i], 1);
+    for (int i = 0; i < kPairStages; ++i) mbar_init(&full[i], 1), mbar_init(&empty[i], 1);
     for (int i = 0; i < 2; ++i) mbar_init(&acc_full[i], 1), mbar_init(&acc_empty[i], 2 * kPairEpiWarps);
     gave_up = 0;
     mbar_fence_init();
@@ -592,9 +617,12 @@ __global__ void __launch_bounds__(kPairThreads, 1) lm_gemm_pair_kernel(const __g
       int it = 0, ahead = 0, st = 0;
       uint32_t ph = 0;
       bool ok = true;
+      const uint32_t full0 = map_to_cta(full, 0);
+      // CTA 0 announces the bytes of both: a stage is complete when it has done so and all of them have landed.  (CTA 1's may
+      // land first.  It reuses a stage once `empty` says that the MMAs have read it, so never two phases ahead.)
       auto load_w = [&](int stage, int k, int item) {
-        mbar_arrive_expect_tx(&full[stage], (uint32_t)kPairStageBytes);
-        tma_load_2d(smem + stage * kPairStageBytes + kABytes, &wmap, k * kTileK, (item / mt % nt) * kPairN + rank * 128, &full[stage]);
+        if (rank == 0) mbar_arrive_expect_tx(&full[stage], 2u * kPairStageBytes);
+        pair_load_2d(smem + stage * kPairStageBytes + kABytes, &wmap, k * kTileK, (item / mt % nt) * kPairN + rank * 128, full0 + 8 * stage);
       };
       {  // the weights do not depend on the previous kernel, the activations do: fill the ring with weights first
         int k0, k1;
@@ -611,15 +639,18 @@ __global__ void __launch_bounds__(kPairThreads, 1) lm_gemm_pair_kernel(const __g
             break;
           }
           if (it >= ahead) load_w(st, k, item);
-          tma_load_2d(smem + st * kPairStageBytes, &amap, k * kTileK, (item % mt) * 2 * kTileM + rank * kTileM, &full[st]);
+          pair_load_2d(smem + st * kPairStageBytes, &amap, k * kTileK, (item % mt) * 2 * kTileM + rank * kTileM, full0 + 8 * st);
           if (++st == kPairStages) st = 0, ph ^= 1u;
         }
       }
       if (!ok) gave_up = 1;
-      // nothing in flight when the CTA leaves: the last copies of every stage have landed
-      for (int i = it > kPairStages ? it - kPairStages : 0; !ok && i < it; ++i) mbar_wait_bounded(&full[i % kPairStages], (i / kPairStages) & 1);
+      // nothing in flight when the CTA leaves.  (After a wait that ran out the phases of `full` say nothing about this CTA's copies:
+      // 10 ms is a thousand times what one takes.)
+      const long long t0 = clock64();
+      while (!ok && clock64() - t0 < (1ll << 24)) {
+      }
     }
-  } else if (warp == 1) {
+  } else if (warp == 1 && rank == 0) {
     const bool leader = elect_one_sync();
     const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kPairN >> 3) << 17) | ((uint32_t)(2 * kTileM >> 4) << 24);
     const uint32_t smem0 = (smem_u32(tc_smem_raw) + 1023u) & ~1023u;
@@ -630,37 +661,32 @@ __global__ void __launch_bounds__(kPairThreads, 1) lm_gemm_pair_kernel(const __g
       int k0, k1;
       k_range(item, k0, k1);
       const int buf = t & 1;
-      if (rank == 0 && t >= 2) ok = __all_sync(0xffffffffu, !gave_up && mbar_wait_bounded(&acc_empty[buf], ((t >> 1) & 1) ^ 1));
+      if (t >= 2) ok = __all_sync(0xffffffffu, !gave_up && pair_wait_bounded(&acc_empty[buf], ((t >> 1) & 1) ^ 1));
       tc_fence_after();
       for (int k = k0; k < k1 && ok; ++k) {
         ok = __all_sync(0xffffffffu, !gave_up && mbar_wait_bounded(&full[st], ph));
         if (!ok) break;
-        if (rank == 0) {
-          ok = __all_sync(0xffffffffu, !gave_up && mbar_wait_bounded(&peer_full[st], ph));
-          if (!ok) break;
-          tc_fence_after();
-          // (operands are values of the whole warp, outside of the elected lane's branch: see above)
-          const uint32_t a = smem0 + (uint32_t)(st * kPairStageBytes);
-          const uint64_t ad = swizzled_desc(a), bd = swizzled_desc(a + kABytes);
-          if (leader) {
+        tc_fence_after();
+        // (operands are values of the whole warp, outside of the elected lane's branch: see above)
+        const uint32_t a = smem0 + (uint32_t)(st * kPairStageBytes);
+        const uint64_t ad = swizzled_desc(a), bd = swizzled_desc(a + kABytes);
+        if (leader) {
 #pragma unroll
-            for (int j = 0; j < kTileK / 16; ++j)
-              pair_mma_f16(tmem + buf * kPairN, ad + j * 2, bd + j * 2, idesc, (k > k0 || j > 0) ? 1u : 0u);
-            pair_commit(&empty[st]);
-          }
-        } else if (leader) {
-          arrive_at_cta0(&peer_full[st]);
+          for (int j = 0; j < kTileK / 16; ++j)
+            pair_mma_f16(tmem + buf * kPairN, ad + j * 2, bd + j * 2, idesc, (k > k0 || j > 0) ? 1u : 0u);
+          pair_commit(&empty[st]);
         }
         __syncwarp();
         if (++st == kPairStages) st = 0, ph ^= 1u;
       }
-      if (ok && rank == 0 && leader) pair_commit(&acc_full[buf]);
+      if (ok && leader) pair_commit(&acc_full[buf]);
       __syncwarp();
     }
     if (!ok) gave_up = 1;
-  } else {
+  } else if (warp >= 2) {
     pdl_wait_prior();  // outputs may still be read by the kernel before
     const int quarter = warp & 3, c_begin = (warp - 2) / 4 * kPairEpiCols;
+    const uint32_t acc_empty0 = map_to_cta(acc_empty, 0);
     int t = 0;
     for (int item = pair; item < items; item += pairs, ++t) {
       const int buf = t & 1;
@@ -686,7 +712,7 @@ __global__ void __launch_bounds__(kPairThreads, 1) lm_gemm_pair_kernel(const __g
       }
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) arrive_at_cta0(&acc_empty[buf]);
+      if (lane == 0) arrive_at_cta0(acc_empty0 + 8 * buf);
     }
   }
   tc_fence_before();
