@@ -88,44 +88,65 @@ struct CkSmem {
   static_assert(kTotal <= 227 * 1024, "shared memory");
 };
 
-// mbar_wait_bounded on a shared-memory address, the whole warp: one outcome
+// mbar_wait_bounded on a shared-memory address, the whole warp: one outcome.  CLUSTER: for arrivals of the other CTA
+template <bool CLUSTER>
 __device__ __forceinline__ bool ck_try_wait(uint32_t bar, uint32_t parity) {
   uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(bar), "r"(parity)
-      : "memory");
+  if constexpr (CLUSTER)
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+  else
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
   return ok != 0;
 }
+template <bool CLUSTER>
 __device__ __noinline__ bool ck_wait_slow(uint32_t bar, uint32_t parity) {
   const long long t0 = clock64();
-  while (!ck_try_wait(bar, parity))
+  while (!ck_try_wait<CLUSTER>(bar, parity))
     if (clock64() - t0 > (1ll << 31)) {
       atomicOr(&g_device_status, kDevStatusTimeout);
       return false;
     }
   return true;
 }
+template <bool CLUSTER = false>
 __device__ __forceinline__ bool ck_wait(uint32_t bar, uint32_t parity) {
-  bool ok = ck_try_wait(bar, parity);
+  bool ok = ck_try_wait<CLUSTER>(bar, parity);
   if (__all_sync(0xffffffffu, ok)) return true;
-  ok = ok || ck_wait_slow(bar, parity);
+  ok = ok || ck_wait_slow<CLUSTER>(bar, parity);
   return __all_sync(0xffffffffu, ok);
 }
-// arrival on this CTA's barrier, or (a pair) on the one of CTA 0 that has its place there
+// Arrival on this CTA's barrier, or (from CTA 1 of a pair) on the one of CTA 0 that has its place there.  That one is relaxed: it hands
+// on tensor memory alone, which the tcgen05 waits and fences around it order between threads of a cluster.
 template <bool PAIR>
-__device__ __forceinline__ void ck_arrive(uint32_t bar) {
-  if constexpr (PAIR)
+__device__ __forceinline__ void ck_arrive(uint32_t bar, int rank) {
+  if (PAIR && rank != 0)
     asm volatile(
         "{\n\t.reg .b32 r;\n\t"
         "mapa.shared::cluster.u32 r, %0, 0;\n\t"
-        "mbarrier.arrive.shared::cluster.b64 _, [r];\n\t}" ::"r"(bar)
+        "mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [r];\n\t}" ::"r"(bar)
         : "memory");
   else
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+// ... that also hands on what this thread has seen arrive in shared memory
+__device__ __forceinline__ void ck_release_to_cta0(uint32_t bar) {
+  asm volatile(
+      "{\n\t.reg .b32 r;\n\t"
+      "mapa.shared::cluster.u32 r, %0, 0;\n\t"
+      "mbarrier.arrive.release.cluster.shared::cluster.b64 _, [r];\n\t}" ::"r"(bar)
+      : "memory");
 }
 // arrival once the MMAs issued so far have completed, on both CTAs' barriers for a pair
 template <bool PAIR>
@@ -213,7 +234,7 @@ __global__ void __launch_bounds__(kCkThreads, 1) w4a32_gemm_chunk_kernel(const _
   uint8_t* smem_ptr = smem_raw + (smem - smem_u32(smem_raw));
   const uint32_t raw_full = smem;                       // [kStages]  loaded data arrived
   const uint32_t raw_free = raw_full + kStages * 8;     // [kStages]  the MMAs that read a stage completed
-  const uint32_t a_full = raw_free + kStages * 8;       // [kAStages] operand written (a pair: by both, in CTA 0)
+  const uint32_t a_full = raw_free + kStages * 8;       // [kAStages] operand written (a pair: by both, in CTA 0; CTA 1's rows of x arrived)
   const uint32_t a_free = a_full + kAStages * 8;        // [kAStages] operand read
   const uint32_t acc_full = a_free + kAStages * 8;      // [2] a chunk's sums are complete
   const uint32_t acc_free = acc_full + 16;              // [2] ... and are in registers (a pair: both, in CTA 0)
@@ -248,7 +269,7 @@ __global__ void __launch_bounds__(kCkThreads, 1) w4a32_gemm_chunk_kernel(const _
     for (int i = 0; i < kBars; ++i) {
       const bool written = i >= 2 * kStages && i < 2 * kStages + kAStages;  // a_full: a warp writes two K-groups of its 32 rows
       const bool fetched = i >= kBars - 2;                                  // acc_free
-      mbar_init(&bars[i], (written ? 2 * kGroups : fetched ? kCkDqWarps : 1) * ((written || fetched) && kPair ? 2 : 1));
+      mbar_init(&bars[i], (written ? 2 * kGroups : fetched ? kCkDqWarps : 1) * ((written || fetched) && kPair ? 2 : 1) + (written && kPair ? 1 : 0));
     }
     mbar_fence_init();
   }
@@ -313,12 +334,12 @@ __global__ void __launch_bounds__(kCkThreads, 1) w4a32_gemm_chunk_kernel(const _
         for (int v = it * parts + parts - 1; v < (it + steps) * parts && ok; v += parts)
           // arrived on by warps that saw raw_full complete: orders the stage's copies too.  (Of two parts the last: the
           // same warps wrote the first before it.)
-          ok = ck_wait(a_full + (uint32_t)(v % kAStages) * 8, (uint32_t)(v / kAStages) & 1u);
+          ok = ck_wait<kPair>(a_full + (uint32_t)(v % kAStages) * 8, (uint32_t)(v / kAStages) & 1u);
         left -= steps;
 #pragma unroll
         for (int h = 0; h < kHalves; ++h) {
           const int slot = kPair ? h : c & 1, use = kPair ? c : c >> 1;
-          if (ok && accumulate == 0 && use > 0) ok = ck_wait(acc_free + (uint32_t)slot * 8, (uint32_t)(use - 1) & 1u);
+          if (ok && accumulate == 0 && use > 0) ok = ck_wait<kPair>(acc_free + (uint32_t)slot * 8, (uint32_t)(use - 1) & 1u);
           if (!ok) break;
           tc_fence_after();
           const uint32_t d = tmem_base + (uint32_t)(slot * S::kSlotCols);
@@ -359,6 +380,17 @@ __global__ void __launch_bounds__(kCkThreads, 1) w4a32_gemm_chunk_kernel(const _
           accumulate = 0;
         }
       }
+    } else {
+      // CTA 1 of a pair: its rows of x, read by instructions that CTA 0 issues, are announced there by a thread that saw them arrive
+      // (one that has nothing else to do: the release would hold up the dequant warps)
+      bool ok = true;
+      for (int v = 0; v < k_tiles * parts && ok; ++v) {
+        const int it = v / parts;
+        ok = ck_wait(raw_full + (uint32_t)(it % kStages) * 8, (uint32_t)(it / kStages) & 1u);
+        if (ok && v >= kAStages) ok = ck_wait(a_free + (uint32_t)(v % kAStages) * 8, (uint32_t)(v / kAStages - 1) & 1u);
+        if (ok && lane == 0) ck_release_to_cta0(a_full + (uint32_t)(v % kAStages) * 8);
+        __syncwarp();
+      }
     }
   } else {
     // ------------------------------------------------------------ dequant and sums
@@ -395,7 +427,7 @@ __global__ void __launch_bounds__(kCkThreads, 1) w4a32_gemm_chunk_kernel(const _
         }
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) ck_arrive<kPair>(acc_free + slot * 8);
+        if (lane == 0) ck_arrive<kPair>(acc_free + slot * 8, rank);
       }
     };
     const int own = kPair ? turn : turn >> 1, half = kPair ? 0 : turn & 1;  // stage of a span, pair of its K-groups
@@ -456,7 +488,7 @@ __global__ void __launch_bounds__(kCkThreads, 1) w4a32_gemm_chunk_kernel(const _
           tmem_st_wait();
           tc_fence_before();
           __syncwarp();
-          if (lane == 0) ck_arrive<kPair>(a_full + sa * 8);
+          if (lane == 0) ck_arrive<kPair>(a_full + sa * 8, rank);
         }
       }
       while (ok && drained_end <= span) drain();
