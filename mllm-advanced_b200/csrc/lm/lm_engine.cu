@@ -232,10 +232,11 @@ int create(Engine* e, const mllmb200_lm_layer* descs) {
   e->f32 = c.dtype == MLLMB200_LM_F32;
   e->elt = e->f32 ? 4 : 2;
   e->widthp = pad_to(c.width, 64);
-  if (e->widthp > 8192 || (size_t)c.conv_taps * e->widthp * 4 > 200 * 1024) return fail(e, MLLMB200_UNSUPPORTED, "width %d with %d taps", c.width, c.conv_taps);
+  if (e->widthp > 8192 || (size_t)c.conv_taps * e->widthp * 4 > kNormSmemMax) return fail(e, MLLMB200_UNSUPPORTED, "width %d with %d taps", c.width, c.conv_taps);
   LM_CUDA(cudaStreamCreateWithFlags(&e->stream, cudaStreamNonBlocking));
   LM_CUDA(cudaEventCreateWithFlags(&e->meta_free, cudaEventDisableTiming));
   LM_CUDA(linear_configure());
+  LM_CUDA(norm_configure());
   LM_CUDA(attention_configure());
   LM_CUDA(retention_configure());
   LM_CUDA(latent_configure());

@@ -377,28 +377,37 @@ __global__ void __launch_bounds__(kRowsWarps<NVW> * 32) lm_norm_rows_kernel(Norm
   }
 }
 
+template <int NVW>
+constexpr size_t rows_smem(int ldx) { return (size_t)kRowsWarps<NVW> * ldx * sizeof(float); }
+
 template <class T, int NVW>
 cudaError_t launch_norm_rows(cudaStream_t s, NormArgs a) {
   const int halo = a.taps ? a.taps - 1 : 0;
   a.rows_per_cta = std::min(std::max(4, (a.rows + kSms - 1) / kSms), kRowsWarps<NVW> - halo);
   const dim3 grid((a.rows + a.rows_per_cta - 1) / a.rows_per_cta), block(kRowsWarps<NVW> * 32);
   if (a.taps == 0) return launch_pdl(lm_norm_rows_kernel<T, NVW, false>, grid, block, 0, s, a);
-  const size_t smem = (size_t)kRowsWarps<NVW> * a.ldx * sizeof(float);  // 192 KB at the widest, 4096
-  if (smem > 40 * 1024) {
-    const cudaError_t r = cudaFuncSetAttribute(lm_norm_rows_kernel<T, NVW, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (r != cudaSuccess) return r;
-  }
-  return launch_pdl(lm_norm_rows_kernel<T, NVW, true>, grid, block, smem, s, a);
+  return launch_pdl(lm_norm_rows_kernel<T, NVW, true>, grid, block, rows_smem<NVW>(a.ldx), s, a);
 }
 
 template <class T, int NV>
 cudaError_t launch_norm_nv(cudaStream_t s, const NormArgs& a) {
   const size_t smem = (size_t)a.taps * a.ldx * sizeof(float);
-  if (smem > 48 * 1024) {
-    const cudaError_t r = cudaFuncSetAttribute(lm_norm_kernel<T, NV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (r != cudaSuccess) return r;
-  }
   return launch_pdl(lm_norm_kernel<T, NV>, dim3((a.rows + a.rows_per_cta - 1) / a.rows_per_cta), dim3(kNormThreads), smem, s, a);
+}
+// The most that any engine asks of each kernel, set when an engine is made: the limit belongs to the function, so a launch that set it to
+// its own need would lower it under the launch of an engine of another width in another thread.
+template <class T>
+cudaError_t configure_norm_t() {
+  const auto most = [](auto* f, size_t bytes) { return cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes); };
+  cudaError_t r = most(lm_norm_rows_kernel<T, 8, true>, rows_smem<8>(1024));
+  if (r == cudaSuccess) r = most(lm_norm_rows_kernel<T, 12, true>, rows_smem<12>(1536));
+  if (r == cudaSuccess) r = most(lm_norm_rows_kernel<T, 16, true>, rows_smem<16>(2048));
+  if (r == cudaSuccess) r = most(lm_norm_rows_kernel<T, 32, true>, rows_smem<32>(4096));
+  if (r == cudaSuccess) r = most(lm_norm_kernel<T, 1>, kNormSmemMax);
+  if (r == cudaSuccess) r = most(lm_norm_kernel<T, 2>, kNormSmemMax);
+  if (r == cudaSuccess) r = most(lm_norm_kernel<T, 4>, kNormSmemMax);
+  if (r == cudaSuccess) r = most(lm_norm_kernel<T, 8>, kNormSmemMax);
+  return r;
 }
 template <class T>
 cudaError_t launch_norm_t(cudaStream_t s, const NormArgs& a) {
@@ -643,6 +652,10 @@ __global__ void __launch_bounds__(256) lm_argmax_kernel(const float* __restrict_
 
 }  // namespace
 
+cudaError_t norm_configure() {
+  const cudaError_t r = configure_norm_t<float>();
+  return r != cudaSuccess ? r : configure_norm_t<__nv_bfloat16>();
+}
 cudaError_t launch_norm(cudaStream_t s, bool f32, const NormArgs& a) {
   return f32 ? launch_norm_t<float>(s, a) : launch_norm_t<__nv_bfloat16>(s, a);
 }

@@ -178,6 +178,8 @@ cudaError_t launch_pack_heads_transposed(cudaStream_t s, const __nv_bfloat16* sr
                                          int rankp, int dimp);
 cudaError_t launch_pack_rows(cudaStream_t s, const __nv_bfloat16* src, int n, int k, __nv_bfloat16* dst, int ldk, int row_block,
                              int row_block_pad, int row_mul, int row_off, int col_block, int col_block_pad);
+constexpr size_t kNormSmemMax = 200 * 1024;  // taps x padded width in fp32, at most
+cudaError_t norm_configure();
 cudaError_t launch_norm(cudaStream_t s, bool f32, const NormArgs& a);
 cudaError_t launch_post_norm(cudaStream_t s, bool f32, const PostNormArgs& a);
 bool fused_router(int rows);  // whether launch_post_norm takes a router with that many rows

@@ -2,6 +2,7 @@
 of a block recomputed) and one token a sequence, over taps and widths at the edges of what a thread and a warp hold."""
 import os
 import sys
+import threading
 
 import numpy as np
 import pytest
@@ -35,3 +36,34 @@ def test_convolution_in_steps(width, taps, dtype, tmp_path):
     for g, o, a in zip(got, want, at):
         c.check(np.concatenate(g), o[:a])
     c.model.close()
+
+
+def test_engines_of_two_widths_in_two_threads(tmp_path):
+    """Widths that share the kernels of the norms but not the shared memory these ask for: neither engine's launches may set a limit
+    that the other's, from another host thread, then exceed."""
+    cases = []
+    for width in (1152, 1536):  # many rows: one instance; and one instance of the kernel for many taps
+        for taps in (4, 12):
+            cfg = M.config(width, 60, [M.layer("attention", M.attention(1, 1, 16, 16, 25))] * 4, taps=taps)
+            c = Case(M.write(tmp_path / f"{width}_{taps}", cfg, M.weights(cfg, 5)), V, cfg, None, "bfloat16", max_seqs=1, max_ctx=320, max_rows=320)
+            toks = c.tokens(300)
+            cases.append((c, toks, c.run(toks)))
+    errors = []
+
+    def step(c, toks, want):
+        try:
+            for _ in range(150):
+                slot = c.model.acquire()
+                got = c.model.step([(slot, toks)], list(range(len(toks))))
+                c.model.release(slot)
+                np.testing.assert_array_equal(got, want)
+        except Exception as e:
+            errors.append(e)
+    jobs = [threading.Thread(target=step, args=a) for a in cases]
+    for j in jobs:
+        j.start()
+    for j in jobs:
+        j.join()
+    for c, _, _ in cases:
+        c.model.close()
+    assert not errors, errors[0]
