@@ -167,6 +167,10 @@ MLLMB200_API int mllmb200_w4a32_linear_forward_grouped(const float* x_dev, int M
  * itself, above the form with chunked sums). */
 MLLMB200_API int mllmb200_w4a32_select_kernel(int M, int K, int N);
 
+/* What linear_forward_ex launches for kernel = 0 or 5 (with its flags): 1, 2, 3, 4 or 7 as above, 8 the tcgen05 tile GEMM with
+ * chunked sums; 0 for other arguments.  Host only, for tests. */
+MLLMB200_API int mllmb200_w4a32_plan_kernel(int M, int K, int N, int kernel);
+
 /* Several INDEPENDENT linears in one launch: count in [1,8] matrices [N[i], K[i]], each with its own
  * activations x_dev[i] [M, ldx[i]] (pointers may repeat) and output y_dev[i] [M, ldy[i]], M <= 4.  The
  * seven linears of one decoder layer at decode are such a set.  Every matrix gets a
@@ -392,8 +396,7 @@ MLLMB200_API int mllmb200_qwen2_batch_read(void* handle, int seq, int first, int
  *   linear_forward_tp  y[:, r N/g : (r+1) N/g] = x W_r^T + b_r on this rank, delivered to all ranks:
  *                    gather_mode 2 = the kernels' epilogues store every finished element into every rank's buffer
  *                    (plain stores over NVLink while other tiles are still computed: the single-launch GEMV for
- *                    M <= 4, the fp16 tensor-core GEMM for kernel policies 4 / 5 at M >= 128, and from M = 64 for
- *                    shards of at least 8192 rows with K <= 4096; other kernels
+ *                    M <= 4, the fp16 tensor-core GEMM where `kernel` is 4 or 5 takes it for the shard; other kernels
  *                    compute the block and push it with strided device copies), then each rank flags every peer
  *                    and waits - bounded, MLLMB200_TIMEOUT through mllmb200_check_device_status - for theirs;
  *                    1 = NCCL baseline (ncclAllGather of the blocks + a re-assembly kernel; needs the
@@ -401,6 +404,7 @@ MLLMB200_API int mllmb200_qwen2_batch_read(void* handle, int seq, int first, int
  *                    N must be a multiple of 32 * nranks.  All ranks must make the same sequence of calls.
  *                    Not capturable in a CUDA graph (a call counter is baked into the launches).
  *   tp_output        the buffer again (device pointer, bytes).
+ *   tp_peer_kernel   whose epilogue gather mode 2 uses for a shard: 1 the GEMV, 4 the fp16 tensor-core GEMM, 0 none (host only).
  * ------------------------------------------------------------------------------------------ */
 MLLMB200_API int mllmb200_w4a32_tp_init(int nranks, int rank, void* nccl_comm, void** handle);
 MLLMB200_API int mllmb200_w4a32_tp_alloc_output(void* handle, size_t y_bytes, float** y_dev, void* stream);
@@ -409,6 +413,7 @@ MLLMB200_API int mllmb200_w4a32_tp_ipc_import(void* handle, const void* all_blob
 MLLMB200_API int mllmb200_w4a32_linear_forward_tp(void* handle, const float* x_dev, const void* tiled_shard_dev,
                                                   void* ws_dev, int M, int K, int N_total, int ldx, int kernel,
                                                   int gather_mode, void* stream);
+MLLMB200_API int mllmb200_w4a32_tp_peer_kernel(int M, int K, int N_shard, int kernel);
 MLLMB200_API int mllmb200_w4a32_tp_output(void* handle, float** y_dev, size_t* bytes);
 MLLMB200_API void mllmb200_w4a32_tp_destroy(void* handle);
 

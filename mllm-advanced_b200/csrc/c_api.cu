@@ -90,12 +90,10 @@ static inline size_t ws_rec_bytes(int m, int k) {
   big = big > mma ? big : mma;
   return align_up(big > blk16 ? big : blk16, 256);
 }
-size_t w4a32_ws_rec_bytes(int m, int k) { return ws_rec_bytes(m, k); }  // for tp.cu
 // the K-split counters of the fp16 tile GEMM: behind the row headers of a workspace of workspace_size(m, k) bytes
-int* w4a32_ws_split_sync(void* ws_dev, int m, int k) {
+static int* ws_split_sync(void* ws_dev, int m, int k) {
   return reinterpret_cast<int*>(static_cast<uint8_t*>(ws_dev) + ws_rec_bytes(m, k) + align_up((size_t)m * sizeof(float2), 256));
 }
-int w4a32_ws_split_sync_ints() { return kSplitSyncInts; }
 
 static W4Blocks blocks_at(W4Form form, int M, int K, int m_pad, void* ws) {
   W4Blocks b = {};
@@ -105,7 +103,7 @@ static W4Blocks blocks_at(W4Form form, int M, int K, int m_pad, void* ws) {
   b.blocks = static_cast<uint8_t*>(ws);
   if (!ws) return b;
   b.hdr = reinterpret_cast<float2*>(b.blocks + ws_rec_bytes(M, K));
-  if (form == kW4Tile) b.clear = w4a32_ws_split_sync(ws, M, K), b.clear_count = kSplitSyncInts;
+  if (form == kW4Tile) b.clear = ws_split_sync(ws, M, K), b.clear_count = kSplitSyncInts;
   return b;
 }
 W4Blocks w4a32_blocks_for(int M, int K, int count, const int* N, int policy_and_flags, void* ws) {
@@ -125,6 +123,7 @@ W4Blocks w4a32_blocks_for(int M, int K, int count, const int* N, int policy_and_
   for (int i = 0; i < count && tiles; ++i) tiles = mllmb200_w4a32_select_kernel(M, K, N[i]) == 3;
   return tiles ? blocks_at(kW4Chunk, M, K, 0, ws) : none;
 }
+W4Blocks w4a32_tile_blocks(int M, int K, int N, void* ws) { return blocks_at(kW4Tile, M, K, w4a32_gemm_tcf16_m_pad(M, N), ws); }
 cudaError_t w4a32_forward_blocks(const W4Blocks& b, int M, int K, int count, const void* const* tiled, float* const* y, const int* N,
                                  const int* ldy, int use_pdl, cudaStream_t stream) {
   switch (b.form) {
@@ -246,6 +245,16 @@ int mllmb200_w4a32_select_kernel(int M, int K, int N) {
   return 2;
 }
 
+int mllmb200_w4a32_plan_kernel(int M, int K, int N, int kernel) {
+  if (M <= 0 || K <= 0 || N <= 0 || ((kernel & 0xFF) != 0 && (kernel & 0xFF) != 5)) return 0;
+  switch (w4a32_blocks_for(M, K, 1, &N, kernel, nullptr).form) {
+    case kW4Stream: return 7;
+    case kW4Tile: return 4;
+    case kW4Chunk: return 8;
+    default: return mllmb200_w4a32_select_kernel(M, K, N);
+  }
+}
+
 // Shared front half of every forward: validate, quantize the activations into the workspace.
 static int quantize_into_ws(const float* x_dev, void* ws_dev, int M, int K, int ldx, int use_pdl, cudaStream_t st,
                             uint8_t** a_rec, float2** a_hdr, bool tc_blocks = false) {
@@ -305,7 +314,7 @@ int mllmb200_w4a32_linear_forward_ex(const float* x_dev, const void* tiled_dev, 
   if (kernel == 3 && !w4a32_gemm_tc_supported(M, K, N)) return MLLMB200_UNSUPPORTED;
   if (kernel == 4) {  // fp16 tensor-core path: its own activation layout
     if (!w4a32_gemm_tcf16_supported(M, K, N)) return MLLMB200_UNSUPPORTED;
-    return forward_through_blocks(blocks_at(kW4Tile, M, K, w4a32_gemm_tcf16_m_pad(M, N), ws_dev), x_dev, M, K, ldx, 1, &tiled_dev, &y_dev, &N, &ldy,
+    return forward_through_blocks(w4a32_tile_blocks(M, K, N, ws_dev), x_dev, M, K, ldx, 1, &tiled_dev, &y_dev, &N, &ldy,
                                   use_pdl, st);
   }
   uint8_t* a_rec;

@@ -25,6 +25,8 @@ struct W4Blocks {
 // What linear_forward_ex (count 1) or linear_forward_grouped with policy 0 or 5 (and the flag of fp16-encoded scales) runs for these
 // shapes, with its places in a workspace of workspace_size(M, K) bytes.
 W4Blocks w4a32_blocks_for(int M, int K, int count, const int* N, int policy_and_flags, void* ws);
+// The places of kernel 4 by name (gemm_tcf16.cu).
+W4Blocks w4a32_tile_blocks(int M, int K, int N, void* ws);
 // The launch behind the blocks.
 cudaError_t w4a32_forward_blocks(const W4Blocks& b, int M, int K, int count, const void* const* tiled, float* const* y, const int* N,
                                  const int* ldy, int use_pdl, cudaStream_t stream);

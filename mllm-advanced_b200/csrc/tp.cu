@@ -26,24 +26,31 @@
 
 #include "../../include/mllmb200.h"
 #include "device_common.cuh"
+#include "linear_blocks.h"
 
 namespace mllmb200 {
 int record_cuda_failure(cudaError_t e);
-size_t w4a32_ws_rec_bytes(int m, int k);
-int* w4a32_ws_split_sync(void* ws_dev, int m, int k);
-int w4a32_ws_split_sync_ints();
 cudaError_t launch_w4a32_gemv_stream(int count, const float* const* x, const int* ldx, const uint8_t* const* a_rec,
                                      const float2* const* a_hdr, int m, const int* k, const void* const* tiled,
                                      float* const* y, const int* n, const int* ldy, int use_pdl, cudaStream_t stream,
                                      int num_peers, float* const* y_peers);
 bool w4a32_gemv_stream_supported(int m, int count, const int* k, const int* n);
 bool w4a32_gemm_tcf16_preferred(int m, int k, int n);
-int w4a32_gemm_tcf16_m_pad(int m, int n);
 cudaError_t launch_act_quant_blocks_f16(const float*, int, int, int, int, uint8_t*, float2*, cudaStream_t, int use_pdl = 0,
                                         int* clear_ints = nullptr, int clear_count = 0);
 cudaError_t launch_w4a32_gemm_tcf16_grouped(const uint8_t*, const float2*, int, int, int, const void* const*, float* const*,
                                             const int*, const int*, cudaStream_t, int num_peers, float* const* y_peers,
                                             int use_pdl = 0, int* split_sync = nullptr, int split_sync_ints = 0);
+
+// Gather mode 2: the kernel whose epilogue stores into the peers' y (1 the GEMV, 4 the fp16 tile GEMM), where that is also what
+// linear_forward_ex - gather modes 0 and 1 - runs for the shard: the modes have the same bits.  0: another kernel computes the
+// shard, the block is pushed with device copies.
+static int peer_kernel(int M, int K, int n_shard, int kernel) {
+  const int policy = kernel & 0xFF;
+  if (M <= 4 && (policy == 0 || policy == 1 || policy == 5) && w4a32_gemv_stream_supported(M, 1, &K, &n_shard)) return 1;
+  if (policy == 4) return w4a32_gemm_tcf16_preferred(M, K, n_shard) ? 4 : 0;
+  return policy == 5 && w4a32_blocks_for(M, K, 1, &n_shard, kernel, nullptr).form == kW4Tile ? 4 : 0;
+}
 
 constexpr int kTpMaxRanks = 8;
 constexpr long long kTpWaitTicks = 1ll << 32;  // ~2 s: ranks reach a collective call milliseconds apart at worst
@@ -223,7 +230,6 @@ int mllmb200_w4a32_linear_forward_tp(void* handle, const float* x_dev, const voi
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   float* y_blk = h->y_local + (size_t)r * nl;  // this rank's column block inside the full [M, N_total]
   const int use_pdl = (kernel >> 8) & 1;
-  const int policy = kernel & 0xFF;
 
   if (gather_mode == 0 || g == 1) {
     return mllmb200_w4a32_linear_forward_ex(x_dev, tiled_shard_dev, y_blk, ws_dev, M, K, nl, ldx, N_total, kernel, stream);
@@ -258,18 +264,15 @@ int mllmb200_w4a32_linear_forward_tp(void* handle, const float* x_dev, const voi
   cudaError_t e = cudaSuccess;
   const void* tiled = tiled_shard_dev;
   int ldy = N_total;
-  if (M <= 4 && (policy == 0 || policy == 1 || policy == 5) && w4a32_gemv_stream_supported(M, 1, &K, &nl)) {
+  const int by = peer_kernel(M, K, nl, kernel);
+  if (by == 1) {
     e = launch_w4a32_gemv_stream(1, &x_dev, &ldx, nullptr, nullptr, M, &K, &tiled, &y_blk, &nl, &ldy, use_pdl, s, np, peers);
-  } else if ((policy == 4 || policy == 5) && w4a32_gemm_tcf16_preferred(M, K, nl)) {
+  } else if (by == 4) {
     if (!ws_dev || (reinterpret_cast<uintptr_t>(ws_dev) & 255u)) return MLLMB200_INVALID_ARG;
-    uint8_t* blocks = static_cast<uint8_t*>(ws_dev);
-    float2* hdr = reinterpret_cast<float2*>(blocks + w4a32_ws_rec_bytes(M, K));
-    // with the K-split counters, as the public forward: every gather mode computes a shard with the same launch
-    int* sync = w4a32_ws_split_sync(ws_dev, M, K);
-    const int sync_ints = w4a32_ws_split_sync_ints();
-    e = launch_act_quant_blocks_f16(x_dev, M, w4a32_gemm_tcf16_m_pad(M, nl), K, ldx, blocks, hdr, s, 0, sync, sync_ints);
+    const W4Blocks b = w4a32_tile_blocks(M, K, nl, ws_dev);
+    e = launch_act_quant_blocks_f16(x_dev, M, b.m_pad, K, ldx, b.blocks, b.hdr, s, 0, b.clear, b.clear_count);
     if (e == cudaSuccess)
-      e = launch_w4a32_gemm_tcf16_grouped(blocks, hdr, M, K, 1, &tiled, &y_blk, &nl, &ldy, s, np, peers, 0, sync, sync_ints);
+      e = launch_w4a32_gemm_tcf16_grouped(b.blocks, b.hdr, M, K, 1, &tiled, &y_blk, &nl, &ldy, s, np, peers, 0, b.clear, b.clear_count);
   } else {
     // kernels without a peer epilogue: compute the block, then push it to every peer with strided device copies
     const int st = mllmb200_w4a32_linear_forward_ex(x_dev, tiled_shard_dev, y_blk, ws_dev, M, K, nl, ldx, N_total, kernel, stream);
@@ -285,6 +288,10 @@ int mllmb200_w4a32_linear_forward_tp(void* handle, const float* x_dev, const voi
   tp_signal_wait_kernel<<<1, 32, 0, s>>>(fp, h->flags_local, g, r, epoch, kTpWaitTicks);
   e = cudaGetLastError();
   return e == cudaSuccess ? MLLMB200_OK : tp_fail(e);
+}
+
+int mllmb200_w4a32_tp_peer_kernel(int M, int K, int N_shard, int kernel) {
+  return M > 0 && K > 0 && N_shard > 0 ? peer_kernel(M, K, N_shard, kernel) : 0;
 }
 
 int mllmb200_w4a32_tp_output(void* handle, float** y_dev, size_t* bytes) {

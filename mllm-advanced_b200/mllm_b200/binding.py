@@ -56,6 +56,8 @@ def lib():
         "mllmb200_w4a32_linear_forward_grouped": ([vp, C.c_int, C.c_int, C.c_int, C.c_int, vp, vp, vp, vp, vp, C.c_int,
                                                    vp], C.c_int),
         "mllmb200_w4a32_select_kernel": ([C.c_int, C.c_int, C.c_int], C.c_int),
+        "mllmb200_w4a32_plan_kernel": ([C.c_int] * 4, C.c_int),
+        "mllmb200_w4a32_tp_peer_kernel": ([C.c_int] * 4, C.c_int),
         "mllmb200_w4a32_gemv_trace": ([vp, C.c_int], C.c_int),
         "mllmb200_w4a32_gemv_plan_check": ([C.c_int, C.c_int, int_p, int_p, int_p, int_p, int_p, int_p, sz_p], C.c_int),
         "mllmb200_w4a32_linear_forward_multi": ([C.c_int, vp, int_p, int_p, vp, vp, int_p, int_p, C.c_int, C.c_int, vp], C.c_int),

@@ -119,6 +119,22 @@ def test_default_kernel_by_batch_size():
     assert L.mllmb200_w4a32_select_kernel(8, 32768, 64) == mb.KERNEL_STREAM_TC               # ... but those of 8 rows do
 
 
+def test_peer_stores_come_from_the_kernel_that_the_forward_runs():
+    """Tensor-parallel gather modes 0 and 1 run the public forward for a shard; the one that stores into the peers from a kernel's epilogue
+    does so only with that same kernel (same bits), and does for each of the kernels that can."""
+    L, seen = mb.lib(), set()
+    for m in (1, 4, 5, 64, 65, 127, 128, 160, 192, 193, 200, 512):
+        for k in (896, 1536, 8960):
+            for n in (32, 256, 1536, 4096, 4128, 8192, 17920):
+                for kernel in (0, 5, 5 | 0x100, 5 | 0x200):
+                    peer, own = L.mllmb200_w4a32_tp_peer_kernel(m, k, n, kernel), L.mllmb200_w4a32_plan_kernel(m, k, n, kernel)
+                    assert peer in (0, own) and own, (m, k, n, kernel, peer, own)
+                    assert (peer != 0) == (own in (1, 4)), (m, k, n, kernel, peer, own)
+                    seen.add((peer, own))
+    assert {(1, 1), (4, 4), (0, 7), (0, 8)} <= seen
+    assert L.mllmb200_w4a32_plan_kernel(128, 1536, 1536, 5) == 7 and L.mllmb200_w4a32_plan_kernel(193, 1536, 1536, 5) == 4
+
+
 def test_workspace_covers_the_tile_gemms_up_to_their_last_row():
     """Where the default takes a tile GEMM above 64 rows, the workspace holds its fp16 activation blocks (64 bytes per row and
     K-group, rows in eights) and the rows' headers; beyond the rows that its launch can cover it takes no tile GEMM."""

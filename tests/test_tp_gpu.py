@@ -93,7 +93,7 @@ def _worker(rank, world, port, results):
         full = mbw.W4A32Weights.from_blob(blob)
         tpl = tp.TensorParallelLinear(blob, 256)
         g = torch.Generator(device="cuda").manual_seed(11)
-        for m, kern in ((1, 0), (3, 0), (8, 0), (64, 0), (200, 5), (256, 4)):
+        for m, kern in ((1, 0), (3, 0), (8, 0), (64, 0), (128, 5), (192, 5), (200, 5), (256, 4)):
             x = torch.randn((m, k), device="cuda", generator=g)
             ref = mbw.linear_forward(x, full, kernel=kern)
             for mode in (tp.GATHER_PEER_STORES, tp.GATHER_NCCL):
@@ -103,7 +103,7 @@ def _worker(rank, world, port, results):
                 y = tpl.forward(x, gather=mode, kernel=kern)
                 torch.cuda.synchronize()
                 mbw.check_device_status()
-                if m <= 4 or kern in (4, 5):
+                if m <= 4 or mbw.lib().mllmb200_w4a32_plan_kernel(m, k, n // world, kern) == 4 or kern == 4:
                     # the GEMV shard splits K over its CTAs differently from the full matrix, and the fp16 tile GEMM
                     # splits K in two on launches that fill under half of the GPU and on the tiles left over after
                     # a launch's last full wave - which tiles those are differs between the full matrix and its
