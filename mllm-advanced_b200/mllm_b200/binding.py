@@ -200,19 +200,24 @@ class W4A32Weights:
         return out.cpu().numpy()
 
 
-_ws_cache = {}
+@functools.lru_cache(maxsize=4096)  # a function of four numbers
+def _scratch_size(m, k, n, kernel):
+    """Bytes of workspace that a call needs: none where the GEMV quantizes x itself."""
+    if kernel == KERNEL_GEMV or (kernel in (KERNEL_AUTO, KERNEL_FASTEST) and lib().mllmb200_w4a32_plan_kernel(m, k, n, kernel) == KERNEL_GEMV):
+        return 0
+    return workspace_size(m, k)
 
 
-def _workspace_for(m, k, device):
-    """One cached workspace per device, grown on demand (the op keeps its own in the C++ backend)."""
+def scratch(nbytes, x, stream):
+    """Memory of one call, from torch's allocator on the stream that the call runs on: calls on other streams, or from other threads,
+    have memory of their own, and what a call drops is reused in its stream's order.  (The op keeps its own in the C++ backend.)"""
     import torch
-    need = workspace_size(m, k)
-    key = device.index
-    ws = _ws_cache.get(key)
-    if ws is None or ws.numel() < need:
-        ws = torch.empty(need, dtype=torch.uint8, device=device)
-        _ws_cache[key] = ws
-    return ws
+    if nbytes == 0:
+        return None
+    if stream is None:
+        return x.new_empty((nbytes,), dtype=torch.uint8)
+    with torch.cuda.stream(stream):
+        return x.new_empty((nbytes,), dtype=torch.uint8)
 
 
 def linear_forward(x, weights, out=None, workspace=None, kernel=KERNEL_AUTO, stream=None, pdl=False):
@@ -224,9 +229,9 @@ def linear_forward(x, weights, out=None, workspace=None, kernel=KERNEL_AUTO, str
     if out is None:
         out = x.new_empty((m, weights.n))
     if workspace is None:
-        workspace = _workspace_for(m, k, x.device)
+        workspace = scratch(_scratch_size(m, k, weights.n, kernel), x, stream)
     _check(lib().mllmb200_w4a32_linear_forward_ex(x.data_ptr(), weights.tiled.data_ptr(), out.data_ptr(),
-                                                  workspace.data_ptr(), m, k, weights.n, x.stride(0), out.stride(0),
+                                                  None if workspace is None else workspace.data_ptr(), m, k, weights.n, x.stride(0), out.stride(0),
                                                   kernel | (KERNEL_FLAG_PDL if pdl else 0) | weights.kernel_flags,
                                                   _stream_ptr(stream)),
            "linear_forward")
@@ -244,13 +249,13 @@ def linear_forward_grouped(x, weights_list, outs=None, workspace=None, stream=No
     if outs is None:
         outs = [torch.empty((m, w.n), dtype=torch.float32, device=x.device) for w in weights_list]
     if workspace is None:
-        workspace = _workspace_for(m, k, x.device)
+        workspace = scratch(max(_scratch_size(m, k, w.n, policy) for w in weights_list), x, stream)
     tiled = (C.c_void_p * cnt)(*[w.tiled.data_ptr() for w in weights_list])
     ys = (C.c_void_p * cnt)(*[o.data_ptr() for o in outs])
     ns = (C.c_int * cnt)(*[w.n for w in weights_list])
     ldy = (C.c_int * cnt)(*[o.stride(0) for o in outs])
     _check(lib().mllmb200_w4a32_linear_forward_grouped(x.data_ptr(), m, k, x.stride(0), cnt, tiled, ys, ns, ldy,
-                                                       workspace.data_ptr(),
+                                                       None if workspace is None else workspace.data_ptr(),
                                                        (KERNEL_FLAG_PDL if pdl else 0) | policy | weights_list[0].kernel_flags,
                                                        _stream_ptr(stream)), "linear_forward_grouped")
     return outs
@@ -322,7 +327,7 @@ def conv3d_forward(x, weights, kernel, stride, stream=None):
     assert k.value == weights.k, (k.value, weights.k)
     ot, oh, ow = [(x.shape[2 + i] - kernel[i]) // stride[i] + 1 for i in range(3)]
     y = torch.empty((x.shape[0], weights.n, ot, oh, ow), dtype=torch.float32, device=x.device)
-    ws = torch.empty(wsb.value + 256, dtype=torch.uint8, device=x.device)
+    ws = scratch(wsb.value + 256, x, stream)
     off = (-ws.data_ptr()) % 256
     _check(lib().mllmb200_conv3d_w4a32_forward(x.data_ptr(), weights.tiled.data_ptr(), y.data_ptr(), ws.data_ptr() + off,
                                                shp, ker, strd, weights.n, _stream_ptr(stream)), "conv3d_forward")

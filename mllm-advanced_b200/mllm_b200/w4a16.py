@@ -6,7 +6,7 @@ import functools
 
 import numpy as np
 
-from .binding import _check, _stream_ptr, lib
+from .binding import _check, _stream_ptr, lib, scratch
 
 
 def prepack_size(n, k, has_bias):
@@ -93,7 +93,7 @@ def linear_forward(x, weights, out=None, workspace=None, stream=None, kernel=KER
     if out is None:
         out = x.new_empty((m, weights.n), dtype=torch.float16)
     if workspace is None:
-        workspace = x.new_empty((workspace_size(m, k, weights.n),), dtype=torch.uint8)
+        workspace = scratch(workspace_size(m, k, weights.n), x, stream)
     _check(lib().mllmb200_w4a16_linear_forward_ex(x.data_ptr(), 1 if x.dtype == torch.float16 else 0,
                                                   weights.tiled.data_ptr(), out.data_ptr(), workspace.data_ptr(), m, k,
                                                   weights.n, x.stride(0), out.stride(0), kernel | (0x100 if pdl else 0),
@@ -112,7 +112,7 @@ def linear_forward_grouped(x, weights_list, outs=None, workspace=None, stream=No
     if outs is None:
         outs = [torch.empty((m, w.n), dtype=torch.float16, device=x.device) for w in weights_list]
     if workspace is None:
-        workspace = torch.empty(max(workspace_size(m, k, w.n) for w in weights_list), dtype=torch.uint8, device=x.device)
+        workspace = scratch(max(workspace_size(m, k, w.n) for w in weights_list), x, stream)
     tiled = (C.c_void_p * cnt)(*[w.tiled.data_ptr() for w in weights_list])
     ys = (C.c_void_p * cnt)(*[o.data_ptr() for o in outs])
     ns = (C.c_int * cnt)(*[w.n for w in weights_list])
