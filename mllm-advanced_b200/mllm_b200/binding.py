@@ -186,15 +186,19 @@ class W4A32Weights:
         row_count = n - row_begin if row_count is None else row_count
         blob_dev = torch.from_numpy(blob).to(device)
         tiled = torch.empty(tiled_size(row_count, k), dtype=torch.uint8, device=device)
+        if stream is not None:
+            torch.cuda.current_stream().synchronize()  # which copies the blob, and may still use what tiled's memory was
         _check(lib().mllmb200_w4a32_repack_device(blob_dev.data_ptr(), n, k, sm, hb, row_begin, row_count,
                                                   tiled.data_ptr(), _stream_ptr(stream)), "repack_device")
-        torch.cuda.current_stream().synchronize()  # blob_dev is released when this returns
+        (stream or torch.cuda.current_stream()).synchronize()  # blob_dev is released when this returns
         return W4A32Weights(tiled, row_count, k, sm, hb, row_begin, n)
 
     def unpack(self, stream=None):
         """Tile layout -> host blob (inverse of the repack), for round-trip checks."""
         import torch
         out = torch.zeros(prepack_size(self.n, self.k, self.has_bias), dtype=torch.uint8, device=self.tiled.device)
+        if stream is not None:
+            torch.cuda.current_stream().synchronize()
         _check(lib().mllmb200_w4a32_unpack_device(self.tiled.data_ptr(), self.n, self.k, out.data_ptr(),
                                                   _stream_ptr(stream)), "unpack_device")
         return out.cpu().numpy()

@@ -74,9 +74,11 @@ class W4A16Weights:
         row_count = n - row_begin if row_count is None else row_count
         blob_dev = torch.from_numpy(blob).to(device)
         tiled = torch.empty(tiled_size(row_count, k), dtype=torch.uint8, device=device)
+        if stream is not None:
+            torch.cuda.current_stream().synchronize()  # which copies the blob, and may still use what tiled's memory was
         _check(lib().mllmb200_w4a16_repack_device(blob_dev.data_ptr(), n, k, hb, row_begin, row_count,
                                                   tiled.data_ptr(), _stream_ptr(stream)), "w4a16_repack_device")
-        torch.cuda.current_stream().synchronize()  # blob_dev is released when this returns
+        (stream or torch.cuda.current_stream()).synchronize()  # blob_dev is released when this returns
         return W4A16Weights(tiled, row_count, k, hb, row_begin, n)
 
 

@@ -46,6 +46,19 @@ def _wrong(calls, order, stream, own):
     return [i for i, y in got if not torch.equal(y, calls[i][1])]
 
 
+def test_weights_loaded_on_a_stream():
+    """The blob's copy belongs to the current stream, its repack to the one that is given, here one with work in front of it."""
+    rng, s = np.random.default_rng(4), torch.cuda.Stream()
+    for pack, load in ((mb.quant_prepack, mb.W4A32Weights), (w4a16.quant_prepack, w4a16.W4A16Weights)):
+        blob = pack((rng.standard_normal((896, 1536)) * 0.02).astype(np.float32))
+        with torch.cuda.stream(s):
+            torch.cuda._sleep(20_000_000)
+        got = load.from_blob(blob, stream=s)
+        assert torch.equal(got.tiled, load.from_blob(blob).tiled)
+        if load is mb.W4A32Weights:
+            assert np.array_equal(got.unpack(stream=s), blob)
+
+
 @pytest.mark.parametrize("own", [True, False])
 def test_two_streams_in_one_thread(calls, own):
     streams, got = [torch.cuda.Stream() for _ in range(2)], []
