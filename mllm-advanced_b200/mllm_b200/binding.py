@@ -166,8 +166,10 @@ def _stream_ptr(stream):
     import torch
     if stream is not None:
         return C.c_void_p(stream.cuda_stream)
-    # torch.cuda.current_stream().cuda_stream without the Python objects around it (3.6 us of a call that takes 18 in all)
-    return C.c_void_p(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))
+    try:  # the next line's answer without the Python objects around it (3.6 us of a call that takes 18 in all)
+        return C.c_void_p(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))
+    except AttributeError:  # (two names that torch does not promise)
+        return C.c_void_p(torch.cuda.current_stream().cuda_stream)
 
 
 class W4A32Weights:

@@ -119,6 +119,22 @@ def test_default_kernel_by_batch_size():
     assert L.mllmb200_w4a32_select_kernel(8, 32768, 64) == mb.KERNEL_STREAM_TC               # ... but those of 8 rows do
 
 
+@pytest.mark.parametrize("name", ["_cuda_getCurrentRawStream", "_cuda_getDevice"])
+def test_current_stream_with_and_without_torchs_short_way(monkeypatch, name):
+    """The calls' stream: through two unpromised functions of torch, or the public way where a torch lacks either."""
+    import types
+
+    import torch
+    from mllm_b200 import binding
+    monkeypatch.setattr(torch._C, "_cuda_getDevice", lambda: 3, raising=False)
+    monkeypatch.setattr(torch._C, "_cuda_getCurrentRawStream", lambda device: 0x1000 + device, raising=False)
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda: types.SimpleNamespace(cuda_stream=0x2000))
+    assert binding._stream_ptr(None).value == 0x1003
+    monkeypatch.delattr(torch._C, name)
+    assert binding._stream_ptr(None).value == 0x2000
+    assert binding._stream_ptr(types.SimpleNamespace(cuda_stream=0x3000)).value == 0x3000
+
+
 def test_peer_stores_come_from_the_kernel_that_the_forward_runs():
     """Tensor-parallel gather modes 0 and 1 run the public forward for a shard; the one that stores into the peers from a kernel's epilogue
     does so only with that same kernel (same bits), and does for each of the kernels that can."""
