@@ -538,8 +538,10 @@ int w4a32_gemm_stream_block_rows(int m) { return ms_block_tiles(m) * 8; }
 // Per-row int8 quantization (the arithmetic of act_quant_records_kernel) into the layout above: for K-group g
 // and row m the four low words (even k of each 8-value item) at [g][m][0..16), the four high words (odd k) at
 // [g][rows + m] of its block of rows.  One CTA per row of the padded batch; padding rows are zeros.  A thread keeps its ITEMS items of 8
-// values in registers between minimum / maximum and quantization (all loads in flight at once); rows that are longer or not
-// 16-byte aligned are read twice.
+// values in registers between minimum / maximum and quantization (all loads in flight at once).  Rows that are longer (ITEMS 0) or not
+// 16-byte aligned are read twice, the former 16 bytes at a time: 14336 -> 4096 with its quantization, us, single floats / so,
+// M = 8 18.0 / 17.0, 16 24.4 / 24.0, 32 30.9 / 28.9, 56 49.5 / 47.9.  (An instance of its own: in the one for up to 12288 values the
+// branch costs 0.1 us at K = 8960.)
 constexpr int kMsQuantThreads = 512;
 template <int ITEMS>
 __global__ void __launch_bounds__(kMsQuantThreads) act_quant_mma_kernel(const float* __restrict__ x, int m_total, int m_pad, int block_rows,
@@ -565,8 +567,8 @@ __global__ void __launch_bounds__(kMsQuantThreads) act_quant_mma_kernel(const fl
     return;
   }
   auto value = [&](int at) { return at < k ? row[at] : 0.0f; };
-  const bool keep = (reinterpret_cast<uintptr_t>(row) & 15u) == 0 && num_items <= ITEMS * kMsQuantThreads;
-  float v[ITEMS][8];
+  const bool aligned = (reinterpret_cast<uintptr_t>(row) & 15u) == 0, keep = ITEMS > 0 && aligned;
+  float v[ITEMS > 0 ? ITEMS : 1][8];
   float mn = 3.402823466e+38f, mx = -3.402823466e+38f;
   if (keep) {
 #pragma unroll
@@ -632,8 +634,14 @@ __global__ void __launch_bounds__(kMsQuantThreads) act_quant_mma_kernel(const fl
   } else {
     for (int item = tid; item < num_items; item += kMsQuantThreads) {
       float f[8];
+      if (ITEMS == 0 && aligned && item * 8 + 8 <= k) {
+        const float4 a = *reinterpret_cast<const float4*>(row + item * 8), b = *reinterpret_cast<const float4*>(row + item * 8 + 4);
+        f[0] = a.x, f[1] = a.y, f[2] = a.z, f[3] = a.w;
+        f[4] = b.x, f[5] = b.y, f[6] = b.z, f[7] = b.w;
+      } else {
 #pragma unroll
-      for (int i = 0; i < 8; ++i) f[i] = value(item * 8 + i);
+        for (int i = 0; i < 8; ++i) f[i] = value(item * 8 + i);
+      }
       emit(item, f);
     }
   }
@@ -747,9 +755,10 @@ cudaError_t launch_act_quant_mma(const float* x, int m, int k, int ldx, uint8_t*
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
   }
-  return num_groups * 4 <= kMsQuantThreads
-             ? cudaLaunchKernelEx(&cfg, act_quant_mma_kernel<1>, x, m, m_pad, ms_block_tiles(m) * 8, k, ldx, num_groups, acts, hdr)
-             : cudaLaunchKernelEx(&cfg, act_quant_mma_kernel<3>, x, m, m_pad, ms_block_tiles(m) * 8, k, ldx, num_groups, acts, hdr);
+  const auto kernel = num_groups * 4 <= kMsQuantThreads       ? act_quant_mma_kernel<1>
+                      : num_groups * 4 <= 3 * kMsQuantThreads ? act_quant_mma_kernel<3>
+                                                              : act_quant_mma_kernel<0>;
+  return cudaLaunchKernelEx(&cfg, kernel, x, m, m_pad, ms_block_tiles(m) * 8, k, ldx, num_groups, acts, hdr);
 }
 
 template <int NT>

@@ -72,6 +72,12 @@ def test_rows_and_outputs_off_16_bytes(m, k, ns):
     _case(m, k, ns, odd=True)
 
 
+# rows that the quantization reads twice: all of them in 16-byte words with half an item at the end, and only every fourth
+@pytest.mark.parametrize("m,k,ns", [(10, 12300, (65,)), (7, 12293, (33,))])
+def test_long_rows(m, k, ns):
+    _case(m, k, ns)
+
+
 # above 64 rows, where the fastest policy takes the kernel: three to six blocks, the borders of its rows, columns and K
 @pytest.mark.parametrize("m,k,ns", [(65, 1024, (31,)), (80, 1536, (1536, 256)), (97, 8960, (1536,)), (127, 4448, (4096,)), (128, 896, (896, 128, 128)),
                                     (161, 4864, (896,)), (192, 2048, (2048, 1024))])
