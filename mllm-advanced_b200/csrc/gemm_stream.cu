@@ -16,9 +16,13 @@
 //     the weights twice from L2, but 1536 x 1536 becomes 96 units on 148 SMs instead of 48 (M = 64: 9.2 -> 6.2 us with the
 //     quantization, in a chain of dependent launches).  S, KS and with them the bits follow from M and K alone: a matrix has
 //     the same bits by itself and in a group.
-//   * a producer warp streams the unit's cells through a ring of 16-group stages (cp.async.bulk + full / empty
+//   * a producer warp streams the unit's cells through a ring of stages (cp.async.bulk + full / empty
 //     mbarriers, weights marked evict-first in L2); under programmatic dependent launch the first stages are
-//     requested before griddepcontrol.wait, the activations after it, in four parts of which the first is enough to start.
+//     requested before griddepcontrol.wait, the activations after it.  A stage is 32 K-groups, two trips of a warp between waits,
+//     where three of those fit beside the activations, else 16 (us, chain of dependent launches, 16 / 32: M = 8 1536 -> 8960 6.8 /
+//     6.4, 2048 -> 17920 13.2 / 12.0, 4096 -> 17920 20.6 / 14.5, 8192 -> 28672 46 / 39; M = 48 8960 -> 1536 17.3 / 16.2; M = 64 8192 ->
+//     28672 131 / 116; a stage may be cut anywhere between K-groups, the bits are the same).  The activations are one copy: in four parts,
+//     of which the first lets the products start, a call of 8 rows takes 0.1 to 0.2 us longer.
 //   * 8 compute warps: warp ks takes the K-groups ks, ks + 8 of a stage.  A cell: one ldmatrix.x4 = the words of four rows
 //     per lane; two LOP3 and a shift make the A fragments of two mma.sync.m16n8k32 (s8: 16 (nibble - 8) in the high half
 //     of each byte, so no zero-point term per group; low nibbles are k 0..15, high nibbles k 16..31 of the instruction, the
@@ -34,10 +38,11 @@
 // What bounds it (M = 64, K = 1536, cycles of an SM): a cell takes 115, of which its tensor instructions need 32 and its
 // packed FP32 instructions 32; the rest is issue (about 80 slots) and dependences.  More warps (16), registers filled one
 // stage ahead and 64 columns per warp were each as slow or slower.  With u8 nibbles, a zero-point term per group, scalar
-// FP32 and 32-bit loads a cell took 150.  us a call with its quantization, before -> now, chain of dependent launches:
-//   1536 -> 17920  M = 8 10.4 -> 10.7, 24 15.5 -> 12.4, 48 22.5 -> 19.7, 64 25.8 -> 21.9
-//   8960 -> 1536   M = 8 12.3 -> 11.4, 24 18.7 -> 11.1, 48 22.7 -> 17.1, 64 30.6 -> 19.3
-//   8192 -> 28672  M = 8 46 -> 46, 24 90 -> 62, 64 292 -> 130
+// FP32 and 32-bit loads a cell took 150.  us a call with its quantization, that form -> now, chain of dependent launches:
+//   1536 -> 17920  M = 8 10.6 -> 10.4, 24 15.7 -> 12.3, 48 22.7 -> 19.1, 64 26.0 -> 21.4
+//   8960 -> 1536   M = 8 12.7 -> 10.3, 24 19.3 -> 10.9, 48 24.0 -> 16.2, 64 30.7 -> 19.6
+//   8192 -> 28672  M = 8 46.4 -> 39.2, 24 90 -> 54, 64 295 -> 116
+//   2048 -> 4096   M = 8 5.57 -> 5.54; 2048 -> 17920 M = 8 11.9 -> 12.0
 // Every wait is bounded; a cluster leaves together (one cluster barrier at the end) so that no CTA's shared memory
 // disappears under a peer.
 #include <algorithm>
@@ -50,10 +55,8 @@ namespace mllmb200 {
 constexpr int kMsCWarps = 8;                  // compute warps
 constexpr int kMsEWarps = 3;                  // epilogue warps; with the producer warp between them 12 warps, 3 per scheduler
 constexpr int kMsThreads = (kMsCWarps + 1 + kMsEWarps) * 32;
-constexpr int kMsBlockGroups = 16;            // K-groups per ring stage
-constexpr int kMsStageBytes = kMsBlockGroups * kCellBytes;  // 9216
+constexpr int kMsStageGroups = 32, kMsSmallStageGroups = 16;  // K-groups per ring stage, where three of 32 fit and else
 constexpr int kMsMaxStages = 6, kMsMinStages = 3;
-constexpr int kMsActChunks = 4;               // parts in which a CTA's activations arrive
 constexpr int kMsMaxProblems = 4;
 constexpr int kMsMaxCluster = 8;
 constexpr int kMsActRowBytes = 32;            // per activation row and K-group: 16 + 16 bytes of int8
@@ -80,11 +83,11 @@ struct MsParams {
 struct MsSmem {
   size_t bars, hdr, flags, acts, ring, red, psum, total;
 };
-__host__ __device__ inline MsSmem ms_smem_layout(int rows, int groups_per_rank, int cluster_size, int stages) {
+__host__ __device__ inline MsSmem ms_smem_layout(int rows, int groups_per_rank, int cluster_size, int stages, int stage_groups) {
   MsSmem L;
   size_t off = 0;
   L.bars = off;
-  off += 256;  // full[6], empty[6], act[4], peer_full[2], peer_free[2], red_full, red_free
+  off += 256;  // full[6], empty[6], act, peer_full[2], peer_free[2], red_full, red_free
   L.hdr = off;
   off += (size_t)rows * 8;
   L.flags = off;
@@ -93,7 +96,7 @@ __host__ __device__ inline MsSmem ms_smem_layout(int rows, int groups_per_rank, 
   off += (size_t)groups_per_rank * rows * kMsActRowBytes;
   off = (off + 127) & ~(size_t)127;
   L.ring = off;
-  off += (size_t)stages * kMsStageBytes;
+  off += (size_t)stages * stage_groups * kCellBytes;
   L.red = off;
   off += (size_t)kMsCWarps * rows * kMsRedCol * 4;
   L.psum = off;
@@ -168,8 +171,8 @@ __device__ __forceinline__ void ms_mma_s8(uint32_t (&d)[4], const uint32_t (&a)[
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "r"(c[0]), "r"(c[1]), "r"(c[2]), "r"(c[3]));
 }
 
-// NT: 8-column tiles of a block of the batch
-template <int NT>
+// NT: 8-column tiles of a block of the batch; SG: K-groups of a ring stage
+template <int NT, int SG>
 __global__ void __launch_bounds__(kMsThreads, 1) w4a32_gemm_stream_kernel(const __grid_constant__ MsParams p) {
   constexpr int KS = kMsCWarps, ROWS = NT * 8;  // (KS: warps that share the K-groups of a stage)
   extern __shared__ __align__(128) uint8_t ms_smem[];
@@ -181,13 +184,13 @@ __global__ void __launch_bounds__(kMsThreads, 1) w4a32_gemm_stream_kernel(const 
   const int first_row = blk * ROWS, n_tiles = min(NT, (p.m_pad >> 3) - blk * NT), rows = n_tiles * 8, m_here = min(rows, p.m - first_row);
   const int g_lo = (int)(((long long)rank * G) / S), g_hi = (int)(((long long)(rank + 1) * G) / S);
   const int ng = g_hi - g_lo;
-  const MsSmem Lo = ms_smem_layout(ROWS, (G + S - 1) / S, S, p.stages);
+  constexpr int kStageBytes = SG * kCellBytes;
   const int NST = p.stages, panel_step = p.num_clusters / p.num_blocks;
-  const int act_chunk = ((ng + kMsActChunks - 1) / kMsActChunks + 15) & ~15;  // K-groups
+  const MsSmem Lo = ms_smem_layout(ROWS, (G + S - 1) / S, S, NST, SG);
   uint64_t* full = reinterpret_cast<uint64_t*>(ms_smem + Lo.bars);
   uint64_t* empty = full + kMsMaxStages;
   uint64_t* act_bar = empty + kMsMaxStages;
-  uint64_t* peer_full = act_bar + kMsActChunks;   // [2] rank 0: the other ranks' partial sums of a unit are in place
+  uint64_t* peer_full = act_bar + 1;   // [2] rank 0: the other ranks' partial sums of a unit are in place
   uint64_t* peer_free = peer_full + 2; // [2] ranks 1..: rank 0 has read the slot
   uint64_t* red_full = peer_free + 2;  // the warps' sums of a unit are in place
   uint64_t* red_free = red_full + 1;   // ... and have been read
@@ -206,7 +209,7 @@ __global__ void __launch_bounds__(kMsThreads, 1) w4a32_gemm_stream_kernel(const 
       mbar_init(&full[i], 1);
       mbar_init(&empty[i], kMsCWarps);
     }
-    for (int i = 0; i < kMsActChunks; ++i) mbar_init(&act_bar[i], 1);
+    mbar_init(act_bar, 1);
     for (int i = 0; i < 2; ++i) {
       mbar_init(&peer_full[i], (uint32_t)max(S - 1, 1));
       mbar_init(&peer_free[i], 1);
@@ -328,18 +331,16 @@ __global__ void __launch_bounds__(kMsThreads, 1) w4a32_gemm_stream_kernel(const 
       bool acts_requested = false;
       auto request_acts = [&] {
         if (p.use_pdl) pdl_wait_prior();  // the activation blocks come from the kernel before this one
-        for (int i = 0, g = 0; g < ng; ++i, g += act_chunk) {
-          const uint32_t bytes = (uint32_t)((size_t)min(act_chunk, ng - g) * group_bytes);
-          mbar_arrive_expect_tx(&act_bar[i], bytes);
-          bulk_g2s(acts + (size_t)g * group_bytes, acts_from + (size_t)(g_lo + g) * group_bytes, bytes, &act_bar[i]);
-        }
+        const uint32_t bytes = (uint32_t)((size_t)ng * group_bytes);
+        mbar_arrive_expect_tx(act_bar, bytes);
+        bulk_g2s(acts, acts_from + (size_t)g_lo * group_bytes, bytes, act_bar);
         acts_requested = true;
       };
       bool ok = true;
       for (int u = first_panel; u < p.total_panels && ok; u += panel_step) {
         const MsProblem& pr = p.prob[problem_of(u)];
         const uint8_t* cells = pr.tiled + sizeof(TiledHeader) + (size_t)(u - pr.panel_begin) * G * kCellBytes;
-        for (int b = g_lo; b < g_hi; b += kMsBlockGroups) {
+        for (int b = g_lo; b < g_hi; b += SG) {
           if (issued == NST && !acts_requested) request_acts();  // the ring is full of weights: now the activations
           if (issued >= NST) {
             if (!mbar_wait_bounded(&empty[st], ph ^ 1u)) {
@@ -348,9 +349,9 @@ __global__ void __launch_bounds__(kMsThreads, 1) w4a32_gemm_stream_kernel(const 
               break;
             }
           }
-          const uint32_t bytes = (uint32_t)(min(kMsBlockGroups, g_hi - b) * kCellBytes);
+          const uint32_t bytes = (uint32_t)(min(SG, g_hi - b) * kCellBytes);
           mbar_arrive_expect_tx(&full[st], bytes);
-          bulk_g2s_hint(ring + (size_t)st * kMsStageBytes, cells + (size_t)b * kCellBytes, bytes, &full[st], stream_once);
+          bulk_g2s_hint(ring + (size_t)st * kStageBytes, cells + (size_t)b * kCellBytes, bytes, &full[st], stream_once);
           ++issued;
           if (++st == NST) {
             st = 0;
@@ -369,7 +370,6 @@ __global__ void __launch_bounds__(kMsThreads, 1) w4a32_gemm_stream_kernel(const 
       if (p.use_pdl) pdl_wait_prior();
       for (int i = tid; i < m_here; i += kMsCWarps * 32) s_hdr[i] = p.a_hdr[first_row + i];
     }
-    int acts_here = 0;  // K-groups of the activations that have arrived
     const uint32_t ring_s = smem_u32(ring), acts_s = smem_u32(acts), red_s = smem_u32(red);
     // matrices of an ldmatrix.x4 of the activations: low and high words of tile t, low and high words of tile t + 1
     const uint32_t b_lane = (uint32_t)(((lane >> 4) * 8 + (lane & 7)) * 16 + ((lane >> 3) & 1) * rows * 16);
@@ -389,22 +389,19 @@ __global__ void __launch_bounds__(kMsThreads, 1) w4a32_gemm_stream_kernel(const 
     uint32_t ph = 0;
     for (int u = first_panel; u < p.total_panels; u += panel_step, ++unit_index) {
       const bool f16 = flags[4 + problem_of(u)] != 0;
-      for (int b = g_lo; b < g_hi && ok; b += kMsBlockGroups) {
-        if (b - g_lo >= acts_here) {  // (the first unit only)
-          ok = mbar_wait_bounded(&act_bar[(b - g_lo) / act_chunk], 0);
-          acts_here += act_chunk;
-        }
+      for (int b = g_lo; b < g_hi && ok; b += SG) {
+        if (unit_index == 0 && b == g_lo) ok = mbar_wait_bounded(act_bar, 0);
         if (!ok || !mbar_wait_bounded(&full[st], ph)) {
           ok = false;
           break;
         }
-        const int cnt = min(kMsBlockGroups, g_hi - b);
+        const int cnt = min(SG, g_hi - b);
         // Two cells per trip (K-groups j and j + KS of the stage), their loads and tensor-core products interleaved:
         // with two warps per scheduler the dependent chain of a single cell would leave the pipes idle.
         for (int j = ks; j < cnt; j += 2 * KS) {
           const bool two = j + KS < cnt;
           uint32_t cell[2], act[2];
-          cell[0] = ring_s + (uint32_t)st * kMsStageBytes + (uint32_t)j * kCellBytes;
+          cell[0] = ring_s + (uint32_t)st * kStageBytes + (uint32_t)j * kCellBytes;
           cell[1] = two ? cell[0] + (uint32_t)KS * kCellBytes : cell[0];
           act[0] = acts_s + (uint32_t)(b - g_lo + j) * (uint32_t)group_bytes;
           act[1] = two ? act[0] + (uint32_t)KS * (uint32_t)group_bytes : act[0];
@@ -649,24 +646,24 @@ __global__ void __launch_bounds__(kMsQuantThreads) act_quant_mma_kernel(const fl
 
 // ------------------------------------------------------------------------------------------------ host side
 struct MsPlan {
-  int m_pad, block_tiles, num_blocks, cluster_size, groups_per_rank, stages, total_panels;
+  int m_pad, block_tiles, num_blocks, cluster_size, groups_per_rank, stages, stage_groups, total_panels;
 };
 
-template <int NT>
+template <int NT, int SG>
 static cudaError_t ms_configure() {
   static bool configured[64] = {};
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
   if (dev >= 0 && dev < 64 && configured[dev]) return cudaSuccess;
-  e = cudaFuncSetAttribute(w4a32_gemm_stream_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMsSmemMax);
+  e = cudaFuncSetAttribute(w4a32_gemm_stream_kernel<NT, SG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMsSmemMax);
   if (e != cudaSuccess) return e;
   if (dev >= 0 && dev < 64) configured[dev] = true;
   return cudaSuccess;
 }
 
 // clusters of `s` CTAs of this kernel that the current device runs at once (148 / s without a device)
-template <int NT>
+template <int NT, int SG>
 static int ms_cluster_capacity(int s, size_t smem) {
   if (s <= 1) return 148;
   int n = 0;
@@ -681,8 +678,8 @@ static int ms_cluster_capacity(int s, size_t smem) {
   attr.val.clusterDim.z = 1;
   cfg.attrs = &attr;
   cfg.numAttrs = 1;
-  if (ms_configure<NT>() != cudaSuccess ||
-      cudaOccupancyMaxActiveClusters(&n, w4a32_gemm_stream_kernel<NT>, &cfg) != cudaSuccess || n <= 0) {
+  if (ms_configure<NT, SG>() != cudaSuccess ||
+      cudaOccupancyMaxActiveClusters(&n, w4a32_gemm_stream_kernel<NT, SG>, &cfg) != cudaSuccess || n <= 0) {
     (void)cudaGetLastError();
     n = 148 / s;
   }
@@ -706,8 +703,11 @@ static bool ms_shape_plan(int m, int k, int count, const int* n, MsPlan* plan) {
   for (int s = G >= 140 && plan->m_pad > 8 ? 2 : 1; s <= kMsMaxCluster && plan->stages == 0; s *= 2) {
     plan->cluster_size = s;
     plan->groups_per_rank = (G + s - 1) / s;
-    for (int stages = kMsMaxStages; stages >= kMsMinStages && plan->stages == 0; --stages)
-      if (ms_smem_layout(plan->block_tiles * 8, plan->groups_per_rank, s, stages).total <= kMsSmemMax) plan->stages = stages;
+    const auto fits = [&](int stages, int groups) { return ms_smem_layout(plan->block_tiles * 8, plan->groups_per_rank, s, stages, groups).total <= kMsSmemMax; };
+    if (!fits(kMsMinStages, kMsSmallStageGroups)) continue;
+    plan->stages = kMsMinStages;
+    plan->stage_groups = fits(kMsMinStages, kMsStageGroups) ? kMsStageGroups : kMsSmallStageGroups;
+    while (plan->stages < (plan->stage_groups == kMsStageGroups ? 4 : kMsMaxStages) && fits(plan->stages + 1, plan->stage_groups)) ++plan->stages;
   }
   long long panels = 0;
   for (int i = 0; i < count; ++i) {
@@ -761,22 +761,22 @@ cudaError_t launch_act_quant_mma(const float* x, int m, int k, int ldx, uint8_t*
   return cudaLaunchKernelEx(&cfg, kernel, x, m, m_pad, ms_block_tiles(m) * 8, k, ldx, num_groups, acts, hdr);
 }
 
-template <int NT>
+template <int NT, int SG>
 static cudaError_t ms_launch_t(MsParams& prm, const MsPlan& plan, cudaStream_t stream) {
-  cudaError_t e = ms_configure<NT>();
+  cudaError_t e = ms_configure<NT, SG>();
   if (e != cudaSuccess) return e;
   const int S = plan.cluster_size;
   static int capacity[64][kMsMaxCluster + 1] = {};  // per device and cluster size (the largest shared-memory need is assumed)
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) dev = 0;
-  if (capacity[dev][S] == 0) capacity[dev][S] = ms_cluster_capacity<NT>(S, kMsSmemMax);
+  if (capacity[dev][S] == 0) capacity[dev][S] = ms_cluster_capacity<NT, SG>(S, kMsSmemMax);
   const int per_block = std::max(1, std::min(capacity[dev][S], 148 / S) / plan.num_blocks);
   prm.num_clusters = std::min(per_block, plan.total_panels) * plan.num_blocks;
   prm.one_unit = plan.total_panels <= per_block;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(prm.num_clusters * S), 1, 1);
   cfg.blockDim = dim3(kMsThreads, 1, 1);
-  cfg.dynamicSmemBytes = ms_smem_layout(plan.block_tiles * 8, plan.groups_per_rank, S, plan.stages).total;
+  cfg.dynamicSmemBytes = ms_smem_layout(plan.block_tiles * 8, plan.groups_per_rank, S, plan.stages, plan.stage_groups).total;
   cfg.stream = stream;
   cudaLaunchAttribute attrs[2];
   int na = 0;
@@ -794,7 +794,13 @@ static cudaError_t ms_launch_t(MsParams& prm, const MsPlan& plan, cudaStream_t s
   }
   cfg.attrs = attrs;
   cfg.numAttrs = na;
-  return cudaLaunchKernelEx(&cfg, w4a32_gemm_stream_kernel<NT>, prm);
+  return cudaLaunchKernelEx(&cfg, w4a32_gemm_stream_kernel<NT, SG>, prm);
+}
+
+template <int NT>
+static cudaError_t ms_launch_tiles(MsParams& prm, const MsPlan& plan, cudaStream_t stream) {
+  return plan.stage_groups == kMsStageGroups ? ms_launch_t<NT, kMsStageGroups>(prm, plan, stream)
+                                             : ms_launch_t<NT, kMsSmallStageGroups>(prm, plan, stream);
 }
 
 // acts / a_hdr: output of launch_act_quant_mma for the same m and k.  Up to four matrices that share them.
@@ -830,10 +836,10 @@ cudaError_t launch_w4a32_gemm_stream(const uint8_t* acts, const float2* a_hdr, i
     begin += (int)th.num_panels;
   }
   switch (plan.block_tiles) {
-    case 1: return ms_launch_t<1>(prm, plan, stream);
-    case 2: return ms_launch_t<2>(prm, plan, stream);
-    case 3: return ms_launch_t<3>(prm, plan, stream);
-    default: return ms_launch_t<4>(prm, plan, stream);
+    case 1: return ms_launch_tiles<1>(prm, plan, stream);
+    case 2: return ms_launch_tiles<2>(prm, plan, stream);
+    case 3: return ms_launch_tiles<3>(prm, plan, stream);
+    default: return ms_launch_tiles<4>(prm, plan, stream);
   }
 }
 

@@ -72,6 +72,13 @@ def test_rows_and_outputs_off_16_bytes(m, k, ns):
     _case(m, k, ns, odd=True)
 
 
+# stages of 32 K-groups: exactly one, one and a K-group, one with the second trip of a few warps, more than the ring in both
+# parts of a cluster; where only 16 fit
+@pytest.mark.parametrize("m,k,ns", [(8, 1024, (40,)), (16, 1056, (4801,)), (40, 608, (5000, 33)), (8, 8225, (64,)), (20, 8992, (2400,)), (56, 12288, (320,))])
+def test_stages_of_32_groups(m, k, ns):
+    _case(m, k, ns)
+
+
 # rows that the quantization reads twice: all of them in 16-byte words with half an item at the end, and only every fourth
 @pytest.mark.parametrize("m,k,ns", [(10, 12300, (65,)), (7, 12293, (33,))])
 def test_long_rows(m, k, ns):
