@@ -247,146 +247,187 @@ __global__ void __launch_bounds__(kNormThreads) lm_norm_single_kernel(NormArgs a
   }
 }
 
-// A row of the sublayer output, column lane + 32 i of float4s in x[i].
-template <int NVW>
-__device__ __forceinline__ void warp_delta(const Delta& d, int row, int lane, int nv, float4 (&x)[NVW]) {
+// A row of the sublayer output, column lane + LANES i of float4s in x[i].
+template <int NV, int LANES>
+__device__ __forceinline__ void warp_delta(const Delta& d, int row, int lane, int nv, float4 (&x)[NV]) {
   const int n_src = d.mix_w ? d.top : 1;
 #pragma unroll
-  for (int i = 0; i < NVW; ++i) x[i] = make_float4(0, 0, 0, 0);
+  for (int i = 0; i < NV; ++i) x[i] = make_float4(0, 0, 0, 0);
   for (int k = 0; k < n_src; ++k) {
     const int pair = row * n_src + k;
     const float g = d.mix_w ? d.mix_w[pair] : 1.0f;
     const float* src = d.p + (size_t)(d.mix_w && d.mix_row ? d.mix_row[pair] : pair) * d.ldx;
     for (int p = 0; p < d.planes; ++p)
 #pragma unroll
-      for (int i = 0; i < NVW; ++i) {
-        const int c = lane + i * 32;
+      for (int i = 0; i < NV; ++i) {
+        const int c = lane + i * LANES;
         if (c < nv) x[i] = fma4(g, *reinterpret_cast<const float4*>(src + p * d.plane + c * 4), x[i]);
       }
   }
 }
 
-// The same for many rows: a warp per row for the sums (no block barrier inside), then - with a convolution - the threads
+// The same for many rows: WPR warps per row for the sums (one, but two above 2048 columns), then - with a convolution - the threads
 // sweep the CTA's rows column by column with the last three rows of h in registers.  All rows of h, the recomputed ones in
-// front of the CTA's own included, wait in shared memory.  A row is its warp's latency, so that of the stream is requested
+// front of the CTA's own included, wait in shared memory.  A row is its warps' latency, so that of the stream is requested
 // along with the sublayer's where the registers hold both, and the rows are dealt out so that no SM gets a second
 // block before each has one.  1500 rows x 1536 behind two planes: 7.2 us alone and 11.5 in a layer, where reading the rows back
-// from memory for the convolution, in blocks of 12, took 13.9 and 22.8; 2048 wide, 1000 rows: 7.2 and 11.8.  (Above 2048 columns
-// the rows in front weigh more: from 7000 rows on 8% slower than blocks of two passes, 10 to 30% faster below.)
-template <int NVW>
-constexpr int kRowsWarps = NVW <= 16 ? 16 : 12;  // rows of a CTA, and what leaves a warp enough registers
-
-template <class T, int NVW, bool CONV>
-__global__ void __launch_bounds__(kRowsWarps<NVW> * 32) lm_norm_rows_kernel(NormArgs a) {
-  constexpr int kWarps = kRowsWarps<NVW>, kThreads = kWarps * 32, kTaps = CONV ? 4 : 1;
-  constexpr bool kAhead = NVW <= 12;
-  extern __shared__ __align__(16) float rows_h[];  // [kWarps][ldx]
-  __shared__ Entry s_e[kWarps];
+// from memory for the convolution, in blocks of 12, took 13.9 and 22.8; 2048 wide, 1000 rows: 7.2 and 11.8.
+// Above 2048 columns a lane of one warp per row would hold 32 float4 and have no registers left for loads in flight, and shared memory
+// holds few rows: two warps take a row, and a CTA makes passes of 8 rows of which the last three stay, so that only its first pass
+// recomputes any.  4096 columns behind two planes, us, one warp a row in blocks of 12 / so: 300 rows 24 / 10, 1000 41 / 21,
+// 7000 280 / 122, 20000 738 / 316; 2560 columns, 1500 rows 51 / 18, 12000 337 / 142.
+template <class T, int NV, int WPR, int ROWS, bool CONV, bool AHEAD>
+__global__ void __launch_bounds__(ROWS* WPR * 32) lm_norm_rows_kernel(NormArgs a) {
+  constexpr int kThreads = ROWS * WPR * 32, kLanes = 32 * WPR, kTaps = CONV ? 4 : 1;
+  constexpr bool kPasses = CONV && WPR > 1;  // several passes of ROWS rows, the last three of each stay
+  // warps without a row skip it, or (with barriers in the sums; and 2048 columns with a convolution, 8% faster so) go along without columns
+  constexpr bool kBranch = WPR == 1 && (NV <= 12 || !CONV);
+  constexpr int kSlots = kPasses ? ROWS + kTaps - 1 : ROWS;
+  extern __shared__ __align__(16) float rows_h[];  // [kSlots][ldx]
+  __shared__ Entry s_e[ROWS];
+  __shared__ float s_sum[2][ROWS][WPR];
   pdl_launch_dependents();
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nv = a.ldx >> 2, keep = a.taps - 1;
+  const int tid = threadIdx.x, row_here = tid / kLanes, lane = tid % kLanes, nv = a.ldx >> 2, keep = a.taps - 1;
   const float g_pre = *a.g_pre, g_post = a.delta.p ? *a.g_post : 0.0f, inv_w = 1.0f / (float)a.width;
   const float4 zero = make_float4(0, 0, 0, 0);
   pdl_wait_prior();
   const int r_begin = blockIdx.x * a.rows_per_cta, r_end = min(r_begin + a.rows_per_cta, a.rows);
-  int t0 = r_begin;
-  if (CONV) {
-    t0 = max(r_begin - keep, a.entries[a.row_entry[r_begin]].row0);
-    if (tid < r_end - t0) s_e[tid] = a.entries[a.row_entry[t0 + tid]];
-  }
-  auto warp_sum = [](float v) {
+  const int t0 = CONV ? max(r_begin - keep, a.entries[a.row_entry[r_begin]].row0) : r_begin;
+  auto row_sum = [&](int which, float v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if (WPR == 1) return v;
+    if ((tid & 31) == 0) s_sum[which][row_here][lane >> 5] = v;
+    __syncthreads();
+    v = 0.0f;
+#pragma unroll
+    for (int i = 0; i < WPR; ++i) v += s_sum[which][row_here][i];
     return v;
   };
-  const int t = t0 + warp;
-  if (t < r_end) {
-    const float4* xr = reinterpret_cast<const float4*>(a.x_in + (size_t)t * a.ldx);
-    float4 x[NVW], ahead[kAhead ? NVW : 1];
-    float ss = 0.0f;
-    if (a.delta.p) {
-      if (kAhead)
-#pragma unroll
-        for (int i = 0; i < NVW; ++i) ahead[i] = lane + i * 32 < nv ? xr[lane + i * 32] : zero;
-      warp_delta<NVW>(a.delta, t, lane, nv, x);
-#pragma unroll
-      for (int i = 0; i < NVW; ++i) ss += dot4(x[i]);
-      const float r = g_post / sqrtf(warp_sum(ss) * inv_w + a.eps);
-      ss = 0.0f;
-#pragma unroll
-      for (int i = 0; i < NVW; ++i) {
-        const int c = lane + i * 32;
-        if (c < nv) x[i] = fma4(r, x[i], kAhead ? ahead[i] : xr[c]);
-        ss += dot4(x[i]);
-      }
-    } else {
-#pragma unroll
-      for (int i = 0; i < NVW; ++i) {
-        const int c = lane + i * 32;
-        x[i] = c < nv ? xr[c] : zero;
-        ss += dot4(x[i]);
-      }
+  for (int p0 = t0; p0 < r_end; p0 += ROWS) {
+    const int rows = min(ROWS, r_end - p0), t = p0 + row_here;
+    const int nv_here = kBranch || t < r_end ? nv : 0;
+    if (CONV) {
+      if (kPasses && p0 > t0) __syncthreads();  // the rows that are overwritten have been swept
+      if (tid < rows) s_e[tid] = a.entries[a.row_entry[p0 + tid]];
     }
-    const float r = g_pre / sqrtf(warp_sum(ss) * inv_w + a.eps);
-    const bool out_x = t >= r_begin && a.x_out;
+    if (!kBranch || t < r_end) {
+      const float4* xr = reinterpret_cast<const float4*>(a.x_in + (size_t)t * a.ldx);
+      float4 x[NV], ahead[AHEAD ? NV : 1];
+      float ss = 0.0f;
+      if (a.delta.p) {
+        if (AHEAD)
 #pragma unroll
-    for (int i = 0; i < NVW; ++i) {
-      const int c = lane + i * 32;
-      if (c >= nv) continue;
-      if (out_x) store4(a.x_out + (size_t)t * a.ldx + c * 4, x[i]);
-      const float4 h = fma4(r, x[i], zero);
-      if (CONV) store4(rows_h + (size_t)warp * a.ldx + c * 4, h);
-      else store4(static_cast<T*>(a.out) + (size_t)t * a.ldx + c * 4, h);
-    }
-  }
-  if (!CONV) return;
-  __syncthreads();
-  for (int c = tid * 4; c < a.ldx; c += kThreads * 4) {
-    float4 w[kTaps], hist[kTaps];  // hist[s]: h of s rows ago
+          for (int i = 0; i < NV; ++i) ahead[i] = lane + i * kLanes < nv_here ? xr[lane + i * kLanes] : zero;
+        if (kBranch || nv_here) {
+          warp_delta<NV, kLanes>(a.delta, t, lane, nv, x);
+        } else {
 #pragma unroll
-    for (int s = 0; s < kTaps; ++s) {
-      w[s] = s <= keep ? __ldg(reinterpret_cast<const float4*>(a.conv_w + (size_t)(keep - s) * a.ldx + c)) : zero;
-      hist[s] = zero;
-    }
-#pragma unroll 4
-    for (int u = 0; u < r_end - t0; ++u) {
-      const Entry e = s_e[u];
-      const int off = t0 + u - e.row0;
-      const float* old_tail = a.tail + ((size_t)e.slot * 2 + e.tail) * keep * a.ldx + c;
-      if (off == 0)  // a sequence's share starts: the rows before it come from its tail, or are zero
+          for (int i = 0; i < NV; ++i) x[i] = zero;
+        }
 #pragma unroll
-        for (int s = 1; s < kTaps; ++s) hist[s] = s <= keep && s <= e.pos0 ? *reinterpret_cast<const float4*>(old_tail + (size_t)(keep - s) * a.ldx) : zero;
-      hist[0] = *reinterpret_cast<const float4*>(rows_h + (size_t)u * a.ldx + c);
-      if (t0 + u >= r_begin) {
-        float4 y = hist[0];
+        for (int i = 0; i < NV; ++i) ss += dot4(x[i]);
+        const float r = g_post / sqrtf(row_sum(0, ss) * inv_w + a.eps);
+        ss = 0.0f;
 #pragma unroll
-        for (int s = 0; s < kTaps; ++s)
-          y = make_float4(fmaf(w[s].x, hist[s].x, y.x), fmaf(w[s].y, hist[s].y, y.y), fmaf(w[s].z, hist[s].z, y.z), fmaf(w[s].w, hist[s].w, y.w));
-        store4(static_cast<T*>(a.out) + (size_t)(t0 + u) * a.ldx + c, y);
-        const int at = keep - (e.count - off);
-        if (at >= 0) {  // among the last rows of its sequence's share: the new tail
-          float* new_tail = a.tail + ((size_t)e.slot * 2 + (e.tail ^ 1)) * keep * a.ldx + c;
-          store4(new_tail + (size_t)at * a.ldx, hist[0]);
-          if (off == e.count - 1)  // a short step: older rows move down
-            for (int j = 0; j + e.count < keep; ++j)
-              store4(new_tail + (size_t)j * a.ldx, *reinterpret_cast<const float4*>(old_tail + (size_t)(j + e.count) * a.ldx));
+        for (int i = 0; i < NV; ++i) {
+          const int c = lane + i * kLanes;
+          if (c < nv_here) x[i] = fma4(r, x[i], AHEAD ? ahead[i] : xr[c]);
+          ss += dot4(x[i]);
+        }
+      } else {
+#pragma unroll
+        for (int i = 0; i < NV; ++i) {
+          const int c = lane + i * kLanes;
+          x[i] = c < nv_here ? xr[c] : zero;
+          ss += dot4(x[i]);
         }
       }
+      const float r = g_pre / sqrtf(row_sum(1, ss) * inv_w + a.eps);
+      const bool out_x = t >= r_begin && a.x_out;
+      float* slot = rows_h + (size_t)(kPasses ? (t - t0) % kSlots : row_here) * a.ldx;
 #pragma unroll
-      for (int s = kTaps - 1; s > 0; --s) hist[s] = hist[s - 1];
+      for (int i = 0; i < NV; ++i) {
+        const int c = lane + i * kLanes;
+        if (c >= nv_here) continue;
+        if (out_x) store4(a.x_out + (size_t)t * a.ldx + c * 4, x[i]);
+        const float4 h = fma4(r, x[i], zero);
+        if (CONV) store4(slot + c * 4, h);
+        else store4(static_cast<T*>(a.out) + (size_t)t * a.ldx + c * 4, h);
+      }
     }
+    if (!CONV) return;  // (one pass)
+    __syncthreads();
+    for (int c = tid * 4; c < a.ldx; c += kThreads * 4) {
+      float4 w[kTaps], hist[kTaps];  // hist[s]: h of s rows ago
+      int at = kPasses ? (p0 - t0) % kSlots : 0;
+#pragma unroll
+      for (int s = 0; s < kTaps; ++s) {
+        w[s] = s <= keep ? __ldg(reinterpret_cast<const float4*>(a.conv_w + (size_t)(keep - s) * a.ldx + c)) : zero;
+        hist[s] = zero;
+      }
+      if (kPasses && p0 > t0) {  // the rows in front of this pass, of the same sequence; before its share the tail, or nothing
+        const Entry e = s_e[0];
+        const int off = p0 - e.row0;
+        const float* old_tail = a.tail + ((size_t)e.slot * 2 + e.tail) * keep * a.ldx + c;
+#pragma unroll
+        for (int s = 1; s < kTaps; ++s) {
+          if (s <= off) hist[s] = *reinterpret_cast<const float4*>(rows_h + (size_t)((p0 - s - t0) % kSlots) * a.ldx + c);
+          else if (s <= keep && s <= e.pos0 + off) hist[s] = *reinterpret_cast<const float4*>(old_tail + (size_t)(keep - (s - off)) * a.ldx);
+        }
+      }
+#pragma unroll 4
+      for (int u = 0; u < rows; ++u) {
+        const Entry e = s_e[u];
+        const int row = p0 + u, off = row - e.row0;
+        const float* old_tail = a.tail + ((size_t)e.slot * 2 + e.tail) * keep * a.ldx + c;
+        if (off == 0)  // a sequence's share starts: the rows before it come from its tail, or are zero
+#pragma unroll
+          for (int s = 1; s < kTaps; ++s) hist[s] = s <= keep && s <= e.pos0 ? *reinterpret_cast<const float4*>(old_tail + (size_t)(keep - s) * a.ldx) : zero;
+        hist[0] = *reinterpret_cast<const float4*>(rows_h + (size_t)at * a.ldx + c);
+        if (++at == kSlots) at = 0;
+        if (row >= r_begin) {
+          float4 y = hist[0];
+#pragma unroll
+          for (int s = 0; s < kTaps; ++s)
+            y = make_float4(fmaf(w[s].x, hist[s].x, y.x), fmaf(w[s].y, hist[s].y, y.y), fmaf(w[s].z, hist[s].z, y.z), fmaf(w[s].w, hist[s].w, y.w));
+          store4(static_cast<T*>(a.out) + (size_t)row * a.ldx + c, y);
+          const int to = keep - (e.count - off);
+          if (to >= 0) {  // among the last rows of its sequence's share: the new tail
+            float* new_tail = a.tail + ((size_t)e.slot * 2 + (e.tail ^ 1)) * keep * a.ldx + c;
+            store4(new_tail + (size_t)to * a.ldx, hist[0]);
+            if (off == e.count - 1)  // a short step: older rows move down
+              for (int j = 0; j + e.count < keep; ++j)
+                store4(new_tail + (size_t)j * a.ldx, *reinterpret_cast<const float4*>(old_tail + (size_t)(j + e.count) * a.ldx));
+          }
+        }
+#pragma unroll
+        for (int s = kTaps - 1; s > 0; --s) hist[s] = hist[s - 1];
+      }
+    }
+    if (!kPasses) return;
   }
 }
 
-template <int NVW>
-constexpr size_t rows_smem(int ldx) { return (size_t)kRowsWarps<NVW> * ldx * sizeof(float); }
+constexpr int kWideRows = 8;  // rows of a pass above 2048 columns (without a convolution 4 or 6 are up to a third slower)
+constexpr size_t rows_smem(int ldx) { return (size_t)(ldx <= 2048 ? 16 : kWideRows + 3) * ldx * sizeof(float); }
 
-template <class T, int NVW>
+template <class T, int NV, int WPR>
 cudaError_t launch_norm_rows(cudaStream_t s, NormArgs a) {
-  const int halo = a.taps ? a.taps - 1 : 0;
-  a.rows_per_cta = std::min(std::max(4, (a.rows + kSms - 1) / kSms), kRowsWarps<NVW> - halo);
-  const dim3 grid((a.rows + a.rows_per_cta - 1) / a.rows_per_cta), block(kRowsWarps<NVW> * 32);
-  if (a.taps == 0) return launch_pdl(lm_norm_rows_kernel<T, NVW, false>, grid, block, 0, s, a);
-  return launch_pdl(lm_norm_rows_kernel<T, NVW, true>, grid, block, rows_smem<NVW>(a.ldx), s, a);
+  constexpr int kRows = WPR == 1 ? 16 : kWideRows;
+  const int per_sm = (a.rows + kSms - 1) / kSms, taps_before = a.taps ? a.taps - 1 : 0;
+  const auto go = [&](auto kernel, int rows, int rows_per_cta, size_t smem) {
+    a.rows_per_cta = rows_per_cta;
+    return launch_pdl(kernel, dim3((a.rows + rows_per_cta - 1) / rows_per_cta), dim3(rows * WPR * 32), smem, s, a);
+  };
+  const int one_pass = std::min(std::max(4, per_sm), kRows - taps_before);
+  if (a.taps) return go(lm_norm_rows_kernel<T, NV, WPR, kRows, true, (NV <= 12)>, kRows, WPR > 1 ? std::max(4, per_sm) : one_pass, rows_smem(a.ldx));
+  // Nothing binds the rows to one CTA.  Where 16 of them are more than a wave, smaller CTAs that do not look ahead keep more warps on an
+  // SM: us, 16 / 8 rows, 1536 columns, 3000 rows 12.4 / 10.8, 12000 51 / 48; at 2048 columns 12 rows, where that saves a wave: 3000 rows
+  // 16.3 / 13.7, 5000 32.0 / 29.1, but 4000 22.9 / 25.9 and 7000 37.0 / 40.2.
+  constexpr int kMany = NV <= 12 ? 8 : 12;
+  if (WPR == 1 && per_sm > kRows && (NV <= 12 || (per_sm <= 40 && (per_sm + 23) / 24 < (per_sm + 15) / 16))) return go(lm_norm_rows_kernel<T, NV, 1, kMany, false, false>, kMany, kMany, 0);
+  return go(lm_norm_rows_kernel<T, NV, WPR, kRows, false, (NV <= 12)>, kRows, one_pass, 0);
 }
 
 template <class T, int NV>
@@ -399,10 +440,10 @@ cudaError_t launch_norm_nv(cudaStream_t s, const NormArgs& a) {
 template <class T>
 cudaError_t configure_norm_t() {
   const auto most = [](auto* f, size_t bytes) { return cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes); };
-  cudaError_t r = most(lm_norm_rows_kernel<T, 8, true>, rows_smem<8>(1024));
-  if (r == cudaSuccess) r = most(lm_norm_rows_kernel<T, 12, true>, rows_smem<12>(1536));
-  if (r == cudaSuccess) r = most(lm_norm_rows_kernel<T, 16, true>, rows_smem<16>(2048));
-  if (r == cudaSuccess) r = most(lm_norm_rows_kernel<T, 32, true>, rows_smem<32>(4096));
+  cudaError_t r = most(lm_norm_rows_kernel<T, 8, 1, 16, true, true>, rows_smem(1024));
+  if (r == cudaSuccess) r = most(lm_norm_rows_kernel<T, 12, 1, 16, true, true>, rows_smem(1536));
+  if (r == cudaSuccess) r = most(lm_norm_rows_kernel<T, 16, 1, 16, true, false>, rows_smem(2048));
+  if (r == cudaSuccess) r = most(lm_norm_rows_kernel<T, 16, 2, kWideRows, true, false>, rows_smem(4096));
   if (r == cudaSuccess) r = most(lm_norm_kernel<T, 1>, kNormSmemMax);
   if (r == cudaSuccess) r = most(lm_norm_kernel<T, 2>, kNormSmemMax);
   if (r == cudaSuccess) r = most(lm_norm_kernel<T, 4>, kNormSmemMax);
@@ -414,10 +455,10 @@ cudaError_t launch_norm_t(cudaStream_t s, const NormArgs& a) {
   // enough rows for a warp each, and a convolution (if any) that fits the register window
   if (a.rows >= 2 * kSms && !a.gather && (a.taps == 0 || (a.taps >= 2 && a.taps <= 4)) && a.ldx <= 4096) {
     const int w = (a.ldx / 4 + 31) / 32;
-    if (w <= 8) return launch_norm_rows<T, 8>(s, a);
-    if (w <= 12) return launch_norm_rows<T, 12>(s, a);
-    if (w <= 16) return launch_norm_rows<T, 16>(s, a);
-    return launch_norm_rows<T, 32>(s, a);
+    if (w <= 8) return launch_norm_rows<T, 8, 1>(s, a);
+    if (w <= 12) return launch_norm_rows<T, 12, 1>(s, a);
+    if (w <= 16) return launch_norm_rows<T, 16, 1>(s, a);
+    return launch_norm_rows<T, 16, 2>(s, a);
   }
   const int per = (a.ldx / 4 + kNormThreads - 1) / kNormThreads;
   // (two float4 columns a thread: more do not fit the registers with all that is in flight)
@@ -522,7 +563,7 @@ __global__ void __launch_bounds__(kNormThreads) lm_post_norm_rows_kernel(PostNor
   if (t >= a.rows) return;
   float4 x[NVW];
   if (a.delta.p) {
-    warp_delta<NVW>(a.delta, t, lane, nv, x);
+    warp_delta<NVW, 32>(a.delta, t, lane, nv, x);
   } else {
 #pragma unroll
     for (int i = 0; i < NVW; ++i) x[i] = make_float4(0, 0, 0, 0);

@@ -38,6 +38,27 @@ def test_convolution_in_steps(width, taps, dtype, tmp_path):
     c.model.close()
 
 
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("width,taps", [(1536, 1), (2048, 1), (2056, 4), (2304, 2), (4096, 3)])
+def test_many_rows_of_wide_models(width, taps, dtype, tmp_path):
+    """Above 2048 columns a block makes passes of 8 rows and keeps three: 18 rows and more a block, sequences that begin and end in every
+    place of a pass, rows in front of a block from the sequence before.  Without a convolution: more rows than one wave of the larger blocks."""
+    cfg = M.config(width, 60, [M.layer("attention", M.attention(1, 1, 16, 16, 25), 64)], taps=taps)
+    w = M.weights(cfg, 5)
+    c = Case(M.write(tmp_path / "m", cfg, w), V, cfg, w, dtype, max_seqs=7, max_ctx=1500, max_rows=2500)
+    steps = [[1, 1100, 2, 700, 3, 400, 260], [1, 1, 200, 500, 1, 900, 740]]
+    toks = [c.tokens(sum(s[i] for s in steps), seed=i) for i in range(7)]
+    want = [c.oracle(t) for t in toks]
+    at, slots = [0] * 7, [c.model.acquire() for _ in toks]
+    for counts in steps:
+        rows = c.model.step([(s, t[a:a + n]) for s, t, a, n in zip(slots, toks, at, counts)], list(range(sum(counts))))
+        c.model.check_device_status()
+        for i, n in enumerate(counts):
+            c.check(rows[sum(counts[:i]):sum(counts[:i + 1])], want[i][at[i]:at[i] + n])
+            at[i] += n
+    c.model.close()
+
+
 def test_engines_of_two_widths_in_two_threads(tmp_path):
     """Widths that share the kernels of the norms but not the shared memory these ask for: neither engine's launches may set a limit
     that the other's, from another host thread, then exceed."""
