@@ -37,6 +37,7 @@
 // kernel (gemm_stream.cu) mostly stays ahead: it needs no 128-row tiles (1536 x 1536, M = 64: 6.2 us; here, M = 65, 13.3).
 // fp16-encoded scales, us: 1536 x 1536, M = 65 19.4, 1536 x 8960, M = 512 87, 8960 x 1536, M = 512 38 (27, 110 and 47 with
 // finished chunks fetched in front of every turn and a wait of the MMA issuer for either part).
+#include <cuda.h>
 #include <cuda_fp16.h>
 
 #include "device_common.cuh"
@@ -84,7 +85,8 @@ struct CkSmem {
   static constexpr int kStageOff = kBarBytes + kHdrBytes;
   static constexpr int kTotal = kStageOff + kStages * kStageBytes + 1024;
   static_assert(kAccCols + kAStages * kACols == 512, "tensor memory");
-  static_assert((2 * kStages + 2 * kAStages + 4) * 8 + 8 <= kBarBytes, "barrier area");
+  static_assert((3 * kStages + 2 * kAStages + 4) * 8 + 8 <= kBarBytes, "barrier area");
+  static_assert(!kPair || (kStageOff % 128 == 0 && kStageBytes % 128 == 0 && kRawBytes % 128 == 0), "a tensor copy's destination");
   static_assert(kTotal <= 227 * 1024, "shared memory");
 };
 
@@ -140,12 +142,14 @@ __device__ __forceinline__ void ck_arrive(uint32_t bar, int rank) {
   else
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
-// ... that also hands on what this thread has seen arrive in shared memory
-__device__ __forceinline__ void ck_release_to_cta0(uint32_t bar) {
+// A box of the activation blocks, [K-group][8 rows of x][512 bytes], into this CTA's shared memory; its bytes are counted on the barrier
+// of CTA 0 that has bar's place there.
+__device__ __forceinline__ void ck_pair_load(uint32_t dst, const CUtensorMap* map, int m8, int group, uint32_t bar) {
   asm volatile(
       "{\n\t.reg .b32 r;\n\t"
-      "mapa.shared::cluster.u32 r, %0, 0;\n\t"
-      "mbarrier.arrive.release.cluster.shared::cluster.b64 _, [r];\n\t}" ::"r"(bar)
+      "mapa.shared::cluster.u32 r, %4, 0;\n\t"
+      "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%5, %2, %3}], [r];\n\t}" ::"r"(dst),
+      "l"(map), "r"(m8), "r"(group), "r"(bar), "r"(0)
       : "memory");
 }
 // arrival once the MMAs issued so far have completed, on both CTAs' barriers for a pair
@@ -225,7 +229,7 @@ __device__ __forceinline__ float ck_clamp(float v) {  // clamp_flt_max: only inf
 }
 
 template <int NT>
-__global__ void __launch_bounds__(kCkThreads, 1) w4a32_gemm_chunk_kernel(const __grid_constant__ CkParams p) {
+__global__ void __launch_bounds__(kCkThreads, 1) w4a32_gemm_chunk_kernel(const __grid_constant__ CkParams p, const __grid_constant__ CUtensorMap amap) {
   using S = CkSmem<NT>;
   constexpr bool kPair = S::kPair;
   constexpr int kStages = S::kStages, kAStages = S::kAStages, kGroups = S::kGroups, kSpan = S::kSpan;
@@ -234,12 +238,15 @@ __global__ void __launch_bounds__(kCkThreads, 1) w4a32_gemm_chunk_kernel(const _
   uint8_t* smem_ptr = smem_raw + (smem - smem_u32(smem_raw));
   const uint32_t raw_full = smem;                       // [kStages]  loaded data arrived
   const uint32_t raw_free = raw_full + kStages * 8;     // [kStages]  the MMAs that read a stage completed
-  const uint32_t a_full = raw_free + kStages * 8;       // [kAStages] operand written (a pair: by both, in CTA 0; CTA 1's rows of x arrived)
+  const uint32_t a_full = raw_free + kStages * 8;       // [kAStages] operand written (a pair: by both, in CTA 0)
   const uint32_t a_free = a_full + kAStages * 8;        // [kAStages] operand read
   const uint32_t acc_full = a_free + kAStages * 8;      // [2] a chunk's sums are complete
   const uint32_t acc_free = acc_full + 16;              // [2] ... and are in registers (a pair: both, in CTA 0)
+  // A pair: the copies of x of both CTAs count on barriers of CTA 0, whose instructions read them.  Those are a_full, one wait for both
+  // (another wait a stage: 15 % of the kernel); of two parts, whose operand stages come round twice as often, barriers of their own.
+  const uint32_t x_own = acc_free + 16;                 // [kStages]
   const uint32_t stages = smem + S::kStageOff;
-  constexpr int kBars = 2 * kStages + 2 * kAStages + 4;
+  constexpr int kXBar = 2 * kStages + 2 * kAStages + 4, kBars = kXBar + (kPair ? kStages : 0);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem_ptr);
   uint32_t* tmem_base_slot = reinterpret_cast<uint32_t*>(bars + kBars);
   float* s_scale = reinterpret_cast<float*>(smem_ptr + S::kBarBytes);
@@ -268,8 +275,8 @@ __global__ void __launch_bounds__(kCkThreads, 1) w4a32_gemm_chunk_kernel(const _
   if (tid == 0) {
     for (int i = 0; i < kBars; ++i) {
       const bool written = i >= 2 * kStages && i < 2 * kStages + kAStages;  // a_full: a warp writes two K-groups of its 32 rows
-      const bool fetched = i >= kBars - 2;                                  // acc_free
-      mbar_init(&bars[i], (written ? 2 * kGroups : fetched ? kCkDqWarps : 1) * ((written || fetched) && kPair ? 2 : 1) + (written && kPair ? 1 : 0));
+      const bool fetched = i >= kXBar - 2 && i < kXBar;                     // acc_free
+      mbar_init(&bars[i], (written ? 2 * kGroups : fetched ? kCkDqWarps : 1) * ((written || fetched) && kPair ? 2 : 1) + (kPair && written && parts == 1 ? 1 : 0));
     }
     mbar_fence_init();
   }
@@ -288,6 +295,8 @@ __global__ void __launch_bounds__(kCkThreads, 1) w4a32_gemm_chunk_kernel(const _
   tc_fence_after();
   const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_base_slot, 0);
 
+  const uint32_t x_full = parts == 1 ? a_full : x_own;
+  static_assert(kStages == kAStages, "a stage's number is that of its operand");
   if (warp == kCkDqWarps) {
     // ------------------------------------------------------------ producer
     const int np = max(0, min(kCkPanels, pr.num_panels - panel0));
@@ -297,13 +306,17 @@ __global__ void __launch_bounds__(kCkThreads, 1) w4a32_gemm_chunk_kernel(const _
     auto request = [&](int it, int which) {  // bit 0: weight cells (and the barrier), bit 1: activation blocks
       const int s = it % kStages, g0 = it * kGroups, ng = min(kGroups, p.num_groups - g0);
       uint8_t* st = smem_ptr + S::kStageOff + s * S::kStageBytes;
-      if ((which & 1) && lane == 0) mbar_arrive_expect_tx(&bars[s], (uint32_t)(np * ng * kCellBytes + ng * b_bytes));
+      if ((which & 1) && lane == 0) mbar_arrive_expect_tx(&bars[s], (uint32_t)(np * ng * kCellBytes + (kPair ? 0 : ng * b_bytes)));
       __syncwarp();
+      if (kPair && (which & 2) && lane == kCkPanels) {  // whole boxes: what lies outside of the blocks arrives as zeros
+        if (rank == 0) mbar_arrive_expect_tx(&bars[(x_full - smem) / 8 + s], 2u * S::kBBytes);
+        ck_pair_load(smem_u32(st) + S::kRawBytes, &amap, b_row0 >> 3, g0, x_full + (uint32_t)s * 8);
+      }
       if ((which & 1) && lane < np)
         bulk_g2s_hint(st + lane * kGroups * kCellBytes,
                       pr.tiled + sizeof(TiledHeader) + ((size_t)(panel0 + lane) * p.num_groups + g0) * kCellBytes,
                       (uint32_t)(ng * kCellBytes), &bars[s], stream_once);
-      else if ((which & 2) && lane >= kCkPanels && lane < kCkPanels + ng && b_bytes > 0)
+      else if (!kPair && (which & 2) && lane >= kCkPanels && lane < kCkPanels + ng && b_bytes > 0)
         bulk_g2s(st + S::kRawBytes + (lane - kCkPanels) * S::kRowsB * 64,
                  p.a_blocks + ((size_t)(g0 + lane - kCkPanels) * p.m8 + (b_row0 >> 3)) * 512, (uint32_t)b_bytes, &bars[s]);
     };
@@ -315,7 +328,12 @@ __global__ void __launch_bounds__(kCkThreads, 1) w4a32_gemm_chunk_kernel(const _
       for (int it = 0; it < first_lap; ++it) request(it, 2);
     }
     for (int it = first_lap; it < k_tiles; ++it) {
-      if (!ck_wait(raw_free + (uint32_t)(it % kStages) * 8, (uint32_t)(it / kStages - 1) & 1u)) break;
+      if (!ck_wait(raw_free + (uint32_t)(it % kStages) * 8, (uint32_t)(it / kStages - 1) & 1u)) {
+        // nothing in flight when the CTA leaves: 10 ms is a thousand times what a copy takes
+        for (const long long t0 = clock64(); clock64() - t0 < (1ll << 24);) {
+        }
+        break;
+      }
       request(it, 3);
     }
   } else if (warp == kCkDqWarps + 1) {
@@ -331,10 +349,12 @@ __global__ void __launch_bounds__(kCkThreads, 1) w4a32_gemm_chunk_kernel(const _
       uint32_t accumulate = 0;
       for (int it = 0; it < k_tiles && ok;) {
         const int steps = min(kStep, left);
-        for (int v = it * parts + parts - 1; v < (it + steps) * parts && ok; v += parts)
+        for (int v = it * parts + parts - 1; v < (it + steps) * parts && ok; v += parts) {
           // arrived on by warps that saw raw_full complete: orders the stage's copies too.  (Of two parts the last: the
           // same warps wrote the first before it.)
           ok = ck_wait<kPair>(a_full + (uint32_t)(v % kAStages) * 8, (uint32_t)(v / kAStages) & 1u);
+          if (kPair && parts > 1 && ok) ok = ck_wait(x_full + (uint32_t)(v / parts % kStages) * 8, (uint32_t)(v / parts / kStages) & 1u);
+        }
         left -= steps;
 #pragma unroll
         for (int h = 0; h < kHalves; ++h) {
@@ -379,17 +399,6 @@ __global__ void __launch_bounds__(kCkThreads, 1) w4a32_gemm_chunk_kernel(const _
           left = min(chunk_tiles, k_tiles - it);
           accumulate = 0;
         }
-      }
-    } else {
-      // CTA 1 of a pair: its rows of x, read by instructions that CTA 0 issues, are announced there by a thread that saw them arrive
-      // (one that has nothing else to do: the release would hold up the dequant warps)
-      bool ok = true;
-      for (int v = 0; v < k_tiles * parts && ok; ++v) {
-        const int it = v / parts;
-        ok = ck_wait(raw_full + (uint32_t)(it % kStages) * 8, (uint32_t)(it / kStages) & 1u);
-        if (ok && v >= kAStages) ok = ck_wait(a_free + (uint32_t)(v % kAStages) * 8, (uint32_t)(v / kAStages - 1) & 1u);
-        if (ok && lane == 0) ck_release_to_cta0(a_full + (uint32_t)(v % kAStages) * 8);
-        __syncwarp();
       }
     }
   } else {
@@ -545,6 +554,25 @@ __global__ void __launch_bounds__(kCkThreads, 1) w4a32_gemm_chunk_kernel(const _
   }
 }
 
+// The activation blocks as a tensor [num_groups][m8][128 words], in boxes of a stage's K-groups and a CTA's half of 256 rows
+static cudaError_t ck_encode(CUtensorMap* map, const CkParams& prm) {
+  using Encode = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
+                              const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+  static const Encode encode = [] {
+    cudaDriverEntryPointQueryResult q;
+    void* f = nullptr;
+    return cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &q) == cudaSuccess ? reinterpret_cast<Encode>(f) : nullptr;
+  }();
+  if (!encode) return cudaErrorSymbolNotFound;
+  using S = CkSmem<256>;
+  const cuuint64_t dims[3] = {128, (cuuint64_t)prm.m8, (cuuint64_t)prm.num_groups}, strides[2] = {512, (cuuint64_t)prm.m8 * 512};
+  const cuuint32_t box[3] = {128, S::kRowsB / 8, S::kGroups}, one[3] = {1, 1, 1};
+  const CUresult r = encode(map, CU_TENSOR_MAP_DATA_TYPE_UINT32, 3, const_cast<uint8_t*>(prm.a_blocks), dims, strides, box, one,
+                            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
+}
+
 template <int NT>
 static cudaError_t ck_launch_t(const CkParams& prm, int tiles, cudaStream_t stream) {
   using S = CkSmem<NT>;
@@ -577,7 +605,9 @@ static cudaError_t ck_launch_t(const CkParams& prm, int tiles, cudaStream_t stre
   }
   cfg.attrs = attrs;
   cfg.numAttrs = na;
-  return cudaLaunchKernelEx(&cfg, w4a32_gemm_chunk_kernel<NT>, prm);
+  CUtensorMap amap = {};
+  if (S::kPair && (e = ck_encode(&amap, prm)) != cudaSuccess) return e;
+  return cudaLaunchKernelEx(&cfg, w4a32_gemm_chunk_kernel<NT>, prm, amap);
 }
 
 // blocks / hdr: output of launch_act_quant_blocks_f16 for the same m and k with rows padded to a multiple of 8.  Up to four
