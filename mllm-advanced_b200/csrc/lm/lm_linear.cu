@@ -516,212 +516,6 @@ __global__ void __launch_bounds__(TcShape<BN>::kThreads, 1) lm_gemm_tc_kernel(co
   if (warp == 1) tmem_dealloc(tmem, S::kTmemCols);
 }
 
-// ------------------------------------------------------------------------------------------ tcgen05 GEMM of CTA pairs
-// 256 rows of x x 256 weight rows by two CTAs (cta_group::2): each loads its 128 rows of x and its 128 weight rows, one instruction
-// of CTA 0 multiplies what lies in both shared memories, and each CTA's tensor memory gets its 128 rows of the result.  What
-// bounds the kernel above with prompts is the way from L2: 48 KB a K tile of 64 for 128 x 256 sums at about 40 bytes a cycle
-// (1230 cycles; the tensor pipe needs 512).  A CTA of a pair loads 32 KB for as many.  us of a prompt of 1500 rows, single CTAs with
-// four epilogue warps and stores of 16 bytes / pairs with eight and of 32: 1536 -> 17920 gated 96 / 78 (pairs with the old
-// epilogue 97, with eight warps 79.5), 8960 -> 1536 48 / 38 (K in two), 1536 -> 6144 35 / 30, 1536 -> 2048 15.5 / 15.2,
-// 1536 -> 1536 14.6 / 13.  Now 1000 cycles a K tile.
-// Barriers: the loads of both CTAs complete on `full` of CTA 0, whose MMA warp is the one that waits for them; commits arrive in
-// both CTAs; the epilogue warps of both free an accumulator in CTA 0.
-constexpr int kPairN = 256, kPairStages = 6, kPairStageBytes = 2 * kABytes;
-constexpr int kPairSmem = kPairStages * kPairStageBytes + 1024;
-constexpr int kPairEpiWarps = 8, kPairEpiCols = kPairN / (kPairEpiWarps / 4);  // epilogue warps, columns of one (and 32 rows)
-constexpr int kPairThreads = 64 + 32 * kPairEpiWarps;  // copy warp, MMA warp, epilogue
-
-// The box goes into this CTA's shared memory, its bytes are counted on a barrier of CTA 0 (bar: an address of the cluster).
-__device__ __forceinline__ void pair_load_2d(void* dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
-  asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
-                   smem_u32(dst)),
-               "l"(map), "r"(x), "r"(y), "r"(bar)
-               : "memory");
-}
-// Hands on tensor-memory reads that tcgen05.wait::ld and a tcgen05 fence have closed: those two and a relaxed arrival order tensor
-// memory between threads of a cluster, stores would need a release.
-__device__ __forceinline__ void arrive_at_cta0(uint32_t bar) {
-  asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-// mbar_wait_bounded for those arrivals
-__device__ __forceinline__ bool pair_try_wait(uint64_t* bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.relaxed.cluster.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-__device__ __forceinline__ bool pair_wait_bounded(uint64_t* bar, uint32_t parity) {
-  if (pair_try_wait(bar, parity)) return true;
-  const long long t0 = clock64();
-  while (!pair_try_wait(bar, parity))
-    if (clock64() - t0 > (1ll << 31)) {
-      atomicOr(&g_device_status, kDevStatusTimeout);
-      return false;
-    }
-  return true;
-}
-__device__ __forceinline__ void pair_commit(uint64_t* bar) {
-  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(smem_u32(bar)),
-               "h"((uint16_t)3)
-               : "memory");
-}
-__device__ __forceinline__ void pair_mma_f16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-
-// Work items as above, a row tile is 256 rows; pair c takes items c, c + pairs, ...
-template <int FORM>
-__global__ void __launch_bounds__(kPairThreads, 1) lm_gemm_pair_kernel(const __grid_constant__ CUtensorMap amap,
-                                                                     const __grid_constant__ CUtensorMap wmap, int M, int N, int K, int splits,
-                                                                     Epi e) {
-  extern __shared__ uint8_t tc_smem_raw[];
-  __shared__ uint64_t full[kPairStages], empty[kPairStages], acc_full[2], acc_empty[2];  // (full and acc_empty: those of CTA 0 are used)
-  __shared__ uint32_t tmem_slot;
-  __shared__ volatile int gave_up;
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(tc_smem_raw) + 1023) & ~(uintptr_t)1023);
-  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
-  const int rank = (int)(blockIdx.x & 1), pair = (int)(blockIdx.x >> 1), pairs = (int)(gridDim.x >> 1);
-  const int mt = (M + 2 * kTileM - 1) / (2 * kTileM), nt = (N + kPairN - 1) / kPairN, kt = K / kTileK, items = mt * nt * splits;
-  if (tid == 0) {
-    for (int i = 0; i < kPairStages; ++i) mbar_init(&full[i], 1), mbar_init(&empty[i], 1);
-    for (int i = 0; i < 2; ++i) mbar_init(&acc_full[i], 1), mbar_init(&acc_empty[i], 2 * kPairEpiWarps);
-    gave_up = 0;
-    mbar_fence_init();
-  }
-  if (warp == 1) {
-    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)), "r"(512u) : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
-  }
-  tc_fence_before();
-  __syncthreads();
-  cluster_sync_all();  // the other CTA's barriers and tensor memory exist
-  tc_fence_after();
-  const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_slot, 0);
-  pdl_launch_dependents();
-  auto k_range = [&](int item, int& k0, int& k1) {
-    const int split = item / (mt * nt);
-    k0 = (int)((long long)kt * split / splits);
-    k1 = (int)((long long)kt * (split + 1) / splits);
-  };
-  if (warp == 0) {
-    if (elect_one_sync()) {
-      int it = 0, ahead = 0, st = 0;
-      uint32_t ph = 0;
-      bool ok = true;
-      const uint32_t full0 = map_to_cta(full, 0);
-      // CTA 0 announces the bytes of both: a stage is complete when it has done so and all of them have landed.  (CTA 1's may
-      // land first.  It reuses a stage once `empty` says that the MMAs have read it, so never two phases ahead.)
-      auto load_w = [&](int stage, int k, int item) {
-        if (rank == 0) mbar_arrive_expect_tx(&full[stage], 2u * kPairStageBytes);
-        pair_load_2d(smem + stage * kPairStageBytes + kABytes, &wmap, k * kTileK, (item / mt % nt) * kPairN + rank * 128, full0 + 8 * stage);
-      };
-      {  // the weights do not depend on the previous kernel, the activations do: fill the ring with weights first
-        int k0, k1;
-        k_range(pair, k0, k1);
-        for (; ahead < kPairStages && ahead < k1 - k0; ++ahead) load_w(ahead, k0 + ahead, pair);
-        pdl_wait_prior();
-      }
-      for (int item = pair; item < items && ok; item += pairs) {
-        int k0, k1;
-        k_range(item, k0, k1);
-        for (int k = k0; k < k1; ++k, ++it) {
-          if (it >= kPairStages && (gave_up || !mbar_wait_bounded(&empty[st], ph ^ 1u))) {
-            ok = false;
-            break;
-          }
-          if (it >= ahead) load_w(st, k, item);
-          pair_load_2d(smem + st * kPairStageBytes, &amap, k * kTileK, (item % mt) * 2 * kTileM + rank * kTileM, full0 + 8 * st);
-          if (++st == kPairStages) st = 0, ph ^= 1u;
-        }
-      }
-      if (!ok) gave_up = 1;
-      // nothing in flight when the CTA leaves.  (After a wait that ran out the phases of `full` say nothing about this CTA's copies:
-      // 10 ms is a thousand times what one takes.)
-      const long long t0 = clock64();
-      while (!ok && clock64() - t0 < (1ll << 24)) {
-      }
-    }
-  } else if (warp == 1 && rank == 0) {
-    const bool leader = elect_one_sync();
-    const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kPairN >> 3) << 17) | ((uint32_t)(2 * kTileM >> 4) << 24);
-    const uint32_t smem0 = (smem_u32(tc_smem_raw) + 1023u) & ~1023u;
-    int st = 0, t = 0;
-    uint32_t ph = 0;
-    bool ok = true;
-    for (int item = pair; item < items && ok; item += pairs, ++t) {
-      int k0, k1;
-      k_range(item, k0, k1);
-      const int buf = t & 1;
-      if (t >= 2) ok = __all_sync(0xffffffffu, !gave_up && pair_wait_bounded(&acc_empty[buf], ((t >> 1) & 1) ^ 1));
-      tc_fence_after();
-      for (int k = k0; k < k1 && ok; ++k) {
-        ok = __all_sync(0xffffffffu, !gave_up && mbar_wait_bounded(&full[st], ph));
-        if (!ok) break;
-        tc_fence_after();
-        // (operands are values of the whole warp, outside of the elected lane's branch: see above)
-        const uint32_t a = smem0 + (uint32_t)(st * kPairStageBytes);
-        const uint64_t ad = swizzled_desc(a), bd = swizzled_desc(a + kABytes);
-        if (leader) {
-#pragma unroll
-          for (int j = 0; j < kTileK / 16; ++j)
-            pair_mma_f16(tmem + buf * kPairN, ad + j * 2, bd + j * 2, idesc, (k > k0 || j > 0) ? 1u : 0u);
-          pair_commit(&empty[st]);
-        }
-        __syncwarp();
-        if (++st == kPairStages) st = 0, ph ^= 1u;
-      }
-      if (ok && leader) pair_commit(&acc_full[buf]);
-      __syncwarp();
-    }
-    if (!ok) gave_up = 1;
-  } else if (warp >= 2) {
-    pdl_wait_prior();  // outputs may still be read by the kernel before
-    const int quarter = warp & 3, c_begin = (warp - 2) / 4 * kPairEpiCols;
-    const uint32_t acc_empty0 = map_to_cta(acc_empty, 0);
-    int t = 0;
-    for (int item = pair; item < items; item += pairs, ++t) {
-      const int buf = t & 1;
-      if (gave_up || !mbar_wait_bounded(&acc_full[buf], (t >> 1) & 1)) {
-        gave_up = 1;
-        break;
-      }
-      tc_fence_after();
-      const int n0 = (item / mt % nt) * kPairN, split = item / (mt * nt);
-      const int m0 = (item % mt) * 2 * kTileM + rank * kTileM + quarter * 32, m = m0 + lane;
-      if (m0 < M) {
-        const uint32_t base = tmem + ((uint32_t)(quarter * 32) << 16) + buf * kPairN;
-#pragma unroll 1
-        for (int c = c_begin; c < c_begin + kPairEpiCols; c += 32) {
-          if (n0 + c >= N) break;
-          uint32_t r0[16], r1[16];
-          tmem_ld16(base + c, r0);
-          tmem_ld16(base + c + 16, r1);
-          tmem_ld_wait();
-          if (m < M) store32<FORM>(e, m, n0 + c, N, r0, r1, split);
-          __syncwarp();
-        }
-      }
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) arrive_at_cta0(acc_empty0 + 8 * buf);
-    }
-  }
-  tc_fence_before();
-  __syncthreads();
-  cluster_sync_all();  // nobody frees tensor memory or leaves while the other still uses it
-  tc_fence_after();
-  if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
-}
-
 // ------------------------------------------------------------------------------------------ packing
 __global__ void lm_pack_rows_kernel(const __nv_bfloat16* __restrict__ src, int n, int k, __nv_bfloat16* __restrict__ dst, int ldk,
                                     int row_block, int row_block_pad, int row_mul, int row_off, int col_block, int col_block_pad) {
@@ -761,18 +555,13 @@ int encode(CUtensorMap* map, const void* base, int rows, int k, int box_rows) {
              : MLLMB200_CUDA_ERROR;
 }
 
-// Tile width (kPairTile: 256 x 256 by pairs of CTAs) and K splits with the smallest estimated time: waves x (K tiles x cycles per
-// K tile + fixed cost).
-constexpr int kPairTile = 512;
-void choose_tile(int M, int mt, int a_rows, int N, int K, int max_splits, bool pairs, int* bn_out, int* splits_out) {
+// Tile width and K splits with the smallest estimated time: waves x (K tiles x cycles per K tile + fixed cost).  Prompts of 256 to 2000
+// rows, 14 shapes of 896 to 2048 columns: the choice is the fastest of all in four cases of five, 25% off at most.  (256 x 256 sums by pairs of
+// CTAs, cta_group::2, a third fewer bytes from L2: slower than 128 x 256 with eight epilogue warps throughout; 1500 rows, us, pairs / this:
+// 1536 -> 17920 gated 85 / 68, 1536 -> 6144 29.7 / 26.3, 8960 -> 1536 36.7 / 34.8; 300 rows 1536 -> 17920 31.7 / 30.6.)
+void choose_tile(int M, int mt, int a_rows, int N, int K, int max_splits, int* bn_out, int* splits_out) {
   const int kt = K / kTileK;
   double best = 1e30;
-  for (int s = 1; pairs && s <= max_splits && s <= kt; ++s) {
-    const long long items = (long long)((M + 255) / 256) * ((N + 255) / 256) * s;
-    const double waves = (double)((items + kSms / 2 - 1) / (kSms / 2));
-    const double t = waves * (((kt + s - 1) / s) * 820.0 + 600.0 + 6.0 * 256) + 1200.0 + (s - 1) * (150.0 + 8.0 * M * N / 2600.0);
-    if (t < best) best = t, *bn_out = kPairTile, *splits_out = s;
-  }
   for (int bn : {256, 128, 64, 32}) {
     const int nt = (N + bn - 1) / bn;
     for (int s = 1; s <= max_splits && s <= kt; ++s) {
@@ -803,36 +592,6 @@ cudaError_t launch_tc(cudaStream_t s, const Linear& w, const ActMap& am, int M, 
   return f == kFormPlanes ? launch_tc_form<BN, kFormPlanes>(s, w, am, M, splits, g, e)
          : f == kFormGate ? launch_tc_form<BN, kFormGate>(s, w, am, M, splits, g, e)
                           : launch_tc_form<BN, kFormScatter>(s, w, am, M, splits, g, e);
-}
-template <int FORM>
-cudaError_t launch_pair_form(cudaStream_t s, const Linear& w, const ActMap& am, int M, int splits, const Epi& e) {
-  const int items = (M + 255) / 256 * ((w.n + 255) / 256) * splits;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)std::min(2 * items, kSms), 1, 1);
-  cfg.blockDim = dim3(kPairThreads, 1, 1);
-  cfg.dynamicSmemBytes = kPairSmem;
-  cfg.stream = s;
-  cudaLaunchAttribute attrs[2];
-  attrs[0].id = cudaLaunchAttributeClusterDimension;
-  attrs[0].val.clusterDim.x = 2;
-  attrs[0].val.clusterDim.y = attrs[0].val.clusterDim.z = 1;
-  attrs[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attrs[1].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attrs;
-  cfg.numAttrs = 2;
-  ++g_launches;
-  return cudaLaunchKernelEx(&cfg, lm_gemm_pair_kernel<FORM>, am.map128, w.map128, M, w.n, w.k, splits, e);
-}
-cudaError_t launch_pair(cudaStream_t s, const Linear& w, const ActMap& am, int M, int splits, const Epi& e) {
-  const Form f = form_of(e);
-  return f == kFormPlanes ? launch_pair_form<kFormPlanes>(s, w, am, M, splits, e)
-         : f == kFormGate ? launch_pair_form<kFormGate>(s, w, am, M, splits, e)
-                          : launch_pair_form<kFormScatter>(s, w, am, M, splits, e);
-}
-cudaError_t configure_pair() {
-  cudaError_t r = cudaFuncSetAttribute(lm_gemm_pair_kernel<kFormPlanes>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmem);
-  if (r == cudaSuccess) r = cudaFuncSetAttribute(lm_gemm_pair_kernel<kFormScatter>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmem);
-  return r != cudaSuccess ? r : cudaFuncSetAttribute(lm_gemm_pair_kernel<kFormGate>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmem);
 }
 template <int BN, int FORM>
 cudaError_t configure_tc() {
@@ -885,7 +644,6 @@ cudaError_t linear_configure() {
   if (r == cudaSuccess) r = configure_tc_forms<128>();
   if (r == cudaSuccess) r = configure_tc_forms<64>();
   if (r == cudaSuccess) r = configure_tc_forms<32>();
-  if (r == cudaSuccess) r = configure_pair();
   if (r == cudaSuccess) r = configure_gemv<float>();
   if (r == cudaSuccess) r = configure_gemv<__nv_bfloat16>();
   return r;
@@ -922,9 +680,8 @@ int launch_linear(cudaStream_t s, bool f32, const Linear& w, const ActMap& am, c
                    static_cast<const float*>(x), w.w, M, w.n, w.k, nullptr, nullptr, e);
   } else {
     int bn = 32;
-    choose_tile(M, (M + kTileM - 1) / kTileM, M >= kTileM ? kTileM : pad_to(M, 16), w.n, w.k, e.kind == kEpiPlanes ? max_splits : 1,
-                M >= 2 * kTileM, &bn, &splits);
-    r = bn == kPairTile ? launch_pair(s, w, am, M, splits, e) : launch_tc_any(s, bn, w, am, M, splits, nullptr, e);
+    choose_tile(M, (M + kTileM - 1) / kTileM, M >= kTileM ? kTileM : pad_to(M, 16), w.n, w.k, e.kind == kEpiPlanes ? max_splits : 1, &bn, &splits);
+    r = launch_tc_any(s, bn, w, am, M, splits, nullptr, e);
   }
   return r == cudaSuccess ? splits : -1;
 }
@@ -940,8 +697,7 @@ int launch_linear_groups(cudaStream_t s, bool f32, const Linear& w, const ActMap
   } else {
     int bn = 32;
     const int per = (g.rows + g.likely_tiles - 1) / g.likely_tiles;
-    choose_tile(g.rows, g.likely_tiles, std::min(kTileM, pad_to(per, 16)), w.n, w.k, e.kind == kEpiPlanes ? max_splits : 1,
-                false, &bn, &splits);
+    choose_tile(g.rows, g.likely_tiles, std::min(kTileM, pad_to(per, 16)), w.n, w.k, e.kind == kEpiPlanes ? max_splits : 1, &bn, &splits);
     r = launch_tc_any(s, bn, w, am, g.rows, splits, &g, e);
   }
   return r == cudaSuccess ? splits : -1;

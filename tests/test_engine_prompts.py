@@ -1,7 +1,6 @@
-"""The engine's GEMM of CTA pairs (256 rows of x x 256 weight rows) with steps of 256 to 1000 rows: queries, keys and values into
-their places, gated products, sums in one and two planes; second CTAs of a pair without rows, weight rows and heads that end
-inside a tile, sizes off the tile's on every side.  At these sizes the cost model takes pairs for every linear of a layer
-from about 500 rows on; bars as everywhere for the bf16 format (lm_case.py)."""
+"""The engine's tile GEMM with steps of 256 to 1000 rows, one to four 256-wide and 128-wide row and weight tiles: queries, keys and values
+into their places, gated products, sums in one and several planes; weight rows and heads that end inside a tile, sizes off the tile's on
+every side.  Bars as everywhere for the bf16 format (lm_case.py)."""
 import os
 import sys
 
@@ -18,7 +17,7 @@ from lm_case import Case  # noqa: E402
 @pytest.mark.parametrize("width,mixer,ff", [(1088, ("attention", M.attention(64, 4, 64, 64, 40)), 2056),
                                             (520, ("attention", M.attention(72, 3, 48, 64, 25)), 4100),
                                             (1032, ("retention", M.retention(24, 48, 80, 48, [0.9 + i / 250 for i in range(24)])), 3000)])
-def test_prompts_in_pairs(width, mixer, ff, tmp_path):
+def test_prompts(width, mixer, ff, tmp_path):
     cfg = M.config(width, 300, [M.layer(*mixer, ff)], taps=3)
     w = M.weights(cfg, 11)
     c = Case(M.write(tmp_path / "m", cfg, w), V, cfg, w, "bfloat16", max_seqs=2, max_ctx=1008, max_rows=1000)
