@@ -555,21 +555,25 @@ int encode(CUtensorMap* map, const void* base, int rows, int k, int box_rows) {
              : MLLMB200_CUDA_ERROR;
 }
 
-// Tile width and K splits with the smallest estimated time: waves x (K tiles x cycles per K tile + fixed cost).  Prompts of 256 to 2000
-// rows, 14 shapes of 896 to 2048 columns: the choice is the fastest of all in four cases of five, 25% off at most.  (256 x 256 sums by pairs of
+// Tile width and K splits with the smallest estimated time: waves x (K tiles x cycles per K tile + fixed cost).  Whole row tiles (128 rows
+// and more): a K tile of 128 x 256 sums costs about 1000 cycles, the way from L2; a narrower one not below 720, the chain from the
+// copy to the freed stage.  Fitted to timings of 128 to 2000 rows, 14 shapes of 896 to 2048 columns, weights from memory: what is chosen
+// is within 3% of the fastest nearly everywhere, 16% off at worst; with 1230 cycles and no least cost, up to 25% off.  (256 x 256 sums by pairs of
 // CTAs, cta_group::2, a third fewer bytes from L2: slower than 128 x 256 with eight epilogue warps throughout; 1500 rows, us, pairs / this:
-// 1536 -> 17920 gated 85 / 68, 1536 -> 6144 29.7 / 26.3, 8960 -> 1536 36.7 / 34.8; 300 rows 1536 -> 17920 31.7 / 30.6.)
+// 1536 -> 17920 gated 85 / 68, 1536 -> 6144 29.7 / 26.3, 8960 -> 1536 36.7 / 34.8.)  Fewer rows are priced as by the bytes alone,
+// too low for narrow tiles: 32 rows, 2048 -> 2048 takes 7.9 us, and 5.1 with tiles of 128 columns and K in eight parts.
 void choose_tile(int M, int mt, int a_rows, int N, int K, int max_splits, int* bn_out, int* splits_out) {
   const int kt = K / kTileK;
+  const bool whole = a_rows == kTileM;
   double best = 1e30;
   for (int bn : {256, 128, 64, 32}) {
     const int nt = (N + bn - 1) / bn;
     for (int s = 1; s <= max_splits && s <= kt; ++s) {
       const long long items = (long long)mt * nt * s;
       const double waves = (double)((items + kSms - 1) / kSms);
-      const double per_k = std::max(2.0 * bn, (a_rows + bn) * 128.0 / 40.0);
+      const double per_k = whole ? std::max(720.0, (a_rows + bn) * 2.6) : std::max(2.0 * bn, (a_rows + bn) * 128.0 / 40.0);
       // more planes are written here and read by the consumer: about 2600 bytes per cycle
-      const double t = waves * (((kt + s - 1) / s) * per_k + 600.0 + 6.0 * bn) + 900.0 + (s - 1) * (150.0 + 8.0 * M * N / 2600.0);
+      const double t = waves * (((kt + s - 1) / s) * per_k + 600.0 + (whole ? 1.5 : 6.0) * bn) + 900.0 + (s - 1) * (150.0 + 8.0 * M * N / 2600.0);
       if (t < best) best = t, *bn_out = bn, *splits_out = s;
     }
   }
