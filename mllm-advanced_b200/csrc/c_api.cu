@@ -274,12 +274,9 @@ static int forward_through_blocks(const W4Blocks& b, const float* x_dev, int M, 
                                       : launch_act_quant_blocks_f16(x_dev, M, b.m_pad, K, ldx, b.blocks, b.hdr, st, use_pdl, b.clear, b.clear_count);
   // The GEMM is a dependent launch of the quantization even where the call itself is not one of what came before: all that it does
   // before that has finished is to read the weights, which nothing of this call writes.  (M = 512, 1536 -> 8960: 28.6 -> 26.7 us a
-  // call; M = 48, 8960 -> 1536: 24.7 -> 19.5.)  Not where its tiles take more than one wave, of which only the first gains: 1536 ->
-  // 17920 in a row, M = 2048 176 us so and 183 as a dependent launch, M = 512 46 and 47; 1536 -> 8960, M = 2048 93 and 96.
-  long long tiles = 0;
-  for (int i = 0; i < count; ++i) tiles += (long long)((N[i] + 127) / 128) * ((M + 255) / 256);
-  const int dependent = use_pdl || b.form == kW4Stream || tiles <= 148;
-  if (e == cudaSuccess) e = w4a32_forward_blocks(b, M, K, count, tiled_dev, y_dev, N, ldy, dependent, st);
+  // call; M = 48, 8960 -> 1536: 24.7 -> 19.5.)  Also where its tiles take many waves: calls in a row, launched in order / so, M = 700, 1536 -> 8960
+  // 51.4 / 49.0, 512, 1536 -> 17920 50.9 / 49.5, "fastest" 39.5 / 37.2; 2048, 1536 -> 17920 185 / 185, 8192 -> 28672 995 / 998.
+  if (e == cudaSuccess) e = w4a32_forward_blocks(b, M, K, count, tiled_dev, y_dev, N, ldy, 1, st);
   return e == cudaSuccess ? MLLMB200_OK : cuda_fail(e);
 }
 

@@ -744,9 +744,7 @@ cudaError_t launch_w4a16_gemm_tcf16_grouped(const uint8_t* a_blocks, int m, int 
   TfParams prm = {};
   prm.a_blocks = a_blocks;
   prm.a_hdr = nullptr;
-  long long t256 = 0;
-  for (int i = 0; i < count; ++i) t256 += (long long)((n[i] + 127) / 128) * ((m + 255) / 256);
-  prm.use_pdl = t256 <= 148;  // (behind its quantization, which is launched in order; not for more than a wave, as in c_api.cu)
+  prm.use_pdl = 1;  // behind its quantization, which is launched in order (as in c_api.cu)
   prm.m = m, prm.k = k;
   prm.num_groups = (k + kGroup - 1) / kGroup;
   prm.m8_pad = (m + nt - 1) / nt * nt / 8;
