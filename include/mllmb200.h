@@ -425,6 +425,14 @@ MLLMB200_API void mllmb200_w4a32_tp_destroy(void* handle);
  * NULL) is 1.  The kernel returns normally; nothing faults. */
 MLLMB200_API int mllmb200_selftest_wait_timeout(long long limit_ticks, int* gave_up_dev, void* stream);
 
+/* The operators in front of the decoder's linears by themselves (tests): op 0 h = a + b (b may be NULL), RMS norm with gain w; op 1
+ * silu(a) * b; then the linear of kernel policy `kernel` (0 or 5, with its flags) on the result.  form 0 = the operator writes fp32 rows
+ * to x_dev [M][K] and the linear quantizes them, 1 = the operator writes the linear's operand blocks (MLLMB200_UNSUPPORTED where the
+ * linear takes none).  a, b, h_out (NULL: none) [M][K], y [M][N] fp32; ws of workspace_size(M, K) bytes. */
+MLLMB200_API int mllmb200_selftest_operator_linear(int op, int form, const float* a_dev, const float* b_dev, const float* w_dev, float eps,
+                                                   int M, int K, int N, const void* tiled_dev, void* ws_dev, float* x_dev, float* h_out_dev,
+                                                   float* y_dev, int kernel, void* stream);
+
 /* The Qwen2 decoder's prompt attention by itself (tests): causal, n tokens from position 0, RoPE with the given tables.
  * form: 0 = what a prompt of n tokens takes, 1 = fp32 on the CUDA cores, 2 = tensor cores.  q_dev and out_dev
  * [n, q_heads * head_dim], k_dev and v_dev [n, kv_heads * head_dim], sin_dev and cos_dev [n, head_dim / 2], caches

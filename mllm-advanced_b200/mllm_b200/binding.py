@@ -64,6 +64,8 @@ def lib():
         "mllmb200_w4a32_quant_activations": ([vp, C.c_int, C.c_int, C.c_int, vp, vp], C.c_int),
         "mllmb200_check_device_status": ([vp], C.c_int),
         "mllmb200_selftest_wait_timeout": ([C.c_longlong, vp, vp], C.c_int),
+        "mllmb200_selftest_operator_linear": ([C.c_int, C.c_int, vp, vp, vp, C.c_float, C.c_int, C.c_int, C.c_int, vp, vp, vp, vp, vp,
+                                               C.c_int, vp], C.c_int),
         "mllmb200_w4a32_tp_init": ([C.c_int, C.c_int, vp, C.POINTER(vp)], C.c_int),
         "mllmb200_w4a32_tp_alloc_output": ([vp, C.c_size_t, C.POINTER(vp), vp], C.c_int),
         "mllmb200_w4a32_tp_ipc_export": ([vp, C.c_size_t, C.POINTER(vp), vp], C.c_int),

@@ -1,5 +1,6 @@
-"""Prompts through the operators that write their linear's operand blocks themselves: one layer at the edges of those kernels, against
-the numpy oracle.  Bar on the 2-norm of the last logits: an int8 activation on a boundary may go the other way, which moves the
+"""Prompts through the operators that write their linear's operand blocks themselves.  Every row of an operator with its linear has the
+bits of the operator followed by the linear's own quantization; and one layer of a decoder at the edges of those kernels, its last row
+(which sees the others through the first norm's keys and values alone) against the numpy oracle.  Bar on the 2-norm of the last logits: an int8 activation on a boundary may go the other way, which moves the
 outputs of one linear by up to a quantum of one of its K inputs, 2^-8 of the row's range over sqrt(K); with a handful of those
 in a layer 5e-3 (LOGIT_TOL of test_decoder.py, there on the largest difference)."""
 import os
@@ -30,3 +31,34 @@ def test_prompt_blocks(hidden, inter, n):
     dec.prefill(prompt)
     got = dec.read(n - 1, 1, want_logits=True)[2].astype(np.float64)
     assert np.linalg.norm(got - want) <= LOGIT_TOL * np.linalg.norm(want)
+
+
+# the same edges row by row: int8 blocks (policy 5 up to 192 rows of a narrow matrix too), fp16 blocks of the tile GEMMs with and without
+# rows of padding, K-split counters; one CTA a row and four; K off 32, 8 and 4
+@pytest.mark.parametrize("op,k", [(0, 64), (0, 72), (0, 1032), (0, 2048), (1, 40), (1, 3073), (1, 3080), (1, 4864), (1, 6152), (1, 8960),
+                                  (1, 9224), (1, 12000)])
+@pytest.mark.parametrize("m,n,kernel", [(5, 96, 0), (33, 40, 5), (41, 64, 0), (64, 64, 5), (65, 64, 0), (128, 96, 5), (130, 40, 0), (200, 64, 5),
+                                        (257, 320, 5)])
+def test_every_row_has_the_bits_of_operator_and_quantization(op, k, m, n, kernel):
+    import ctypes as C
+
+    import torch
+    import mllm_b200 as mb
+    rng = np.random.default_rng(op + k + m)
+    wt = mb.W4A32Weights.from_blob(mb.quant_prepack((rng.standard_normal((n, k)) / np.sqrt(k)).astype(np.float32), rng.standard_normal(n).astype(np.float32)))
+    dev = lambda a: torch.from_numpy(np.asarray(a, np.float32)).cuda()  # noqa: E731
+    a, b, w = dev(rng.standard_normal((m, k)) * 2), dev(rng.standard_normal((m, k))), dev(1 + 0.1 * rng.standard_normal(k))
+    a[m // 2], b[m // 2] = 0, 0
+    out = []
+    for form in (0, 1):
+        x, h, y = (torch.full((m, c), float("nan"), device="cuda") for c in (k, k, n))
+        ws = torch.full((mb.workspace_size(m, k),), 0x7e, dtype=torch.uint8, device="cuda")
+        st = mb.lib().mllmb200_selftest_operator_linear(op, form, a.data_ptr(), b.data_ptr(), w.data_ptr(), 1e-6, m, k, n, wt.tiled.data_ptr(),
+                                                        ws.data_ptr(), x.data_ptr(), h.data_ptr(), y.data_ptr(), kernel,
+                                                        C.c_void_p(torch.cuda.current_stream().cuda_stream))
+        assert st == 0, mb.status_str(st)
+        torch.cuda.synchronize()
+        mb.check_device_status()
+        out.append((y, h))
+    assert torch.isfinite(out[0][0]).all() and torch.equal(out[0][0], out[1][0])
+    assert op == 1 or torch.equal(out[0][1], out[1][1])

@@ -175,6 +175,8 @@ TENSOR_SHAPES = [
     (64, 256, 128, 4), (100, 100, 33, 4), (130, 512, 320, 4), (200, 1176, 1280, 4), (512, 1536, 1536, 4),
     (512, 1536, 8960, 4), (512, 8960, 1536, 4), (300, 1536, 8960, 0), (70, 256, 96, 0), (512, 1536, 256, 2), (130, 512, 320, 2), (63, 8192, 512, 0), (40, 256, 8200, 0), (16, 512, 96, 4),
     (1, 1536, 256, 2), (3, 100, 33, 2), (4, 8960, 1536, 2),   # the record-based dp4a kernel where auto takes the fused one
+    # one tile of x as wide as the rows need where the weight tiles fill the SMs, on both sides of its limits in rows and weight rows
+    (65, 96, 8065, 4), (127, 512, 8200, 4), (64, 96, 8200, 4), (100, 96, 8064, 4), (129, 224, 12673, 4), (255, 96, 12800, 4), (140, 96, 12672, 4),
 ]
 
 
