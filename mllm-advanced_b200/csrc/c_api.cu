@@ -84,7 +84,7 @@ static inline size_t ws_rec_bytes(int m, int k) {
   const size_t blk = w4a32_gemm_tc_supported(m, k, 1) ? (size_t)w4a32_gemm_tc_m_pad(m) * blob_num_blocks(k) * 32 : 0;
   // fp16 operand blocks of the fp16 tensor-core path (64 bytes per row and K-group, rows padded to its widest tile)
   const size_t blk16 = w4a32_gemm_tcf16_supported(m, k, 1) ? (size_t)w4a32_gemm_tcf16_m_pad_max(m) * blob_num_blocks(k) * 64 : 0;
-  // activation blocks of the streaming small-batch GEMM (36 bytes per row and K-group, rows padded to 8)
+  // activation blocks of the streaming small-batch GEMM (32 bytes per row and K-group, sized as 36, rows padded to 8)
   const size_t mma = m <= kStreamGemmMaxM ? w4a32_gemm_stream_act_bytes(m, k) : 0;
   size_t big = rec > blk ? rec : blk;
   big = big > mma ? big : mma;

@@ -68,7 +68,7 @@ constexpr size_t kMsSmemMax = 227 * 1024;
 struct MsProblem {
   const uint8_t* tiled;  // TiledHeader at offset 0
   float* y;
-  int n, ldy, num_panels, panel_begin;  // panels [panel_begin, panel_begin + num_panels) of the launch
+  int n, ldy, panel_begin;  // first panel of the launch
   size_t zsum_off, bias_off;
 };
 struct MsParams {
@@ -195,7 +195,7 @@ __global__ void __launch_bounds__(kMsThreads, 1) w4a32_gemm_stream_kernel(const 
   uint64_t* red_full = peer_free + 2;  // the warps' sums of a unit are in place
   uint64_t* red_free = red_full + 1;   // ... and have been read
   float2* s_hdr = reinterpret_cast<float2*>(ms_smem + Lo.hdr);
-  volatile int* flags = reinterpret_cast<volatile int*>(ms_smem + Lo.flags);  // bad header, wait ran out, -, -, scale encodings
+  volatile int* flags = reinterpret_cast<volatile int*>(ms_smem + Lo.flags);  // bad header, -, start value, -, scale encodings
   uint8_t* acts = ms_smem + Lo.acts;
   uint8_t* ring = ms_smem + Lo.ring;
   float* red = reinterpret_cast<float*>(ms_smem + Lo.red);
@@ -217,7 +217,6 @@ __global__ void __launch_bounds__(kMsThreads, 1) w4a32_gemm_stream_kernel(const 
     mbar_init(red_full, kMsCWarps);
     mbar_init(red_free, kMsEWarps);
     mbar_fence_init();
-    flags[1] = 0;  // set when a wait ran out
     flags[2] = (int)kMsMagic;
   }
   if (warp == 1) {
@@ -344,7 +343,6 @@ __global__ void __launch_bounds__(kMsThreads, 1) w4a32_gemm_stream_kernel(const 
           if (issued == NST && !acts_requested) request_acts();  // the ring is full of weights: now the activations
           if (issued >= NST) {
             if (!mbar_wait_bounded(&empty[st], ph ^ 1u)) {
-              flags[1] = 1;
               ok = false;
               break;
             }
@@ -498,7 +496,6 @@ __global__ void __launch_bounds__(kMsThreads, 1) w4a32_gemm_stream_kernel(const 
       if (lane == 0) mbar_arrive(red_full);
       if (!ok) break;
     }
-    if (!ok && lane == 0) flags[1] = 1;
   } else {
     // =============================== epilogue warps ===============================
     constexpr int kEThreads = kMsEWarps * 32;
@@ -516,7 +513,6 @@ __global__ void __launch_bounds__(kMsThreads, 1) w4a32_gemm_stream_kernel(const 
                  if (lane == 0) mbar_arrive(red_free);
                });
     }
-    if (!ok && lane == 0) flags[1] = 1;
   }
   // Leave together: ranks 1.. hold partial sums that rank 0 reads, rank 0 holds the barriers they arrive on.
   __syncthreads();
@@ -687,7 +683,7 @@ static int ms_cluster_capacity(int s, size_t smem) {
 }
 
 // Nothing here but the number of panels depends on N: a matrix has the same bits whether it is launched alone or grouped.
-// The limit of K is that of 36 bytes per row and group (what callers' workspaces are made for) in eight shares of 112 KB.
+// The limit of K is that of 36 bytes per row and group (as workspaces are sized) in eight shares of 112 KB.
 // The smallest cluster whose shared memory holds the activations, a power of two (us, 8960 -> 1536, M = 16, an earlier form of
 // the kernel: sizes 2 / 3 / 4 / 5 10.4 / 15.4 / 13.0 / 13.3); two from K = 4480 on, where one CTA would walk a unit for longer
 // than the exchange takes (8960 -> 1536, M = 16: 12.7 alone, 10.1; 4864 -> 896, M = 24: 9.8, 8.7), but for a single tile of
@@ -736,7 +732,8 @@ bool w4a32_gemm_stream_preferred(int m, int k, int count, const int* n) {
   return m > kMsNamedMaxM && (m >= 128 || k >= 1024) && ms_shape_plan(m, k, count, n, &plan) && plan.total_panels <= 4096 / kPanelRows;
 }
 
-// bytes of the activation blocks for m rows of k values (rows padded to a multiple of 8; what workspaces are made for)
+// bytes of the activation blocks for m rows of k values (rows padded to a multiple of 8): 32 a row and K-group are written; workspaces, and
+// the limit of K above, go by 36
 size_t w4a32_gemm_stream_act_bytes(int m, int k) {
   return (size_t)((k + kGroup - 1) / kGroup) * (size_t)((m + 7) / 8 * 8) * 36;
 }
@@ -829,7 +826,6 @@ cudaError_t launch_w4a32_gemm_stream(const uint8_t* acts, const float2* a_hdr, i
     prm.prob[i].y = y[i];
     prm.prob[i].n = n[i];
     prm.prob[i].ldy = ldy[i];
-    prm.prob[i].num_panels = (int)th.num_panels;
     prm.prob[i].panel_begin = begin;
     prm.prob[i].zsum_off = th.zsum_off;
     prm.prob[i].bias_off = th.bias_off;
