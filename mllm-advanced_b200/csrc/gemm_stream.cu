@@ -721,15 +721,21 @@ bool w4a32_gemm_stream_supported(int m, int k, int count, const int* n) {
 }
 
 // Where the "fastest" policy (5) takes this kernel above 64 rows: matrices, or groups, of at most 4096 rows, whose 128-row tiles
-// would leave most SMs of the tile GEMMs idle, and up to 192 rows of x, in blocks of 32.  us with the quantization, the tile
-// GEMM that policy took / this kernel: M = 65 (gemm_chunk.cu) 1536 -> 1536 13.3 / 7.8, 8960 -> 1536 50.1 / 19.6, 4864 -> 896
-// 30.0 / 12.7; M = 127 14.7 / 9.2, 54.0 / 26.9, 32.1 / 14.3; M = 192 (gemm_tcf16.cu) 15.6 / 11.5, 33.7 / 33.0, 23.4 / 17.3;
-// M = 256 16.8 / 13.5, 35.2 / 43.5, 24.4 / 20.6; more weight rows: 896 -> 9728, M = 128 10.8 / 19.7.  Error against 64 bits, the
-// same: K = 8960 9.7e-8 / 6.9e-8 (M = 65) and 4.3e-7 / 6.9e-8 (M = 192), K = 1536 5.2e-8 / 5.1e-8 and 7.8e-8 / 5.2e-8, K = 896
-// 4.3e-8 / 4.5e-8 and 9.5e-8 / 4.6e-8: short K below 128 rows stays where it was.
+// would leave most SMs of the tile GEMMs idle, up to 192 rows of x, in blocks of 32, and as long as a CTA has few K-groups to walk
+// through: its time grows with those (0.03 to 0.05 us each), that of the tile GEMMs with K alone.  The lines lie where 243 timings below 128
+// rows and 450 above cross (256 to 4096 weight rows, K = 896 to 14336): what is taken is at most 3% slower than the tile GEMM that policy
+// took.  us with the quantization, that / this kernel: M = 65 (gemm_chunk.cu) 1536 -> 1536 13.3 / 7.8, 8960 -> 1536 50.1 / 19.6,
+// 4864 -> 896 30.0 / 12.7; M = 127 14.7 / 9.2, 54.0 / 26.9, 32.1 / 14.3; M = 192 (gemm_tcf16.cu) 15.9 / 10.8, 33.7 / 33.1, 23.0 / 16.6, 2048 -> 3072
+// 18.2 / 16.9; beyond the lines 896 -> 4096 12.8 / 15.4, 4096 -> 4096 23.3 / 33.1, 14336 -> 4096 51 / 119; M = 256 1536 -> 1536 16.8 / 13.5,
+// 8960 -> 1536 35.2 / 43.5.  Error against 64 bits, the same: K = 8960 9.7e-8 / 6.9e-8 (M = 65) and 4.3e-7 / 6.9e-8 (M = 192), K = 1536
+// 5.2e-8 / 5.1e-8 and 7.8e-8 / 5.2e-8, K = 896 4.3e-8 / 4.5e-8 and 9.5e-8 / 4.6e-8: short K below 128 rows stays where it was.
 bool w4a32_gemm_stream_preferred(int m, int k, int count, const int* n) {
   MsPlan plan;
-  return m > kMsNamedMaxM && (m >= 128 || k >= 1024) && ms_shape_plan(m, k, count, n, &plan) && plan.total_panels <= 4096 / kPanelRows;
+  if (m <= kMsNamedMaxM || (m < 128 && k < 1024) || !ms_shape_plan(m, k, count, n, &plan) || plan.total_panels > 4096 / kPanelRows) return false;
+  const int G = (k + kGroup - 1) / kGroup, S = plan.cluster_size, per_block = std::max(1, 148 / S / plan.num_blocks);
+  const int walk = (plan.total_panels + per_block - 1) / per_block * plan.groups_per_rank;
+  if (m < 128) return walk <= 180 + 16 * G / 5;
+  return walk <= (G < 32 ? 3 * G : S <= 2 ? 170 + 17 * G / 10 : 7 * G / 4);
 }
 
 // bytes of the activation blocks for m rows of k values (rows padded to a multiple of 8): 32 a row and K-group are written; workspaces, and

@@ -638,14 +638,15 @@ static TfTile tf_tile_for(int m, int count, const int* n) {
   // One tile of x as wide as the rows need, where the weight tiles alone give most SMs one: the weights are dequantized once
   // a tile, which costs more than the columns of padding (us with the quantization, 1536 -> 17920 in narrower / one tile:
   // M = 65 23.6 / 14.1, M = 127 24.3 / 15.3, M = 129 27.4 / 19.6, M = 255 28.0 / 21.6; 896 -> 9728, 76 weight tiles, M = 65
-  // 15.6 / 9.9, but M = 160 18.6 / 20.5; 8192 -> 28672 M = 160, 128 / 256 / 256 with 256 weight rows 154 / 127 / 117).
+  // 15.6 / 9.9, but M = 160 18.6 / 20.5; 8192 -> 28672 M = 160, 128 / 256 / 256 with 256 weight rows 154 / 127 / 117).  Up to 74 weight
+  // tiles two narrow tiles of x still are one wave, and one wide one would split K: 1536 -> 8192, M = 65 14.1 / 15.5, 127 14.3 / 17.5.
   if (MLLMB200_TF_WIDE && wide && m > 128 && t256 * ((m + 255) / 256) >= 100) {  // (256 rows x 128: measured slower than 128 x 256, 31 vs 24 us)
     t.rows = 256;
     t.nt = 256;
     return t;
   }
   t.rows = 128;
-  t.nt = (m > 128 && t128 * ((m + 255) / 256) >= 100) ? 256 : (m >= 128 || (m > 64 && t128 >= 64) ? 128 : 64);
+  t.nt = (m > 128 && t128 * ((m + 255) / 256) >= 100) ? 256 : (m >= 128 || (m > 64 && 2 * t128 > 148) ? 128 : 64);
   return t;
 }
 int w4a32_gemm_tcf16_tile(int m, int n) { return tf_tile_for(m, 1, &n).nt; }
@@ -734,7 +735,8 @@ cudaError_t launch_w4a32_gemm_tcf16_grouped(const uint8_t* a_blocks, const float
 int w4a16_gemm_tcf16_tile_grouped(int m, int count, const int* n) {
   long long t128 = 0;
   for (int i = 0; i < count; ++i) t128 += (n[i] + 127) / 128;
-  return (m > 128 && t128 * ((m + 255) / 256) >= 100) ? 256 : (m >= 128 || (m > 64 && t128 >= 64) ? 128 : 64);  // as tf_tile_for
+  // as tf_tile_for, but K is never split here: one wide tile from 64 weight tiles on (896 -> 8192, M = 65, two / one 19.6 / 14.9 us)
+  return (m > 128 && t128 * ((m + 255) / 256) >= 100) ? 256 : (m >= 128 || (m > 64 && t128 >= 64) ? 128 : 64);
 }
 int w4a16_gemm_tcf16_tile(int m, int n) { return w4a16_gemm_tcf16_tile_grouped(m, 1, &n); }
 cudaError_t launch_w4a16_gemm_tcf16_grouped(const uint8_t* a_blocks, int m, int k, int count, const void* const* tiled,

@@ -151,6 +151,14 @@ def test_peer_stores_come_from_the_kernel_that_the_forward_runs():
     assert L.mllmb200_w4a32_plan_kernel(128, 1536, 1536, 5) == 7 and L.mllmb200_w4a32_plan_kernel(193, 1536, 1536, 5) == 4
 
 
+def test_fastest_policy_between_64_and_192_rows():
+    """The streaming GEMM where a CTA has few K-groups to walk through, else the tile GEMM that is faster there (8 with chunked sums, 4)."""
+    for m, k, n, want in ((65, 1536, 1536, 7), (65, 896, 1536, 8), (96, 8960, 1536, 7), (127, 4864, 4096, 7), (127, 12288, 4096, 8), (128, 1536, 4096, 7),
+                          (192, 1536, 4096, 4), (192, 1536, 3584, 7), (128, 896, 1536, 7), (192, 896, 4096, 4), (192, 8960, 1536, 7), (192, 8960, 2048, 4),
+                          (192, 4096, 4096, 4), (128, 14336, 4096, 4), (192, 14336, 1024, 7), (193, 1536, 1536, 4), (128, 1536, 4128, 4), (64, 1536, 1536, 7)):
+        assert mb.lib().mllmb200_w4a32_plan_kernel(m, k, n, 5) == want, (m, k, n)
+
+
 def test_workspace_covers_the_tile_gemms_up_to_their_last_row():
     """Where the default takes a tile GEMM above 64 rows, the workspace holds its fp16 activation blocks (64 bytes per row and
     K-group, rows in eights) and the rows' headers; beyond the rows that its launch can cover it takes no tile GEMM."""
