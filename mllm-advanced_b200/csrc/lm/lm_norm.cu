@@ -3,6 +3,7 @@
 #include <cooperative_groups.h>
 
 #include <algorithm>
+#include <type_traits>
 
 #include "../device_common.cuh"
 #include "lm_route.cuh"
@@ -37,23 +38,17 @@ __device__ __forceinline__ void store4(__nv_bfloat16* p, const float4& v) {
   *reinterpret_cast<uint2*>(p) = make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
 }
 
-// columns [c, c + 4) of a row of the sublayer output.  Four planes, or the rows of four experts, are requested before the first is
-// added (in order): a row by itself is a chain of latencies.
-__device__ __forceinline__ float4 load_planes(const Delta& d, const float* p) {
-  float4 v = make_float4(0, 0, 0, 0);
-  for (int i0 = 0; i0 < d.planes; i0 += 4) {
-    float4 q[4];
-#pragma unroll
-    for (int j = 0; j < 4; ++j)
-      if (i0 + j < d.planes) q[j] = *reinterpret_cast<const float4*>(p + (i0 + j) * d.plane);
-#pragma unroll
-    for (int j = 0; j < 4; ++j)
-      if (i0 + j < d.planes) v = i0 + j == 0 ? q[j] : fma4(1.0f, q[j], v);
-  }
-  return v;
-}
+// columns [c, c + 4) of a row of the sublayer output.  Four experts' rows are requested before the first is added (in order): a row by
+// itself is a chain of latencies.  Planes are left to the compiler, which does the same with less: four requested by hand cost Vupuzen's
+// and dense Taralix' decode steps 1 to 2%.  MIX false: no experts (their code alone costs a dense model of 1536 columns 2% of a step).
+template <bool MIX = true>
 __device__ __forceinline__ float4 load_delta(const Delta& d, int row, int c) {
-  if (!d.mix_w) return load_planes(d, d.p + (size_t)row * d.ldx + c);
+  if (!MIX || !d.mix_w) {
+    const float* p = d.p + (size_t)row * d.ldx + c;
+    float4 v = *reinterpret_cast<const float4*>(p);
+    for (int i = 1; i < d.planes; ++i) v = fma4(1.0f, *reinterpret_cast<const float4*>(p + i * d.plane), v);
+    return v;
+  }
   float4 v = make_float4(0, 0, 0, 0);
   for (int k0 = 0; k0 < d.top; k0 += 4) {
     float w[4];
@@ -474,7 +469,7 @@ cudaError_t launch_norm_t(cudaStream_t s, const NormArgs& a) {
 
 // x' = rms_unit(alpha x + delta) * gain, a CTA per row.  With a router a cluster of CTAs per row: each makes the row and
 // the logits of its share of the experts, the first one keeps the row and chooses.
-template <class T, int NV, bool ROUTER>
+template <class T, int NV, bool ROUTER, bool MIX>
 __global__ void __launch_bounds__(kNormThreads) lm_post_norm_kernel(PostNormArgs a) {
   extern __shared__ __align__(16) float row_x[];  // [ldx], then [experts]; with a router only
   __shared__ float scratch[32];
@@ -499,7 +494,7 @@ __global__ void __launch_bounds__(kNormThreads) lm_post_norm_kernel(PostNormArgs
     const int c = tid + i * kNormThreads;
     x[i] = make_float4(0, 0, 0, 0);
     if (c < nv) {
-      const float4 d = a.delta.p ? load_delta(a.delta, src, c * 4) : x[i];
+      const float4 d = a.delta.p ? load_delta<MIX>(a.delta, src, c * 4) : x[i];
       x[i] = fma4(a.alpha, *reinterpret_cast<const float4*>(a.x_in + (size_t)src * a.ldx + c * 4), d);
     }
     ss += dot4(x[i]);
@@ -592,13 +587,13 @@ __global__ void __launch_bounds__(kNormThreads) lm_post_norm_rows_kernel(PostNor
 
 constexpr int kFusedRouterRows = 2 * kSms;
 
-template <class T, int NV>
+template <class T, int NV, bool MIX>
 cudaError_t launch_post_norm_nv(cudaStream_t s, const PostNormArgs& a) {
-  if (!a.router.w) return launch_pdl(lm_post_norm_kernel<T, NV, false>, dim3(a.rows), dim3(kNormThreads), 0, s, a);
+  if (!a.router.w) return launch_pdl(lm_post_norm_kernel<T, NV, false, MIX>, dim3(a.rows), dim3(kNormThreads), 0, s, a);
   int parts = 8;
   while (parts > 1 && (a.rows * parts > 2 * kSms || a.router.experts < parts * (kNormThreads / 32))) parts /= 2;
   const size_t smem = (size_t)(a.ldx + a.router.experts) * sizeof(float);
-  return launch_pdl_cluster(lm_post_norm_kernel<T, NV, true>, dim3(a.rows, parts), dim3(kNormThreads), dim3(1, parts, 1), smem, s, a);
+  return launch_pdl_cluster(lm_post_norm_kernel<T, NV, true, MIX>, dim3(a.rows, parts), dim3(kNormThreads), dim3(1, parts, 1), smem, s, a);
 }
 template <class T>
 cudaError_t launch_post_norm_t(cudaStream_t s, const PostNormArgs& a) {
@@ -610,11 +605,15 @@ cudaError_t launch_post_norm_t(cudaStream_t s, const PostNormArgs& a) {
     return launch_pdl(lm_post_norm_rows_kernel<T, 32>, grid, dim3(kNormThreads), 0, s, a);
   }
   const int per = (a.ldx / 4 + kNormThreads - 1) / kNormThreads;
-  if (per <= 1) return launch_post_norm_nv<T, 1>(s, a);
-  if (per <= 2) return launch_post_norm_nv<T, 2>(s, a);
-  if (per <= 4) return launch_post_norm_nv<T, 4>(s, a);
-  if (per <= 8) return launch_post_norm_nv<T, 8>(s, a);
-  return cudaErrorInvalidValue;
+  const auto go = [&](auto mix) {
+    constexpr bool kMix = decltype(mix)::value;
+    return per <= 1   ? launch_post_norm_nv<T, 1, kMix>(s, a)
+           : per <= 2 ? launch_post_norm_nv<T, 2, kMix>(s, a)
+           : per <= 4 ? launch_post_norm_nv<T, 4, kMix>(s, a)
+           : per <= 8 ? launch_post_norm_nv<T, 8, kMix>(s, a)
+                      : cudaErrorInvalidValue;
+  };
+  return a.delta.p && a.delta.mix_w ? go(std::true_type()) : go(std::false_type());
 }
 
 template <class T>
