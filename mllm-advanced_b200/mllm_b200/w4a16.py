@@ -6,7 +6,7 @@ import functools
 
 import numpy as np
 
-from .binding import _check, _stream_ptr, lib, scratch
+from .binding import _check, _stream_int, _stream_ptr, lib, scratch
 
 
 def prepack_size(n, k, has_bias):
@@ -94,13 +94,12 @@ def linear_forward(x, weights, out=None, workspace=None, stream=None, kernel=KER
     assert k == weights.k
     if out is None:
         out = x.new_empty((m, weights.n), dtype=torch.float16)
-    if workspace is None:
-        workspace = scratch(workspace_size(m, k, weights.n), x, stream)
-    _check(lib().mllmb200_w4a16_linear_forward_ex(x.data_ptr(), 1 if x.dtype == torch.float16 else 0,
-                                                  weights.tiled.data_ptr(), out.data_ptr(), workspace.data_ptr(), m, k,
-                                                  weights.n, x.stride(0), out.stride(0), kernel | (0x100 if pdl else 0),
-                                                  _stream_ptr(stream)),
-           "w4a16_linear_forward")
+    s = _stream_int(stream)
+    with scratch(workspace_size(m, k, weights.n) if workspace is None else 0, s) as ws:
+        _check(lib().mllmb200_w4a16_linear_forward_ex(x.data_ptr(), 1 if x.dtype == torch.float16 else 0, weights.tiled.data_ptr(), out.data_ptr(),
+                                                      ws if workspace is None else workspace.data_ptr(), m, k, weights.n, x.stride(0),
+                                                      out.stride(0), kernel | (0x100 if pdl else 0), s),
+               "w4a16_linear_forward")
     return out
 
 
@@ -113,14 +112,13 @@ def linear_forward_grouped(x, weights_list, outs=None, workspace=None, stream=No
     assert 1 <= cnt <= 4 and all(w.k == k for w in weights_list)
     if outs is None:
         outs = [torch.empty((m, w.n), dtype=torch.float16, device=x.device) for w in weights_list]
-    if workspace is None:
-        workspace = scratch(max(workspace_size(m, k, w.n) for w in weights_list), x, stream)
     tiled = (C.c_void_p * cnt)(*[w.tiled.data_ptr() for w in weights_list])
     ys = (C.c_void_p * cnt)(*[o.data_ptr() for o in outs])
     ns = (C.c_int * cnt)(*[w.n for w in weights_list])
     ldy = (C.c_int * cnt)(*[o.stride(0) for o in outs])
-    _check(lib().mllmb200_w4a16_linear_forward_grouped(x.data_ptr(), 1 if x.dtype == torch.float16 else 0, m, k,
-                                                       x.stride(0), cnt, tiled, ys, ns, ldy, workspace.data_ptr(),
-                                                       0x100 if pdl else 0, _stream_ptr(stream)),
-           "w4a16_linear_forward_grouped")
+    s = _stream_int(stream)
+    with scratch(max(workspace_size(m, k, w.n) for w in weights_list) if workspace is None else 0, s) as ws:
+        _check(lib().mllmb200_w4a16_linear_forward_grouped(x.data_ptr(), 1 if x.dtype == torch.float16 else 0, m, k, x.stride(0), cnt, tiled, ys, ns,
+                                                           ldy, ws if workspace is None else workspace.data_ptr(), 0x100 if pdl else 0, s),
+               "w4a16_linear_forward_grouped")
     return outs

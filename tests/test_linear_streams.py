@@ -9,7 +9,7 @@ torch = pytest.importorskip("torch")
 pytestmark = pytest.mark.gpu
 
 import mllm_b200 as mb  # noqa: E402
-from mllm_b200 import w4a16  # noqa: E402
+from mllm_b200 import binding, w4a16  # noqa: E402
 
 SHAPES = [(1, 1536, 1536, 0), (8, 1536, 1536, 0), (48, 1536, 1536, 0), (64, 4864, 896, 0), (96, 1536, 1536, 0), (160, 1536, 1536, 5),
           (300, 1536, 1536, 5), (513, 1536, 1536, 0)]
@@ -44,6 +44,31 @@ def _wrong(calls, order, stream, own):
         got = [(i, calls[i][0](stream)) for i in order]
     stream.synchronize()
     return [i for i, y in got if not torch.equal(y, calls[i][1])]
+
+
+def test_a_captured_first_call_and_torchs_public_allocator(monkeypatch):
+    """A captured call's memory is the graph's; and without torch's short way to its allocator the public one serves."""
+    m, k, n = 512, 1536, 8960
+    w = mb.W4A32Weights.from_blob(mb.quant_prepack((np.random.default_rng(5).standard_normal((n, k)) * 0.02).astype(np.float32)))
+    x = torch.randn((m, k), device="cuda")
+    graph, s = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph, stream=s):
+        y = mb.linear_forward(x, w)
+    others = [torch.full((1 << 22,), 0x7f, dtype=torch.uint8, device="cuda") for _ in range(8)]  # whatever the allocator hands out meanwhile
+    y.fill_(float("nan"))
+    graph.replay()
+    torch.cuda.synchronize()
+    assert all(bool((o == 0x7f).all()) for o in others)
+    raw = torch._C._cuda_cudaCachingAllocator_raw_alloc  # (what the public way calls today, under whatever name)
+    monkeypatch.delattr(torch._C, "_cuda_cudaCachingAllocator_raw_alloc")
+    monkeypatch.setattr(torch.cuda, "caching_allocator_alloc", lambda size, device=None, stream=None: raw(size, stream))
+    binding._allocator.cache_clear()
+    again = mb.linear_forward(x, w), mb.linear_forward(x, w, stream=s)
+    torch.cuda.synchronize()
+    binding._allocator.cache_clear()
+    assert torch.equal(y, again[0]) and torch.equal(y, again[1])
+    mb.check_device_status()
 
 
 def test_weights_loaded_on_a_stream():
