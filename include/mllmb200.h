@@ -137,7 +137,8 @@ MLLMB200_API int mllmb200_w4a32_linear_forward(const float* x_dev, const void* t
  * split K between two CTAs per output tile, and y holds one half's partial sums for a moment during the
  * call - deterministic, but y is scratch until the call's work on the stream has finished), 5 fastest: kernel 4
  * for M >= 128 and, at 64 <= M < 128, for matrices (or groups) of at least 8192 rows with K <= 4096; kernel 7's code for
- * 65 <= M <= 192 and matrices (or groups) of at most 4096 rows (below M = 128: K >= 1024); else auto,
+ * 65 <= M <= 192 and matrices (or groups) of at most 4096 rows as far as that is the faster one (few rows or a short K; below
+ * M = 128: K >= 1024; plan_kernel below says which); else auto,
  * 6 the two-launch GEMV (activation-quantization kernel + one-shot GEMV), kept for comparison,
  * 7 streaming tensor-core GEMM for small batches (M <= 64; what auto picks for 5 <= M <= 64): the weight cells are
  * spread over all SMs as in the GEMV, the per-group integer products run as mma.sync s8 x s8 (exact int32 group

@@ -22,7 +22,8 @@
 // CTAs, for launches with few tiles.  576 threads, one CTA per SM:
 //   warps 0-15 dequant: thread = weight row 32 (w % 4) + lane; a turn = two K-groups of the row (32 bytes of nibbles -> 32
 //              tensor-memory columns of fp16); a finished chunk is added to the registers after the turn behind it
-//   warp 16    producer: bulk copies of weight cells (evict-first) and activation blocks
+//   warp 16    producer: bulk copies of weight cells (evict-first) and activation blocks (a pair: tensor copies of both CTAs that
+//              count on the barrier of CTA 0 that its products wait for anyway)
 //   warp 17    MMA issuer (one elected lane; of CTA 0 for a pair) and tensor-memory owner
 // A pair multiplies four stages (256 values of K) for the first half of its columns, then for the second: while one half's
 // finished chunk is fetched the other half's products run, and the next four stages are dequantized.
@@ -35,7 +36,7 @@
 // are of one sign throughout, 1.3e-7 / 1.0e-7 at K = 1536, 3.9e-7 / 5.3e-7 at K = 8960.  M = 65, 17920 x 1536
 // 33 / 24 us; the three matrices of q, k, v, M = 65 (one launch instead of three) 47 / 14 us.  At M <= 64 the streaming
 // kernel (gemm_stream.cu) mostly stays ahead: it needs no 128-row tiles (1536 x 1536, M = 64: 6.2 us; here, M = 65, 13.3).
-// fp16-encoded scales, us: 1536 x 1536, M = 65 19.4, 1536 x 8960, M = 512 87, 8960 x 1536, M = 512 38 (27, 110 and 47 with
+// fp16-encoded scales, us: 1536 x 1536, M = 65 19.4, 1536 x 8960, M = 512 87, 8960 x 1536, M = 512 35 (27, 110 and 47 with
 // finished chunks fetched in front of every turn and a wait of the MMA issuer for either part).
 #include <cuda.h>
 #include <cuda_fp16.h>
