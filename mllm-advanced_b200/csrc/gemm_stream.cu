@@ -19,9 +19,9 @@
 //   * a producer warp streams the unit's cells through a ring of stages (cp.async.bulk + full / empty
 //     mbarriers, weights marked evict-first in L2); under programmatic dependent launch the first stages are
 //     requested before griddepcontrol.wait, the activations after it.  A stage is 32 K-groups, two trips of a warp between waits,
-//     where three of those fit beside the activations, else 16 (us, chain of dependent launches, 16 / 32: M = 8 1536 -> 8960 6.8 /
-//     6.4, 2048 -> 17920 13.2 / 12.0, 4096 -> 17920 20.6 / 14.5, 8192 -> 28672 46 / 39; M = 48 8960 -> 1536 17.3 / 16.2; M = 64 8192 ->
-//     28672 131 / 116; a stage may be cut anywhere between K-groups, the bits are the same).  The activations are one copy: in four parts,
+//     where three of those fit beside the activations, else 16 (us, chain of dependent launches, 16 / 32: M = 8 1536 -> 8960 6.4 /
+//     6.0, 2048 -> 17920 10.5 / 9.6, 4096 -> 17920 16.4 / 14.3, 8192 -> 28672 46 / 38; M = 48 8960 -> 1536 17.1 / 16.1; M = 64 8192 ->
+//     28672 130 / 116; a stage may be cut anywhere between K-groups, the bits are the same).  The activations are one copy: in four parts,
 //     of which the first lets the products start, a call of 8 rows takes 0.1 to 0.2 us longer.
 //   * 8 compute warps: warp ks takes the K-groups ks, ks + 8 of a stage.  A cell: one ldmatrix.x4 = the words of four rows
 //     per lane; two LOP3 and a shift make the A fragments of two mma.sync.m16n8k32 (s8: 16 (nibble - 8) in the high half
@@ -39,10 +39,10 @@
 // packed FP32 instructions 32; the rest is issue (about 80 slots) and dependences.  More warps (16), registers filled one
 // stage ahead and 64 columns per warp were each as slow or slower.  With u8 nibbles, a zero-point term per group, scalar
 // FP32 and 32-bit loads a cell took 150.  us a call with its quantization, that form -> now, chain of dependent launches:
-//   1536 -> 17920  M = 8 10.6 -> 10.4, 24 15.7 -> 12.3, 48 22.7 -> 19.1, 64 26.0 -> 21.4
+//   1536 -> 17920  M = 8 10.6 -> 8.5, 24 15.7 -> 12.1, 48 22.7 -> 18.9, 64 26.0 -> 21.5
 //   8960 -> 1536   M = 8 12.7 -> 10.3, 24 19.3 -> 10.9, 48 24.0 -> 16.2, 64 30.7 -> 19.6
-//   8192 -> 28672  M = 8 46.4 -> 39.2, 24 90 -> 54, 64 295 -> 116
-//   2048 -> 4096   M = 8 5.57 -> 5.54; 2048 -> 17920 M = 8 11.9 -> 12.0
+//   8192 -> 28672  M = 8 46.4 -> 38.2, 24 90 -> 54, 64 295 -> 116
+//   2048 -> 4096   M = 8 5.57 -> 4.96; 2048 -> 17920 M = 8 11.9 -> 9.6
 // Every wait is bounded; a cluster leaves together (one cluster barrier at the end) so that no CTA's shared memory
 // disappears under a peer.
 #include <algorithm>
@@ -64,6 +64,11 @@ constexpr int kMsMaxM = 192, kMsNamedMaxM = 64;  // of a launch; of kernel 7 by 
 constexpr int kMsMaxTiles = 4;                // tiles of 8 rows that a CTA multiplies a cell with
 constexpr int kMsRedCol = 36;                 // floats per column of a panel's sums (32 rows; 36 keep the stores free of bank conflicts)
 constexpr size_t kMsSmemMax = 227 * 1024;
+// Asked for at least: more than half of an SM's 228 KB, so that an SM holds one CTA.  A launch has at most one CTA an SM to give; where two
+// fit (one tile of rows, K below 4064), those of a dependent launch go two by two to the SMs that the launch before it leaves first, and
+// others stay idle.  us, M = 8, two CTAs an SM / one: chain of dependent launches 1536 -> 1536 4.71 / 4.34, 1536 -> 17920 10.3 / 8.6,
+// 3584 -> 18944 17.9 / 13.5 (twice that N in a group 31.7 / 22.7), ordinary launches 5.73 / 5.72, 11.5 / 10.5, 19.7 / 15.3.
+constexpr size_t kMsSmemMin = 114 * 1024;
 
 struct MsProblem {
   const uint8_t* tiled;  // TiledHeader at offset 0
@@ -779,7 +784,7 @@ static cudaError_t ms_launch_t(MsParams& prm, const MsPlan& plan, cudaStream_t s
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(prm.num_clusters * S), 1, 1);
   cfg.blockDim = dim3(kMsThreads, 1, 1);
-  cfg.dynamicSmemBytes = ms_smem_layout(plan.block_tiles * 8, plan.groups_per_rank, S, plan.stages, plan.stage_groups).total;
+  cfg.dynamicSmemBytes = std::max(kMsSmemMin, ms_smem_layout(plan.block_tiles * 8, plan.groups_per_rank, S, plan.stages, plan.stage_groups).total);
   cfg.stream = stream;
   cudaLaunchAttribute attrs[2];
   int na = 0;
